@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(128, 3) decode_kernel(const __grid_constant__ 
     // a ragged batch with as many tokens as sequences: mine only if the prefix kernel found one token in each (then
     // sequence n is token n, as in a fixed batch)
     if (a.short_flag != nullptr && *a.short_flag != 2) return;
+    if (a.short_flag == nullptr && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t chain = blockIdx.x;
     const int64_t n = chain / a.H;          // sequence = token index (T == 1)
@@ -171,7 +172,6 @@ int launch_decode_ragged(const TwoPassArgs& a, cudaStream_t stream) {
 int launch_decode(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     TwoPassArgs a;
     fill_args(p, &a);
-    if (cudaMemsetAsync(p.workspace, 0, 16, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;  // header: device status
     const int64_t chains = p.N * p.H;
     if (chains > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
     decode_kernel<<<(unsigned)chains, 128, 0, stream>>>(a);

@@ -4,6 +4,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
+
+#include <atomic>
 #include <stdint.h>
 
 #include "../../include/flashkda_b200.h"
@@ -76,6 +78,20 @@ int launch_short(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches)
 bool short_ragged_candidate(const fkda_fwd_params& p);
 int launch_short_ragged(const TwoPassArgs& a, cudaStream_t stream);
 int launch_decode_ragged(const TwoPassArgs& a, cudaStream_t stream);   // as many tokens as sequences: maybe one each
+
+// Allows a kernel its dynamic shared memory on the current device.  The attribute belongs to the function and the device,
+// so it is set once for each and remembered (a driver call on every launch is half a microsecond of host time).
+template <auto kKernel>
+inline bool allow_smem(int bytes) {
+    static std::atomic<uint64_t> devices{0};   // bit d: set on device d
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;
+    if ((devices.load(std::memory_order_acquire) & bit) != 0) return true;
+    if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    devices.fetch_or(bit, std::memory_order_release);
+    return true;
+}
 
 // Fills the kernel arguments common to both implementations (pointers, strides, gate scale,
 // workspace carving).

@@ -60,7 +60,7 @@ size_t fkda_noalloc_scratch_bytes(void) { return (size_t)FKDA_NOALLOC_SCRATCH_BY
 int fkda_fwd_noalloc(const fkda_fwd_params* p, void* stream_v) {
     if (p == nullptr) return FKDA_ERR_NULL_POINTER;
     if (p->B <= 0 || p->T < 0 || p->H <= 0 || p->N <= 0) return FKDA_ERR_BAD_SHAPE;
-    const size_t need = fkda_workspace_bytes_for(p);  // by the path this call takes: a decode step needs 256 bytes
+    const size_t need = fkda_workspace_bytes_for(p);  // by the path this call takes: a decode step needs nothing
     if (need > (size_t)FKDA_NOALLOC_SCRATCH_BYTES) return FKDA_ERR_NOALLOC_TOO_LARGE;
     void* scratch = nullptr;
     int rc = scratch_for_current_device(&scratch);

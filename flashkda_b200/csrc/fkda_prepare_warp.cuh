@@ -372,11 +372,8 @@ __global__ void __launch_bounds__(kPwWarpsPerCta * 32, 1) prepare_warp_kernel(co
 template <bool kTc>
 inline int launch_prepare_warp(const TwoPassArgs& a, cudaStream_t stream, int max_ctas = 0) {
     const int smem = (int)sizeof(PrepWarpSmem) * kPwWarpsPerCta;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(prepare_warp_kernel<kTc>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return FKDA_ERR_LAUNCH;
+    if (!allow_smem<prepare_warp_kernel<kTc>>(smem)) return FKDA_ERR_LAUNCH;
+    const int sms = device_sm_count();
     const int64_t n_units = (a.slab_chunks > 0 ? a.N * (int64_t)a.slab_chunks : a.total_tiles) * a.H;
     int64_t ctas = (n_units + kPwWarpsPerCta - 1) / kPwWarpsPerCta;
     if (ctas > sms) ctas = sms;

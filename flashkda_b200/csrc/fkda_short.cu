@@ -2,7 +2,7 @@
 // holds more than 16 (ONE chunk per sequence), the step between a decode step (one token, fkda_decode.cu) and
 // prefill -- e.g. the verification pass of speculative decoding.  Such a batch is bound by HBM traffic on the [128,128] states (read once, written once), so the whole
 // forward of a (sequence, head) chain runs in ONE kernel with nothing staged in HBM: no chunk records, no second
-// launch, 256 bytes of workspace.
+// launch, no workspace.
 //
 // One 128-thread CTA per FOUR chains, three CTAs per SM:
 //   * first every warp runs the prepare stage of one of the four chunks (the same warp-per-chunk routine as the
@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(128, 3) short_kernel(const __grid_constant__ T
     // a ragged batch that the prefix kernel has given to other kernels (a longer sequence: the general ones; one token
     // each: the decode kernel)
     if (a.short_flag != nullptr && *a.short_flag != 1) return;
+    if (a.short_flag == nullptr && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
     const int64_t n_chains = a.N * a.H;
     const int64_t chain0 = (int64_t)blockIdx.x * kShortChainsPerCta;
     const int row0 = warp * 32 + g;           // my rows: row0 + 16 mt + 8 hi
@@ -326,8 +327,7 @@ bool short_ragged_candidate(const fkda_fwd_params& p) {
 int launch_short_ragged(const TwoPassArgs& a, cudaStream_t stream) {
     const int64_t chains = a.N * a.H;
     if (chains > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
-    if (cudaFuncSetAttribute(short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kShortSmemBytes) != cudaSuccess)
-        return FKDA_ERR_LAUNCH;
+    if (!allow_smem<short_kernel>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
     const int64_t ctas = (chains + kShortChainsPerCta - 1) / kShortChainsPerCta;
     short_kernel<<<(unsigned)ctas, 128, kShortSmemBytes, stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? FKDA_OK : FKDA_ERR_LAUNCH;
@@ -336,11 +336,9 @@ int launch_short_ragged(const TwoPassArgs& a, cudaStream_t stream) {
 int launch_short(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     TwoPassArgs a;
     fill_args(p, &a);
-    if (cudaMemsetAsync(p.workspace, 0, 16, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;  // header: device status
     const int64_t chains = p.N * p.H;
     if (chains > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
-    if (cudaFuncSetAttribute(short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kShortSmemBytes) != cudaSuccess)
-        return FKDA_ERR_LAUNCH;
+    if (!allow_smem<short_kernel>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
     const int64_t ctas = (chains + kShortChainsPerCta - 1) / kShortChainsPerCta;
     short_kernel<<<(unsigned)ctas, 128, kShortSmemBytes, stream>>>(a);
     if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;

@@ -295,8 +295,8 @@ static TcCarve tc_carve(const fkda_fwd_params& p, int sms) {
     return c;
 }
 size_t tc_workspace_bytes_for(const fkda_fwd_params& p) {
-    if (decode_eligible(p) && !(p.flags & FKDA_FLAG_NO_DECODE) && p.chunk_states == nullptr) return kWsHeaderBytes;  // status word only
-    if (short_eligible(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) return kWsHeaderBytes;
+    if (decode_eligible(p) && !(p.flags & FKDA_FLAG_NO_DECODE) && p.chunk_states == nullptr) return 0;   // one kernel, nothing staged
+    if (short_eligible(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) return 0;
     const TcCarve c = tc_carve(p, device_sm_count());
     return kWsHeaderBytes + ws_prefix_bytes(p.N) + c.slots + c.states + c.records;
 }
@@ -364,9 +364,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
          !encode_token_map(&maps.out, p.out, T_total, p.H, p.token_stride)))
         return FKDA_ERR_LAUNCH;
     const int wide_smem = kWideSmemBytes;
-    if (do_rec && wide &&
-        cudaFuncSetAttribute(recurrence_tc_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem) != cudaSuccess)
-        return FKDA_ERR_LAUNCH;
+    if (do_rec && wide && !allow_smem<recurrence_tc_wide_kernel>(wide_smem)) return FKDA_ERR_LAUNCH;
 
     // ---- few chains on a fixed batch: the recurrence is a serial walk on `chains` SMs and leaves the others
     //      idle, so the forward is cut into slabs of chunks and the prepare stage of slab i+1 runs on the idle SMs
@@ -452,9 +450,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
             recurrence_tc_wide_kernel<<<(unsigned)ctas, kWideThreads, wide_smem, stream>>>(a, maps);
         } else {
             // three chains per CTA, state copy and 16-deep A operands in tensor memory
-            if (cudaFuncSetAttribute(recurrence_tc_ts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes) !=
-                cudaSuccess)
-                return FKDA_ERR_LAUNCH;
+            if (!allow_smem<recurrence_tc_ts_kernel>(kTsSmemBytes)) return FKDA_ERR_LAUNCH;
             recurrence_tc_ts_kernel<<<(unsigned)ctas, kTcChains * 128, kTsSmemBytes, stream>>>(a, maps);
         }
         ++launches;

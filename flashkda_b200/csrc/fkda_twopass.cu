@@ -285,7 +285,8 @@ void fill_args(const fkda_fwd_params& p, TwoPassArgs* out) {
     a.total_tiles = varlen ? ws_tiles_upper_bound(T_total, p.N) : p.N * ((p.T + kChunk - 1) / kChunk);
     uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace);
     a.queue = reinterpret_cast<int32_t*>(base);
-    a.status = reinterpret_cast<int32_t*>(base) + 1;
+    // (a one-kernel path needs no workspace; where the caller gave one, its status word is kept)
+    a.status = base != nullptr && p.workspace_bytes >= kWsHeaderBytes && ((uintptr_t)base & 255u) == 0 ? reinterpret_cast<int32_t*>(base) + 1 : nullptr;
     a.short_flag = nullptr;
     a.qslots = nullptr;
     a.seg_state = nullptr;
@@ -315,10 +316,7 @@ int launch_twopass(const fkda_fwd_params& p, cudaStream_t stream, int* n_launche
         if (launch_prepare_warp<false>(a, stream) != FKDA_OK) return FKDA_ERR_LAUNCH;
         ++launches;
     }
-    // per device and cheap, so set on every call rather than cached per process
-    if (cudaFuncSetAttribute(recurrence_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(RecSmem)) != cudaSuccess)
-        return FKDA_ERR_LAUNCH;
+    if (!allow_smem<recurrence_kernel>((int)sizeof(RecSmem))) return FKDA_ERR_LAUNCH;
     if (do_rec) {
         dim3 grid2((unsigned)p.N, (unsigned)p.H);
         recurrence_kernel<<<grid2, 128, sizeof(RecSmem), stream>>>(a);

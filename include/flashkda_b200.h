@@ -116,7 +116,8 @@ enum {
 size_t fkda_workspace_bytes(int64_t T_total, int64_t H, int64_t N, int32_t algo);
 
 /* Scratch bytes THIS call needs (<= fkda_workspace_bytes for the same totals): a fixed batch with at most 16 tokens
- * per sequence (a decode step, T == 1, or a short step, T <= 16) needs only the 256-byte header, other calls their
+ * per sequence (a decode step, T == 1, or a short step, T <= 16) needs nothing (where a workspace is given all the same,
+ * its status word is kept), other calls their header,
  * records and queue.  No counterpart in the reference. */
 size_t fkda_workspace_bytes_for(const fkda_fwd_params* p);
 
@@ -151,7 +152,7 @@ int fkda_device_status(const void* workspace, void* stream);
  * Limit: fkda_workspace_bytes_for(p) must not exceed FKDA_NOALLOC_SCRATCH_BYTES.  With the default
  * algorithm a chunk record takes 14 656 bytes and a (sequence, head) chain 32 KB of hand-over state when
  * the call may be pipelined or queued, so about H * (B*T/16) <= 2 250 chunk records minus 2.2 records per
- * chain (algo = twopass: 13 824-byte records, about 2 400); a decode step (T == 1) needs 256 bytes whatever
+ * chain (algo = twopass: 13 824-byte records, about 2 400); a decode step (T == 1) needs nothing whatever
  * its batch size.  Larger problems return FKDA_ERR_NOALLOC_TOO_LARGE and launch nothing.
  * The call itself performs no cudaMalloc/cudaFree and allocates no device memory through any library.
  * The first call on each device looks up the array's device address (cudaGetSymbolAddress); the first
