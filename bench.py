@@ -331,12 +331,12 @@ def run_ours(a):
 
     # ---- each kernel of the forward alone (CUDA events on the launching stream); the slower one is
     #      the dominant kernel the roofline line describes ----
-    # (the tensor-core recurrence has a one-chain-per-CTA variant that the launcher picks when there are no more
+    # (the tensor-core recurrence has a row-slice variant that the launcher picks when there are no more
     #  (sequence, head) chains than SMs; otherwise the three-chains-per-CTA kernel runs)
     n_seqs = (len(inp["cu_seqlens"]) - 1) if inp.get("cu_seqlens") is not None else w_local.B
-    wide = n_seqs * w.H <= torch.cuda.get_device_properties(dev).multi_processor_count
+    rows = n_seqs * w.H <= torch.cuda.get_device_properties(dev).multi_processor_count
     names = {"twopass": ("fkda::prepare_warp_kernel", "fkda::recurrence_kernel")}.get(
-        algo, ("fkda::prepare_warp_kernel", "fkda::recurrence_tc_wide_kernel" if wide else "fkda::recurrence_tc_ts_kernel"))
+        algo, ("fkda::prepare_warp_kernel", "fkda::recurrence_rows_kernel" if rows else "fkda::recurrence_tc_ts_kernel"))
     kernel_times = {}
     n_phase = 3
     barrier()

@@ -14,7 +14,7 @@
 //   * the other element-wise steps (bf16 roundings, beta) by the same threads (thread v = TMEM lane v of
 //     D1/D2/D3), reading accumulators with tcgen05.ld.
 // The kernels live in their own files and share the helpers below: fkda_tc_ts.cuh (three chains per CTA: the
-// default for more chains than SMs) and fkda_tc_wide.cuh (one chain per CTA, for no more chains than SMs).
+// default for more chains than SMs) and fkda_rows.cuh (row slices of a chain on mma.sync, for no more chains than SMs).
 //
 // Numerics: steps B1-B7 of the reference's contract (tests/torch_ref.py:231-251; the reference's own
 // recurrence is csrc/smxx/fwd_kernel2.cuh:434-742, built on mma.sync with register transposes).
@@ -51,7 +51,7 @@ struct alignas(64) TcMaps {
 };
 
 // ---------------------------------------------------------------------------------
-// Pieces shared by the recurrence kernels of this file and of fkda_tc_wide.cuh / fkda_tc_ts.cuh.
+// Pieces shared by the recurrence kernels of this file and of fkda_rows.cuh / fkda_tc_ts.cuh.
 
 // Where the tokens and records of one (sequence, head) chain live.
 struct TcChain {
@@ -198,7 +198,7 @@ __device__ __forceinline__ void tc_store_out(const uint32_t (&r)[32], unsigned s
 }  // namespace fkda
 
 #include "fkda_tc_ts.cuh"
-#include "fkda_tc_wide.cuh"
+#include "fkda_rows.cuh"
 
 namespace fkda {
 
@@ -242,7 +242,7 @@ static size_t seg_slots_bytes(int64_t T_total, int64_t H, int64_t N, int sms) {
 }
 // Few chains on a fixed batch may run as a slab pipeline (see launch_tc); its chain states travel through the
 // same hand-over buffer as the segments of the work queue (32 KB per chain).
-static bool slabs_possible(int64_t chains, int sms) { return chains <= sms - 32; }
+static bool slabs_possible(int64_t chains, int sms) { return chains * kRowSplit <= sms - 32; }   // SMs left for the prepare stage
 static size_t seg_state_bytes(int64_t H, int64_t N, bool needed) { return needed ? (size_t)(H * N) * 32768 : 0; }
 
 // Side stream and events of the slab pipeline, one set per device, created on first use.
@@ -318,15 +318,18 @@ static EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-static bool encode_token_map(CUtensorMap* m, const void* base, int64_t T_total, int64_t H, int64_t token_stride) {
+// Map over a [token][head][128] tensor with tiles of 16 tokens x `cols` columns of one head.  `swizzle`: the 16-byte pieces
+// of a tile row are permuted by the row, so that transposing accesses to the tile (8 rows of one piece) do not collide.
+static bool encode_token_map(CUtensorMap* m, const void* base, int64_t T_total, int64_t H, int64_t token_stride, int cols,
+                             CUtensorMapSwizzle swizzle) {
     EncodeTiledFn encode = encode_tiled_fn();
     if (encode == nullptr) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)H, (cuuint64_t)(T_total > 0 ? T_total : 1)};
     const cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)token_stride * 2};  // bytes, dims 1 and 2
-    const cuuint32_t box[3] = {(cuuint32_t)kD, 1u, (cuuint32_t)kChunk};
+    const cuuint32_t box[3] = {(cuuint32_t)cols, 1u, (cuuint32_t)kChunk};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
-                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -355,39 +358,44 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         a.workspace = base + c.slots + c.states;
     }
     const int64_t chains = p.N * p.H;
-    const bool wide = chains <= sms && !(p.flags & FKDA_FLAG_NO_WIDE);
+    const bool rows = chains <= sms && !(p.flags & FKDA_FLAG_NO_WIDE);
     TcMaps maps;
     memset(&maps, 0, sizeof(maps));
     // (an empty batch has no tiles to move: its chains only pass their state through)
     if (do_rec && T_total > 0 &&
-        (!encode_token_map(&maps.v, p.v, T_total, p.H, p.token_stride) ||
-         !encode_token_map(&maps.out, p.out, T_total, p.H, p.token_stride)))
+        (!encode_token_map(&maps.v, p.v, T_total, p.H, p.token_stride, rows ? kRowCols : kD,
+                           rows ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE) ||
+         (!rows && !encode_token_map(&maps.out, p.out, T_total, p.H, p.token_stride, kD, CU_TENSOR_MAP_SWIZZLE_NONE))))
         return FKDA_ERR_LAUNCH;
-    const int wide_smem = kWideSmemBytes;
-    if (do_rec && wide && !allow_smem<recurrence_tc_wide_kernel>(wide_smem)) return FKDA_ERR_LAUNCH;
+    const auto rows_kernel = a.chunk_states != nullptr ? recurrence_rows_kernel<true> : recurrence_rows_kernel<false>;
+    if (do_rec && rows && !(a.chunk_states != nullptr ? allow_smem<recurrence_rows_kernel<true>>(kRowSmemBytes)
+                                                       : allow_smem<recurrence_rows_kernel<false>>(kRowSmemBytes)))
+        return FKDA_ERR_LAUNCH;
 
     // ---- few chains on a fixed batch: the recurrence is a serial walk on `chains` SMs and leaves the others
     //      idle, so the forward is cut into slabs of chunks and the prepare stage of slab i+1 runs on the idle SMs
     //      (side stream) while the recurrence walks slab i; the state of a chain travels through seg_state.
     //      Only stream order and events connect the launches: no kernel waits for another one. ----
     const int64_t tps = (p.T + kChunk - 1) / kChunk;
-    const int idle_sms = sms - (int)chains;
-    if (wide && !varlen && p.phase_mask == 0 && slabs_possible(chains, sms) && tps >= 64 && !(p.flags & FKDA_FLAG_NO_SLABS)) {
+    const int idle_sms = sms - (int)chains * kRowSplit;
+    if (rows && !varlen && p.phase_mask == 0 && slabs_possible(chains, sms) && tps >= 64 && !(p.flags & FKDA_FLAG_NO_SLABS)) {
         SlabStreams* ss = slab_streams(dev);
         if (ss == nullptr) return FKDA_ERR_LAUNCH;
         // host threads that call concurrently on one device share the side stream and its events
         std::lock_guard<std::mutex> enqueue_lock(ss->launch_mu);
-        // Slab boundaries.  The prepare of slab i+1 (on idle_sms SMs, about 5.2 ns per (chunk, head) on the whole
-        // GPU) must be done when the recurrence (about 1.18 us per chunk) has walked slab i.  When prepare is at
-        // least twice as fast (x <= 0.5) the slabs grow, 1/8, 1/4, 5/16, 5/16 of the chunks (1/3, 2/3 for two), so
-        // that little prepare work goes first, unhidden; otherwise they are equal.
+        // Slab boundaries.  The prepare of slab i+1 (on idle_sms SMs, about 5.2 ns per (chunk, head) on the whole GPU) must
+        // be done when the recurrence (about 0.52 us per chunk) has walked slab i, and the prepare of the first slab is
+        // not hidden at all: the slabs grow by the ratio of the two speeds, at most by 2 (equal when prepare is slower).
         const int n_slabs = tps >= 256 ? kMaxSlabs : 2;
-        const double x = (double)chains * (double)sms / ((double)idle_sms * 227.0);
-        static const double grow4[kMaxSlabs + 1] = {0.0, 0.125, 0.375, 0.6875, 1.0}, grow2[3] = {0.0, 1.0 / 3.0, 1.0};
+        const double x = (double)chains * (double)sms / ((double)idle_sms * 100.0);
+        const double grow = x >= 1.0 ? 1.0 : (x <= 0.5 ? 2.0 : 1.0 / x);
         int bounds[kMaxSlabs + 1];
-        for (int i = 0; i <= n_slabs; ++i) {
-            const double frac = x <= 0.5 ? (n_slabs == 2 ? grow2[i] : grow4[i]) : (double)i / n_slabs;
-            bounds[i] = (int)((int64_t)(frac * (double)tps + 1.0) / 2 * 2);  // even
+        double total = 0.0, part = 1.0, run = 0.0;
+        for (int i = 0; i < n_slabs; ++i, part *= grow) total += part;
+        part = 1.0;
+        for (int i = 0; i <= n_slabs; ++i, part *= grow) {
+            bounds[i] = (int)((int64_t)(run / total * (double)tps + 1.0) / 2 * 2);  // even
+            run += part;
         }
         bounds[0] = 0;
         bounds[n_slabs] = (int)tps;
@@ -410,7 +418,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         for (int i = 0; i < n_slabs; ++i) {
             if (bounds[i + 1] <= bounds[i]) continue;
             if (i > 0 && cudaStreamWaitEvent(stream, ss->done[i], 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
-            recurrence_tc_wide_kernel<<<(unsigned)chains, kWideThreads, wide_smem, stream>>>(slab_args(i), maps);
+            rows_kernel<<<(unsigned)(chains * kRowSplit), kRowThreads, kRowSmemBytes, stream>>>(slab_args(i), maps);
             ++launches;
         }
         if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
@@ -445,9 +453,9 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         int64_t ctas = chains;  // one chain per SM while they last, then two, then three
         if (ctas > sms) ctas = sms;
         if (ctas < 1) ctas = 1;
-        if (wide) {
-            // few chains: one per CTA, the idle warpgroups help with the state update
-            recurrence_tc_wide_kernel<<<(unsigned)ctas, kWideThreads, wide_smem, stream>>>(a, maps);
+        if (rows) {
+            // few chains: every chain cut into row slices
+            rows_kernel<<<(unsigned)(chains * kRowSplit), kRowThreads, kRowSmemBytes, stream>>>(a, maps);
         } else {
             // three chains per CTA, state copy and 16-deep A operands in tensor memory
             if (!allow_smem<recurrence_tc_ts_kernel>(kTsSmemBytes)) return FKDA_ERR_LAUNCH;
