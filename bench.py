@@ -331,20 +331,20 @@ def run_ours(a):
 
     # ---- each kernel of the forward alone (CUDA events on the launching stream); the slower one is
     #      the dominant kernel the roofline line describes ----
-    # (the tensor-core recurrence has a row-slice variant that the launcher picks when there are no more
-    #  (sequence, head) chains than SMs; otherwise the three-chains-per-CTA kernel runs)
-    n_seqs = (len(inp["cu_seqlens"]) - 1) if inp.get("cu_seqlens") is not None else w_local.B
-    rows = n_seqs * w.H <= torch.cuda.get_device_properties(dev).multi_processor_count
+    # (with enough (sequence, head) chains to fill the GPU the forward is one kernel, otherwise a prepare and a recurrence
+    #  kernel; a ragged batch has a prefix kernel in front)
     names = {"twopass": ("fkda::prepare_warp_kernel", "fkda::recurrence_kernel")}.get(
-        algo, ("fkda::prepare_warp_kernel", "fkda::recurrence_rows_kernel" if rows else "fkda::recurrence_tc_ts_kernel"))
+        algo, ("fkda::prepare_warp_kernel", "fkda::recurrence_rows_kernel"))
     kernel_times = {}
     n_phase = 3
     barrier()
     decode = w_local.T == 1 and inp.get("cu_seqlens") is None and algo != "twopass" and not (a.flags & 1)
     short = 2 <= w_local.T <= 16 and inp.get("cu_seqlens") is None and algo != "twopass" and not (a.flags & 8)
-    if (decode or short) and not cp_mode and a.seq_parts == 1:
-        # at most one chunk per sequence: the library runs ONE kernel (no phases to time apart)
-        kernel_name, kernel_ms = ("fkda::decode_kernel" if decode else "fkda::short_kernel"), ms_step
+    one_kernel = launches_per_step == (1 if inp.get("cu_seqlens") is None else 2)
+    if one_kernel and not cp_mode and a.seq_parts == 1:
+        # the library runs ONE kernel (no phases to time apart)
+        kernel_name = "fkda::decode_kernel" if decode else ("fkda::short_kernel" if short else "fkda::fused_kernel")
+        kernel_ms = ms_step
         kernel_times[kernel_name] = ms_step
     elif not cp_mode and a.seq_parts == 1:
         step()
@@ -418,7 +418,7 @@ def run_ours(a):
     state_bytes = alg_bytes - th * 1282 if not cp_mode else 0
     rec = {"twopass": 13824}.get(algo, 14656)
     own = {"fkda::prepare_warp_kernel": th * 770 + units * rec,
-           "fkda::decode_kernel": alg_bytes, "fkda::short_kernel": alg_bytes}
+           "fkda::decode_kernel": alg_bytes, "fkda::short_kernel": alg_bytes, "fkda::fused_kernel": alg_bytes}
     for n in names[1:]:
         own[n] = units * rec + th * 512 + state_bytes
     tdb = json.load(open(os.path.join(ROOT, "profiles", "traffic.json"))) \

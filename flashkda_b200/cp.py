@@ -259,12 +259,12 @@ class SequenceSplit:
         self.prepared = False   # whether self.ws holds the chunk records of this shard
 
     def _fwd(self, v, h0, hT):
-        """One operator call on the batch of pieces; the first one also runs the prepare stage, later ones
-        walk the records it left in the workspace."""
+        """One operator call on the batch of pieces; the first one asks for both stages by name, so that it leaves its
+        chunk records in the workspace, later ones walk them."""
         from . import _lib
         qb, kb, _, gb, bb = self.t
         self.F.fwd(qb, kb, v, gb, bb, self.scale, self.out, *self.args, h0, hT, None, workspace=self.ws,
-                   phase_mask=_lib.PHASE_RECURRENCE if self.prepared else 0)
+                   phase_mask=_lib.PHASE_RECURRENCE if self.prepared else _lib.PHASE_PREPARE | _lib.PHASE_RECURRENCE)
         self.prepared = True
 
     def maps(self, total: bool = True):

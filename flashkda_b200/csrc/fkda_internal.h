@@ -23,17 +23,14 @@ struct TwoPassArgs {
     int32_t* tile_prefix;  // [N + 1] chunk-count prefix (varlen only)
     const int32_t* seq_order;  // [N] sequences by decreasing length (varlen with N <= kSeqOrderMaxN, else nullptr)
     uint8_t* workspace;    // [H][total_tiles] per-chunk records
-    int32_t* queue;        // header word 0: tail / queue ticket counter of the persistent recurrence (zeroed per call)
+    int32_t* queue;        // header word 0: ticket counter of the one-kernel forward (zeroed per call)
     int32_t* status;       // header word 1: device status, 0 ok, else the code of a bounded wait that gave up
     int32_t* short_flag;   // header word 8, or null: written by the prefix kernel of a ragged batch that MAY consist of
                            // one-chunk sequences; the kernels that can serve the call are all enqueued and all but one
                            // return at once: 2 = every sequence has exactly one token (decode kernel), 1 = no sequence is
                            // longer than one chunk (fused short-sequence kernel), 0 = the general kernels
-                           // (header words 2, 3: push counter and finished-chain counter of the segment queue;
-                           //  words 4..6: claim counters of the three layers of first segments)
-    int32_t* qslots;       // segment queue: slot i receives the i-th pushed item (-1 = not yet pushed)
-    uint32_t* seg_state;   // [chain][16][128] uint4: bf16 state handed from one segment of a chain to the next
-    int32_t seg_chunks;    // chunks per scheduling segment (0 = whole chains)
+    int32_t* range_flags;  // one-kernel forward: walking warps of each range that have published their rows of its state
+    uint32_t* seg_state;   // bf16 states in fragment order, handed from range to range (one-kernel forward) or slab to slab
     int32_t slab_c0, slab_chunks;  // fixed batches only: this launch covers chunks [slab_c0, slab_c0 + slab_chunks) of
                                    // every sequence (slab_chunks == 0: all chunks); a chain's state travels from one
                                    // slab to the next through seg_state
@@ -43,13 +40,13 @@ struct TwoPassArgs {
     __nv_bfloat16* chunk_states;   // optional export of the state before every cs_every-th chunk (see fkda_fwd_params)
     const int32_t* cs_prefix;      // [N] first export slot of every sequence (varlen; fixed batches compute it)
     int32_t cs_every;
-    uint64_t wait_ns;      // limit of every bounded device-side wait (mbarrier, queue slot)
+    uint64_t wait_ns;      // limit of every bounded device-side wait (mbarrier, range flag)
     bool state_fp32;
-    bool test_drop_push;   // test hook (FKDA_FLAG_TEST_DROP_PUSH): finished segments do not queue their follow-up
+    bool test_drop_push;   // test hook (FKDA_FLAG_TEST_DROP_PUSH): ranges do not publish the state they hand over
 };
 
 // Workspace layout of both two-pass implementations:
-//   [0, 256)  header: int32 ticket counter, device status, push counter, finished-chain counter, 3 layer counters
+//   [0, 256)  header: int32 ticket counter, device status, word 8: path decision of a ragged batch
 //   [256, ..) tile prefix (N + 1 int32, padded to 256 B)
 //   then      H * total_tiles records
 constexpr size_t kWsHeaderBytes = 256;
@@ -96,9 +93,9 @@ inline bool allow_smem(int bytes) {
 // Fills the kernel arguments common to both implementations (pointers, strides, gate scale,
 // workspace carving).
 void fill_args(const fkda_fwd_params& p, TwoPassArgs* a);
-void launch_tile_prefix(const int64_t* cu_seqlens, int64_t N, int32_t* prefix, int32_t* seq_order, int32_t* cs_prefix,
-                        int cs_tokens, int32_t* short_flag, bool decode_enqueued, int32_t* critical_chunks, int64_t heads,
-                        int chain_slots, cudaStream_t stream);
+// The prefix kernel of a ragged batch: chunk (and state-export) prefix tables, the length order if asked for, and the path
+// decision if a.short_flag is set.
+void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream);
 // First state-export slot of sequence n.
 __device__ __forceinline__ int64_t cs_first_slot(const TwoPassArgs& a, int64_t n) {
     if (a.cu_seqlens != nullptr) return a.cs_prefix[n];

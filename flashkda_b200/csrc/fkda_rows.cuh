@@ -22,7 +22,7 @@ constexpr int kRowThreads = (kRowWarps + 1) * 32;
 constexpr int kRowVBytes = kChunk * kRowCols * 2;              // value tile [16 tokens][64] bf16, 128-byte swizzle
 constexpr int kRowV = 0;                                       // (1024-byte aligned for the swizzle)
 constexpr int kRowOut = kRowV + kRowStages * kRowVBytes;       // per warp an out tile [16 tokens][16] bf16
-constexpr int kRowRec = kRowOut + kRowWarps * 512;         // chunk records
+constexpr int kRowRec = kRowOut + kRowWarps * 512;             // chunk records
 constexpr int kRowStaging = kRowRec + kRowStages * kTcRecord;  // per warp one staging tile for states
 constexpr int kRowCtrl = kRowStaging + kRowWarps * kWalkStageBytes;
 struct RowCtrl {
@@ -34,10 +34,11 @@ constexpr int kRowSmemBytes = kRowCtrl + (int)sizeof(RowCtrl) + 1024;
 static_assert(kRowCols == 64 && kRowVBytes % 1024 == 0 && kRowOut % 256 == 0 && kRowRec % 16 == 0 && kRowStaging % 16 == 0 && kRowCtrl % 8 == 0,
               "tile alignments");
 
-// kExport: the states before every cs_every-th chunk are written out as well
-template <bool kExport>
+// kExport: the states before every cs_every-th chunk are written out as well.  kLoop: a CTA takes several slices in turn
+// (for launches that mostly return at once, see launch_tc; the loop alone makes a step 15 % longer).
+template <bool kExport, bool kLoop>
 __global__ void __launch_bounds__(kRowThreads, 2)
-recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ TcMaps maps) {
+recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap map) {
     // (a ragged batch that a one-kernel path has served: nothing to do)
     if (a.short_flag != nullptr && *a.short_flag != 0) return;
     extern __shared__ uint8_t smem_dyn[];
@@ -56,36 +57,39 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
     }
     __syncthreads();
 
-    const int64_t chain = blockIdx.x / kRowSplit;
-    const int slice = (int)(blockIdx.x % kRowSplit);
+    const int64_t n_items = a.N * a.H * kRowSplit;
+    bool failed = false;
+    int k0 = 0;   // chunks of the items before: the stages and their phases run on from item to item
+    for (int64_t item = blockIdx.x; item < n_items && !failed; item = kLoop ? item + gridDim.x : n_items) {
+    const int64_t chain = item / kRowSplit;
+    const int slice = (int)(item % kRowSplit);
     const TcChain ch = tc_locate_chain(a, chain);
     const int h = ch.h;
     // chunk range of this launch: all chunks, or one slab of a pipelined forward (fixed batches)
     const int c0 = a.slab_chunks > 0 ? a.slab_c0 : 0;
     const int c1 = (a.slab_chunks > 0 && c0 + a.slab_chunks < ch.n_chunks) ? c0 + a.slab_chunks : ch.n_chunks;
-    bool failed = false;
-
     if (warp == kRowWarps) {
         // =========================== control warp: keeps the stages filled ===========================
         if (elect_one()) {
             int t = c0;
             for (; t < c1; ++t) {
-                const int i = t - c0, s = i % kRowStages;
-                if (i >= kRowStages && !mbar_wait_bounded(&ctl.empty[s], (uint32_t)((i / kRowStages - 1) & 1), abort_flag, a.wait_ns)) {
+                const int k = k0 + t - c0, s = k % kRowStages;
+                if (k >= kRowStages && !mbar_wait_bounded(&ctl.empty[s], (uint32_t)((k / kRowStages - 1) & 1), abort_flag, a.wait_ns)) {
                     failed = true;
                     break;
                 }
                 mbar_arrive_expect_tx(&ctl.full[s], (uint32_t)(kTcRecord + kRowVBytes));
                 bulk_g2s(sm + kRowRec + s * kTcRecord, ch.rec_base + (int64_t)t * kTcRecord, kTcRecord, &ctl.full[s]);
                 // rows past the end of the tensor arrive as zeros; rows of the next sequence are never used
-                tma_load_3d(sm + kRowV + s * kRowVBytes, &maps.v, slice * kRowCols, h, (int)(ch.bos + (int64_t)t * kChunk), &ctl.full[s]);
+                tma_load_3d(sm + kRowV + s * kRowVBytes, &map.v, slice * kRowCols, h, (int)(ch.bos + (int64_t)t * kChunk), &ctl.full[s]);
             }
             if (failed) {   // the copies in flight land before this CTA's shared memory goes
                 *abort_flag = 1;
-                for (int i = max(0, t - c0 - kRowStages); i < t - c0; ++i)
-                    mbar_wait_bounded(&ctl.full[i % kRowStages], (uint32_t)((i / kRowStages) & 1), nullptr, 100000000ull);
+                for (int k = max(0, k0 + t - c0 - kRowStages); k < k0 + t - c0; ++k)
+                    mbar_wait_bounded(&ctl.full[k % kRowStages], (uint32_t)((k / kRowStages) & 1), nullptr, 100000000ull);
             }
         }
+        failed = __any_sync(0xffffffffu, failed) != 0;
     } else {
         // =========================== walking warps ===========================
         const int row0 = slice * kRowCols + warp * 16;   // my first state row
@@ -113,18 +117,13 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
                 w.s[0][j][0] = x.x; w.s[0][j][1] = x.y; w.s[0][j][2] = x.z; w.s[0][j][3] = x.w;
             }
         } else if (a.initial_state != nullptr) {
-            walk_load_tile(w.s[0], stage_tile,
-                           a.state_fp32 ? (const void*)(reinterpret_cast<const float*>(a.initial_state) + st_base)
-                                        : (const void*)(reinterpret_cast<const unsigned short*>(a.initial_state) + st_base),
-                           a.state_fp32, lane);
+            if (a.state_fp32) walk_load_tiles<1, true>(w.s, stage_tile, reinterpret_cast<const float*>(a.initial_state) + st_base, lane);
+            else walk_load_tiles<1, false>(w.s, stage_tile, reinterpret_cast<const unsigned short*>(a.initial_state) + st_base, lane);
         } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) w.s[0][j][e] = 0u;
+            w.clear();
         }
-        auto full_bar = [&](int i) { return &ctl.full[i % kRowStages]; };
-        auto full_phase = [&](int i) { return (uint32_t)((i / kRowStages) & 1); };
+        auto full_bar = [&](int i) { return &ctl.full[(k0 + i) % kRowStages]; };
+        auto full_phase = [&](int i) { return (uint32_t)(((k0 + i) / kRowStages) & 1); };
         auto wait_full = [&](int i) {
             return __all_sync(0xffffffffu, mbar_wait_bounded(full_bar(i), full_phase(i), abort_flag, a.wait_ns)) != 0;
         };
@@ -139,11 +138,11 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         if (n > 0) {
             if (!wait_full(0)) failed = true;
             else {
-                w.first(rec0, wl);
-                fetch_head(0, left);
+                w.first(rec0 + k0 % kRowStages * kTcRecord, wl);
+                fetch_head(k0 % kRowStages, left);
             }
         }
-        int s = 0;            // stage of the current chunk
+        int s = k0 % kRowStages;   // stage of the current chunk
         bool ready = false;   // the next chunk's operands have been seen
         for (int i = 0; i < n && !failed; ++i) {
             if (kExport && (c0 + i) % a.cs_every == 0)   // the state before this group of chunks
@@ -186,6 +185,8 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         } else {
             *abort_flag = 1;   // the other warps leave their waits
         }
+    }
+    if constexpr (kLoop) k0 += max(0, c1 - c0);
     }
     if (failed) atomicExch(a.status, FKDA_ERR_DEVICE_STATUS);
     __syncthreads();   // shared memory stays until every warp, and every copy of the control warp, is done with it

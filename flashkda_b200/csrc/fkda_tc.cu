@@ -1,23 +1,18 @@
-// Tensor-core two-pass KDA forward for sm_100a: the token-parallel prepare kernel writes per-chunk
-// operand records already laid out as tcgen05 (UMMA) shared-memory operands; a persistent
-// recurrence kernel walks the chunks of each (sequence, head) chain with
-//   * per chunk one bulk asynchronous copy of the record plus one tiled TMA load (tensor map) of the
-//     [16,128] value tile, multi-buffered on mbarriers; out tiles leave through a tiled TMA store,
-//   * all contractions on tcgen05.mma with fp32 accumulators in tensor memory (M = 128 always):
-//        D1[V,32]   = S[V,K] . [kd; qd]^T         (8 x M128 N32 K16; A = the bf16 state copy in tensor memory)
-//        D2[V,16]   = u'^T[V,16] . INV^T          (M128 N16 K16)
-//        D3[V,16]   = U^T[V,16] . Mqk^T           (M128 N16 K16)
-//        DST[V,K]   = U^T[V,16] . kr[16,K]        (M128 N128 K16; the state update)
-//   * the bf16 state held twice: in the registers of its owner threads (thread v owns S[v,:]) for the
-//     element-wise update S[v,k] = bf(fma(S[v,k], E_tot[k], DST[v,k])), and as the tensor-memory copy that the
-//     next chunk's first MMA reads as its A operand,
-//   * the other element-wise steps (bf16 roundings, beta) by the same threads (thread v = TMEM lane v of
-//     D1/D2/D3), reading accumulators with tcgen05.ld.
-// The kernels live in their own files and share the helpers below: fkda_tc_ts.cuh (three chains per CTA: the
-// default for more chains than SMs) and fkda_rows.cuh (row slices of a chain on mma.sync, for no more chains than SMs).
+// Tensor-core KDA forward for sm_100a: dispatch and launches.
 //
-// Numerics: steps B1-B7 of the reference's contract (tests/torch_ref.py:231-251; the reference's own
-// recurrence is csrc/smxx/fwd_kernel2.cuh:434-742, built on mma.sync with register transposes).
+// Two forms of the forward, both on the same chunk operands (a 14 656-byte record per (chunk, head), fkda_common.cuh), the same
+// chunk step on mma.sync with the state in registers (fkda_walk.cuh), and with bit-identical results:
+//   * fkda_fused.cuh: one persistent kernel whose CTAs prepare the records in shared memory and walk them, for batches with
+//     enough chains to fill the GPU: no record ever reaches HBM;
+//   * fkda_prepare_warp.cuh + fkda_rows.cuh: a prepare kernel writes the records to the workspace, a recurrence kernel walks
+//     row slices of the chains; the slices of few chains spread over more SMs than there are chains, and the prepare stage of
+//     later chunks runs on the SMs that are left (the slab pipeline below).
+// An earlier form of both recurrences ran the products on tcgen05 with accumulators in tensor memory: the hand-overs between
+// registers and tensor memory (a store takes 180 cycles, a commit and its wait as long) cost more than products that are 16 to
+// 128 columns wide and 16 deep take on mma.sync (a chunk step of one chain per SM: 1.11 us against 0.52).
+//
+// Numerics: steps B1-B7 of the reference's contract (tests/torch_ref.py:231-251; the reference's own recurrence is
+// csrc/smxx/fwd_kernel2.cuh:434-742).
 #include <cuda.h>
 #include <string.h>
 
@@ -31,27 +26,6 @@
 namespace fkda {
 
 using namespace sm100;
-
-constexpr int kTcChains = 3;    // chains (warpgroups) per CTA
-constexpr int kTcStages = 3;    // chunk records in flight per chain
-constexpr int kTcTmemCols = 512;
-constexpr int kTcStageBytes = kTcRecord;   // one chunk record per stage
-
-struct TcCtrl {
-    uint64_t full[kTcChains][kTcStages];
-    uint64_t mma[kTcChains];
-    uint32_t tmem_base;
-    int32_t next_chain[kTcChains];
-    int32_t abort_flag;
-};
-
-// Tensor maps over v and out viewed as [token][head][128] bf16 (box = 16 tokens x 1 head x 128).
-struct alignas(64) TcMaps {
-    CUtensorMap v, out;
-};
-
-// ---------------------------------------------------------------------------------
-// Pieces shared by the recurrence kernels of this file and of fkda_rows.cuh / fkda_tc_ts.cuh.
 
 // Where the tokens and records of one (sequence, head) chain live.
 struct TcChain {
@@ -85,119 +59,9 @@ __device__ __forceinline__ TcChain tc_locate_chain(const TwoPassArgs& a, int64_t
     return c;
 }
 
-// Next work item of a chain slot (called by ONE thread of the slot's warpgroup).  An item is one segment
-// (seg_chunks chunks) of one chain; item id = seg * n_chains + chain.
-//
-// First segments are CLAIMED, never assigned: nothing waits for a CTA that is not resident (SMs held by another
-// kernel, or a second persistent launch on another stream), so the kernel makes progress with whatever CTAs run.
-//   * The first kTcChains * gridDim chains form kTcChains layers of gridDim entries.  Warpgroup j's first claim
-//     comes from layer j (an atomic counter per layer), so few chains spread one per SM before any SM takes a
-//     second; odd layers are handed out backwards, so with chains ordered by decreasing length the longest of one
-//     layer meet the shortest of the next on an SM.
-//   * Every later claim first looks for entries that are still unclaimed in any layer (left by CTAs that have not
-//     started), then takes the chains beyond the layers in order (the tail counter).
-//   * When all first segments are taken, the tail counter hands out queue tickets: ticket q reads slot q, which
-//     the finisher of some segment fills with the follow-up segment, so chains take turns on the chain slots
-//     (first come, first served) and more chains than slots still share the machine evenly.  Only warpgroups that
-//     run hold tickets, and every unfinished chain is either being walked by a running warpgroup or sits in a
-//     slot, so a waiter never depends on a CTA that has not started.
-// Returns the item, -2 when nothing is left to do, -3 when the bounded wait gave up.
-__device__ __forceinline__ int tc_layer_item(int j, int x, int cnt) {
-    return j * (int)gridDim.x + ((j & 1) ? cnt - 1 - x : x);
-}
-__device__ __forceinline__ int tc_next_item(const TwoPassArgs& a, bool first_claim, int wg, int64_t n_chains,
-                                            volatile int* abort_flag) {
-    const int G = (int)gridDim.x;
-    int32_t* layer = a.queue + 4;   // header words 4 .. 4 + kTcChains - 1
-    auto layer_count = [&](int j) {
-        const int64_t c = n_chains - (int64_t)j * G;
-        return (int)(c < 0 ? 0 : (c > G ? G : c));
-    };
-    if (first_claim) {
-        const int cnt = layer_count(wg);
-        if (cnt > 0) {
-            const int x = atomicAdd(layer + wg, 1);
-            if (x < cnt) return tc_layer_item(wg, x, cnt);
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < kTcChains; ++j) {
-            const int cnt = layer_count(j);
-            if (*reinterpret_cast<volatile int32_t*>(layer + j) < cnt) {
-                const int x = atomicAdd(layer + j, 1);
-                if (x < cnt) return tc_layer_item(j, x, cnt);
-            }
-        }
-    }
-    const int64_t n_tail = n_chains > (int64_t)kTcChains * G ? n_chains - (int64_t)kTcChains * G : 0;
-    const int t = atomicAdd(a.queue, 1);
-    if (t < n_tail) return kTcChains * G + t;
-    int item = -2;
-    if (a.seg_chunks > 0) {
-        volatile int32_t* slot = a.qslots + (t - (int)n_tail);
-        volatile int32_t* finished = a.queue + 3;
-        const uint64_t t0 = global_timer_ns();
-        uint32_t spins = 0;
-        for (;;) {
-            const int x = *slot;
-            if (x >= 0) { item = x; break; }
-            if (*finished >= (int)n_chains) break;
-            if ((++spins & 63u) == 0 && (*abort_flag != 0 || global_timer_ns() - t0 > a.wait_ns)) { item = -3; break; }
-            __nanosleep(200);
-        }
-        __threadfence();  // the pusher's state stores are visible before we read them
-    }
-    return item;
-}
-// The finisher of a non-final segment queues the follow-up segment (ONE thread, after the state hand-over
-// stores of all threads have been fenced and a barrier has passed).
-__device__ __forceinline__ void tc_push_followup(const TwoPassArgs& a, int item, int64_t n_chains) {
-    if (a.test_drop_push) return;  // test hook: starve the queue so that its bounded waits give up
-    const int pos = atomicAdd(a.queue + 2, 1);
-    __threadfence();
-    *reinterpret_cast<volatile int32_t*>(a.qslots + pos) = item + (int)n_chains;
-}
-
-// sigmoid(beta) of the 16 rows as bf16x2 pairs (the record holds them as 16 bf16 values)
-__device__ __forceinline__ void tc_load_beta(const uint8_t* rec, uint32_t (&bpk)[8]) {
-    const uint4* bp = reinterpret_cast<const uint4*>(rec + kTcBeta);
-    const uint4 x = bp[0], y = bp[1];
-    bpk[0] = x.x; bpk[1] = x.y; bpk[2] = x.z; bpk[3] = x.w;
-    bpk[4] = y.x; bpk[5] = y.y; bpk[6] = y.z; bpk[7] = y.w;
-}
-// value column v of the chunk from the [16][128] tile (zero past the sequence end)
-__device__ __forceinline__ void tc_load_v_column(const uint8_t* v_tile, int v, int len, unsigned short (&v_cur)[kChunk]) {
-    const unsigned short* vt = reinterpret_cast<const unsigned short*>(v_tile) + v;
-    if (len == kChunk) {  // the common case without per-row masks
-#pragma unroll
-        for (int i = 0; i < kChunk; ++i) v_cur[i] = vt[i * kD];
-    } else {
-#pragma unroll
-        for (int i = 0; i < kChunk; ++i) v_cur[i] = (i < len) ? vt[i * kD] : (unsigned short)0;
-    }
-}
-// out = bf(o0) (+) bf(Mqk U) for V row v; r holds D3 in 0-15 and o0 in 16-31.  Full chunks go through the out
-// tile (one TMA store later), ragged tails straight to global memory, valid rows only.
-__device__ __forceinline__ void tc_store_out(const uint32_t (&r)[32], unsigned short* out_tile, unsigned short* out_global,
-                                             int64_t tstride, int v, int len) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t o = bf2_add(pack_bf2(__uint_as_float(r[16 + 2 * i]), __uint_as_float(r[16 + 2 * i + 1])),
-                                   pack_bf2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
-        if (len == kChunk) {
-            out_tile[(2 * i) * kD + v] = (unsigned short)(o & 0xffffu);
-            out_tile[(2 * i + 1) * kD + v] = (unsigned short)(o >> 16);
-        } else {
-            unsigned short* dst = out_global + (int64_t)(2 * i) * tstride;
-            if (2 * i < len) dst[0] = (unsigned short)(o & 0xffffu);
-            if (2 * i + 1 < len) dst[tstride] = (unsigned short)(o >> 16);
-        }
-    }
-}
-
 }  // namespace fkda
 
-#include "fkda_tc_ts.cuh"
+#include "fkda_fused.cuh"
 #include "fkda_rows.cuh"
 
 namespace fkda {
@@ -217,33 +81,58 @@ int device_sm_count() {
     return cache[dev];
 }
 
-// Segment scheduling is used when there are more chains than the GPU can hold at once (3 per SM);
-// with fewer chains every chain has its own slot and whole chains are the work items.
-constexpr int kSegChunksMax = 64, kSegChunksMin = 16;
-// Segment length: 64 chunks when there is plenty of work (the hand-over of a 32 KB state costs about one chunk
-// step), shorter when the whole problem is only a few segments per chain slot, so that 512 chains of 64 chunks
-// do not run as one full round plus a nearly empty one.  Even, so that the stage parity of a segment's
-// first chunk is fixed.  A function of (T_total, H, N) only: the workspace is sized with the same value.
-static int seg_chunks_for(int64_t T_total, int64_t H, int64_t N, int sms) {
-    const int64_t chain_slots = (int64_t)sms * kTcChains;
-    int64_t seg = H * ws_tiles_upper_bound(T_total, N) / (4 * chain_slots);  // aim at >= 4 segments per chain slot
-    seg = seg / 2 * 2;
-    if (seg > kSegChunksMax) seg = kSegChunksMax;
-    if (seg < kSegChunksMin) seg = kSegChunksMin;
-    return (int)seg;
+constexpr size_t kStateBytes = (size_t)kD * kD * 2;   // a chain's state as bf16 (hand-over buffers)
+
+// Few chains on a fixed batch may run as a slab pipeline (see launch_tc): at least 32 SMs are left beside the row slices.
+static bool slabs_possible(int64_t chains, int sms) { return chains * kRowSplit <= sms - 32; }
+
+// The one-kernel forward serves whole forwards with more than one chunk per chain on average and more row slices than SMs.
+// While every slice has an SM of its own, a step of the row-slice kernel takes 0.52 us against 1.05 us here, which pays for the
+// prepare kernel in front of it (64 chains of 512 chunks: 0.50 ms against 0.57; 96 chains: 0.71 against 0.57).  A ragged batch
+// whose lengths the host does not know may consist of a few long chains, whose walk is then the whole time (128 chains of 1
+// to 32 chunks: 52 us in two kernels against 82): it needs two chains per SM.
+static bool fused_eligible(const fkda_fwd_params& p, int sms) {
+    if (p.phase_mask != 0 || p.B * p.T <= kChunk * p.N || p.token_stride >= ((int64_t)1 << 27)) return false;
+    const int64_t chains = p.N * p.H;
+    return (p.cu_seqlens != nullptr ? chains >= 2 * sms : chains * kRowSplit > sms) || (p.flags & FKDA_FLAG_NO_WIDE);
 }
-static bool use_segments(int64_t H, int64_t N, int sms) { return H * N > (int64_t)sms * kTcChains; }
-// slots of the segment queue: sized for the shortest segment length a call may ask for (8 chunks), plus one
-// ticket per resident warpgroup at the end
-static size_t seg_slots_bytes(int64_t T_total, int64_t H, int64_t N, int sms) {
-    if (!use_segments(H, N, sms)) return 0;
-    const size_t count = (size_t)(H * (ws_tiles_upper_bound(T_total, N) / 8 + N) + 4096);
-    return (count * 4 + 255) / 256 * 256;
+static size_t fused_flag_bytes(int sms) { return (size_t)(sms * 4 + 255) / 256 * 256; }
+// header | prefix tables | one flag and one hand-over state per range
+static size_t fused_bytes(int64_t N, int sms) { return kWsHeaderBytes + ws_prefix_bytes(N) + fused_flag_bytes(sms) + (size_t)sms * kStateBytes; }
+
+// The two-kernel form: header | prefix tables | hand-over states of the slab pipeline | records.  A function of the shapes
+// only, not of phase_mask or flags, so that calls which share a workspace find the records in the same place.
+struct TcCarve {
+    size_t states, records;
+};
+static TcCarve tc_carve(const fkda_fwd_params& p, int sms) {
+    const int64_t chains = p.N * p.H;
+    const bool varlen = p.cu_seqlens != nullptr;
+    TcCarve c;
+    c.states = !varlen && slabs_possible(chains, sms) ? (size_t)chains * kStateBytes : 0;
+    const int64_t tiles = varlen ? ws_tiles_upper_bound(p.B * p.T, p.N) : p.N * ((p.T + kChunk - 1) / kChunk);
+    c.records = (size_t)p.H * (size_t)tiles * (size_t)kTcRecord;
+    return c;
 }
-// Few chains on a fixed batch may run as a slab pipeline (see launch_tc); its chain states travel through the
-// same hand-over buffer as the segments of the work queue (32 KB per chain).
-static bool slabs_possible(int64_t chains, int sms) { return chains * kRowSplit <= sms - 32; }   // SMs left for the prepare stage
-static size_t seg_state_bytes(int64_t H, int64_t N, bool needed) { return needed ? (size_t)(H * N) * 32768 : 0; }
+
+// Upper bound over every call with these totals (the caller may not know yet whether the batch is ragged).
+size_t tc_workspace_bytes(int64_t T_total, int64_t H, int64_t N) {
+    const int sms = device_sm_count();
+    const size_t two_pass = kWsHeaderBytes + ws_prefix_bytes(N) + (slabs_possible(H * N, sms) ? (size_t)(H * N) * kStateBytes : 0) +
+                            (size_t)H * (size_t)ws_tiles_upper_bound(T_total, N) * (size_t)kTcRecord;
+    const size_t fused = fused_bytes(N, sms);
+    return two_pass > fused ? two_pass : fused;
+}
+
+// What one particular call needs.
+size_t tc_workspace_bytes_for(const fkda_fwd_params& p) {
+    if (decode_eligible(p) && !(p.flags & FKDA_FLAG_NO_DECODE) && p.chunk_states == nullptr) return 0;   // one kernel, nothing staged
+    if (short_eligible(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) return 0;
+    const int sms = device_sm_count();
+    if (fused_eligible(p, sms)) return fused_bytes(p.N, sms);
+    const TcCarve c = tc_carve(p, sms);
+    return kWsHeaderBytes + ws_prefix_bytes(p.N) + c.states + c.records;
+}
 
 // Side stream and events of the slab pipeline, one set per device, created on first use.
 constexpr int kMaxSlabs = 4;
@@ -269,38 +158,6 @@ static SlabStreams* slab_streams(int dev) {
     return &t;
 }
 
-// Upper bound over every call with these totals (the caller may not know yet whether the batch is ragged).
-size_t tc_workspace_bytes(int64_t T_total, int64_t H, int64_t N) {
-    const int sms = device_sm_count();
-    const bool states = use_segments(H, N, sms) || slabs_possible(H * N, sms);
-    return kWsHeaderBytes + ws_prefix_bytes(N) + seg_slots_bytes(T_total, H, N, sms) + seg_state_bytes(H, N, states) +
-           (size_t)H * (size_t)ws_tiles_upper_bound(T_total, N) * (size_t)kTcRecord;
-}
-
-// What one particular call needs: the same carving as launch_tc (a function of the shapes only, not of
-// phase_mask or flags, so that calls which share a workspace find the records in the same place).
-struct TcCarve {
-    size_t slots, states, records;
-    bool segments;
-};
-static TcCarve tc_carve(const fkda_fwd_params& p, int sms) {
-    const int64_t T_total = p.B * p.T, chains = p.N * p.H;
-    const bool varlen = p.cu_seqlens != nullptr;
-    TcCarve c;
-    c.segments = use_segments(p.H, p.N, sms);
-    c.slots = seg_slots_bytes(T_total, p.H, p.N, sms);
-    c.states = seg_state_bytes(p.H, p.N, c.segments || (!varlen && slabs_possible(chains, sms)));
-    const int64_t tiles = varlen ? ws_tiles_upper_bound(T_total, p.N) : p.N * ((p.T + kChunk - 1) / kChunk);
-    c.records = (size_t)p.H * (size_t)tiles * (size_t)kTcRecord;
-    return c;
-}
-size_t tc_workspace_bytes_for(const fkda_fwd_params& p) {
-    if (decode_eligible(p) && !(p.flags & FKDA_FLAG_NO_DECODE) && p.chunk_states == nullptr) return 0;   // one kernel, nothing staged
-    if (short_eligible(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) return 0;
-    const TcCarve c = tc_carve(p, device_sm_count());
-    return kWsHeaderBytes + ws_prefix_bytes(p.N) + c.slots + c.states + c.records;
-}
-
 // The driver entry point is looked up through the runtime (no link-time dependency on libcuda, so
 // the library also loads on a machine without a driver).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -318,19 +175,42 @@ static EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// Map over a [token][head][128] tensor with tiles of 16 tokens x `cols` columns of one head.  `swizzle`: the 16-byte pieces
-// of a tile row are permuted by the row, so that transposing accesses to the tile (8 rows of one piece) do not collide.
-static bool encode_token_map(CUtensorMap* m, const void* base, int64_t T_total, int64_t H, int64_t token_stride, int cols,
-                             CUtensorMapSwizzle swizzle) {
+// Map over v viewed as [token][head][128] bf16 with tiles of 16 tokens x 64 columns of one head; the 16-byte pieces of a tile
+// row are permuted by the row (128-byte swizzle), so that transposing reads of the tile (8 rows of one piece) do not collide.
+static bool encode_v_map(CUtensorMap* m, const fkda_fwd_params& p) {
     EncodeTiledFn encode = encode_tiled_fn();
     if (encode == nullptr) return false;
-    const cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)H, (cuuint64_t)(T_total > 0 ? T_total : 1)};
-    const cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)token_stride * 2};  // bytes, dims 1 and 2
-    const cuuint32_t box[3] = {(cuuint32_t)cols, 1u, (cuuint32_t)kChunk};
+    const cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)p.H, (cuuint64_t)(p.B * p.T)};
+    const cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)p.token_stride * 2};  // bytes, dims 1 and 2
+    const cuuint32_t box[3] = {(cuuint32_t)kD / 2, 1u, (cuuint32_t)kChunk};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
-    return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
-                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                                  CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p.v), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+static_assert(kRowCols == kD / 2, "a CTA of the row-slice kernel takes one half of a value row");
+
+// One kernel (and the prefix kernel of a ragged batch).
+static int launch_fused(const fkda_fwd_params& p, TwoPassArgs& a, int sms, cudaStream_t stream, int* n_launches) {
+    const int64_t chains = p.N * p.H;
+    uint8_t* flags = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes + ws_prefix_bytes(p.N);
+    a.range_flags = reinterpret_cast<int32_t*>(flags);
+    a.seg_state = reinterpret_cast<uint32_t*>(flags + fused_flag_bytes(sms));
+    if (cudaMemsetAsync(p.workspace, 0, 64, stream) != cudaSuccess || cudaMemsetAsync(flags, 0, fused_flag_bytes(sms), stream) != cudaSuccess)
+        return FKDA_ERR_LAUNCH;
+    int launches = 0;
+    if (p.cu_seqlens != nullptr) {
+        launch_tile_prefix(a, nullptr, false, stream);
+        ++launches;
+    }
+    VMap map;
+    if (!encode_v_map(&map.v, p)) return FKDA_ERR_LAUNCH;
+    const bool exports = a.chunk_states != nullptr;
+    if (!(exports ? allow_smem<fused_kernel<true>>(kFusedSmemBytes) : allow_smem<fused_kernel<false>>(kFusedSmemBytes))) return FKDA_ERR_LAUNCH;
+    (exports ? fused_kernel<true> : fused_kernel<false>)<<<(unsigned)(chains < sms ? chains : sms), kFusedThreads, kFusedSmemBytes, stream>>>(a, map);
+    ++launches;
+    if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
+    *n_launches = launches;
+    return FKDA_OK;
 }
 
 int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
@@ -343,42 +223,41 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return FKDA_ERR_LAUNCH;
     const int sms = device_sm_count();
-    const int64_t T_total = p.B * p.T;
-    if (cudaMemsetAsync(p.workspace, 0, 64, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;  // header counters
-    {   // carve the segment queue and the hand-over states in front of the records
-        uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes + ws_prefix_bytes(p.N);
-        const TcCarve c = tc_carve(p, sms);
-        if (c.segments) {
-            a.qslots = reinterpret_cast<int32_t*>(base);
-            const int forced = ((p.flags >> 8) & 0xff) / 2 * 2;
-            a.seg_chunks = forced >= 8 ? forced : seg_chunks_for(T_total, p.H, p.N, sms);
-            if (do_rec && cudaMemsetAsync(a.qslots, 0xff, c.slots, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;
-        }
-        a.seg_state = reinterpret_cast<uint32_t*>(base + c.slots);
-        a.workspace = base + c.slots + c.states;
-    }
-    const int64_t chains = p.N * p.H;
-    const bool rows = chains <= sms && !(p.flags & FKDA_FLAG_NO_WIDE);
-    TcMaps maps;
-    memset(&maps, 0, sizeof(maps));
+    const int64_t T_total = p.B * p.T, chains = p.N * p.H;
+    if (fused_eligible(p, sms)) return launch_fused(p, a, sms, stream, n_launches);
+    if (chains * kRowSplit > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
+    if (cudaMemsetAsync(p.workspace, 0, 64, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;  // header: status, decisions
+    const TcCarve carve = tc_carve(p, sms);
+    uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes + ws_prefix_bytes(p.N);
+    a.seg_state = reinterpret_cast<uint32_t*>(base);
+    a.workspace = base + carve.states;
+    VMap map;
+    memset(&map, 0, sizeof(map));
     // (an empty batch has no tiles to move: its chains only pass their state through)
-    if (do_rec && T_total > 0 &&
-        (!encode_token_map(&maps.v, p.v, T_total, p.H, p.token_stride, rows ? kRowCols : kD,
-                           rows ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE) ||
-         (!rows && !encode_token_map(&maps.out, p.out, T_total, p.H, p.token_stride, kD, CU_TENSOR_MAP_SWIZZLE_NONE))))
-        return FKDA_ERR_LAUNCH;
-    const auto rows_kernel = a.chunk_states != nullptr ? recurrence_rows_kernel<true> : recurrence_rows_kernel<false>;
-    if (do_rec && rows && !(a.chunk_states != nullptr ? allow_smem<recurrence_rows_kernel<true>>(kRowSmemBytes)
-                                                       : allow_smem<recurrence_rows_kernel<false>>(kRowSmemBytes)))
-        return FKDA_ERR_LAUNCH;
+    if (do_rec && T_total > 0 && !encode_v_map(&map.v, p)) return FKDA_ERR_LAUNCH;
+    // A ragged batch whose sequences MAY all fit one chunk (the host sees only the totals): the prefix kernel decides, the
+    // one-chunk kernels and the general kernels are all enqueued and all but one return at once.
+    if (short_ragged_candidate(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) a.short_flag = a.queue + 8;
+    auto rows_kernel = recurrence_rows_kernel<false, false>;
+    bool smem_ok = true;
+    if (a.short_flag != nullptr) {   // (such a batch exports no states)
+        rows_kernel = recurrence_rows_kernel<false, true>;
+        smem_ok = allow_smem<recurrence_rows_kernel<false, true>>(kRowSmemBytes);
+    } else if (a.chunk_states != nullptr) {
+        rows_kernel = recurrence_rows_kernel<true, false>;
+        smem_ok = allow_smem<recurrence_rows_kernel<true, false>>(kRowSmemBytes);
+    } else {
+        smem_ok = allow_smem<recurrence_rows_kernel<false, false>>(kRowSmemBytes);
+    }
+    if (!smem_ok) return FKDA_ERR_LAUNCH;
 
-    // ---- few chains on a fixed batch: the recurrence is a serial walk on `chains` SMs and leaves the others
+    // ---- few chains on a fixed batch: the recurrence is a serial walk on 2 x chains SMs and leaves the others
     //      idle, so the forward is cut into slabs of chunks and the prepare stage of slab i+1 runs on the idle SMs
     //      (side stream) while the recurrence walks slab i; the state of a chain travels through seg_state.
     //      Only stream order and events connect the launches: no kernel waits for another one. ----
     const int64_t tps = (p.T + kChunk - 1) / kChunk;
-    const int idle_sms = sms - (int)chains * kRowSplit;
-    if (rows && !varlen && p.phase_mask == 0 && slabs_possible(chains, sms) && tps >= 64 && !(p.flags & FKDA_FLAG_NO_SLABS)) {
+    if (!varlen && p.phase_mask == 0 && slabs_possible(chains, sms) && tps >= 64 && !(p.flags & FKDA_FLAG_NO_SLABS)) {
+        const int idle_sms = sms - (int)chains * kRowSplit;
         SlabStreams* ss = slab_streams(dev);
         if (ss == nullptr) return FKDA_ERR_LAUNCH;
         // host threads that call concurrently on one device share the side stream and its events
@@ -418,7 +297,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         for (int i = 0; i < n_slabs; ++i) {
             if (bounds[i + 1] <= bounds[i]) continue;
             if (i > 0 && cudaStreamWaitEvent(stream, ss->done[i], 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
-            rows_kernel<<<(unsigned)(chains * kRowSplit), kRowThreads, kRowSmemBytes, stream>>>(slab_args(i), maps);
+            rows_kernel<<<(unsigned)(chains * kRowSplit), kRowThreads, kRowSmemBytes, stream>>>(slab_args(i), map);
             ++launches;
         }
         if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
@@ -426,15 +305,10 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         return FKDA_OK;
     }
 
-    // A ragged batch whose sequences MAY all fit one chunk (the host sees only the totals): the prefix kernel decides,
-    // the fused short-sequence kernel and the general kernels are both enqueued and one side returns at once.
-    if (short_ragged_candidate(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) a.short_flag = a.queue + 8;
     // as many tokens as sequences: they may have one token each, the decode kernel's case
     const bool try_decode = a.short_flag != nullptr && T_total == p.N && !(p.flags & FKDA_FLAG_NO_DECODE);
     if (varlen && do_prep) {
-        launch_tile_prefix(p.cu_seqlens, p.N, a.tile_prefix, const_cast<int32_t*>(a.seq_order),
-                           a.chunk_states != nullptr ? const_cast<int32_t*>(a.cs_prefix) : nullptr, 16 * a.cs_every,
-                           a.short_flag, try_decode, a.qslots != nullptr ? a.queue + 9 : nullptr, p.H, sms * kTcChains, stream);
+        launch_tile_prefix(a, const_cast<int32_t*>(a.seq_order), try_decode, stream);
         ++launches;
     }
     if (try_decode) {
@@ -450,17 +324,10 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         ++launches;
     }
     if (do_rec) {
-        int64_t ctas = chains;  // one chain per SM while they last, then two, then three
-        if (ctas > sms) ctas = sms;
-        if (ctas < 1) ctas = 1;
-        if (rows) {
-            // few chains: every chain cut into row slices
-            rows_kernel<<<(unsigned)(chains * kRowSplit), kRowThreads, kRowSmemBytes, stream>>>(a, maps);
-        } else {
-            // three chains per CTA, state copy and 16-deep A operands in tensor memory
-            if (!allow_smem<recurrence_tc_ts_kernel>(kTsSmemBytes)) return FKDA_ERR_LAUNCH;
-            recurrence_tc_ts_kernel<<<(unsigned)ctas, kTcChains * 128, kTsSmemBytes, stream>>>(a, maps);
-        }
+        // (behind a device-side decision this launch mostly returns at once: a grid that is resident in one go)
+        int64_t ctas = chains * kRowSplit;
+        if (a.short_flag != nullptr && ctas > 2 * sms) ctas = 2 * sms;
+        rows_kernel<<<(unsigned)ctas, kRowThreads, kRowSmemBytes, stream>>>(a, map);
         ++launches;
     }
     if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;

@@ -12,6 +12,8 @@
 // reads them is issued, so the eight dependent products of D1 run inside the update instead of after it.
 #pragma once
 
+#include <cuda.h>
+
 #include "fkda_common.cuh"
 #include "fkda_internal.h"
 #include "fkda_sm100.cuh"
@@ -60,6 +62,11 @@ __device__ __forceinline__ uint32_t update_pair(uint32_t s, const float2& e, flo
     fma2_rn(y0, y1, bf_lo(s), bf_hi(s), e.x, e.y, d0, d1);
     return pack_bf2(y0, y1);
 }
+
+// Tensor map over v (see encode_v_map).
+struct alignas(64) VMap {
+    CUtensorMap v;
+};
 
 // Per-lane byte offsets into a record (ldmatrix: lane 8m + r addresses row r of the m-th 8x8 matrix)
 struct WalkLane {
@@ -121,6 +128,14 @@ struct WalkState {
     float u0[kMt][2][4];       // S . kd^T of the current chunk, token tiles 0 and 1
     float o0[kMt][2][4];       // S . qd^T
 
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int mt = 0; mt < kMt; ++mt)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[mt][j][e] = 0u;
+    }
     // K step j of D1: kd fragments b[0..3], qd fragments b[4..7]
     __device__ __forceinline__ void fetch_d1(uint32_t (&b)[8], uint32_t rec, const WalkLane& wl, int j) {
         ldmatrix_x4_a(b[0], b[1], b[2], b[3], rec + wl.b1 + 2 * j * kTcB1Lbo);
@@ -243,35 +258,35 @@ struct WalkState {
 constexpr int kWalkStageBytes = 16 * 256;
 __device__ __forceinline__ uint32_t walk_stage_off(int r, int piece) { return (uint32_t)(r * 256 + ((piece ^ (r & 7)) << 4)); }
 
-// `src` = element (first row of the tile, column 0); fp32 states are rounded to bf16
-__device__ __forceinline__ void walk_load_tile(uint32_t (&s)[8][4], uint8_t* stage, const void* src, bool fp32, int lane) {
-    if (fp32) {
-        const float4* p = reinterpret_cast<const float4*>(src);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float4 x[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) x[i] = __ldg(p + 32 * (8 * h + i) + lane);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)   // row i, columns 4 lane ..: half (lane & 1) of piece lane / 2
-                *reinterpret_cast<uint2*>(stage + walk_stage_off(8 * h + i, lane >> 1) + 8 * (lane & 1)) =
-                    make_uint2(pack_bf2(x[i].x, x[i].y), pack_bf2(x[i].z, x[i].w));
-        }
-    } else {
-        const uint4* p = reinterpret_cast<const uint4*>(src);
-        uint4 x[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = __ldg(p + 32 * i + lane);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)   // row 2 i + lane / 16, piece lane % 16
-            *reinterpret_cast<uint4*>(stage + walk_stage_off(2 * i + (lane >> 4), lane & 15)) = x[i];
-    }
-    __syncwarp();
+// kMt consecutive row tiles; `src` = element (first row, column 0); fp32 states are rounded to bf16.  The loads of all tiles
+// are in flight before the first is staged.
+template <int kMt, bool kFp32>
+__device__ __forceinline__ void walk_load_tiles(uint32_t (&s)[kMt][8][4], uint8_t* stage, const void* src, int lane) {
     const uint32_t base = sm100::smem_u32(stage);
     const int r = (lane & 7) + 8 * ((lane >> 3) & 1), c = lane >> 4;
+    const uint4* p = reinterpret_cast<const uint4*>(src) + lane;
+    constexpr int kPer = kFp32 ? 16 : 8;   // 16-byte pieces per lane and tile
+    uint4 x[kMt][kPer];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ldmatrix_x4_a(s[j][0], s[j][1], s[j][2], s[j][3], base + walk_stage_off(r, 2 * j + c));
-    __syncwarp();
+    for (int mt = 0; mt < kMt; ++mt)
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) x[mt][i] = __ldg(p + 32 * (kPer * mt + i));
+#pragma unroll
+    for (int mt = 0; mt < kMt; ++mt) {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            if constexpr (kFp32)   // row i, columns 4 lane ..: half (lane & 1) of piece lane / 2
+                *reinterpret_cast<uint2*>(stage + walk_stage_off(i, lane >> 1) + 8 * (lane & 1)) =
+                    make_uint2(pack_bf2(__uint_as_float(x[mt][i].x), __uint_as_float(x[mt][i].y)),
+                               pack_bf2(__uint_as_float(x[mt][i].z), __uint_as_float(x[mt][i].w)));
+            else                   // row 2 i + lane / 16, piece lane % 16
+                *reinterpret_cast<uint4*>(stage + walk_stage_off(2 * i + (lane >> 4), lane & 15)) = x[mt][i];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ldmatrix_x4_a(s[mt][j][0], s[mt][j][1], s[mt][j][2], s[mt][j][3], base + walk_stage_off(r, 2 * j + c));
+        __syncwarp();
+    }
 }
 __device__ __forceinline__ void walk_store_tile(const uint32_t (&s)[8][4], uint8_t* stage, void* dst, bool fp32, int lane) {
     const uint32_t base = sm100::smem_u32(stage);

@@ -47,7 +47,8 @@ enum { FKDA_PHASE_PREPARE = 1, FKDA_PHASE_RECURRENCE = 2 };
 enum {
     FKDA_ALGO_AUTO = 0,
     FKDA_ALGO_TWOPASS = 1, /* prepare kernel -> HBM workspace -> recurrence kernel (CUDA cores) */
-    FKDA_ALGO_TC = 2       /* prepare kernel -> HBM workspace -> persistent tcgen05/TMEM recurrence; a fixed batch
+    FKDA_ALGO_TC = 2       /* tensor cores: one persistent kernel where the chains fill the GPU, otherwise prepare kernel ->
+                              workspace -> recurrence on row slices; a fixed batch
                               with T == 1 (decode step) runs one state read-modify-write kernel instead, one with
                               2 <= T <= 16 one fused kernel per (sequence, head) */
 };
@@ -82,9 +83,9 @@ typedef struct fkda_fwd_params {
     double lower_bound;        /* gate lower bound, -5 <= lower_bound <= 0 */
     void* workspace;           /* >= fkda_workspace_bytes(B*T, H, N, algo) bytes, 256-byte aligned */
     size_t workspace_bytes;
-    int32_t phase_mask;        /* measurement aid for multi-kernel algos: 0 = whole forward; otherwise a
-                                  bit set of FKDA_PHASE_* to launch (the workspace must then already hold
-                                  what the skipped phases produce) */
+    int32_t phase_mask;        /* 0 = whole forward, by whatever kernels serve it best; otherwise a bit set of FKDA_PHASE_*
+                                  to launch in the two-kernel form, which leaves (PREPARE) or expects (RECURRENCE)
+                                  the chunk records in the workspace */
     int32_t flags;             /* 0 for normal use; FKDA_FLAG_* bits select kernel variants for tests and tuning */
     void* chunk_states;        /* optional bf16 [slots, H, 128 (V), 128 (K)]: the state of every sequence BEFORE each group
                                   of `chunk_states_every` chunks (16 * every tokens), i.e. before tokens 0, 16*every,
@@ -100,13 +101,13 @@ typedef struct fkda_fwd_params {
 /* fkda_fwd_params.flags.  All zero is the production setting. */
 enum {
     FKDA_FLAG_NO_DECODE = 1,       /* run a T == 1 batch through the chunked kernels instead of the decode kernel */
-    FKDA_FLAG_NO_WIDE = 2,         /* never pick the one-chain-per-CTA recurrence */
+    FKDA_FLAG_NO_WIDE = 2,         /* run a whole forward of few chains through the one-kernel form instead of row slices */
     FKDA_FLAG_NO_SLABS = 4,        /* no slab pipeline (prepare of the next slab beside the recurrence) */
     FKDA_FLAG_NO_SHORT = 8,        /* run a batch of sequences of at most 16 tokens each through the general kernels */
-    FKDA_FLAG_TEST_DROP_PUSH = 16  /* TEST ONLY: finished segments do not queue their follow-up, so that the
-                                      work queue starves and its bounded waits give up */
+    FKDA_FLAG_TEST_DROP_PUSH = 16  /* TEST ONLY: the one-kernel form does not publish the states it hands over, so that
+                                      the waiters starve and their bounded waits give up */
 };
-/* bits 8..15: segment length of the work queue in chunks (0 = automatic; tuning aid)
+/* bits 8..15: no effect (once the segment length of a work queue)
  * bits 16..29: limit of every bounded device-side wait in milliseconds (0 = the default of 2000) */
 #define FKDA_FLAGS_SEG_CHUNKS(x) (((x) & 0xff) << 8)
 #define FKDA_FLAGS_WAIT_MS(x) (((x) & 0x3fff) << 16)
@@ -122,8 +123,9 @@ size_t fkda_workspace_bytes(int64_t T_total, int64_t H, int64_t N, int32_t algo)
 size_t fkda_workspace_bytes_for(const fkda_fwd_params* p);
 
 /* Enqueues the forward pass on `stream` (a cudaStream_t passed as void*).
- * Paths: a fixed batch with T == 1 is one state read-modify-write kernel, with 2 <= T <= 16 one fused kernel, anything
- * else the prepare kernel plus the tensor-core recurrence.  For a ragged batch (cu_seqlens) the host knows only the
+ * Paths: a fixed batch with T == 1 is one state read-modify-write kernel, with 2 <= T <= 16 one fused kernel, a batch
+ * with enough (sequence, head) pairs to fill the GPU one persistent kernel, anything else the prepare kernel plus the
+ * recurrence on row slices.  For a ragged batch (cu_seqlens) the host knows only the
  * totals: when there are at most 16 tokens per sequence on average (and at least 64 (sequence, head) pairs), a prefix
  * kernel decides on the device whether every sequence has one token, or at most 16, and the kernels of the paths that
  * may apply are all enqueued; those that are not needed return at once.  Results do not depend on the path
