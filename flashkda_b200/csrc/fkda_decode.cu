@@ -12,9 +12,24 @@
 // accumulation in the dot products, tanh.approx / ex2.approx / rsqrt.approx, state rounded to bf16.
 #include "fkda_common.cuh"
 #include "fkda_internal.h"
-#include "fkda_prepare_warp.cuh"
 
 namespace fkda {
+
+// Sum of squares of one 128-wide row held 4 columns per lane, in the contract's order: FMA chain
+// over columns 8m..8m+7 (lanes 2m then 2m+1), then xor-butterfly with offsets 8,4,2,1 over the 16
+// groups.  All lanes return the row total.
+__device__ __forceinline__ float row_sumsq(const float (&x)[4], int lane) {
+    float p = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) p = __fmaf_rn(x[i], x[i], p);
+    const float first = __shfl_sync(0xffffffffu, p, lane & ~1);  // partial of the even lane of my pair
+    float c = first;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c = __fmaf_rn(x[i], x[i], c);     // odd lanes: chain continued over their 4
+#pragma unroll
+    for (int off = 16; off >= 2; off >>= 1) c = __fadd_rn(c, __shfl_xor_sync(0xffffffffu, c, off));
+    return __shfl_sync(0xffffffffu, c, lane | 1);                 // the odd lanes hold the group sums
+}
 
 // x[i] holds this lane's partial sum of row i (32 rows).  Returns the warp total of row `lane`:
 // at each halving step a lane keeps the half of the rows whose index bit matches its lane bit and

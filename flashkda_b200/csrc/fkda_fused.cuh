@@ -123,6 +123,10 @@ struct FusedCtrl {
     int32_t abort_flag;
 };
 constexpr int kFusedSmemBytes = kFusedCtrl + (int)sizeof(FusedCtrl) + 1024;
+// Two producers may wait on one slot, for units a whole round apart, but the later one only after the unit before the earlier
+// one's was consumed (it had to be, for the later one's previous unit to get its slot): with more producers than slots that
+// no longer holds and the parities of the rounds become ambiguous.
+static_assert(kFusedPrep <= kFusedSlots, "no more preparing warps than slots");
 static_assert(kFusedVTile == 4096 && kFusedWalkers * kFusedCols == kD && kFusedOut % 256 == 0 && kFusedStaging % 16 == 0 &&
               kFusedRec % 16 == 0 && kFusedCtrl % 8 == 0 && kFusedSmemBytes <= 232448, "shared-memory layout");
 
@@ -165,8 +169,6 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
     if (warp >= kFusedWalkers) {
         // =========================== preparing warps ===========================
         reg_dealloc<144>();
-        int slot = (warp - kFusedWalkers) % kFusedSlots;
-        uint32_t phase = 1;   // of empty[slot]: the first round finds the blocks free
         FusedSeq sq;          // the sequence of the current unit
         sq.begin = sq.end = sq.n_chunks = -1;
         int h = 0, t = 0;     // its head and chunk
@@ -191,35 +193,35 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
             PrepHead x;
             const PrepSrc src = prep_src(a, t0, len, h, lane);
             prep_load(a, src, t0, len, h, lane, x);
-            if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.empty[slot], phase, abort_flag, a.wait_ns)) == 0) {
+            const int slot = u % kFusedSlots;
+            const uint32_t phase = 1u ^ ((u / kFusedSlots) & 1);   // of empty[slot]: the first round finds the slots free
+            uint8_t* rec = sm + kFusedRec + slot * kTcRecord;
+            auto acquire = [&]() {   // the slot is free: leave the note and ask for the value tile
+                if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.empty[slot], phase, abort_flag, a.wait_ns)) == 0) return false;
+                if (lane == 0) {
+                    FusedInfo& f = ctl.info[slot];
+                    f.tok0 = t0;
+                    f.n = sq.n; f.h = h; f.chunk = t;
+                    f.left = (int)min((int64_t)0x7fffffff, sq.seq_len - (int64_t)t * kChunk);
+                    f.rest = (int)min(end - p, (int64_t)(sq.n_chunks - t));
+                    f.last = f.rest == sq.n_chunks - t;
+                    // rows past the end of the tensor arrive as zeros; rows of the next sequence are never used
+                    mbar_arrive_expect_tx(&ctl.full[slot], kFusedVTile);
+                    tma_load_3d(sm + kFusedV + slot * kFusedVTile, &map.v, 0, h, (int)t0, &ctl.full[slot]);
+                    tma_load_3d(sm + kFusedV + slot * kFusedVTile + kFusedVTile / 2, &map.v, kD / 2, h, (int)t0, &ctl.full[slot]);
+                }
+                __syncwarp();
+                return true;
+            };
+            if (!prep_compute(a, src, len, rec, lane, x, acquire, [] {})) {
                 failed = true;
                 *abort_flag = 1;
-                // my value tiles in flight (of my last two units at most) land before this CTA's shared memory goes
-                for (int v = u - kFusedPrep; v >= 0 && v >= u - 2 * kFusedPrep; v -= kFusedPrep)
+                // my value tiles in flight (of my last units, as many as there are slots) land before this CTA's shared memory goes
+                for (int v = u - kFusedPrep; v >= 0 && v > u - kFusedSlots - kFusedPrep; v -= kFusedPrep)
                     mbar_wait_bounded(&ctl.full[v % kFusedSlots], (uint32_t)((v / kFusedSlots) & 1), nullptr, 100000000ull);
                 break;
             }
-            if (lane == 0) {
-                FusedInfo& f = ctl.info[slot];
-                f.tok0 = t0;
-                f.n = sq.n; f.h = h; f.chunk = t;
-                f.left = (int)min((int64_t)0x7fffffff, sq.seq_len - (int64_t)t * kChunk);
-                f.rest = (int)min(end - p, (int64_t)(sq.n_chunks - t));
-                f.last = f.rest == sq.n_chunks - t;
-                // rows past the end of the tensor arrive as zeros; rows of the next sequence are never used
-                mbar_arrive_expect_tx(&ctl.full[slot], kFusedVTile);
-                tma_load_3d(sm + kFusedV + slot * kFusedVTile, &map.v, 0, h, (int)t0, &ctl.full[slot]);
-                tma_load_3d(sm + kFusedV + slot * kFusedVTile + kFusedVTile / 2, &map.v, kD / 2, h, (int)t0, &ctl.full[slot]);
-            }
-            __syncwarp();
-            uint8_t* rec = sm + kFusedRec + slot * kTcRecord;
-            prep_compute(a, src, len, rec, lane, x);
-            if (lane == 0) mbar_arrive(&ctl.full[slot]);
-            slot += kFusedPrep;
-            if (slot >= kFusedSlots) {
-                slot -= kFusedSlots;
-                phase ^= 1u;
-            }
+            mbar_arrive_lane0(&ctl.full[slot], lane);
         }
     } else {
         // =========================== walking warps ===========================

@@ -71,27 +71,28 @@ struct PrepHead {
     float a_log;
     __nv_bfloat16 beta;   // logit of row `lane` (lanes below 16; 0 past the end, as zero padding does)
 };
-// Where a unit's rows are: the lane's columns of its first row in each tensor (offsets inside a unit fit 32 bits).
+// Where a unit's rows are: the lane's columns of its first row in each tensor.
 struct PrepSrc {
-    const __nv_bfloat16 *q, *k, *g;
-    uint32_t step;        // elements between rows
+    const uint4 *q, *k, *g;
+    uint32_t step;        // 16-byte pieces between rows
     int row0, last;       // my first row, the unit's last row
 };
 __device__ __forceinline__ PrepSrc prep_src(const TwoPassArgs& a, int64_t t0, int len, int h, int lane) {
     const int64_t off = t0 * a.token_stride + (int64_t)h * kD + 8 * (lane & 15);
-    return PrepSrc{a.q + off, a.k + off, a.g + off, (uint32_t)a.token_stride, 8 * (lane >> 4), len - 1};
+    return PrepSrc{reinterpret_cast<const uint4*>(a.q + off), reinterpret_cast<const uint4*>(a.k + off),
+                   reinterpret_cast<const uint4*>(a.g + off), (uint32_t)(a.token_stride >> 3), 8 * (lane >> 4), len - 1};
 }
 // Row i of my half; a row past the end reads the last valid row (its factors are zero).
 __device__ __forceinline__ void prep_load_row(const PrepSrc& s, int i, PrepRow& x) {
-    const uint32_t off = (uint32_t)min(s.row0 + i, s.last) * s.step;
-    x.k = __ldg(reinterpret_cast<const uint4*>(s.k + off));
-    x.q = __ldg(reinterpret_cast<const uint4*>(s.q + off));
-    x.g = __ldg(reinterpret_cast<const uint4*>(s.g + off));
+    const uint64_t off = (uint64_t)(uint32_t)min(s.row0 + i, s.last) * s.step;
+    x.k = __ldg(s.k + off);
+    x.q = __ldg(s.q + off);
+    x.g = __ldg(s.g + off);
 }
 __device__ __forceinline__ void prep_load(const TwoPassArgs& a, const PrepSrc& s, int64_t t0, int len, int h, int lane, PrepHead& x) {
-    const __nv_bfloat16* g = a.g + t0 * a.token_stride + (int64_t)h * kD + 4 * lane;
+    const uint2* g = reinterpret_cast<const uint2*>(a.g + t0 * a.token_stride + (int64_t)h * kD + 4 * lane);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x.g7[i] = __ldg(reinterpret_cast<const uint2*>(g + (uint32_t)min(i, s.last) * s.step));
+    for (int i = 0; i < 8; ++i) x.g7[i] = __ldg(g + (uint64_t)(uint32_t)min(i, s.last) * (2 * s.step));
 #pragma unroll
     for (int i = 0; i < 2; ++i) prep_load_row(s, i, x.row[i]);
     const float4* dt = reinterpret_cast<const float4*>(a.dt_bias + (int64_t)h * kD);
@@ -135,17 +136,16 @@ __device__ __forceinline__ f2_t prep_add_gate(f2_t run, uint32_t g, f2_t dt, f2_
     return f2_add(run, f2_pack(__fmul_rn(gs, y0), __fmul_rn(gs, y1)));
 }
 
-// One warp, one unit of `len` tokens (asked for with prep_load): fills the record block.
-__device__ __forceinline__ void prep_compute(const TwoPassArgs& a, const PrepSrc& src, int len, uint8_t* rec_ptr, int lane, PrepHead& x) {
+// One warp, one unit of `len` tokens (asked for with prep_load): fills the record block.  `acquire()` is called before the first
+// write to the block, after work that needs none: it returns whether the block may be written.  `next()` is called when the
+// unit's inputs are used up, before the products: it may load the next unit's head into `x`.
+template <class Acquire, class Next>
+__device__ __forceinline__ bool prep_compute(const TwoPassArgs& a, const PrepSrc& src, int len, uint8_t* rec_ptr, int lane, PrepHead& x,
+                                             Acquire&& acquire, Next&& next) {
     const uint32_t rec = sm100::smem_u32(rec_ptr);
     const int c = lane & 15, hh = lane >> 4;
     const uint32_t b1 = rec + kTcB1 + c * kTcB1Lbo + hh * 128, kip = rec + kTcKr + c * kPrepKiLbo + hh * 128;
     float* beta_act = reinterpret_cast<float*>(rec_ptr + kTcInv);
-    if (lane < kChunk) {   // sigmoid(beta) of row `lane`
-        const float sb = sigmoid_tanh(bf2f(x.beta));
-        beta_act[lane] = sb;
-        reinterpret_cast<__nv_bfloat16*>(rec_ptr + kTcBeta)[lane] = f2bf(sb);
-    }
     const float a_exp_half = __fmul_rn(ex2_approx(__fmul_rn(x.a_log, 1.4426950408889634f)), 0.5f);
     const f2_t ae = f2_pack(a_exp_half, a_exp_half);
     // ---- the gate sum over rows 0-7, from which the lanes of rows 8-15 go on: 4 columns per lane ----
@@ -167,6 +167,12 @@ __device__ __forceinline__ void prep_compute(const TwoPassArgs& a, const PrepSrc
             const float y0 = __shfl_sync(0xffffffffu, s[2 * (p & 1)], 2 * c + (p >> 1)), y1 = __shfl_sync(0xffffffffu, s[2 * (p & 1) + 1], 2 * c + (p >> 1));
             run[p] = f2_pack(hh ? y0 : 0.0f, hh ? y1 : 0.0f);
         }
+    }
+    if (!acquire()) return false;
+    if (lane < kChunk) {   // sigmoid(beta) of row `lane`
+        const float sb = sigmoid_tanh(bf2f(x.beta));
+        beta_act[lane] = sb;
+        reinterpret_cast<__nv_bfloat16*>(rec_ptr + kTcBeta)[lane] = f2bf(sb);
     }
     // ---- rows: kd, qd, ki; one bf16 rounding per element and operation ----
     const f2_t dt[4] = {f2_pack(x.dt0.x, x.dt0.y), f2_pack(x.dt0.z, x.dt0.w), f2_pack(x.dt1.x, x.dt1.y), f2_pack(x.dt1.z, x.dt1.w)};
@@ -231,6 +237,7 @@ __device__ __forceinline__ void prep_compute(const TwoPassArgs& a, const PrepSrc
         }
     }
     __syncwarp();
+    next();
     // ---- L = fp16(kd ki^T) masked * fp16(beta), Mqk = bf16(qd ki^T) masked ----
     Frag16 lfrag;  // L as the A / C fragment the inverse starts from
     {
@@ -285,6 +292,7 @@ __device__ __forceinline__ void prep_compute(const TwoPassArgs& a, const PrepSrc
     }
     neumann_inverse_warp<true>(lfrag, rec_ptr + kTcInv, lane);
     __syncwarp();
+    return true;
 }
 
 }  // namespace fkda

@@ -23,7 +23,7 @@
 // csrc/smxx/fwd_kernel1.cuh / fwd_kernel2.cuh).
 #include "fkda_common.cuh"
 #include "fkda_internal.h"
-#include "fkda_prepare_warp.cuh"
+#include "fkda_prep.cuh"
 
 namespace fkda {
 
@@ -97,9 +97,10 @@ __global__ void __launch_bounds__(128, 3) short_kernel(const __grid_constant__ T
         int len;
         locate(n, &t0, &len);
         if (len > 0) {
-            PrepPrefetch pf;
-            prep_prefetch(a, t0, len, h, lane, pf);
-            prepare_chunk_warp<true, true>(a, t0, len, h, rec, *reinterpret_cast<PrepWarpSmem*>(rec), lane, pf, false, 0, 0, 0);
+            PrepHead x;
+            const PrepSrc src = prep_src(a, t0, len, h, lane);
+            prep_load(a, src, t0, len, h, lane, x);
+            prep_compute(a, src, len, rec, lane, x, [] { return true; }, [] {});
         }
     }
     __syncthreads();   // the four records are complete

@@ -92,7 +92,7 @@ static bool slabs_possible(int64_t chains, int sms) { return chains * kRowSplit 
 // whose lengths the host does not know may consist of a few long chains, whose walk is then the whole time (128 chains of 1
 // to 32 chunks: 52 us in two kernels against 82): it needs two chains per SM.
 static bool fused_eligible(const fkda_fwd_params& p, int sms) {
-    if (p.phase_mask != 0 || p.B * p.T <= kChunk * p.N || p.token_stride >= ((int64_t)1 << 27)) return false;
+    if (p.phase_mask != 0 || p.B * p.T <= kChunk * p.N) return false;
     const int64_t chains = p.N * p.H;
     return (p.cu_seqlens != nullptr ? chains >= 2 * sms : chains * kRowSplit > sms) || (p.flags & FKDA_FLAG_NO_WIDE);
 }
