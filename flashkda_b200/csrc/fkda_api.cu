@@ -95,9 +95,9 @@ int fkda_fwd(const fkda_fwd_params* p, void* stream_v) {
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
     int launches = 0;
     int rc;
-    if (algo == FKDA_ALGO_TC && fkda::decode_eligible(*p) && !(p->flags & FKDA_FLAG_NO_DECODE) && p->chunk_states == nullptr)
+    if (algo == FKDA_ALGO_TC && fkda::decode_eligible(*p))
         rc = fkda::launch_decode(*p, stream, &launches);  // one token per sequence: state read-modify-write
-    else if (algo == FKDA_ALGO_TC && fkda::short_eligible(*p) && !(p->flags & FKDA_FLAG_NO_SHORT))
+    else if (algo == FKDA_ALGO_TC && fkda::short_eligible(*p))
         rc = fkda::launch_short(*p, stream, &launches);   // at most one chunk per sequence: one fused kernel
     else if (algo == FKDA_ALGO_TC)
         rc = fkda::launch_tc(*p, stream, &launches);

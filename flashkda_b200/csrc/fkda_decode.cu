@@ -3,7 +3,8 @@
 // With a single valid row the chunk algebra of the forward collapses (the in-chunk triangular system is
 // the identity, Mqk is one number), and the step is a read-modify-write of the [128,128] state per
 // (sequence, head): it is bound by HBM traffic on the states (2 x 32 KB in bf16, 2 x 64 KB in fp32),
-// not by the tensor cores.  One 128-thread CTA per (sequence, head); warp w owns state rows 32w..32w+31,
+// not by the tensor cores.  For small batches (decode_max_chains): the shortest way from the token to the state, no staging and
+// no hand-overs.  One 128-thread CTA per (sequence, head); warp w owns state rows 32w..32w+31,
 // lane l columns 4l..4l+3 of each, so every state row is read and written once as one coalesced
 // 256-byte (bf16) or 512-byte (fp32) warp access, and stays in registers in between.
 //
@@ -171,10 +172,6 @@ __global__ void __launch_bounds__(128, 3) decode_kernel(const __grid_constant__ 
             *reinterpret_cast<uint2*>(dst) = make_uint2(y0, y1);
         }
     }
-}
-
-bool decode_eligible(const fkda_fwd_params& p) {
-    return p.cu_seqlens == nullptr && p.T == 1 && (p.phase_mask == 0 || p.phase_mask == (FKDA_PHASE_PREPARE | FKDA_PHASE_RECURRENCE));
 }
 
 int launch_decode_ragged(const TwoPassArgs& a, cudaStream_t stream) {

@@ -1,6 +1,7 @@
 // Internal host/device declarations shared by the translation units of the library.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -65,6 +66,11 @@ int device_sm_count();
 void* noalloc_scratch_or_null();
 int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches);
 // Decode step (fixed batch, T == 1): one read-modify-write kernel over the states, no workspace records.
+// (sequence, head) pairs up to which the decode kernel serves it; beyond, the short-sequence kernel, whose state loads never
+// pause.  The line is where the two cross (B200): with bf16 states after two waves of the decode kernel (896 pairs 12.6 us
+// against 15.0, 2 048: 30.9 against 28.8, 32 768: 404 against 340); with fp32 states, where the decode kernel's loads are
+// twice as wide, far up (4 096: 85 against 88, 32 768: 655 against 646).
+inline int64_t decode_max_chains(const fkda_fwd_params& p) { return p.state_dtype == FKDA_STATE_FP32 ? 16384 : 1024; }
 bool decode_eligible(const fkda_fwd_params& p);
 int launch_decode(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches);
 // Short sequences (fixed batch, 2 <= T <= 16): one fused kernel per (sequence, head), no workspace records.
@@ -73,7 +79,10 @@ int launch_short(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches)
 // Ragged batches: whether the call MAY consist of sequences of at most one chunk each (the host knows only the totals;
 // the prefix kernel decides on the device), and the launch of the fused kernel behind that decision.
 bool short_ragged_candidate(const fkda_fwd_params& p);
-int launch_short_ragged(const TwoPassArgs& a, cudaStream_t stream);
+int launch_short_ragged(const fkda_fwd_params& p, const TwoPassArgs& a, cudaStream_t stream);
+// Tensor maps over v and over the states (fkda_tc.cu).
+bool encode_v_map(CUtensorMap* m, const fkda_fwd_params& p);
+bool encode_state_map(CUtensorMap* m, const void* base, int64_t chains, bool fp32);
 int launch_decode_ragged(const TwoPassArgs& a, cudaStream_t stream);   // as many tokens as sequences: maybe one each
 
 // Allows a kernel its dynamic shared memory on the current device.  The attribute belongs to the function and the device,

@@ -139,7 +139,9 @@ __device__ __forceinline__ f2_t prep_add_gate(f2_t run, uint32_t g, f2_t dt, f2_
 // One warp, one unit of `len` tokens (asked for with prep_load): fills the record block.  `acquire()` is called before the first
 // write to the block, after work that needs none: it returns whether the block may be written.  `next()` is called when the
 // unit's inputs are used up, before the products: it may load the next unit's head into `x`.
-template <class Acquire, class Next>
+// kFewRows: units of 8 tokens or fewer are common, their missing rows are skipped (the code for it costs the others 2 %, and
+// the walking warps beside them in fkda_fused.cuh 20 % in registers).
+template <bool kFewRows, class Acquire, class Next>
 __device__ __forceinline__ bool prep_compute(const TwoPassArgs& a, const PrepSrc& src, int len, uint8_t* rec_ptr, int lane, PrepHead& x,
                                              Acquire&& acquire, Next&& next) {
     const uint32_t rec = sm100::smem_u32(rec_ptr);
@@ -177,8 +179,9 @@ __device__ __forceinline__ bool prep_compute(const TwoPassArgs& a, const PrepSrc
     // ---- rows: kd, qd, ki; one bf16 rounding per element and operation ----
     const f2_t dt[4] = {f2_pack(x.dt0.x, x.dt0.y), f2_pack(x.dt0.z, x.dt0.w), f2_pack(x.dt1.x, x.dt1.y), f2_pack(x.dt1.z, x.dt1.w)};
     const uint32_t sc2 = pack_bf2(a.scale, a.scale);
+    const int rows = !kFewRows || len > 8 ? 8 : (len + 1) & ~1;   // rows of each half that are gone through
 #pragma unroll 1
-    for (int ib = 0; ib < 8; ib += 2) {
+    for (int ib = 0; ib < rows; ib += 2) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int i = ib + u;
@@ -216,6 +219,14 @@ __device__ __forceinline__ bool prep_compute(const TwoPassArgs& a, const PrepSrc
             prep_sts(b1 + 16 * i, kd[0], kd[1], kd[2], kd[3]);
             prep_sts(b1 + 256 + 16 * i, qd[0], qd[1], qd[2], qd[3]);   // rows 16..31 = two row groups further
             prep_sts(kip + 16 * i, ki[0], ki[1], ki[2], ki[3]);
+        }
+    }
+    if constexpr (kFewRows) {
+#pragma unroll 1
+        for (int i = rows; i < 8; ++i) {   // the other rows are zeros
+            prep_sts(b1 + 16 * i, 0u, 0u, 0u, 0u);
+            prep_sts(b1 + 256 + 16 * i, 0u, 0u, 0u, 0u);
+            prep_sts(kip + 16 * i, 0u, 0u, 0u, 0u);
         }
     }
     // E_tot = 2^(sum over all rows): known to the lanes of rows 8-15; as bf16 also to the others, for kr

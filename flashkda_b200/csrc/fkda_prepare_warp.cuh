@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32, 1) prepare_warp_kernel(const 
     while (valid) {
         const bool next_valid = locate(u + stride, &tile_n, &t0n, &lenn, &hn);
         uint8_t* ws = a.workspace + ((int64_t)h * a.total_tiles + tile) * (int64_t)(kTc ? kTcRecord : kWsRecord);
-        prep_compute(a, src, len, rec, lane, x,
+        prep_compute<false>(a, src, len, rec, lane, x,
                      [&]() {   // the previous record has left the block
                          if (kTc && lane == 0) sm100::bulk_wait_group_read<0>();
                          __syncwarp();

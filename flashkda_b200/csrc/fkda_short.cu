@@ -1,350 +1,376 @@
-// Short sequences: a fixed batch whose sequences hold 2 .. 16 tokens each, or a ragged batch in which no sequence
-// holds more than 16 (ONE chunk per sequence), the step between a decode step (one token, fkda_decode.cu) and
-// prefill -- e.g. the verification pass of speculative decoding.  Such a batch is bound by HBM traffic on the [128,128] states (read once, written once), so the whole
-// forward of a (sequence, head) chain runs in ONE kernel with nothing staged in HBM: no chunk records, no second
-// launch, no workspace.
+// Short sequences: a fixed batch whose sequences hold 1 .. 16 tokens each, or a ragged batch in which no sequence holds more
+// than 16 (ONE chunk per sequence): a decode step of a large batch, the verification pass of speculative decoding.  Such a
+// batch is bound by HBM traffic on the [128,128] states (read once, written once), so the whole forward of a (sequence, head)
+// chain runs in ONE kernel with nothing staged in HBM and no workspace, and the kernel is built to keep state loads and
+// stores in flight on every SM all the time:
 //
-// One 128-thread CTA per FOUR chains, three CTAs per SM:
-//   * first every warp runs the prepare stage of one of the four chunks (the same warp-per-chunk routine as the
-//     prefill path), record left in shared memory: the prepare stage is a long serial instruction stream, so four
-//     of them run side by side instead of three warps waiting for one;
-//   * after one block barrier the four chains are walked one after the other by all four warps: every warp brings
-//     its 32 state rows into mma.sync A-fragment registers (thread g = lane / 4, tq = lane % 4 of warp w holds rows
-//     32 w + 16 mt + {g, g + 8}, columns 16 j + {2tq, 2tq+1, 2tq+8, 2tq+9} for the row tiles mt = 0, 1 and the K steps
-//     j = 0 .. 7): whole rows from global memory (512 contiguous bytes per warp instruction) into a 4 KB staging tile
-//     per warp, from there with ldmatrix; then it runs the chunk step on mma.sync, state in registers throughout:
-//       D1[V,32] = S . [kd; qd]^T   (8 K steps in order: the reference's accumulation order)
-//       u' = (v (-) bf(u0)) (*) bf(beta),  U = bf(u' INV^T),  out = bf(o0) (+) bf(U Mqk^T)
-//       DST[V,K] = U^T . kr,  S[v,k] = bf(fma(S[v,k], E_tot[k], DST[v,k]))  (accumulator and A fragments of a
-//       16 x 16 block hold the same elements, so the update runs fragment on fragment)
-//     and the refreshed rows leave the same way, fragments into the staging tile, whole rows out.
-// Numerics and results: those of the chunked kernels on the same inputs (tests/torch_ref.py:153-251 of the
-// reference; the reference itself runs such batches through its two general kernels,
-// csrc/smxx/fwd_kernel1.cuh / fwd_kernel2.cuh).
+// One persistent CTA per SM (12 warps), chains blockIdx.x, blockIdx.x + gridDim.x, ...
+//   * two groups of four walking warps; each group owns two 32 KB stages of shared memory.  A stage takes the whole state of a
+//     chain (bf16) or 64 of its rows (fp32: the groups share a chain).  A stage is filled by TMA, its rows go through the
+//     registers of the walking warps (fkda_walk.cuh) and back into the stage in place, and leave by TMA; the group's other
+//     stage is refilled meanwhile, so 64 KB of loads per SM are in flight beside the stores.  128-byte swizzle on both
+//     ways: whole 128-byte lines for global memory, no bank conflicts for fragments;
+//   * four preparing warps build the chunk operands of the coming chains in a ring of records (fkda_prep.cuh), the inputs of
+//     their next chain in registers ahead of time.
+// Everything is handed over through mbarriers with bounded waits.
+// Bound by HBM: 32 768 chains of 2 tokens take 344 us with bf16 and 653 us with fp32 states, 0.98 and 1.02 of the copy bandwidth
+// (554 and 833 us for the predecessor, whose four warps loaded, computed and stored one chain after the other); with 16
+// tokens 472 and 757 us (776, 1 083), where the preparing warps take as long as the states.
+// Numerics and results: those of the chunked kernels on the same inputs (tests/torch_ref.py:153-251 of the reference; the
+// reference itself runs such batches through its two general kernels, csrc/smxx/fwd_kernel1.cuh / fwd_kernel2.cuh).
+#include <cuda.h>
+#include <string.h>
+
 #include "fkda_common.cuh"
 #include "fkda_internal.h"
 #include "fkda_prep.cuh"
+#include "fkda_walk.cuh"
 
 namespace fkda {
 
-// B operand fragments of mma.sync m16n8k16 for n-tile rows r = 8 nt + g of a K-major [rows, K] tile in the record's
-// B1 layout (byte = (k/8)*528 + (r/8)*128 + (r%8)*16 + (k%8)*2): b0 = (k 16j + 2tq, +1), b1 = (k 16j + 8 + 2tq, +1)
-__device__ __forceinline__ void short_b1_frag(const uint8_t* b1, int r, int j, int tq, uint32_t& b0, uint32_t& b1r) {
-    const uint8_t* p = b1 + (2 * j) * kTcB1Lbo + (r >> 3) * 128 + (r & 7) * 16 + tq * 4;
-    b0 = *reinterpret_cast<const uint32_t*>(p);
-    b1r = *reinterpret_cast<const uint32_t*>(p + kTcB1Lbo);
+using namespace sm100;
+
+constexpr int kShortGroups = 2, kShortWalkers = 4 * kShortGroups, kShortPrep = 4;
+constexpr int kShortThreads = (kShortWalkers + kShortPrep) * 32;
+constexpr int kShortSlots = 4;                       // records (and value tiles) in the ring
+constexpr int kShortStage = 32768;                   // state stage: 128 rows of bf16 or 64 rows of fp32
+constexpr int kShortV = kShortGroups * 2 * kShortStage;                   // value tiles: two halves [16][64] bf16 each
+constexpr int kShortVTile = kChunk * kD * 2;
+constexpr int kShortOut = kShortV + kShortSlots * kShortVTile;            // per walking warp up to two out tiles [16][16]
+constexpr int kShortRec = kShortOut + kShortWalkers * 2 * 512;
+constexpr int kShortCtrl = kShortRec + kShortSlots * kTcRecord;
+struct ShortCtrl {
+    uint64_t full[kShortSlots];           // a record is complete and its value tile has landed
+    uint64_t empty[kShortSlots];          // a slot has been read by all walking warps of its chain
+    uint64_t sfull[kShortGroups][2];      // a state stage has landed
+    uint64_t sdone[kShortGroups];         // the walking warps of a group have put their rows back
+    int32_t len[kShortSlots];             // tokens of the slot's chain
+    int32_t abort_flag;
+};
+constexpr int kShortSmemBytes = kShortCtrl + (int)sizeof(ShortCtrl) + 1024;
+static_assert(kShortRec % 16 == 0 && kShortCtrl % 8 == 0 && kShortSmemBytes <= 232448, "shared-memory layout");
+static_assert(kShortPrep <= kShortSlots, "no more preparing warps than slots (see fkda_fused.cuh)");
+
+struct alignas(64) ShortMaps {
+    CUtensorMap v, h0, hT;
+};
+
+// Where the fragments of row tile `row` (first row, inside the stage) and K step j live in a state stage.
+// bf16: two boxes of 64 columns; lane's ldmatrix / stmatrix row.
+__device__ __forceinline__ uint32_t short_bf16_off(int row, int j, int lane) {
+    const int r = row + (lane & 7) + 8 * ((lane >> 3) & 1), piece = 2 * j + (lane >> 4);
+    return (uint32_t)((piece >> 3) * 16384 + r * 128 + (((piece & 7) ^ (lane & 7)) << 4));
 }
-// Four 8x8 b16 matrices, transposed on the way: lane 8m + r gives the address of row r (16 bytes) of matrix m; thread
-// (g, tq) receives elements (rows 2tq, 2tq+1; column g) of each, i.e. mma.sync B fragments of row-major [K, N] tiles.
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row_ptr) {
-    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(row_ptr);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"(addr));
+// fp32: four boxes of 32 columns; my element pair e of the fragment
+__device__ __forceinline__ uint32_t short_fp32_off(int row, int j, int e, int lane) {
+    const int g = lane >> 2, tq = lane & 3, piece = 4 * (j & 1) + 2 * (e >> 1) + (tq >> 1);
+    return (uint32_t)((j >> 1) * 8192 + (row + g + 8 * (e & 1)) * 128 + ((piece ^ g) << 4) + 8 * (tq & 1));
+}
+template <int kMt, bool kFp32>
+__device__ __forceinline__ void short_get(uint32_t (&s)[kMt][8][4], uint32_t stage, int row, int lane) {
+#pragma unroll
+    for (int mt = 0; mt < kMt; ++mt)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if constexpr (kFp32) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 x = lds_f2(stage + short_fp32_off(row + 16 * mt, j, e, lane));
+                    s[mt][j][e] = pack_bf2(x.x, x.y);
+                }
+            } else {
+                ldmatrix_x4_a(s[mt][j][0], s[mt][j][1], s[mt][j][2], s[mt][j][3], stage + short_bf16_off(row + 16 * mt, j, lane));
+            }
+        }
+}
+template <int kMt, bool kFp32>
+__device__ __forceinline__ void short_put(const uint32_t (&s)[kMt][8][4], uint32_t stage, int row, int lane) {
+#pragma unroll
+    for (int mt = 0; mt < kMt; ++mt)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if constexpr (kFp32) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(stage + short_fp32_off(row + 16 * mt, j, e, lane)),
+                                 "f"(bf_lo(s[mt][j][e])), "f"(bf_hi(s[mt][j][e]))
+                                 : "memory");
+            } else {
+                stmatrix_x4(stage + short_bf16_off(row + 16 * mt, j, lane), s[mt][j][0], s[mt][j][1], s[mt][j][2], s[mt][j][3]);
+            }
+        }
 }
 
-constexpr int kShortChainsPerCta = 4;
-// Per warp, a staging tile of 16 state rows as bf16 (256 bytes a row): the states travel between global memory and the
-// fragment registers through it, so that global memory sees whole rows (512 contiguous bytes per warp instruction)
-// instead of 4-byte pieces.  The 16-byte piece c of row r sits at r * 256 + ((c ^ (r & 7)) * 16): rows 8 apart in
-// banks, so the 8-row reads of ldmatrix and the fragment stores do not collide.
-constexpr int kShortStageBytes = 16 * 256;
-constexpr int kShortSmemBytes = kShortChainsPerCta * kTcRecord + 4 * kShortStageBytes + 16;
-__device__ __forceinline__ int short_stage_off(int r, int piece) { return r * 256 + ((piece ^ (r & 7)) << 4); }
-
-__global__ void __launch_bounds__(128, 3) short_kernel(const __grid_constant__ TwoPassArgs a) {
-    extern __shared__ uint8_t short_smem[];
-    uint8_t* recs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(short_smem) + 15) & ~(uintptr_t)15);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, tq = lane & 3;
+template <bool kFp32>
+__global__ void __launch_bounds__(kShortThreads, 1)
+short_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ ShortMaps maps) {
     // a ragged batch that the prefix kernel has given to other kernels (a longer sequence: the general ones; one token
     // each: the decode kernel)
     if (a.short_flag != nullptr && *a.short_flag != 1) return;
+    extern __shared__ uint8_t smem_dyn[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+    ShortCtrl& ctl = *reinterpret_cast<ShortCtrl*>(sm + kShortCtrl);
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    const int lane = threadIdx.x & 31;
+    volatile int* abort_flag = &ctl.abort_flag;
     if (a.short_flag == nullptr && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
-    const int64_t n_chains = a.N * a.H;
-    const int64_t chain0 = (int64_t)blockIdx.x * kShortChainsPerCta;
-    const int row0 = warp * 32 + g;           // my rows: row0 + 16 mt + 8 hi
-    uint8_t* stage = recs + kShortChainsPerCta * kTcRecord + warp * kShortStageBytes;   // my warp's staging tile
-    // The state of the chain that comes next is asked into L2 one chain ahead (the first before the prepare stage), so
-    // that its loads find it there: one chain ahead only, more than that competes with the loads that are needed now.
-    auto prefetch_state = [&](int64_t chain) {
-        if (a.initial_state == nullptr || chain >= n_chains) return;
-        const int64_t bytes = (int64_t)kD * kD * (a.state_fp32 ? 4 : 2);
-        const char* base = reinterpret_cast<const char*>(a.initial_state) + chain * bytes;
-        for (int64_t off = (int64_t)threadIdx.x * 128; off < bytes; off += 128 * 128)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(base + off));
-    };
-    prefetch_state(chain0);
-    // first token and length (0 .. 16 tokens: at most one chunk) of sequence n
-    auto locate = [&](int64_t n, int64_t* t0, int* len) {
-        if (a.cu_seqlens != nullptr) {
-            const int64_t b = a.cu_seqlens[n], e = a.cu_seqlens[n + 1];
-            *t0 = b;
-            *len = e > b ? (int)(e - b) : 0;
-        } else {
-            *t0 = n * a.T;
-            *len = (int)a.T;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kShortSlots; ++s) {
+            mbar_init(&ctl.full[s], 2);
+            mbar_init(&ctl.empty[s], kFp32 ? kShortWalkers : 4);
         }
-    };
-
-    // ---- the operands of the four chunks: warp w runs the prepare stage of chain chain0 + w, record left in
-    //      shared memory (layout of fkda_common.cuh) ----
-    if (chain0 + warp < n_chains) {
-        const int64_t n = (chain0 + warp) / a.H;
-        const int h = (int)(chain0 + warp - n * a.H);
-        uint8_t* rec = recs + warp * kTcRecord;
-        int64_t t0;
-        int len;
-        locate(n, &t0, &len);
-        if (len > 0) {
-            PrepHead x;
-            const PrepSrc src = prep_src(a, t0, len, h, lane);
-            prep_load(a, src, t0, len, h, lane, x);
-            prep_compute(a, src, len, rec, lane, x, [] { return true; }, [] {});
+        for (int g = 0; g < kShortGroups; ++g) {
+            mbar_init(&ctl.sfull[g][0], 1);
+            mbar_init(&ctl.sfull[g][1], 1);
+            mbar_init(&ctl.sdone[g], 4);
         }
+        ctl.abort_flag = 0;
+        mbar_fence_init();
     }
-    __syncthreads();   // the four records are complete
+    __syncthreads();
+    const int64_t n_chains = a.N * a.H;
+    const int n_local = (int)((n_chains - blockIdx.x + gridDim.x - 1) / gridDim.x);   // (the grid is no larger than n_chains)
+    bool failed = false;
 
-#pragma unroll 1
-    for (int ci = 0; ci < kShortChainsPerCta; ++ci) {
-    const int64_t chain = chain0 + ci;
-    if (chain >= n_chains) break;
-    const int64_t n = chain / a.H;
-    const int h = (int)(chain - n * a.H);
-    int64_t t0;
-    int len;
-    locate(n, &t0, &len);
-    const uint8_t* rec = recs + ci * kTcRecord;
-    if (ci + 1 < kShortChainsPerCta) prefetch_state(chain + 1);
-
-    // ---- state rows into A-fragment registers: sreg[mt][j][e], e = {row g: cols 2tq | row g+8 | row g: cols 2tq+8 | row g+8},
-    //      16 rows (one row tile mt) at a time through the warp's staging tile ----
-    uint32_t sreg[2][8][4];
-    const int64_t st_chain = chain * (int64_t)(kD * kD);
-    if (a.initial_state != nullptr) {
-        if (a.state_fp32) {
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                // 16 rows x 512 bytes: piece p = 32 i + lane is 4 floats, row p / 32, columns 4 (p % 32) ..
-                const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.initial_state) + st_chain +
-                                                                    (int64_t)(warp * 32 + 16 * mt) * kD);
-                float4 x[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) x[i] = __ldg(src + 32 * i + lane);
-#pragma unroll
-                for (int i = 0; i < 16; ++i)   // row i, columns 4 lane .. 4 lane + 3: half (lane & 1) of piece lane / 2
-                    *reinterpret_cast<uint2*>(stage + short_stage_off(i, lane >> 1) + 8 * (lane & 1)) =
-                        make_uint2(pack_bf2(x[i].x, x[i].y), pack_bf2(x[i].z, x[i].w));
-                __syncwarp();
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    ldmatrix_x4(sreg[mt][j][0], sreg[mt][j][1], sreg[mt][j][2], sreg[mt][j][3],
-                                stage + short_stage_off((lane & 7) + 8 * ((lane >> 3) & 1), 2 * j + (lane >> 4)));
-                __syncwarp();
+    if (warp >= kShortWalkers) {
+        // =========================== preparing warps ===========================
+        const int p = warp - kShortWalkers;
+        // first token, length (0 .. 16 tokens) and head of local chain i
+        auto locate = [&](int i, int64_t* t0, int* len, int* h) {
+            const int64_t chain = blockIdx.x + (int64_t)i * gridDim.x, n = chain / a.H;
+            *h = (int)(chain - n * a.H);
+            if (a.cu_seqlens != nullptr) {
+                const int64_t b = a.cu_seqlens[n], e = a.cu_seqlens[n + 1];
+                *len = e > b ? (int)(e - b) : 0;
+                *t0 = *len > 0 ? b : 0;   // (an empty sequence: any address inside the tensors)
+            } else {
+                *t0 = n * a.T;
+                *len = (int)a.T;
             }
-        } else {
-            // 32 rows x 256 bytes: piece p = 32 i + lane is 8 bf16, row p / 16, columns 8 (p % 16) ..; both row tiles are
-            // fetched before the first is staged
-            const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.initial_state) + st_chain +
-                                                              (int64_t)(warp * 32) * kD);
-            uint4 x[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) x[i] = __ldg(src + 32 * i + lane);
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i)   // row 2 i + lane / 16 of the tile, piece lane % 16
-                    *reinterpret_cast<uint4*>(stage + short_stage_off(2 * i + (lane >> 4), lane & 15)) = x[8 * mt + i];
+        };
+        PrepHead x;
+        PrepSrc src;
+        int64_t t0 = 0, t0n = 0;
+        int len = 0, h = 0, lenn = 0, hn = 0;
+        if (p < n_local) {
+            locate(p, &t0, &len, &h);
+            src = prep_src(a, t0, max(len, 1), h, lane);
+            prep_load(a, src, t0, max(len, 1), h, lane, x);
+        }
+        for (int i = p; i < n_local; i += kShortPrep) {
+            const int slot = i % kShortSlots;
+            const uint32_t phase = 1u ^ ((i / kShortSlots) & 1);   // of empty[slot]: the first round finds the slots free
+            const bool next_valid = i + kShortPrep < n_local;
+            if (next_valid) locate(i + kShortPrep, &t0n, &lenn, &hn);
+            uint8_t* rec = sm + kShortRec + slot * kTcRecord;
+            auto acquire = [&]() {   // the slot is free: ask for the value tile
+                if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.empty[slot], phase, abort_flag, a.wait_ns)) == 0) return false;
+                if (lane == 0) {
+                    ctl.len[slot] = len;
+                    // (tokens past the sequence end are masked by the walking warps)
+                    mbar_arrive_expect_tx(&ctl.full[slot], kShortVTile);
+                    tma_load_3d(sm + kShortV + slot * kShortVTile, &maps.v, 0, h, (int)t0, &ctl.full[slot]);
+                    tma_load_3d(sm + kShortV + slot * kShortVTile + kShortVTile / 2, &maps.v, kD / 2, h, (int)t0, &ctl.full[slot]);
+                }
                 __syncwarp();
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    ldmatrix_x4(sreg[mt][j][0], sreg[mt][j][1], sreg[mt][j][2], sreg[mt][j][3],
-                                stage + short_stage_off((lane & 7) + 8 * ((lane >> 3) & 1), 2 * j + (lane >> 4)));
-                __syncwarp();
+                return true;
+            };
+            auto next = [&]() {   // the inputs of my next chain travel while the products and the inverse run
+                if (next_valid) {
+                    src = prep_src(a, t0n, max(lenn, 1), hn, lane);
+                    prep_load(a, src, t0n, max(lenn, 1), hn, lane, x);
+                }
+            };
+            if (!prep_compute<true>(a, src, len, rec, lane, x, acquire, next)) {
+                failed = true;
+                *abort_flag = 1;
+                // my value tile in flight lands before this CTA's shared memory goes
+                if (i >= kShortPrep) mbar_wait_bounded(&ctl.full[slot], phase, nullptr, 100000000ull);
+                break;
             }
+            mbar_arrive_lane0(&ctl.full[slot], lane);
+            t0 = t0n; len = lenn; h = hn;
         }
     } else {
+        // =========================== walking warps ===========================
+        constexpr int kMt = kFp32 ? 1 : 2;
+        const int group = warp >> 2, wiw = warp & 3;
+        const bool leader = wiw == 0 && lane == 0;
+        const int row = wiw * 16 * kMt;                                // my first row in a stage
+        const int vrow = (kFp32 ? 64 * group : 0) + row;               // my first state row = value column
+        const int per = kFp32 ? 1 : kShortGroups;                      // my group takes local chains first, first + per, ...
+        const int first = kFp32 ? 0 : group;
+        const int n_items = n_local > first ? (n_local - first + per - 1) / per : 0;
+        const bool has_in = a.initial_state != nullptr, has_out = a.final_state != nullptr;
+        const WalkLane wl = walk_lane(lane);
+        const uint32_t rec0 = smem_u32(sm + kShortRec);
+        uint8_t* const stages = sm + group * 2 * kShortStage;
+        uint32_t v_off[kMt];   // my value columns in a value tile (layout as in fused_kernel)
+        const int v_tok = (lane & 7) + 8 * (lane >> 4);
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) sreg[mt][j][e] = 0u;
-    }
-    // A row tile of the refreshed state leaves through the staging tile: fragments in, whole rows out.
-    auto stage_frag = [&](int j, const uint32_t (&y)[4]) {   // fragment j of the tile: (row g | g+8) x (piece 2j | 2j+1)
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            *reinterpret_cast<uint32_t*>(stage + short_stage_off(g + 8 * (e & 1), 2 * j + (e >> 1)) + 4 * tq) = y[e];
-    };
-    auto flush_tile = [&](int mt) {
-        __syncwarp();
-        if (a.state_fp32) {
-            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.final_state) + st_chain + (int64_t)(warp * 32 + 16 * mt) * kD);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const uint2 y = *reinterpret_cast<const uint2*>(stage + short_stage_off(i, lane >> 1) + 8 * (lane & 1));
-                dst[32 * i + lane] = make_float4(bf_lo(y.x), bf_hi(y.x), bf_lo(y.y), bf_hi(y.y));
+        for (int mt = 0; mt < kMt; ++mt) {
+            const int piece = (vrow + 16 * mt) / 8 + ((lane >> 3) & 1);   // 16-byte piece of a 256-byte value row
+            v_off[mt] = smem_u32(sm + kShortV) + (uint32_t)((piece >> 3) * (kShortVTile / 2) + v_tok * 128 + (((piece & 7) ^ (lane & 7)) << 4));
+        }
+        const uint32_t o_tile = smem_u32(sm + kShortOut + warp * 2 * 512);
+        const uint32_t o_frag = o_tile + (uint32_t)(v_tok * 32 + ((((lane >> 3) & 1) ^ ((v_tok >> 2) & 1)) << 4));
+        const uint32_t o_row = o_tile + (uint32_t)((lane >> 1) * 32 + (((lane & 1) ^ ((lane >> 3) & 1)) << 4));
+        auto chain_of = [&](int k) { return blockIdx.x + (int64_t)(first + k * per) * gridDim.x; };
+        // (leader) item k's rows between global memory and stage k & 1
+        auto state_load = [&](int k) {
+            uint8_t* st = stages + (k & 1) * kShortStage;
+            uint64_t* bar = &ctl.sfull[group][k & 1];
+            const int y = (int)(chain_of(k) * kD) + (kFp32 ? 64 * group : 0);
+            mbar_arrive_expect_tx(bar, kShortStage);
+            if constexpr (kFp32) {
+                for (int b = 0; b < 4; ++b) tma_load_2d(st + 8192 * b, &maps.h0, 32 * b, y, bar);
+            } else {
+                for (int b = 0; b < 2; ++b) tma_load_2d(st + 16384 * b, &maps.h0, 64 * b, y, bar);
             }
-        } else {
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(a.final_state) + st_chain + (int64_t)(warp * 32 + 16 * mt) * kD);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                dst[32 * i + lane] = *reinterpret_cast<const uint4*>(stage + short_stage_off(2 * i + (lane >> 4), lane & 15));
-        }
-        __syncwarp();
-    };
-    if (len == 0) {   // an empty sequence of a ragged batch: its state passes through (rounded to bf16, as everywhere)
-        if (a.final_state != nullptr) {
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) stage_frag(j, sreg[mt][j]);
-                flush_tile(mt);
+        };
+        auto state_store = [&](int k) {
+            const uint8_t* st = stages + (k & 1) * kShortStage;
+            const int y = (int)(chain_of(k) * kD) + (kFp32 ? 64 * group : 0);
+            if constexpr (kFp32) {
+                for (int b = 0; b < 4; ++b) tma_store_2d(&maps.hT, 32 * b, y, st + 8192 * b);
+            } else {
+                for (int b = 0; b < 2; ++b) tma_store_2d(&maps.hT, 64 * b, y, st + 16384 * b);
             }
-        }
-        continue;
-    }
-    // value tile in A-fragment layout (zero past the sequence end), straight from global memory
-    uint32_t vfr[2][4];
-    {
-        const unsigned short* vp = reinterpret_cast<const unsigned short*>(a.v) + t0 * a.token_stride + (int64_t)h * kD;
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int row = row0 + 16 * mt + 8 * (e & 1), tok = 2 * tq + 8 * (e >> 1);
-                const uint32_t lo = tok < len ? vp[(int64_t)tok * a.token_stride + row] : 0u;
-                const uint32_t hi = tok + 1 < len ? vp[(int64_t)(tok + 1) * a.token_stride + row] : 0u;
-                vfr[mt][e] = lo | (hi << 16);
+            bulk_commit_group();
+        };
+        int loads = 0;   // (leader) items whose load has been issued
+        if (leader && has_in)
+            for (; loads < 2 && loads < n_items; ++loads) state_load(loads);
+        WalkState<kMt> w;
+        WalkHead<kMt> hd;
+        auto wait_all = [&](uint64_t* bar, uint32_t ph) { return __all_sync(0xffffffffu, mbar_wait_bounded(bar, ph, abort_flag, a.wait_ns)) != 0; };
+#pragma unroll 1
+        for (int k = 0; k < n_items; ++k) {
+            const int i = first + k * per, slot = i % kShortSlots;
+            const int64_t chain = chain_of(k), n = chain / a.H;
+            const int h = (int)(chain - n * a.H);
+            const uint32_t stage = smem_u32(stages + (k & 1) * kShortStage);
+            if (has_in) {
+                if (!wait_all(&ctl.sfull[group][k & 1], (uint32_t)((k >> 1) & 1))) { failed = true; break; }
+                short_get<kMt, kFp32>(w.s, stage, row, lane);
+            } else {
+                w.clear();
             }
-        }
-    }
-
-    // ---- D1[V,32] = S . [kd; qd]^T: rows 0-15 of B1 are kd (-> u0), rows 16-31 qd (-> o0) ----
-    float d1[2][4][4];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) d1[mt][nt][i] = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            uint32_t b0, b1;
-            short_b1_frag(rec + kTcB1, 8 * nt + g, j, tq, b0, b1);
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
-                mma_bf16_f32acc(d1[mt][nt], sreg[mt][j][0], sreg[mt][j][1], sreg[mt][j][2], sreg[mt][j][3], b0, b1);
-        }
-    }
-    // ---- u' = (v (-) bf(u0)) (*) bf(beta);  U = bf(u' INV^T);  out = bf(o0) (+) bf(U Mqk^T) ----
-    const uint32_t* beta32 = reinterpret_cast<const uint32_t*>(rec + kTcBeta);
-    const uint32_t bp0 = beta32[tq], bp1 = beta32[tq + 4];
-    uint32_t invb[2][2], mqkb[2][2];
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-        invb[nt][0] = *reinterpret_cast<const uint32_t*>(rec + kTcInv + tc_sq_off(8 * nt + g, 2 * tq));
-        invb[nt][1] = *reinterpret_cast<const uint32_t*>(rec + kTcInv + tc_sq_off(8 * nt + g, 2 * tq + 8));
-        mqkb[nt][0] = *reinterpret_cast<const uint32_t*>(rec + kTcMqk + tc_sq_off(8 * nt + g, 2 * tq));
-        mqkb[nt][1] = *reinterpret_cast<const uint32_t*>(rec + kTcMqk + tc_sq_off(8 * nt + g, 2 * tq + 8));
-    }
-    uint32_t ufr[2][4];
-    unsigned short* og = reinterpret_cast<unsigned short*>(a.out) + t0 * a.token_stride + (int64_t)h * kD;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-        uint32_t up[4];   // accumulator tiles nt = 0, 1 of D1 are u0 for tokens 0-7, 8-15: {c0,c1 | c2,c3} = {row g | row g+8}
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const uint32_t u0 = pack_bf2(d1[mt][e >> 1][2 * (e & 1)], d1[mt][e >> 1][2 * (e & 1) + 1]);
-            up[e] = bf2_mul(bf2_sub(vfr[mt][e], u0), (e >> 1) ? bp1 : bp0);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            float c[4] = {0.f, 0.f, 0.f, 0.f};
-            mma_bf16_f32acc(c, up[0], up[1], up[2], up[3], invb[nt][0], invb[nt][1]);
-            ufr[mt][2 * nt] = pack_bf2(c[0], c[1]);
-            ufr[mt][2 * nt + 1] = pack_bf2(c[2], c[3]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            float c[4] = {0.f, 0.f, 0.f, 0.f};
-            mma_bf16_f32acc(c, ufr[mt][0], ufr[mt][1], ufr[mt][2], ufr[mt][3], mqkb[nt][0], mqkb[nt][1]);
-#pragma unroll
-            for (int hi = 0; hi < 2; ++hi) {
-                const uint32_t o = bf2_add(pack_bf2(d1[mt][2 + nt][2 * hi], d1[mt][2 + nt][2 * hi + 1]), pack_bf2(c[2 * hi], c[2 * hi + 1]));
-                const int row = row0 + 16 * mt + 8 * hi, tok = 8 * nt + 2 * tq;
-                if (tok < len) og[(int64_t)tok * a.token_stride + row] = (unsigned short)(o & 0xffffu);
-                if (tok + 1 < len) og[(int64_t)(tok + 1) * a.token_stride + row] = (unsigned short)(o >> 16);
+            if (leader && k > 0) {
+                // the other stage's rows have left (their store was issued an item ago): refill it
+                bulk_wait_group_read<0>();
+                if (has_in && loads < n_items) state_load(loads++);
             }
+            __syncwarp();
+            if (!wait_all(&ctl.full[slot], (uint32_t)((i / kShortSlots) & 1))) { failed = true; break; }
+            const uint32_t rec = rec0 + slot * kTcRecord;
+            const int len = ctl.len[slot];
+            w.first(rec, wl);
+            hd.fetch(rec, wl);
+#pragma unroll
+            for (int mt = 0; mt < kMt; ++mt) ldmatrix_x4_t(hd.v[mt][0], hd.v[mt][1], hd.v[mt][2], hd.v[mt][3], v_off[mt] + slot * kShortVTile);
+            hd.mask(len, lane & 3);
+            const int64_t t0 = a.cu_seqlens != nullptr ? a.cu_seqlens[n] : n * a.T;
+            __nv_bfloat16* og = a.out + (t0 + (lane >> 1)) * a.token_stride + (int64_t)h * kD + vrow + 8 * (lane & 1);
+            uint32_t o[kMt][4];
+            uint4 orow[kMt];
+            w.template chunk<false>(rec, rec, wl, hd, o, [&](int j) {
+                if (j == 3) {   // the out rows: fragments through a 512-byte tile, 32 contiguous bytes per token to global memory
+#pragma unroll
+                    for (int mt = 0; mt < kMt; ++mt) stmatrix_x4_t(o_frag + mt * 512, o[mt][0], o[mt][1], o[mt][2], o[mt][3]);
+                    __syncwarp();
+                }
+                if (j == 4) {
+#pragma unroll
+                    for (int mt = 0; mt < kMt; ++mt) orow[mt] = lds_u4(o_row + mt * 512);
+                }
+                if (j == 6 && (lane >> 1) < len) {
+#pragma unroll
+                    for (int mt = 0; mt < kMt; ++mt) *reinterpret_cast<uint4*>(og + mt * 16) = orow[mt];
+                }
+            });
+            __syncwarp();
+            mbar_arrive_lane0(&ctl.empty[slot], lane);   // (my warp's last reads of this slot are done)
+            if (has_out) {
+                short_put<kMt, kFp32>(w.s, stage, row, lane);
+                fence_proxy_async_smem();
+            }
+            __syncwarp();
+            mbar_arrive_lane0(&ctl.sdone[group], lane);   // my rows are back in the stage
+            if (leader) {
+                if (!mbar_wait_bounded(&ctl.sdone[group], (uint32_t)(k & 1), abort_flag, a.wait_ns)) failed = true;
+                else if (has_out) state_store(k);
+            }
+            failed = __any_sync(0xffffffffu, failed) != 0;
+            if (failed) break;
+        }
+        if (failed) *abort_flag = 1;
+        if (leader) {
+            if (failed && has_in)   // loads in flight land before this CTA's shared memory goes
+                for (int k = max(0, loads - 2); k < loads; ++k)
+                    mbar_wait_bounded(&ctl.sfull[group][k & 1], (uint32_t)((k >> 1) & 1), nullptr, 100000000ull);
+            bulk_wait_group<0>();   // the states are written
         }
     }
-    if (a.final_state == nullptr) continue;
-
-    // ---- DST[V,K] = U^T . kr and S[v,k] = bf(fma(S[v,k], E_tot[k], DST[v,k])), 16 state columns (K step j) at a time;
-    //      the refreshed fragments go straight to the final state ----
-    const float* et = reinterpret_cast<const float*>(rec + kTcEt);
-    // KR tile: kr[token i][column k] at (i/8)*2304 + (k/8)*144 + (i%8)*16 + (k%8)*2: 8x8 blocks with tokens as rows.
-    // ldmatrix lane 8m + r: matrix m = (token group m & 1, column block 2j + (m >> 1)), row r = token
-    const uint8_t* kr_row = rec + kTcKr + ((lane >> 3) & 1) * kTcKrLbo + (lane >> 4) * kTcKrSbo + (lane & 7) * 16;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            uint32_t b00, b01, b10, b11;   // column block 2j: tokens 0-7, 8-15; column block 2j+1: tokens 0-7, 8-15
-            ldmatrix_x4_trans(b00, b01, b10, b11, kr_row + (2 * j) * kTcKrSbo);
-            const float2 e0 = *reinterpret_cast<const float2*>(et + 16 * j + 2 * tq);        // E_tot of columns 16j + 2tq, +1
-            const float2 e1 = *reinterpret_cast<const float2*>(et + 16 * j + 8 + 2 * tq);    // 16j + 8 + 2tq, +1
-            float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-            mma_bf16_f32acc(c0, ufr[mt][0], ufr[mt][1], ufr[mt][2], ufr[mt][3], b00, b01);   // columns 16j + 0..7
-            mma_bf16_f32acc(c1, ufr[mt][0], ufr[mt][1], ufr[mt][2], ufr[mt][3], b10, b11);   // columns 16j + 8..15
-            const uint32_t s0 = sreg[mt][j][0], s1 = sreg[mt][j][1], s2 = sreg[mt][j][2], s3 = sreg[mt][j][3];
-            const uint32_t y[4] = {
-                pack_bf2(__fmaf_rn(bf_lo(s0), e0.x, c0[0]), __fmaf_rn(bf_hi(s0), e0.y, c0[1])),    // row g
-                pack_bf2(__fmaf_rn(bf_lo(s1), e0.x, c0[2]), __fmaf_rn(bf_hi(s1), e0.y, c0[3])),    // row g+8
-                pack_bf2(__fmaf_rn(bf_lo(s2), e1.x, c1[0]), __fmaf_rn(bf_hi(s2), e1.y, c1[1])),
-                pack_bf2(__fmaf_rn(bf_lo(s3), e1.x, c1[2]), __fmaf_rn(bf_hi(s3), e1.y, c1[3]))};
-            stage_frag(j, y);
-        }
-        flush_tile(mt);
+    if (failed) {
+        *abort_flag = 1;
+        if (a.status != nullptr) atomicExch(a.status, FKDA_ERR_DEVICE_STATUS);
     }
-    }   // chains of this CTA
+    __syncthreads();
 }
 
+// ---------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------
+static bool whole_forward(const fkda_fwd_params& p) {
+    return p.phase_mask == 0 || p.phase_mask == (FKDA_PHASE_PREPARE | FKDA_PHASE_RECURRENCE);
+}
+
+// A fixed batch of 2 .. 16 tokens per sequence, or a decode step (one token) with more chains than the decode kernel is for.
 bool short_eligible(const fkda_fwd_params& p) {
-    return p.cu_seqlens == nullptr && p.T >= 2 && p.T <= kChunk && p.chunk_states == nullptr &&
-           (p.phase_mask == 0 || p.phase_mask == (FKDA_PHASE_PREPARE | FKDA_PHASE_RECURRENCE));
+    if (p.cu_seqlens != nullptr || p.T < 1 || p.T > kChunk || p.chunk_states != nullptr || !whole_forward(p)) return false;
+    if (p.flags & FKDA_FLAG_NO_SHORT) return false;
+    return p.T > 1 || (p.N * p.H > decode_max_chains(p) && !(p.flags & FKDA_FLAG_NO_DECODE));
+}
+// A decode step of a fixed batch for the decode kernel.
+bool decode_eligible(const fkda_fwd_params& p) {
+    return p.cu_seqlens == nullptr && p.T == 1 && p.chunk_states == nullptr && whole_forward(p) && !(p.flags & FKDA_FLAG_NO_DECODE) &&
+           (p.N * p.H <= decode_max_chains(p) || (p.flags & FKDA_FLAG_NO_SHORT));
 }
 
 bool short_ragged_candidate(const fkda_fwd_params& p) {
     // tokens <= 16 per sequence on average is necessary for "no sequence longer than a chunk"; a handful of chains is
     // not worth two extra launches
-    return p.cu_seqlens != nullptr && p.N > 0 && p.B * p.T <= kChunk * p.N && p.N * p.H >= 64 &&
-           p.chunk_states == nullptr && (p.phase_mask == 0 || p.phase_mask == (FKDA_PHASE_PREPARE | FKDA_PHASE_RECURRENCE));
+    return p.cu_seqlens != nullptr && p.N > 0 && p.T > 0 && p.B * p.T <= kChunk * p.N && p.N * p.H >= 64 &&
+           p.chunk_states == nullptr && whole_forward(p);
 }
 
-int launch_short_ragged(const TwoPassArgs& a, cudaStream_t stream) {
-    const int64_t chains = a.N * a.H;
-    if (chains > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
-    if (!allow_smem<short_kernel>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
-    const int64_t ctas = (chains + kShortChainsPerCta - 1) / kShortChainsPerCta;
-    short_kernel<<<(unsigned)ctas, 128, kShortSmemBytes, stream>>>(a);
+template <bool kFp32>
+static int launch_short_typed(const fkda_fwd_params& p, const TwoPassArgs& a, int sms, cudaStream_t stream) {
+    const int64_t chains = p.N * p.H;
+    ShortMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    if (!encode_v_map(&maps.v, p)) return FKDA_ERR_LAUNCH;
+    if (p.initial_state != nullptr && !encode_state_map(&maps.h0, p.initial_state, chains, kFp32)) return FKDA_ERR_LAUNCH;
+    if (p.final_state != nullptr && !encode_state_map(&maps.hT, p.final_state, chains, kFp32)) return FKDA_ERR_LAUNCH;
+    if (!allow_smem<short_kernel<kFp32>>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
+    short_kernel<kFp32><<<(unsigned)(chains < sms ? chains : sms), kShortThreads, kShortSmemBytes, stream>>>(a, maps);
     return cudaGetLastError() == cudaSuccess ? FKDA_OK : FKDA_ERR_LAUNCH;
+}
+
+int launch_short_ragged(const fkda_fwd_params& p, const TwoPassArgs& a, cudaStream_t stream) {
+    // (state rows are counted in 32 bits: half a terabyte of states)
+    if (p.N * p.H > 0xffffff && (p.initial_state != nullptr || p.final_state != nullptr)) return FKDA_ERR_BAD_SHAPE;
+    const int sms = device_sm_count();
+    return a.state_fp32 ? launch_short_typed<true>(p, a, sms, stream) : launch_short_typed<false>(p, a, sms, stream);
 }
 
 int launch_short(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     TwoPassArgs a;
     fill_args(p, &a);
-    const int64_t chains = p.N * p.H;
-    if (chains > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
-    if (!allow_smem<short_kernel>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
-    const int64_t ctas = (chains + kShortChainsPerCta - 1) / kShortChainsPerCta;
-    short_kernel<<<(unsigned)ctas, 128, kShortSmemBytes, stream>>>(a);
-    if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
-    *n_launches = 1;
-    return FKDA_OK;
+    const int rc = launch_short_ragged(p, a, stream);
+    if (rc == FKDA_OK) *n_launches = 1;
+    return rc;
 }
 
 }  // namespace fkda

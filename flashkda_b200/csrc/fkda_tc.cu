@@ -126,8 +126,7 @@ size_t tc_workspace_bytes(int64_t T_total, int64_t H, int64_t N) {
 
 // What one particular call needs.
 size_t tc_workspace_bytes_for(const fkda_fwd_params& p) {
-    if (decode_eligible(p) && !(p.flags & FKDA_FLAG_NO_DECODE) && p.chunk_states == nullptr) return 0;   // one kernel, nothing staged
-    if (short_eligible(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) return 0;
+    if (decode_eligible(p) || short_eligible(p)) return 0;   // one kernel, nothing staged
     const int sms = device_sm_count();
     if (fused_eligible(p, sms)) return fused_bytes(p.N, sms);
     const TcCarve c = tc_carve(p, sms);
@@ -175,17 +174,29 @@ static EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// Map over v viewed as [token][head][128] bf16 with tiles of 16 tokens x 64 columns of one head; the 16-byte pieces of a tile
-// row are permuted by the row (128-byte swizzle), so that transposing reads of the tile (8 rows of one piece) do not collide.
-static bool encode_v_map(CUtensorMap* m, const fkda_fwd_params& p) {
+static bool encode_map(CUtensorMap* m, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims,
+                       const cuuint64_t* strides, const cuuint32_t* box) {
     EncodeTiledFn encode = encode_tiled_fn();
     if (encode == nullptr) return false;
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    return encode(m, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// Map over v viewed as [token][head][128] bf16 with tiles of 16 tokens x 64 columns of one head; the 16-byte pieces of a tile
+// row are permuted by the row (128-byte swizzle), so that transposing reads of the tile (8 rows of one piece) do not collide.
+bool encode_v_map(CUtensorMap* m, const fkda_fwd_params& p) {
     const cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)p.H, (cuuint64_t)(p.B * p.T)};
     const cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)p.token_stride * 2};  // bytes, dims 1 and 2
     const cuuint32_t box[3] = {(cuuint32_t)kD / 2, 1u, (cuuint32_t)kChunk};
-    const cuuint32_t estr[3] = {1u, 1u, 1u};
-    return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p.v), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, p.v, dims, strides, box);
+}
+// Map over states viewed as [chains * 128 rows][128 columns], in tiles 128 bytes wide: 128 rows of 64 bf16 or 64 rows of 32
+// fp32 columns (16 or 8 KB), swizzled as above.
+bool encode_state_map(CUtensorMap* m, const void* base, int64_t chains, bool fp32) {
+    const cuuint64_t dims[2] = {(cuuint64_t)kD, (cuuint64_t)(chains * kD)};
+    const cuuint64_t strides[1] = {(cuuint64_t)kD * (fp32 ? 4 : 2)};
+    const cuuint32_t box[2] = {fp32 ? 32u : 64u, fp32 ? 64u : 128u};
+    return encode_map(m, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box);
 }
 static_assert(kRowCols == kD / 2, "a CTA of the row-slice kernel takes one half of a value row");
 
@@ -306,7 +317,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     }
 
     // as many tokens as sequences: they may have one token each, the decode kernel's case
-    const bool try_decode = a.short_flag != nullptr && T_total == p.N && !(p.flags & FKDA_FLAG_NO_DECODE);
+    const bool try_decode = a.short_flag != nullptr && T_total == p.N && chains <= decode_max_chains(p) && !(p.flags & FKDA_FLAG_NO_DECODE);
     if (varlen && do_prep) {
         launch_tile_prefix(a, const_cast<int32_t*>(a.seq_order), try_decode, stream);
         ++launches;
@@ -316,7 +327,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         ++launches;
     }
     if (a.short_flag != nullptr) {
-        if (launch_short_ragged(a, stream) != FKDA_OK) return FKDA_ERR_LAUNCH;
+        if (launch_short_ragged(p, a, stream) != FKDA_OK) return FKDA_ERR_LAUNCH;
         ++launches;
     }
     if (a.total_tiles > 0 && do_prep) {

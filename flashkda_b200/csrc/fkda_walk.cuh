@@ -165,9 +165,10 @@ struct WalkState {
     }
     // One chunk, record at shared-memory address `rec`, operands of its head in `hd`; D1 of the chunk at `next` is formed on
     // the way (`next` = `rec` when there is none: it is then not used).  `mid(j)` is called after block j of the update:
-    // the caller fetches the next head and finishes the out rows there, in the shadow of the products.
+    // the caller fetches the next head and finishes the out rows there, in the shadow of the products.  kNext = false: this is
+    // the only chunk.
     // o[mt] = out of tokens 8 (i >> 1) + 2tq, +1 of row g + 8 (i & 1), i = 0 .. 3, complete after block 2.
-    template <class Mid>
+    template <bool kNext = true, class Mid>
     __device__ __forceinline__ void chunk(uint32_t rec, uint32_t next, const WalkLane& wl, const WalkHead<kMt>& hd, uint32_t (&o)[kMt][4], Mid&& mid) {
         constexpr int kAhead = 2;   // blocks whose operands (kr, E_tot, [kd; qd]) are fetched ahead of their products
         uint32_t kr[8][4], b[8][8];
@@ -179,7 +180,7 @@ struct WalkState {
         };
 #pragma unroll
         for (int j = 0; j < kAhead; ++j) fetch_kr(j);
-        fetch_d1(b[0], next, wl, 0);
+        if constexpr (kNext) fetch_d1(b[0], next, wl, 0);
         // ---- u' = (v (-) bf(u0)) (*) bf(beta);  U = bf(u' INV^T) as A fragments (tokens are the K dimension) ----
         uint32_t up[kMt][4], ufr[kMt][4];
 #pragma unroll
@@ -220,7 +221,7 @@ struct WalkState {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (j + kAhead < 8) fetch_kr(j + kAhead);
-            if (j + 1 < 8) fetch_d1(b[j + 1], next, wl, j + 1);
+            if (kNext && j + 1 < 8) fetch_d1(b[j + 1], next, wl, j + 1);
             if (j == 0) {   // the out term U Mqk^T
 #pragma unroll
                 for (int mt = 0; mt < kMt; ++mt) {
@@ -235,9 +236,9 @@ struct WalkState {
                 s[mt][j][2] = update_pair(s[mt][j][2], et[j][1], d[j][mt][1][0], d[j][mt][1][1]);
                 s[mt][j][3] = update_pair(s[mt][j][3], et[j][1], d[j][mt][1][2], d[j][mt][1][3]);
             }
-            d1_half(u0, b[j], j);
+            if constexpr (kNext) d1_half(u0, b[j], j);
             if (j + 2 < 8) dst(j + 2);
-            if (j > 0) d1_half(o0, b[j - 1] + 4, j - 1);
+            if (kNext && j > 0) d1_half(o0, b[j - 1] + 4, j - 1);
             if (j == 2) {   // out = bf(o0) (+) bf(U Mqk^T)
 #pragma unroll
                 for (int mt = 0; mt < kMt; ++mt)
@@ -247,7 +248,7 @@ struct WalkState {
             }
             mid(j);
         }
-        d1_half(o0, b[7] + 4, 7);
+        if constexpr (kNext) d1_half(o0, b[7] + 4, 7);
     }
 };
 

@@ -1,0 +1,63 @@
+"""The one-chunk kernel (sequences of 1 .. 16 tokens, persistent CTAs that stream states through shared memory) against the general
+kernels, bit for bit: chain counts around its grid, its two groups and its ring, both state types, missing states, a final
+state written over the initial one, and decode steps on both sides of the dispatch line."""
+import pytest
+import torch
+
+import flashkda_b200
+from flashkda_b200 import _lib
+from flashkda_b200.synth import Workload, make_inputs, to_device
+
+pytestmark = pytest.mark.gpu
+GENERAL = _lib.FLAG_NO_DECODE | _lib.FLAG_NO_SHORT
+
+
+def _call(d, flags=0, h0="initial_state"):
+    out = torch.zeros_like(d["out"])
+    h_in = None if d["initial_state"] is None else d["initial_state"].clone()
+    hT = h_in if h0 == "in place" else (None if d["final_state"] is None else torch.zeros_like(d["final_state"]))
+    flashkda_b200.fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], d["scale"], out, d["A_log"], d["dt_bias"], d["lower_bound"],
+                      h_in, hT, d["cu_seqlens"], flags=flags)
+    return out, hT
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 2, 1), (147, 9, 1), (149, 8, 1), (74, 7, 4), (297, 16, 3), (150, 1, 9)])
+@pytest.mark.parametrize("state_in,state_out", [("bf16", "bf16"), ("fp32", "fp32"), (None, "bf16"), ("fp32", None), (None, None)])
+def test_fixed_batches_equal_the_general_kernels(B, T, H, state_in, state_out):
+    d = to_device(make_inputs(Workload("oc", B, T, H, state_in=state_in, state_out=state_out, lower_bound=-2.0), seed=B + T), "cuda")
+    got = _call(d)
+    assert flashkda_b200.last_launch_count() == 1
+    ref = _call(d, GENERAL)
+    assert flashkda_b200.last_launch_count() >= 1
+    exact = T > 1 or "fp32" not in (state_in, state_out)   # (a decode step of so few fp32 states: the decode kernel)
+    for x, y in zip(got, ref):
+        if x is not None:
+            assert torch.equal(x, y) if exact else torch.allclose(x.float(), y.float(), atol=2e-2)
+
+
+@pytest.mark.parametrize("state", ["bf16", "fp32"])
+def test_final_state_over_the_initial_state(state):
+    d = to_device(make_inputs(Workload("ip", 160, 5, 4, state_in=state, state_out=state, lower_bound=-2.0), seed=3), "cuda")
+    ref, got = _call(d), _call(d, h0="in place")
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("chains", [1024, 1025])
+def test_decode_steps_on_both_sides_of_the_dispatch_line(chains):
+    d = to_device(make_inputs(Workload("dl", chains, 1, 1, state_in="bf16", state_out="bf16", lower_bound=-2.0), seed=5), "cuda")
+    got = _call(d)
+    assert flashkda_b200.last_launch_count() == 1
+    ref = _call(d, GENERAL)
+    if chains > 1024:   # (the decode kernel sums its dot products in another order)
+        assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+    assert torch.allclose(got[0].float(), ref[0].float(), atol=2e-2) and torch.allclose(got[1].float(), ref[1].float(), atol=2e-2)
+
+
+@pytest.mark.parametrize("state", ["bf16", "fp32"])
+def test_ragged_with_empty_sequences_over_several_rounds(state):
+    g = torch.Generator().manual_seed(2)
+    lens = torch.randint(0, 17, (333,), generator=g).tolist()
+    lens[0] = lens[-1] = 0
+    d = to_device(make_inputs(Workload("re", 1, sum(lens), 4, state_in=state, state_out=state, lower_bound=-2.0, seq_lens=lens), seed=6), "cuda")
+    got, ref = _call(d), _call(d, GENERAL)
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
