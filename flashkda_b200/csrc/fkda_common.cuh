@@ -54,6 +54,13 @@ __host__ __device__ constexpr int tc_sq_off(int i, int j) {
     return (j >> 3) * 256 + (i >> 3) * 128 + (i & 7) * 16 + (j & 7) * 2;
 }
 
+// ---- programmatic dependent launch: a kernel launched with launch_dependent (fkda_internal.h) may start before the kernel in
+//      front of it has ended; grid_dep_wait() returns when that one is complete and its writes are visible (at once in a
+//      kernel launched otherwise), so every such kernel calls it before anything else.  Each kernel of a call waits for
+//      the one before it, so the one before that is complete as well. ----
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- approximate transcendentals: the instructions are part of the contract ----
 __device__ __forceinline__ float ex2_approx(float x) {
     float r;

@@ -157,9 +157,10 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
             mbar_init(&ctl.empty[s], kFusedWalkers);
         }
         ctl.abort_flag = 0;
-        ctl.range = atomicAdd(a.queue, 1);
         mbar_fence_init();
     }
+    grid_dep_wait();
+    if (threadIdx.x == 0) ctl.range = atomicAdd(a.queue, 1);
     __syncthreads();
     const int range = ctl.range;
     const FusedRange r = fused_range(a, range);

@@ -99,12 +99,29 @@ inline bool allow_smem(int bytes) {
     return true;
 }
 
+// Launches a kernel that begins with grid_dep_wait() (fkda_common.cuh) behind the previous kernel of the same call: its launch
+// and start overlap that kernel's end.
+template <typename... KernelArgs, typename... Args>
+inline bool launch_dependent(void (*kernel)(KernelArgs...), int64_t ctas, int threads, int smem, cudaStream_t stream, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+}
+
 // Fills the kernel arguments common to both implementations (pointers, strides, gate scale,
 // workspace carving).
 void fill_args(const fkda_fwd_params& p, TwoPassArgs* a);
 // The prefix kernel of a ragged batch: chunk (and state-export) prefix tables, the length order if asked for, and the path
-// decision if a.short_flag is set.
-void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream);
+// decision if a.short_flag is set; clears the header and `n_flags` range flags.
+void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags = 0);
 // First state-export slot of sequence n.
 __device__ __forceinline__ int64_t cs_first_slot(const TwoPassArgs& a, int64_t n) {
     if (a.cu_seqlens != nullptr) return a.cs_prefix[n];

@@ -61,6 +61,10 @@ __device__ __forceinline__ void prep_export_plain(uint8_t* ws, const uint8_t* re
 
 template <bool kTc>
 __global__ void __launch_bounds__(kPrepWarps * 32, 1) prepare_warp_kernel(const __grid_constant__ TwoPassArgs a) {
+    // (no early grid_dep_launch(): the recurrence's CTAs would fill the first SMs that fall free two by two)
+    grid_dep_wait();
+    // the first launch of a fixed batch's forward clears the device status (the prefix kernel that of a ragged batch)
+    if (a.cu_seqlens == nullptr && a.slab_c0 == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
     // (a ragged batch that the fused short-sequence kernel has served: nothing to do)
     if (a.short_flag != nullptr && *a.short_flag != 0) return;
     extern __shared__ uint8_t prep_smem[];
@@ -127,9 +131,10 @@ __global__ void __launch_bounds__(kPrepWarps * 32, 1) prepare_warp_kernel(const 
     sm100::bulk_wait_group<0>();  // (lane 0) the last records have landed
 }
 
-// max_ctas > 0 caps the grid (a launch that shares the GPU with a concurrent recurrence kernel)
+// max_ctas > 0 caps the grid (a launch that shares the GPU with a concurrent recurrence kernel); dependent: behind another
+// kernel of the same call
 template <bool kTc>
-inline int launch_prepare_warp(const TwoPassArgs& a, cudaStream_t stream, int max_ctas = 0) {
+inline int launch_prepare_warp(const TwoPassArgs& a, cudaStream_t stream, int max_ctas = 0, bool dependent = false) {
     if (!allow_smem<prepare_warp_kernel<kTc>>(kPrepSmemBytes)) return FKDA_ERR_LAUNCH;
     const int sms = device_sm_count();
     const int64_t n_units = (a.slab_chunks > 0 ? a.N * (int64_t)a.slab_chunks : a.total_tiles) * a.H;
@@ -140,6 +145,7 @@ inline int launch_prepare_warp(const TwoPassArgs& a, cudaStream_t stream, int ma
     int64_t ctas = (n_units + warps - 1) / warps;
     if (ctas > max_grid) ctas = max_grid;
     if (ctas < 1) ctas = 1;
+    if (dependent) return launch_dependent(prepare_warp_kernel<kTc>, ctas, warps * 32, warps * kTcRecord + 128, stream, a) ? FKDA_OK : FKDA_ERR_LAUNCH;
     prepare_warp_kernel<kTc><<<(unsigned)ctas, warps * 32, warps * kTcRecord + 128, stream>>>(a);
     return FKDA_OK;
 }

@@ -39,8 +39,6 @@ static_assert(kRowCols == 64 && kRowVBytes % 1024 == 0 && kRowOut % 256 == 0 && 
 template <bool kExport, bool kLoop>
 __global__ void __launch_bounds__(kRowThreads, 2)
 recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap map) {
-    // (a ragged batch that a one-kernel path has served: nothing to do)
-    if (a.short_flag != nullptr && *a.short_flag != 0) return;
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     RowCtrl& ctl = *reinterpret_cast<RowCtrl*>(sm + kRowCtrl);
@@ -55,6 +53,9 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         ctl.abort_flag = 0;
         mbar_fence_init();
     }
+    grid_dep_wait();
+    // (a ragged batch that a one-kernel path has served: nothing to do)
+    if (a.short_flag != nullptr && *a.short_flag != 0) return;
     __syncthreads();
 
     const int64_t n_items = a.N * a.H * kRowSplit;

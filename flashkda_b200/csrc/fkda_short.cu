@@ -104,6 +104,7 @@ __device__ __forceinline__ void short_put(const uint32_t (&s)[kMt][8][4], uint32
 template <bool kFp32>
 __global__ void __launch_bounds__(kShortThreads, 1)
 short_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ ShortMaps maps) {
+    grid_dep_wait();
     // a ragged batch that the prefix kernel has given to other kernels (a longer sequence: the general ones; one token
     // each: the decode kernel)
     if (a.short_flag != nullptr && *a.short_flag != 1) return;
@@ -354,7 +355,10 @@ static int launch_short_typed(const fkda_fwd_params& p, const TwoPassArgs& a, in
     if (p.initial_state != nullptr && !encode_state_map(&maps.h0, p.initial_state, chains, kFp32)) return FKDA_ERR_LAUNCH;
     if (p.final_state != nullptr && !encode_state_map(&maps.hT, p.final_state, chains, kFp32)) return FKDA_ERR_LAUNCH;
     if (!allow_smem<short_kernel<kFp32>>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
-    short_kernel<kFp32><<<(unsigned)(chains < sms ? chains : sms), kShortThreads, kShortSmemBytes, stream>>>(a, maps);
+    const int64_t ctas = chains < sms ? chains : sms;
+    if (a.short_flag != nullptr)   // behind the prefix kernel
+        return launch_dependent(short_kernel<kFp32>, ctas, kShortThreads, kShortSmemBytes, stream, a, maps) ? FKDA_OK : FKDA_ERR_LAUNCH;
+    short_kernel<kFp32><<<(unsigned)ctas, kShortThreads, kShortSmemBytes, stream>>>(a, maps);
     return cudaGetLastError() == cudaSuccess ? FKDA_OK : FKDA_ERR_LAUNCH;
 }
 

@@ -203,21 +203,30 @@ static_assert(kRowCols == kD / 2, "a CTA of the row-slice kernel takes one half 
 // One kernel (and the prefix kernel of a ragged batch).
 static int launch_fused(const fkda_fwd_params& p, TwoPassArgs& a, int sms, cudaStream_t stream, int* n_launches) {
     const int64_t chains = p.N * p.H;
-    uint8_t* flags = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes + ws_prefix_bytes(p.N);
+    // the flags directly behind the header for a fixed batch (it has no prefix tables): one stretch to clear; the prefix
+    // kernel clears both for a ragged batch
+    uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes;
+    uint8_t* flags = base + (p.cu_seqlens != nullptr ? ws_prefix_bytes(p.N) : 0);
     a.range_flags = reinterpret_cast<int32_t*>(flags);
-    a.seg_state = reinterpret_cast<uint32_t*>(flags + fused_flag_bytes(sms));
-    if (cudaMemsetAsync(p.workspace, 0, 64, stream) != cudaSuccess || cudaMemsetAsync(flags, 0, fused_flag_bytes(sms), stream) != cudaSuccess)
-        return FKDA_ERR_LAUNCH;
+    a.seg_state = reinterpret_cast<uint32_t*>(base + ws_prefix_bytes(p.N) + fused_flag_bytes(sms));
     int launches = 0;
     if (p.cu_seqlens != nullptr) {
-        launch_tile_prefix(a, nullptr, false, stream);
+        launch_tile_prefix(a, nullptr, false, stream, sms);
         ++launches;
+    } else if (cudaMemsetAsync(p.workspace, 0, kWsHeaderBytes + (size_t)sms * 4, stream) != cudaSuccess) {
+        return FKDA_ERR_LAUNCH;
     }
     VMap map;
     if (!encode_v_map(&map.v, p)) return FKDA_ERR_LAUNCH;
     const bool exports = a.chunk_states != nullptr;
     if (!(exports ? allow_smem<fused_kernel<true>>(kFusedSmemBytes) : allow_smem<fused_kernel<false>>(kFusedSmemBytes))) return FKDA_ERR_LAUNCH;
-    (exports ? fused_kernel<true> : fused_kernel<false>)<<<(unsigned)(chains < sms ? chains : sms), kFusedThreads, kFusedSmemBytes, stream>>>(a, map);
+    const auto kernel = exports ? fused_kernel<true> : fused_kernel<false>;
+    const int64_t ctas = chains < sms ? chains : sms;
+    if (p.cu_seqlens != nullptr) {
+        if (!launch_dependent(kernel, ctas, kFusedThreads, kFusedSmemBytes, stream, a, map)) return FKDA_ERR_LAUNCH;
+    } else {
+        kernel<<<(unsigned)ctas, kFusedThreads, kFusedSmemBytes, stream>>>(a, map);
+    }
     ++launches;
     if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
     *n_launches = launches;
@@ -237,7 +246,8 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     const int64_t T_total = p.B * p.T, chains = p.N * p.H;
     if (fused_eligible(p, sms)) return launch_fused(p, a, sms, stream, n_launches);
     if (chains * kRowSplit > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
-    if (cudaMemsetAsync(p.workspace, 0, 64, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;  // header: status, decisions
+    // (the header is cleared by the first kernel where there is one: the prefix kernel, or the prepare stage of a fixed batch)
+    if (!(do_prep && (varlen || a.total_tiles > 0)) && cudaMemsetAsync(p.workspace, 0, 64, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;
     const TcCarve carve = tc_carve(p, sms);
     uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes + ws_prefix_bytes(p.N);
     a.seg_state = reinterpret_cast<uint32_t*>(base);
@@ -331,14 +341,18 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         ++launches;
     }
     if (a.total_tiles > 0 && do_prep) {
-        if (launch_prepare_warp<true>(a, stream) != FKDA_OK) return FKDA_ERR_LAUNCH;
+        if (launch_prepare_warp<true>(a, stream, 0, varlen) != FKDA_OK) return FKDA_ERR_LAUNCH;
         ++launches;
     }
     if (do_rec) {
         // (behind a device-side decision this launch mostly returns at once: a grid that is resident in one go)
         int64_t ctas = chains * kRowSplit;
         if (a.short_flag != nullptr && ctas > 2 * sms) ctas = 2 * sms;
-        rows_kernel<<<(unsigned)ctas, kRowThreads, kRowSmemBytes, stream>>>(a, map);
+        if (launches > 0) {
+            if (!launch_dependent(rows_kernel, ctas, kRowThreads, kRowSmemBytes, stream, a, map)) return FKDA_ERR_LAUNCH;
+        } else {
+            rows_kernel<<<(unsigned)ctas, kRowThreads, kRowSmemBytes, stream>>>(a, map);
+        }
         ++launches;
     }
     if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;

@@ -22,9 +22,13 @@ namespace fkda {
 __global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __restrict__ cu, int64_t N,
                                                            int32_t* __restrict__ prefix, int32_t* __restrict__ order,
                                                            int32_t* __restrict__ cs_prefix, int cs_tokens,
-                                                           int32_t* __restrict__ short_flag, int decode_enqueued) {
+                                                           int32_t* __restrict__ short_flag, int decode_enqueued,
+                                                           int32_t* __restrict__ header, int32_t* __restrict__ flags, int n_flags) {
+    grid_dep_launch();
     __shared__ int64_t part[1024];
     const int tid = threadIdx.x;
+    if (tid < 8) header[tid] = 0;   // ticket counter, device status
+    for (int i = tid; i < n_flags; i += 1024) flags[i] = 0;
     const int64_t per = (N + 1023) / 1024;
     const int64_t lo = tid * per, hi = (lo + per < N) ? lo + per : N;
     // exclusive prefix over the sequences of ceil(len / unit): chunks (unit 16), or state-export groups
@@ -237,10 +241,10 @@ __global__ void __launch_bounds__(128) recurrence_kernel(TwoPassArgs a) {
 // ---------------------------------------------------------------------------------
 // host launcher
 // ---------------------------------------------------------------------------------
-void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream) {
+void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags) {
     tile_prefix_kernel<<<1, 1024, 0, stream>>>(a.cu_seqlens, a.N, a.tile_prefix, seq_order,
                                                a.chunk_states != nullptr ? const_cast<int32_t*>(a.cs_prefix) : nullptr, 16 * a.cs_every,
-                                               a.short_flag, decode_enqueued ? 1 : 0);
+                                               a.short_flag, decode_enqueued ? 1 : 0, a.queue, a.range_flags, n_flags);
 }
 
 size_t twopass_workspace_bytes(int64_t T_total, int64_t H, int64_t N) {
