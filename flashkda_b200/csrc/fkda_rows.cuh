@@ -17,31 +17,38 @@ namespace fkda {
 constexpr int kRowWarps = 4;                      // walking warps per CTA, 16 state rows each
 constexpr int kRowSplit = kD / (16 * kRowWarps);  // CTAs per chain
 constexpr int kRowCols = 16 * kRowWarps;          // value columns (= state rows) of a CTA
-constexpr int kRowStages = 4;
 constexpr int kRowThreads = (kRowWarps + 1) * 32;
 constexpr int kRowVBytes = kChunk * kRowCols * 2;              // value tile [16 tokens][64] bf16, 128-byte swizzle
-constexpr int kRowV = 0;                                       // (1024-byte aligned for the swizzle)
-constexpr int kRowOut = kRowV + kRowStages * kRowVBytes;       // per warp an out tile [16 tokens][16] bf16
-constexpr int kRowRec = kRowOut + kRowWarps * 512;             // chunk records
-constexpr int kRowStaging = kRowRec + kRowStages * kTcRecord;  // per warp one staging tile for states
-constexpr int kRowCtrl = kRowStaging + kRowWarps * kWalkStageBytes;
-struct RowCtrl {
-    uint64_t full[kRowStages];    // operands of a chunk have landed (transaction bytes)
-    uint64_t empty[kRowStages];   // a stage has been read by all walking warps
-    int32_t abort_flag;
+static_assert(kRowCols == 64 && kRowVBytes % 1024 == 0, "tile alignments");
+
+// Shared memory of a CTA with kStages chunks in flight
+template <int kStages>
+struct RowSmem {
+    static constexpr int kV = 0;                                        // value tiles (1024-byte aligned for the swizzle)
+    static constexpr int kOut = kV + kStages * kRowVBytes;              // per warp an out tile [16 tokens][16] bf16
+    static constexpr int kRec = kOut + kRowWarps * 512;                 // chunk records
+    static constexpr int kStaging = kRec + kStages * kTcRecord;         // per warp one staging tile for states
+    static constexpr int kCtrl = kStaging + kRowWarps * kWalkStageBytes;
+    struct Ctrl {
+        uint64_t full[kStages];    // operands of a chunk have landed (transaction bytes)
+        uint64_t empty[kStages];   // a stage has been read by all walking warps
+        int32_t abort_flag;
+    };
+    static constexpr int kBytes = kCtrl + (int)sizeof(Ctrl) + 1024;
+    static_assert(kOut % 256 == 0 && kRec % 16 == 0 && kStaging % 16 == 0 && kCtrl % 8 == 0, "tile alignments");
 };
-constexpr int kRowSmemBytes = kRowCtrl + (int)sizeof(RowCtrl) + 1024;
-static_assert(kRowCols == 64 && kRowVBytes % 1024 == 0 && kRowOut % 256 == 0 && kRowRec % 16 == 0 && kRowStaging % 16 == 0 && kRowCtrl % 8 == 0,
-              "tile alignments");
 
 // kExport: the states before every cs_every-th chunk are written out as well.  kLoop: a CTA takes several slices in turn
-// (for launches that mostly return at once, see launch_tc; the loop alone makes a step 15 % longer).
-template <bool kExport, bool kLoop>
+// (for launches that mostly return at once, see launch_tc; the loop alone makes a step 15 % longer).  kRowStages: 8 when every
+// slice has an SM of its own (with the prepare stage of the next slab loading the memory, records arrive up to four steps
+// late: 131 072 tokens, 32 heads: 4.58 -> 4.31 ms against 4 stages), otherwise 4, so that two CTAs fit an SM.
+template <bool kExport, bool kLoop, int kRowStages>
 __global__ void __launch_bounds__(kRowThreads, 2)
 recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap map) {
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-    RowCtrl& ctl = *reinterpret_cast<RowCtrl*>(sm + kRowCtrl);
+    using L = RowSmem<kRowStages>;
+    typename L::Ctrl& ctl = *reinterpret_cast<typename L::Ctrl*>(sm + L::kCtrl);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &ctl.abort_flag;
@@ -80,9 +87,9 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
                     break;
                 }
                 mbar_arrive_expect_tx(&ctl.full[s], (uint32_t)(kTcRecord + kRowVBytes));
-                bulk_g2s(sm + kRowRec + s * kTcRecord, ch.rec_base + (int64_t)t * kTcRecord, kTcRecord, &ctl.full[s]);
+                bulk_g2s(sm + L::kRec + s * kTcRecord, ch.rec_base + (int64_t)t * kTcRecord, kTcRecord, &ctl.full[s]);
                 // rows past the end of the tensor arrive as zeros; rows of the next sequence are never used
-                tma_load_3d(sm + kRowV + s * kRowVBytes, &map.v, slice * kRowCols, h, (int)(ch.bos + (int64_t)t * kChunk), &ctl.full[s]);
+                tma_load_3d(sm + L::kV + s * kRowVBytes, &map.v, slice * kRowCols, h, (int)(ch.bos + (int64_t)t * kChunk), &ctl.full[s]);
             }
             if (failed) {   // the copies in flight land before this CTA's shared memory goes
                 *abort_flag = 1;
@@ -95,14 +102,14 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         // =========================== walking warps ===========================
         const int row0 = slice * kRowCols + warp * 16;   // my first state row
         const WalkLane wl = walk_lane(lane);
-        uint8_t* stage_tile = sm + kRowStaging + warp * kWalkStageBytes;
-        const uint32_t rec0 = smem_u32(sm + kRowRec);
+        uint8_t* stage_tile = sm + L::kStaging + warp * kWalkStageBytes;
+        const uint32_t rec0 = smem_u32(sm + L::kRec);
         // my value columns in the [16 tokens][64] tile: token (lane & 7) + 8 (lane / 16), 16-byte piece 2 warp + (lane / 8) % 2
-        const uint32_t v_off = smem_u32(sm + kRowV) + (uint32_t)(((lane & 7) + 8 * (lane >> 4)) * 128 + (((2 * warp + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+        const uint32_t v_off = smem_u32(sm + L::kV) + (uint32_t)(((lane & 7) + 8 * (lane >> 4)) * 128 + (((2 * warp + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
         // out tile of my warp, [16 tokens][16] with the two 16-byte pieces of a token swapped in every other group of four:
         // fragments in (token (lane & 7) + 8 (lane / 16), piece (lane / 8) % 2), rows out (token lane / 2, piece lane % 2)
         const int o_tok = (lane & 7) + 8 * (lane >> 4);
-        const uint32_t o_tile = smem_u32(sm + kRowOut + warp * 512);
+        const uint32_t o_tile = smem_u32(sm + L::kOut + warp * 512);
         const uint32_t o_frag = o_tile + (uint32_t)(o_tok * 32 + ((((lane >> 3) & 1) ^ ((o_tok >> 2) & 1)) << 4));
         const uint32_t o_row = o_tile + (uint32_t)((lane >> 1) * 32 + (((lane & 1) ^ ((lane >> 3) & 1)) << 4));
         const int64_t o_step = kChunk * a.token_stride;

@@ -259,16 +259,19 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     // A ragged batch whose sequences MAY all fit one chunk (the host sees only the totals): the prefix kernel decides, the
     // one-chunk kernels and the general kernels are all enqueued and all but one return at once.
     if (short_ragged_candidate(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) a.short_flag = a.queue + 8;
-    auto rows_kernel = recurrence_rows_kernel<false, false>;
+    // every slice has an SM of its own (and the launch is not one that mostly returns at once)
+    const bool roomy = a.short_flag == nullptr && chains * kRowSplit <= sms;
+    const int rows_smem = roomy ? RowSmem<8>::kBytes : RowSmem<4>::kBytes;
+    auto rows_kernel = recurrence_rows_kernel<false, true, 4>;
     bool smem_ok = true;
     if (a.short_flag != nullptr) {   // (such a batch exports no states)
-        rows_kernel = recurrence_rows_kernel<false, true>;
-        smem_ok = allow_smem<recurrence_rows_kernel<false, true>>(kRowSmemBytes);
+        smem_ok = allow_smem<recurrence_rows_kernel<false, true, 4>>(rows_smem);
     } else if (a.chunk_states != nullptr) {
-        rows_kernel = recurrence_rows_kernel<true, false>;
-        smem_ok = allow_smem<recurrence_rows_kernel<true, false>>(kRowSmemBytes);
+        rows_kernel = roomy ? recurrence_rows_kernel<true, false, 8> : recurrence_rows_kernel<true, false, 4>;
+        smem_ok = roomy ? allow_smem<recurrence_rows_kernel<true, false, 8>>(rows_smem) : allow_smem<recurrence_rows_kernel<true, false, 4>>(rows_smem);
     } else {
-        smem_ok = allow_smem<recurrence_rows_kernel<false, false>>(kRowSmemBytes);
+        rows_kernel = roomy ? recurrence_rows_kernel<false, false, 8> : recurrence_rows_kernel<false, false, 4>;
+        smem_ok = roomy ? allow_smem<recurrence_rows_kernel<false, false, 8>>(rows_smem) : allow_smem<recurrence_rows_kernel<false, false, 4>>(rows_smem);
     }
     if (!smem_ok) return FKDA_ERR_LAUNCH;
 
@@ -283,12 +286,18 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         if (ss == nullptr) return FKDA_ERR_LAUNCH;
         // host threads that call concurrently on one device share the side stream and its events
         std::lock_guard<std::mutex> enqueue_lock(ss->launch_mu);
-        // Slab boundaries.  The prepare of slab i+1 (on idle_sms SMs, about 5.2 ns per (chunk, head) on the whole GPU) must
-        // be done when the recurrence (about 0.52 us per chunk) has walked slab i, and the prepare of the first slab is
-        // not hidden at all: the slabs grow by the ratio of the two speeds, at most by 2 (equal when prepare is slower).
-        const int n_slabs = tps >= 256 ? kMaxSlabs : 2;
-        const double x = (double)chains * (double)sms / ((double)idle_sms * 100.0);
-        const double grow = x >= 1.0 ? 1.0 : (x <= 0.5 ? 2.0 : 1.0 / x);
+        // Slab boundaries.  The prepare of slab i+1 (on idle_sms SMs, about 5.8 ns per (chunk, head) on the whole GPU) must
+        // be done when the recurrence (about 0.52 us per chunk) has walked slab i: the slabs grow (or shrink) by the ratio
+        // of the two speeds (the factor 1.1 measured: 0.9 .. 1.4 tried).  Two or four slabs: more of them leave less of the prepare stage in front of the first one,
+        // unhidden, and cost a hand-over of the states and a launch each, about 5 us.
+        const double prep_us = 0.0058 * (double)(chains * tps), walk_us = 0.52 * (double)tps;
+        const double fit = 1.1 * walk_us * (double)idle_sms / (prep_us * (double)sms);
+        const double grow = fit < 0.6 ? 0.6 : (fit > 8.0 ? 8.0 : fit);
+        int n_slabs = 2;
+        if (tps >= 256) {
+            const double first2 = prep_us / (1.0 + grow), first4 = prep_us / (1.0 + grow + grow * grow + grow * grow * grow);
+            if (first2 > (first4 > 6.0 ? first4 : 6.0) + 10.0) n_slabs = kMaxSlabs;
+        }
         int bounds[kMaxSlabs + 1];
         double total = 0.0, part = 1.0, run = 0.0;
         for (int i = 0; i < n_slabs; ++i, part *= grow) total += part;
@@ -318,7 +327,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         for (int i = 0; i < n_slabs; ++i) {
             if (bounds[i + 1] <= bounds[i]) continue;
             if (i > 0 && cudaStreamWaitEvent(stream, ss->done[i], 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
-            rows_kernel<<<(unsigned)(chains * kRowSplit), kRowThreads, kRowSmemBytes, stream>>>(slab_args(i), map);
+            rows_kernel<<<(unsigned)(chains * kRowSplit), kRowThreads, rows_smem, stream>>>(slab_args(i), map);
             ++launches;
         }
         if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
@@ -349,9 +358,9 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         int64_t ctas = chains * kRowSplit;
         if (a.short_flag != nullptr && ctas > 2 * sms) ctas = 2 * sms;
         if (launches > 0) {
-            if (!launch_dependent(rows_kernel, ctas, kRowThreads, kRowSmemBytes, stream, a, map)) return FKDA_ERR_LAUNCH;
+            if (!launch_dependent(rows_kernel, ctas, kRowThreads, rows_smem, stream, a, map)) return FKDA_ERR_LAUNCH;
         } else {
-            rows_kernel<<<(unsigned)ctas, kRowThreads, kRowSmemBytes, stream>>>(a, map);
+            rows_kernel<<<(unsigned)ctas, kRowThreads, rows_smem, stream>>>(a, map);
         }
         ++launches;
     }

@@ -25,8 +25,8 @@ __global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __rest
                                                            int32_t* __restrict__ short_flag, int decode_enqueued,
                                                            int32_t* __restrict__ header, int32_t* __restrict__ flags, int n_flags) {
     grid_dep_launch();
-    __shared__ int64_t part[1024];
-    const int tid = threadIdx.x;
+    __shared__ int64_t part[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < 8) header[tid] = 0;   // ticket counter, device status
     for (int i = tid; i < n_flags; i += 1024) flags[i] = 0;
     const int64_t per = (N + 1023) / 1024;
@@ -39,23 +39,33 @@ __global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __rest
             if (len < 0) len = 0;
             s += (len + unit - 1) / unit;
         }
-        __syncthreads();
-        part[tid] = s;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {
-            int64_t add = (tid >= off) ? part[tid - off] : 0;
-            __syncthreads();
-            part[tid] += add;
-            __syncthreads();
+        int64_t inc = s;   // inclusive over my warp, then over the warps
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int64_t x = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += x;
         }
-        int64_t run = (tid == 0) ? 0 : part[tid - 1];
+        __syncthreads();
+        if (lane == 31) part[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            int64_t w = part[lane];
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int64_t x = __shfl_up_sync(0xffffffffu, w, off);
+                if (lane >= off) w += x;
+            }
+            part[lane] = w;
+        }
+        __syncthreads();
+        int64_t run = inc - s + (warp > 0 ? part[warp - 1] : 0);
         for (int64_t n = lo; n < hi; ++n) {
             out[n] = (int32_t)run;
             int64_t len = cu[n + 1] - cu[n];
             if (len < 0) len = 0;
             run += (len + unit - 1) / unit;
         }
-        if (tid == 1023) out[N] = (int32_t)part[1023];
+        if (tid == 1023) out[N] = (int32_t)part[31];
     };
     scan(kChunk, prefix);
     if (cs_prefix != nullptr) scan(cs_tokens, cs_prefix);
@@ -70,15 +80,15 @@ __global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __rest
         not_one = __syncthreads_or(not_one);
         if (tid == 0) *short_flag = longer ? 0 : ((decode_enqueued && !not_one) ? 2 : 1);
     }
-    if (order != nullptr) {
-        for (int64_t n = tid; n < N; n += 1024) {
-            const int64_t len_n = cu[n + 1] - cu[n];
+    if (order != nullptr) {   // (N <= kSeqOrderMaxN)
+        __shared__ int32_t chunks[kSeqOrderMaxN];
+        for (int n = tid; n < (int)N; n += 1024) chunks[n] = (int32_t)((cu[n + 1] - cu[n] + kChunk - 1) / kChunk);
+        __syncthreads();
+        for (int n = tid; n < (int)N; n += 1024) {
+            const int32_t mine = chunks[n];
             int rank = 0;
-            for (int64_t m = 0; m < N; ++m) {
-                const int64_t len_m = cu[m + 1] - cu[m];
-                rank += (len_m > len_n || (len_m == len_n && m < n)) ? 1 : 0;
-            }
-            order[rank] = (int32_t)n;
+            for (int m = 0; m < (int)N; ++m) rank += (chunks[m] > mine || (chunks[m] == mine && m < n)) ? 1 : 0;
+            order[rank] = n;
         }
     }
 }
