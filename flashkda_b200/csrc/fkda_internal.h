@@ -67,10 +67,10 @@ void* noalloc_scratch_or_null();
 int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches);
 // Decode step (fixed batch, T == 1): one read-modify-write kernel over the states, no workspace records.
 // (sequence, head) pairs up to which the decode kernel serves it; beyond, the short-sequence kernel, whose state loads never
-// pause.  The line is where the two cross (B200): with bf16 states after two waves of the decode kernel (896 pairs 12.6 us
-// against 15.0, 2 048: 30.9 against 28.8, 32 768: 404 against 340); with fp32 states, where the decode kernel's loads are
-// twice as wide, far up (4 096: 85 against 88, 32 768: 655 against 646).
-inline int64_t decode_max_chains(const fkda_fwd_params& p) { return p.state_dtype == FKDA_STATE_FP32 ? 16384 : 1024; }
+// pause.  The line is where the two cross with bf16 states (2 048 pairs: 30.8 us both, 1 024: 14.4 against 16.8, 32 768: 435
+// against 373); with fp32 states, where the decode kernel's loads are twice as wide, it is the faster one throughout
+// (32 768 pairs: 631 against 671).
+inline int64_t decode_max_chains(const fkda_fwd_params& p) { return p.state_dtype == FKDA_STATE_FP32 ? 0x7fffffff / 4 : 2048; }
 bool decode_eligible(const fkda_fwd_params& p);
 int launch_decode(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches);
 // Short sequences (fixed batch, 2 <= T <= 16): one fused kernel per (sequence, head), no workspace records.
