@@ -35,6 +35,7 @@ struct TwoPassArgs {
     int32_t slab_c0, slab_chunks;  // fixed batches only: this launch covers chunks [slab_c0, slab_c0 + slab_chunks) of
                                    // every sequence (slab_chunks == 0: all chunks); a chain's state travels from one
                                    // slab to the next through seg_state
+    int32_t layer;         // row slices by decreasing length: CTAs of the first layer (one per SM), 0 = no particular order
     int64_t T, H, N, total_tiles;
     int64_t token_stride, beta_token_stride;
     float scale, gate_scale;

@@ -39,8 +39,9 @@ __device__ __forceinline__ bool locate_tile(const TwoPassArgs& a, int64_t tile, 
     return true;
 }
 
-constexpr int kPrepWarps = 12;   // 168 registers each; 15 record blocks would fit the shared memory: spills, 14 % slower
-constexpr int kPrepSmemBytes = kPrepWarps * kTcRecord + 128;
+// Warps per CTA: 12 with 168 registers each; 15, as many as have room for a record block, with 128 and spills, 14 % slower
+// per unit, where that makes one round of units out of two (2 176 units: 23 -> 19 us with the prefix kernel).
+constexpr int kPrepWarps = 12, kPrepWarpsMost = 15;
 
 // The plain record of the CUDA-core recurrence (kWs* layout): kd, qd, kr row-major, INV and Mqk row-major.
 __device__ __forceinline__ void prep_export_plain(uint8_t* ws, const uint8_t* rec_ptr, int lane) {
@@ -59,8 +60,8 @@ __device__ __forceinline__ void prep_export_plain(uint8_t* ws, const uint8_t* re
     *reinterpret_cast<uint4*>(ws + kWsMqk + (i * kChunk + j) * 2) = prep_lds(rec + kTcMqk + tc_sq_off(i, j));
 }
 
-template <bool kTc>
-__global__ void __launch_bounds__(kPrepWarps * 32, 1) prepare_warp_kernel(const __grid_constant__ TwoPassArgs a) {
+template <bool kTc, int kMaxWarps>
+__global__ void __launch_bounds__(kMaxWarps * 32, 1) prepare_warp_kernel(const __grid_constant__ TwoPassArgs a) {
     // (no early grid_dep_launch(): the recurrence's CTAs would fill the first SMs that fall free two by two)
     grid_dep_wait();
     // the first launch of a fixed batch's forward clears the device status (the prefix kernel that of a ragged batch)
@@ -135,18 +136,23 @@ __global__ void __launch_bounds__(kPrepWarps * 32, 1) prepare_warp_kernel(const 
 // kernel of the same call
 template <bool kTc>
 inline int launch_prepare_warp(const TwoPassArgs& a, cudaStream_t stream, int max_ctas = 0, bool dependent = false) {
-    if (!allow_smem<prepare_warp_kernel<kTc>>(kPrepSmemBytes)) return FKDA_ERR_LAUNCH;
     const int sms = device_sm_count();
     const int64_t n_units = (a.slab_chunks > 0 ? a.N * (int64_t)a.slab_chunks : a.total_tiles) * a.H;
     // few units: spread over all SMs, with as many warps per CTA as that takes
     const int64_t max_grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
     const int64_t per = (n_units + max_grid - 1) / max_grid;
-    const int warps = (int)(per < 1 ? 1 : (per < kPrepWarps ? per : kPrepWarps));
+    const bool most = per > kPrepWarps && per <= kPrepWarpsMost;   // one round instead of two
+    const int max_warps = most ? kPrepWarpsMost : kPrepWarps;
+    if (!(most ? allow_smem<prepare_warp_kernel<kTc, kPrepWarpsMost>>(kPrepWarpsMost * kTcRecord + 128)
+               : allow_smem<prepare_warp_kernel<kTc, kPrepWarps>>(kPrepWarps * kTcRecord + 128)))
+        return FKDA_ERR_LAUNCH;
+    const auto kernel = most ? prepare_warp_kernel<kTc, kPrepWarpsMost> : prepare_warp_kernel<kTc, kPrepWarps>;
+    const int warps = (int)(per < 1 ? 1 : (per < max_warps ? per : max_warps));
     int64_t ctas = (n_units + warps - 1) / warps;
     if (ctas > max_grid) ctas = max_grid;
     if (ctas < 1) ctas = 1;
-    if (dependent) return launch_dependent(prepare_warp_kernel<kTc>, ctas, warps * 32, warps * kTcRecord + 128, stream, a) ? FKDA_OK : FKDA_ERR_LAUNCH;
-    prepare_warp_kernel<kTc><<<(unsigned)ctas, warps * 32, warps * kTcRecord + 128, stream>>>(a);
+    if (dependent) return launch_dependent(kernel, ctas, warps * 32, warps * kTcRecord + 128, stream, a) ? FKDA_OK : FKDA_ERR_LAUNCH;
+    kernel<<<(unsigned)ctas, warps * 32, warps * kTcRecord + 128, stream>>>(a);
     return FKDA_OK;
 }
 

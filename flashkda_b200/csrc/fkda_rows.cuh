@@ -69,8 +69,11 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
     bool failed = false;
     int k0 = 0;   // chunks of the items before: the stages and their phases run on from item to item
     for (int64_t item = blockIdx.x; item < n_items && !failed; item = kLoop ? item + gridDim.x : n_items) {
-    const int64_t chain = item / kRowSplit;
-    const int slice = (int)(item % kRowSplit);
+    // chains come longest first; the second layer of CTAs runs backwards, so that the SMs with the longest chains get the
+    // shortest ones beside them (or none)
+    const int64_t place = !kLoop && a.layer > 0 && item >= a.layer ? n_items - 1 - (item - a.layer) : item;
+    const int64_t chain = place / kRowSplit;
+    const int slice = (int)(place % kRowSplit);
     const TcChain ch = tc_locate_chain(a, chain);
     const int h = ch.h;
     // chunk range of this launch: all chunks, or one slab of a pipelined forward (fixed batches)

@@ -356,6 +356,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     if (do_rec) {
         // (behind a device-side decision this launch mostly returns at once: a grid that is resident in one go)
         int64_t ctas = chains * kRowSplit;
+        if (a.seq_order != nullptr && ctas > sms && ctas <= 2 * sms) a.layer = sms;
         if (a.short_flag != nullptr && ctas > 2 * sms) ctas = 2 * sms;
         if (launches > 0) {
             if (!launch_dependent(rows_kernel, ctas, kRowThreads, rows_smem, stream, a, map)) return FKDA_ERR_LAUNCH;
