@@ -126,7 +126,6 @@ template <int kMt>
 struct WalkState {
     uint32_t s[kMt][8][4];     // my state rows, A fragments
     float u0[kMt][2][4];       // S . kd^T of the current chunk, token tiles 0 and 1
-    float o0[kMt][2][4];       // S . qd^T
 
     __device__ __forceinline__ void clear() {
 #pragma unroll
@@ -136,12 +135,14 @@ struct WalkState {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) s[mt][j][e] = 0u;
     }
-    // K step j of D1: kd fragments b[0..3], qd fragments b[4..7]
-    __device__ __forceinline__ void fetch_d1(uint32_t (&b)[8], uint32_t rec, const WalkLane& wl, int j) {
+    // B fragments of K step j of D1: kd (the token tiles 0 and 1)
+    __device__ __forceinline__ void fetch_kd(uint32_t (&b)[4], uint32_t rec, const WalkLane& wl, int j) {
         ldmatrix_x4_a(b[0], b[1], b[2], b[3], rec + wl.b1 + 2 * j * kTcB1Lbo);
-        ldmatrix_x4_a(b[4], b[5], b[6], b[7], rec + wl.b1 + 2 * j * kTcB1Lbo + 256);
     }
-    __device__ __forceinline__ void d1_half(float (&acc)[kMt][2][4], const uint32_t* b, int j) {
+    __device__ __forceinline__ void fetch_qd(uint32_t (&b)[4], uint32_t rec, const WalkLane& wl, int j) {
+        ldmatrix_x4_a(b[0], b[1], b[2], b[3], rec + wl.b1 + 2 * j * kTcB1Lbo + 256);
+    }
+    __device__ __forceinline__ void d1_step(float (&acc)[kMt][2][4], const uint32_t (&b)[4], int j) {
 #pragma unroll
         for (int mt = 0; mt < kMt; ++mt) {
             if (j == 0) {
@@ -153,34 +154,38 @@ struct WalkState {
             }
         }
     }
-    // D1 of the first chunk of a walk
+    // S . kd^T of the first chunk of a walk
     __device__ __forceinline__ void first(uint32_t rec, const WalkLane& wl) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            uint32_t b[8];
-            fetch_d1(b, rec, wl, j);
-            d1_half(u0, b, j);
-            d1_half(o0, b + 4, j);
+            uint32_t b[4];
+            fetch_kd(b, rec, wl, j);
+            d1_step(u0, b, j);
         }
     }
-    // One chunk, record at shared-memory address `rec`, operands of its head in `hd`; D1 of the chunk at `next` is formed on
-    // the way (`next` = `rec` when there is none: it is then not used).  `mid(j)` is called after block j of the update:
+    // One chunk, record at shared-memory address `rec`, operands of its head in `hd`; S . kd^T of the chunk at `next` is formed
+    // on the way (`next` = `rec` when there is none: it is then not used).  `mid(j)` is called after block j of the update:
     // the caller fetches the next head and finishes the out rows there, in the shadow of the products.  kNext = false: this is
     // the only chunk.
+    // The chain of a chunk is u' -> U -> DST -> update -> the next u0; at its start the tensor pipe would be idle, so that is
+    // where most of the out term's S . qd^T goes, which only has to read each 16 columns of the state before they are updated
+    // (all of D1 inside the update: 0.515 us per chunk step of recurrence_rows_kernel).
     // o[mt] = out of tokens 8 (i >> 1) + 2tq, +1 of row g + 8 (i & 1), i = 0 .. 3, complete after block 2.
     template <bool kNext = true, class Mid>
     __device__ __forceinline__ void chunk(uint32_t rec, uint32_t next, const WalkLane& wl, const WalkHead<kMt>& hd, uint32_t (&o)[kMt][4], Mid&& mid) {
-        constexpr int kAhead = 2;   // blocks whose operands (kr, E_tot, [kd; qd]) are fetched ahead of their products
-        uint32_t kr[8][4], b[8][8];
+        constexpr int kAhead = 2;   // blocks whose operands (kr, E_tot, kd) are fetched ahead of their products
+        uint32_t kr[8][4], b[8][4], q[8][4];
         float2 et[8][2];
+        float o0[kMt][2][4];   // S . qd^T
         auto fetch_kr = [&](int j) {
             ldmatrix_x4_t(kr[j][0], kr[j][1], kr[j][2], kr[j][3], rec + wl.kr + 2 * j * kTcKrSbo);
             et[j][0] = lds_f2(rec + wl.et + 64 * j);
             et[j][1] = lds_f2(rec + wl.et + 64 * j + 32);
         };
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j) fetch_kr(j);
-        if constexpr (kNext) fetch_d1(b[0], next, wl, 0);
+        for (int j = 0; j < 4; ++j) fetch_qd(q[j], rec, wl, j);
+        d1_step(o0, q[0], 0);
+        d1_step(o0, q[1], 1);
         // ---- u' = (v (-) bf(u0)) (*) bf(beta);  U = bf(u' INV^T) as A fragments (tokens are the K dimension) ----
         uint32_t up[kMt][4], ufr[kMt][4];
 #pragma unroll
@@ -190,19 +195,24 @@ struct WalkState {
                 const uint32_t x = pack_bf2(u0[mt][e >> 1][2 * (e & 1)], u0[mt][e >> 1][2 * (e & 1) + 1]);
                 up[mt][e] = bf2_mul(bf2_sub(hd.v[mt][e], x), hd.bp[e >> 1]);
             }
-        {
-            float c[kMt][2][4];
+        float c[kMt][2][4];
 #pragma unroll
-            for (int mt = 0; mt < kMt; ++mt) {
-                mma_zero(c[mt][0], up[mt], hd.inv[0], hd.inv[1]);
-                mma_zero(c[mt][1], up[mt], hd.inv[2], hd.inv[3]);
-            }
-#pragma unroll
-            for (int mt = 0; mt < kMt; ++mt)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) ufr[mt][i] = pack_bf2(c[mt][i >> 1][2 * (i & 1)], c[mt][i >> 1][2 * (i & 1) + 1]);
+        for (int mt = 0; mt < kMt; ++mt) {
+            mma_zero(c[mt][0], up[mt], hd.inv[0], hd.inv[1]);
+            mma_zero(c[mt][1], up[mt], hd.inv[2], hd.inv[3]);
         }
-        // ---- blocks of 16 state columns: DST = U^T . kr two blocks ahead, the update, K step j of the next D1 ----
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) fetch_kr(j);
+        if constexpr (kNext) fetch_kd(b[0], next, wl, 0);
+        fetch_qd(q[4], rec, wl, 4);
+        fetch_qd(q[5], rec, wl, 5);
+        d1_step(o0, q[2], 2);
+        d1_step(o0, q[3], 3);
+#pragma unroll
+        for (int mt = 0; mt < kMt; ++mt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ufr[mt][i] = pack_bf2(c[mt][i >> 1][2 * (i & 1)], c[mt][i >> 1][2 * (i & 1) + 1]);
+        // ---- blocks of 16 state columns: DST = U^T . kr two blocks ahead, the update, K step j of the next S . kd^T ----
         float d[8][kMt][2][4], m[kMt][2][4];
         auto dst = [&](int j) {
 #pragma unroll
@@ -213,21 +223,15 @@ struct WalkState {
         };
         dst(0);
         dst(1);
-        uint32_t o0p[kMt][4];
-#pragma unroll
-        for (int mt = 0; mt < kMt; ++mt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) o0p[mt][i] = pack_bf2(o0[mt][i >> 1][2 * (i & 1)], o0[mt][i >> 1][2 * (i & 1) + 1]);
+        d1_step(o0, q[4], 4);
+        d1_step(o0, q[5], 5);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (j + kAhead < 8) fetch_kr(j + kAhead);
-            if (kNext && j + 1 < 8) fetch_d1(b[j + 1], next, wl, j + 1);
-            if (j == 0) {   // the out term U Mqk^T
-#pragma unroll
-                for (int mt = 0; mt < kMt; ++mt) {
-                    mma_zero(m[mt][0], ufr[mt], hd.mqk[0], hd.mqk[1]);
-                    mma_zero(m[mt][1], ufr[mt], hd.mqk[2], hd.mqk[3]);
-                }
+            if (kNext && j + 1 < 8) fetch_kd(b[j + 1], next, wl, j + 1);
+            if (j == 0) {
+                fetch_qd(q[6], rec, wl, 6);
+                fetch_qd(q[7], rec, wl, 7);
             }
 #pragma unroll
             for (int mt = 0; mt < kMt; ++mt) {
@@ -236,19 +240,29 @@ struct WalkState {
                 s[mt][j][2] = update_pair(s[mt][j][2], et[j][1], d[j][mt][1][0], d[j][mt][1][1]);
                 s[mt][j][3] = update_pair(s[mt][j][3], et[j][1], d[j][mt][1][2], d[j][mt][1][3]);
             }
-            if constexpr (kNext) d1_half(u0, b[j], j);
+            if constexpr (kNext) d1_step(u0, b[j], j);
             if (j + 2 < 8) dst(j + 2);
-            if (kNext && j > 0) d1_half(o0, b[j - 1] + 4, j - 1);
+            if (j == 0) {
+                d1_step(o0, q[6], 6);
+                d1_step(o0, q[7], 7);
+            }
+            if (j == 1) {   // the out term U Mqk^T
+#pragma unroll
+                for (int mt = 0; mt < kMt; ++mt) {
+                    mma_zero(m[mt][0], ufr[mt], hd.mqk[0], hd.mqk[1]);
+                    mma_zero(m[mt][1], ufr[mt], hd.mqk[2], hd.mqk[3]);
+                }
+            }
             if (j == 2) {   // out = bf(o0) (+) bf(U Mqk^T)
 #pragma unroll
                 for (int mt = 0; mt < kMt; ++mt)
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
-                        o[mt][i] = bf2_add(o0p[mt][i], pack_bf2(m[mt][i >> 1][2 * (i & 1)], m[mt][i >> 1][2 * (i & 1) + 1]));
+                        o[mt][i] = bf2_add(pack_bf2(o0[mt][i >> 1][2 * (i & 1)], o0[mt][i >> 1][2 * (i & 1) + 1]),
+                                           pack_bf2(m[mt][i >> 1][2 * (i & 1)], m[mt][i >> 1][2 * (i & 1) + 1]));
             }
             mid(j);
         }
-        if constexpr (kNext) d1_half(o0, b[7] + 4, 7);
     }
 };
 
