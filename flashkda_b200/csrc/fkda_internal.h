@@ -36,6 +36,7 @@ struct TwoPassArgs {
                                    // every sequence (slab_chunks == 0: all chunks); a chain's state travels from one
                                    // slab to the next through seg_state
     int32_t layer;         // row slices by decreasing length: CTAs of the first layer (one per SM), 0 = no particular order
+    int32_t chain_weight;  // one-kernel forward: what the start and the end of a chain cost, in chunk steps (see chain_weight)
     int64_t T, H, N, total_tiles;
     int64_t token_stride, beta_token_stride;
     float scale, gate_scale;

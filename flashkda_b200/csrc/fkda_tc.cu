@@ -200,9 +200,20 @@ bool encode_state_map(CUtensorMap* m, const void* base, int64_t chains, bool fp3
 }
 static_assert(kRowCols == kD / 2, "a CTA of the row-slice kernel takes one half of a value row");
 
+// What the start and the end of a chain cost a CTA of the one-kernel forward, in chunk steps: the loads and stores of its state,
+// which nothing hides (a chain of c chunks takes 1.2 c + 3.9 us with bf16 states in and out and 1.2 c + 5.7 us with fp32
+// states).  Measured best among 0 .. 8 on sequences of 1 to 2 u tokens, u = 2 to 64 chunks, 512 to 12 800 chains: 1 without
+// states, 3 with bf16 states, 4 with fp32 states (12 800 chains of 4 chunks on average, us by weight 0, 1, 3, 4, 8: no states
+// 663, 587, 635, 655, 710; bf16 1115, 962, 853, 872, 925; fp32 1452, 1246, 1038, 1033, 1089).
+static int chain_weight(const fkda_fwd_params& p) {
+    const int each = p.state_dtype == FKDA_STATE_FP32 ? 3 : 2;
+    return (2 + (p.initial_state != nullptr ? each : 0) + (p.final_state != nullptr ? each : 0)) / 2;
+}
+
 // One kernel (and the prefix kernel of a ragged batch).
 static int launch_fused(const fkda_fwd_params& p, TwoPassArgs& a, int sms, cudaStream_t stream, int* n_launches) {
     const int64_t chains = p.N * p.H;
+    a.chain_weight = chain_weight(p);
     // the flags directly behind the header for a fixed batch (it has no prefix tables): one stretch to clear; the prefix
     // kernel clears both for a ragged batch
     uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes;

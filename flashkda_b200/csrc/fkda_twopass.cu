@@ -301,6 +301,7 @@ void fill_args(const fkda_fwd_params& p, TwoPassArgs* out) {
     a.slab_c0 = 0;
     a.slab_chunks = 0;
     a.layer = 0;
+    a.chain_weight = 0;
     a.tile_prefix = reinterpret_cast<int32_t*>(base + kWsHeaderBytes);
     a.seq_order = (varlen && p.N <= kSeqOrderMaxN) ? a.tile_prefix + (p.N + 1) : nullptr;
     a.cs_prefix = a.tile_prefix + (2 * p.N + 1);
