@@ -90,11 +90,17 @@ static bool slabs_possible(int64_t chains, int sms) { return chains * kRowSplit 
 // While every slice has an SM of its own, a step of the row-slice kernel takes 0.52 us against 1.05 us here, which pays for the
 // prepare kernel in front of it (64 chains of 512 chunks: 0.50 ms against 0.57; 96 chains: 0.71 against 0.57).  A ragged batch
 // whose lengths the host does not know may consist of a few long chains, whose walk is then the whole time (128 chains of 1
-// to 32 chunks: 52 us in two kernels against 82): it needs two chains per SM.
+// to 32 chunks: 52 us in two kernels against 82): it needs two chains per SM, or 1.6 with more than ten chunks per sequence
+// on average (256 and 288 chains: 16 chunks 47 to 93 us against 51 to 112, 256 chunks 425 to 568 against 645 to 873, but 4
+// chunks 39 against 34; 192 chains go either way).  With fp32 states to load and to store, which nothing hides here, it needs
+// more than four chunks per sequence on average (3 840 chains of 2 chunks 256 us against 214, of 4 chunks 318 against 289).
 static bool fused_eligible(const fkda_fwd_params& p, int sms) {
     if (p.phase_mask != 0 || p.B * p.T <= kChunk * p.N) return false;
-    const int64_t chains = p.N * p.H;
-    return (p.cu_seqlens != nullptr ? chains >= 2 * sms : chains * kRowSplit > sms) || (p.flags & FKDA_FLAG_NO_WIDE);
+    if (p.flags & FKDA_FLAG_NO_WIDE) return true;
+    const int64_t chains = p.N * p.H, tokens = p.B * p.T;
+    if (p.state_dtype == FKDA_STATE_FP32 && p.initial_state != nullptr && p.final_state != nullptr && tokens <= 4 * kChunk * p.N) return false;
+    if (p.cu_seqlens == nullptr) return chains * kRowSplit > sms;
+    return chains >= 2 * sms || (5 * chains >= 8 * sms && tokens > 10 * kChunk * p.N);
 }
 static size_t fused_flag_bytes(int sms) { return (size_t)(sms * 4 + 255) / 256 * 256; }
 // header | prefix tables | one flag and one hand-over state per range

@@ -65,3 +65,26 @@ def test_dispatch_line():
     for n, expect in ((2 * sms - 1, 3), (2 * sms, 2)):
         _call(make_inputs(Workload("l", 1, 18 * n, 1, seq_lens=[18] * n), seed=1))
         assert flashkda_b200.last_launch_count() == expect
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+@pytest.mark.parametrize("length", [64, 65])
+def test_dispatch_line_of_short_sequences(dtype, length):
+    """fp32 states in and out: the one kernel from more than four chunks per sequence, with the same results."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for w, one in ((Workload("s", sms, length, 1, state_in=dtype, state_out=dtype), 1),
+                   (Workload("s", 1, length * 2 * sms, 1, state_in=dtype, state_out=dtype, seq_lens=[length] * (2 * sms)), 2)):
+        inp = make_inputs(w, seed=3)
+        out, hT, _ = _call(inp)
+        assert flashkda_b200.last_launch_count() == one + (1 if dtype == "fp32" and length == 64 else 0)
+        out2, hT2, _ = _call(inp, flags=_lib.FLAG_NO_WIDE)
+        assert torch.equal(out, out2) and torch.equal(hT, hT2)
+
+
+def test_dispatch_line_of_long_ragged_sequences():
+    """Ragged batches of more than ten chunks per sequence take the one kernel from 1.6 chains per SM."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = (8 * sms + 4) // 5
+    for count, length, expect in ((n, 161, 2), (n, 160, 3), (n - 1, 161, 3)):
+        _call(make_inputs(Workload("l", 1, length * count, 1, seq_lens=[length] * count), seed=1))
+        assert flashkda_b200.last_launch_count() == expect
