@@ -1,6 +1,7 @@
 """The one-chunk kernel (sequences of 1 .. 16 tokens, persistent CTAs that stream states through shared memory) against the general
-kernels, bit for bit: chain counts around its grid, its two groups and its ring, both state types, missing states, a final
-state written over the initial one, and decode steps on both sides of the dispatch line."""
+kernels, bit for bit: chain counts around its grid, its two groups and its ring, many rounds per CTA with and without states to
+load, both state types, missing states, a final state written over the initial one, and decode steps on both sides of the
+dispatch line."""
 import pytest
 import torch
 
@@ -61,3 +62,19 @@ def test_ragged_with_empty_sequences_over_several_rounds(state):
     d = to_device(make_inputs(Workload("re", 1, sum(lens), 4, state_in=state, state_out=state, lower_bound=-2.0, seq_lens=lens), seed=6), "cuda")
     got, ref = _call(d), _call(d, GENERAL)
     assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("T", [2, 16])
+@pytest.mark.parametrize("state_in,state_out", [(None, "bf16"), (None, "fp32"), ("bf16", "bf16"), ("fp32", "fp32")])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_many_rounds_per_cta(T, state_in, state_out, ragged):
+    """Dozens of chains per CTA, repeated: nothing but the kernel's own barriers keeps the warps of a group in step, and without
+    states to load there is no arrival of a load to hold one back."""
+    n, H = 1100, 4
+    lens = [T] * n if ragged else None
+    w = Workload("mr", 1 if ragged else n, n * T if ragged else T, H, state_in=state_in, state_out=state_out, lower_bound=-2.0, seq_lens=lens)
+    d = to_device(make_inputs(w, seed=T), "cuda")
+    ref = _call(d, GENERAL)
+    for _ in range(10):
+        got = _call(d)
+        assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
