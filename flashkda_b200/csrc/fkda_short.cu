@@ -101,20 +101,22 @@ __device__ __forceinline__ void short_put(const uint32_t (&s)[kMt][8][4], uint32
         }
 }
 
-template <bool kFp32>
+// kRagged: a ragged batch behind the prefix kernel's decision; it may hold empty sequences (a check for them in the build for fixed
+// batches as well: 357 -> 382 us for 32 768 decode steps)
+template <bool kFp32, bool kRagged>
 __global__ void __launch_bounds__(kShortThreads, 1)
 short_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ ShortMaps maps) {
     grid_dep_wait();
     // a ragged batch that the prefix kernel has given to other kernels (a longer sequence: the general ones; one token
     // each: the decode kernel)
-    if (a.short_flag != nullptr && *a.short_flag != 1) return;
+    if (kRagged && *a.short_flag != 1) return;
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     ShortCtrl& ctl = *reinterpret_cast<ShortCtrl*>(sm + kShortCtrl);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &ctl.abort_flag;
-    if (a.short_flag == nullptr && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
+    if (!kRagged && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kShortSlots; ++s) {
             mbar_init(&ctl.full[s], 2);
@@ -140,7 +142,7 @@ short_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ Shor
         auto locate = [&](int i, int64_t* t0, int* len, int* h) {
             const int64_t chain = blockIdx.x + (int64_t)i * gridDim.x, n = chain / a.H;
             *h = (int)(chain - n * a.H);
-            if (a.cu_seqlens != nullptr) {
+            if (kRagged) {
                 const int64_t b = a.cu_seqlens[n], e = a.cu_seqlens[n + 1];
                 *len = e > b ? (int)(e - b) : 0;
                 *t0 = *len > 0 ? b : 0;   // (an empty sequence: any address inside the tensors)
@@ -271,7 +273,7 @@ short_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ Shor
 #pragma unroll
             for (int mt = 0; mt < kMt; ++mt) ldmatrix_x4_t(hd.v[mt][0], hd.v[mt][1], hd.v[mt][2], hd.v[mt][3], v_off[mt] + slot * kShortVTile);
             hd.mask(len, lane & 3);
-            const int64_t t0 = a.cu_seqlens != nullptr ? a.cu_seqlens[n] : n * a.T;
+            const int64_t t0 = kRagged ? a.cu_seqlens[n] : n * a.T;
             __nv_bfloat16* og = a.out + (t0 + (lane >> 1)) * a.token_stride + (int64_t)h * kD + vrow + 8 * (lane & 1);
             uint32_t o[kMt][4];
             uint4 orow[kMt];
@@ -297,6 +299,10 @@ short_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ Shor
             // (Of six ways to order this, among them a barrier per stage, and all warps waiting for item k itself: 154 us
             // for 12 288 chains of 5 tokens with bf16 states, the others 154 to 167.)
             if (k > 0 && !wait_all(&ctl.sdone[group], (uint32_t)((k - 1) & 1))) { failed = true; break; }
+            if (kRagged && len == 0) {   // an empty sequence: its state passes through, whatever the record holds
+                if (has_in) short_get<kMt, kFp32>(w.s, stage, row, lane);
+                else w.clear();
+            }
             if (has_out) {
                 short_put<kMt, kFp32>(w.s, stage, row, lane);
                 fence_proxy_async_smem();
@@ -359,11 +365,13 @@ static int launch_short_typed(const fkda_fwd_params& p, const TwoPassArgs& a, in
     if (!encode_v_map(&maps.v, p)) return FKDA_ERR_LAUNCH;
     if (p.initial_state != nullptr && !encode_state_map(&maps.h0, p.initial_state, chains, kFp32)) return FKDA_ERR_LAUNCH;
     if (p.final_state != nullptr && !encode_state_map(&maps.hT, p.final_state, chains, kFp32)) return FKDA_ERR_LAUNCH;
-    if (!allow_smem<short_kernel<kFp32>>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
     const int64_t ctas = chains < sms ? chains : sms;
-    if (a.short_flag != nullptr)   // behind the prefix kernel
-        return launch_dependent(short_kernel<kFp32>, ctas, kShortThreads, kShortSmemBytes, stream, a, maps) ? FKDA_OK : FKDA_ERR_LAUNCH;
-    short_kernel<kFp32><<<(unsigned)ctas, kShortThreads, kShortSmemBytes, stream>>>(a, maps);
+    if (a.short_flag != nullptr) {   // behind the prefix kernel
+        if (!allow_smem<short_kernel<kFp32, true>>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
+        return launch_dependent(short_kernel<kFp32, true>, ctas, kShortThreads, kShortSmemBytes, stream, a, maps) ? FKDA_OK : FKDA_ERR_LAUNCH;
+    }
+    if (!allow_smem<short_kernel<kFp32, false>>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
+    short_kernel<kFp32, false><<<(unsigned)ctas, kShortThreads, kShortSmemBytes, stream>>>(a, maps);
     return cudaGetLastError() == cudaSuccess ? FKDA_OK : FKDA_ERR_LAUNCH;
 }
 

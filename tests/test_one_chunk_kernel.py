@@ -78,3 +78,24 @@ def test_many_rounds_per_cta(T, state_in, state_out, ragged):
     for _ in range(10):
         got = _call(d)
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("state", ["bf16", "fp32"])
+def test_empty_sequences_pass_their_state_through(state):
+    """Bit for bit, whatever the state holds (signed zeros, infinities, NaN) and whatever the tokens of other sequences hold: the
+    batch's first token is made of NaN."""
+    lens = [5, 0, 16, 0, 1, 0] * 24
+    d = to_device(make_inputs(Workload("ep", 1, sum(lens), 3, state_in=state, state_out=state, lower_bound=-2.0, seq_lens=lens), seed=8), "cuda")
+    for name in "qkvg":
+        d[name][0, 0] = float("nan")
+    h0 = d["initial_state"]
+    h0[1, :, 3] = -0.0
+    h0[3, :, 5, 7], h0[3, :, 6] = float("inf"), float("nan")
+    got, ref = _call(d), _call(d, GENERAL)
+    assert flashkda_b200.last_launch_count() == 3
+    bits = lambda x: x.contiguous().view(torch.int16 if x.dtype == torch.bfloat16 else torch.int32)
+    empty, rest = [i for i, n in enumerate(lens) if n == 0], [i for i, n in enumerate(lens) if n > 0 and i > 0]
+    want = h0[empty].to(torch.bfloat16).to(h0.dtype)
+    assert torch.equal(bits(got[1][empty]), bits(ref[1][empty]))
+    assert torch.allclose(got[1][empty], want, rtol=0, atol=0, equal_nan=True)
+    assert torch.equal(got[1][rest], ref[1][rest]) and torch.equal(got[0][0, 5:], ref[0][0, 5:])
