@@ -260,7 +260,7 @@ class SequenceSplit:
 
     def _fwd(self, v, h0, hT):
         """One operator call on the batch of pieces; the first one asks for both stages by name, so that it leaves its
-        chunk records in the workspace, later ones walk them."""
+        chunk records in the workspace (pieces of one chunk: the second one does), later ones walk them."""
         from . import _lib
         qb, kb, _, gb, bb = self.t
         self.F.fwd(qb, kb, v, gb, bb, self.scale, self.out, *self.args, h0, hT, None, workspace=self.ws,

@@ -64,7 +64,10 @@ __global__ void __launch_bounds__(128, 4) decode_kernel(const __grid_constant__ 
     // a ragged batch with as many tokens as sequences: mine only if the prefix kernel found one token in each (then
     // sequence n is token n, as in a fixed batch)
     if (a.short_flag != nullptr && *a.short_flag != 2) return;
-    if (a.short_flag == nullptr && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
+    if (a.short_flag == nullptr && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.status = 0;
+        *a.records = 0;
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t chain = blockIdx.x / kSplit;
     const int my_row = lane / kSplit;       // the row whose u, v and out are mine

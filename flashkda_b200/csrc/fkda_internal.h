@@ -30,6 +30,10 @@ struct TwoPassArgs {
                            // one-chunk sequences; the kernels that can serve the call are all enqueued and all but one
                            // return at once: 2 = every sequence has exactly one token (decode kernel), 1 = no sequence is
                            // longer than one chunk (fused short-sequence kernel), 0 = the general kernels
+    uint64_t* records;     // header words 16, 17, or null without a header: which chunk records the workspace holds (records_tag of
+                           // the call that wrote them; 0: none, the last forward on this workspace kept them on the SMs)
+    uint64_t records_tag;  // of this call
+    bool on_demand;        // the recurrence alone was asked for: the records are prepared if the workspace does not hold them
     int32_t* range_flags;  // one-kernel forward: walking warps of each range that have published their rows of its state
     uint32_t* seg_state;   // bf16 states in fragment order, handed from range to range (one-kernel forward) or slab to slab
     int32_t slab_c0, slab_chunks;  // fixed batches only: this launch covers chunks [slab_c0, slab_c0 + slab_chunks) of
@@ -49,7 +53,8 @@ struct TwoPassArgs {
 };
 
 // Workspace layout of both two-pass implementations:
-//   [0, 256)  header: int32 ticket counter, device status, word 8: path decision of a ragged batch
+//   [0, 256)  header: int32 ticket counter, device status, word 8: path decision of a ragged batch, words 16, 17: which chunk
+//             records are behind it
 //   [256, ..) tile prefix (N + 1 int32, padded to 256 B)
 //   then      H * total_tiles records
 constexpr size_t kWsHeaderBytes = 256;
@@ -122,7 +127,8 @@ inline bool launch_dependent(void (*kernel)(KernelArgs...), int64_t ctas, int th
 // workspace carving).
 void fill_args(const fkda_fwd_params& p, TwoPassArgs* a);
 // The prefix kernel of a ragged batch: chunk (and state-export) prefix tables, the length order if asked for, and the path
-// decision if a.short_flag is set; clears the header and `n_flags` range flags.
+// decision if a.short_flag is set; clears the header (the note on the records only if the call is going to write new ones
+// or none) and `n_flags` range flags.
 void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags = 0);
 // First state-export slot of sequence n.
 __device__ __forceinline__ int64_t cs_first_slot(const TwoPassArgs& a, int64_t n) {

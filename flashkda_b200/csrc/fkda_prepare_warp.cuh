@@ -68,6 +68,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) prepare_warp_kernel(const _
     if (a.cu_seqlens == nullptr && a.slab_c0 == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
     // (a ragged batch that the fused short-sequence kernel has served: nothing to do)
     if (a.short_flag != nullptr && *a.short_flag != 0) return;
+    if (a.on_demand) {   // (these records get no note: CTAs that start later still have to find none)
+        if (*a.records == a.records_tag) return;
+    } else if (a.slab_c0 == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.records = a.records_tag;
+    }
     extern __shared__ uint8_t prep_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint8_t* rec = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(prep_smem) + 127) & ~(uintptr_t)127) + warp * kTcRecord;

@@ -116,7 +116,10 @@ short_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ Shor
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &ctl.abort_flag;
-    if (!kRagged && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
+    if (!kRagged && a.status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.status = 0;
+        *a.records = 0;
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kShortSlots; ++s) {
             mbar_init(&ctl.full[s], 2);

@@ -121,6 +121,13 @@ static TcCarve tc_carve(const fkda_fwd_params& p, int sms) {
     return c;
 }
 
+// Names the records that a call writes or expects: everything that decides where each of them lies.
+static uint64_t records_tag(const fkda_fwd_params& p) {
+    uint64_t x = p.cu_seqlens != nullptr ? 2 : 1;
+    for (const int64_t y : {p.B, p.T, p.H, p.N}) x = (x ^ (uint64_t)y) * 0x9e3779b97f4a7c15ull, x ^= x >> 29;
+    return x | 1;
+}
+
 // Upper bound over every call with these totals (the caller may not know yet whether the batch is ragged).
 size_t tc_workspace_bytes(int64_t T_total, int64_t H, int64_t N) {
     const int sms = device_sm_count();
@@ -263,8 +270,11 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     const int64_t T_total = p.B * p.T, chains = p.N * p.H;
     if (fused_eligible(p, sms)) return launch_fused(p, a, sms, stream, n_launches);
     if (chains * kRowSplit > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
+    a.records_tag = records_tag(p);
+    a.on_demand = do_rec && !do_prep;
+    const bool tables = do_prep || do_rec;   // (a phase mask may also name neither)
     // (the header is cleared by the first kernel where there is one: the prefix kernel, or the prepare stage of a fixed batch)
-    if (!(do_prep && (varlen || a.total_tiles > 0)) && cudaMemsetAsync(p.workspace, 0, 64, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;
+    if (!(varlen ? tables : do_prep && a.total_tiles > 0) && cudaMemsetAsync(p.workspace, 0, 64, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;
     const TcCarve carve = tc_carve(p, sms);
     uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes + ws_prefix_bytes(p.N);
     a.seg_state = reinterpret_cast<uint32_t*>(base);
@@ -354,7 +364,10 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
 
     // as many tokens as sequences: they may have one token each, the decode kernel's case
     const bool try_decode = a.short_flag != nullptr && T_total == p.N && chains <= decode_max_chains(p) && !(p.flags & FKDA_FLAG_NO_DECODE);
-    if (varlen && do_prep) {
+    // The recurrence alone takes the records that an earlier call on this workspace left.  That call may have been one that leaves
+    // none (the one-kernel forms), so the tables of a ragged batch are made again and the prepare stage is enqueued in any
+    // case: it returns at once where the records are there.
+    if (varlen && tables) {
         launch_tile_prefix(a, const_cast<int32_t*>(a.seq_order), try_decode, stream);
         ++launches;
     }
@@ -366,7 +379,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         if (launch_short_ragged(p, a, stream) != FKDA_OK) return FKDA_ERR_LAUNCH;
         ++launches;
     }
-    if (a.total_tiles > 0 && do_prep) {
+    if (a.total_tiles > 0 && tables) {
         if (launch_prepare_warp<true>(a, stream, 0, varlen) != FKDA_OK) return FKDA_ERR_LAUNCH;
         ++launches;
     }

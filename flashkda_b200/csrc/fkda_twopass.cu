@@ -23,11 +23,13 @@ __global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __rest
                                                            int32_t* __restrict__ prefix, int32_t* __restrict__ order,
                                                            int32_t* __restrict__ cs_prefix, int cs_tokens,
                                                            int32_t* __restrict__ short_flag, int decode_enqueued,
-                                                           int32_t* __restrict__ header, int32_t* __restrict__ flags, int n_flags) {
+                                                           int32_t* __restrict__ header, int keep_records, int32_t* __restrict__ flags,
+                                                           int n_flags) {
     grid_dep_launch();
     __shared__ int64_t part[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < 8) header[tid] = 0;   // ticket counter, device status
+    if (!keep_records && (tid == 16 || tid == 17)) header[tid] = 0;
     for (int i = tid; i < n_flags; i += 1024) flags[i] = 0;
     const int64_t per = (N + 1023) / 1024;
     const int64_t lo = tid * per, hi = (lo + per < N) ? lo + per : N;
@@ -254,7 +256,7 @@ __global__ void __launch_bounds__(128) recurrence_kernel(TwoPassArgs a) {
 void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags) {
     tile_prefix_kernel<<<1, 1024, 0, stream>>>(a.cu_seqlens, a.N, a.tile_prefix, seq_order,
                                                a.chunk_states != nullptr ? const_cast<int32_t*>(a.cs_prefix) : nullptr, 16 * a.cs_every,
-                                               a.short_flag, decode_enqueued ? 1 : 0, a.queue, a.range_flags, n_flags);
+                                               a.short_flag, decode_enqueued ? 1 : 0, a.queue, a.on_demand ? 1 : 0, a.range_flags, n_flags);
 }
 
 size_t twopass_workspace_bytes(int64_t T_total, int64_t H, int64_t N) {
@@ -295,6 +297,9 @@ void fill_args(const fkda_fwd_params& p, TwoPassArgs* out) {
     a.queue = reinterpret_cast<int32_t*>(base);
     // (a one-kernel path needs no workspace; where the caller gave one, its status word is kept)
     a.status = base != nullptr && p.workspace_bytes >= kWsHeaderBytes && ((uintptr_t)base & 255u) == 0 ? reinterpret_cast<int32_t*>(base) + 1 : nullptr;
+    a.records = a.status != nullptr ? reinterpret_cast<uint64_t*>(base) + 8 : nullptr;
+    a.records_tag = 0;
+    a.on_demand = false;
     a.short_flag = nullptr;
     a.range_flags = nullptr;
     a.seg_state = nullptr;
@@ -313,7 +318,7 @@ int launch_twopass(const fkda_fwd_params& p, cudaStream_t stream, int* n_launche
     fill_args(p, &a);
     const bool varlen = p.cu_seqlens != nullptr;
     int launches = 0;
-    if (cudaMemsetAsync(p.workspace, 0, 16, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;  // queue + status
+    if (cudaMemsetAsync(p.workspace, 0, kWsHeaderBytes, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;
     const bool do_prep = p.phase_mask == 0 || (p.phase_mask & FKDA_PHASE_PREPARE);
     const bool do_rec = p.phase_mask == 0 || (p.phase_mask & FKDA_PHASE_RECURRENCE);
     if (varlen && do_prep) {

@@ -84,8 +84,10 @@ typedef struct fkda_fwd_params {
     void* workspace;           /* >= fkda_workspace_bytes(B*T, H, N, algo) bytes, 256-byte aligned */
     size_t workspace_bytes;
     int32_t phase_mask;        /* 0 = whole forward, by whatever kernels serve it best; otherwise a bit set of FKDA_PHASE_*
-                                  to launch in the two-kernel form, which leaves (PREPARE) or expects (RECURRENCE)
-                                  the chunk records in the workspace */
+                                  to run in the two-kernel form (sequences of at most 16 tokens, both bits: as 0).
+                                  PREPARE leaves the chunk records in the workspace.  RECURRENCE alone walks the records
+                                  that the last call on this workspace left there, if its shapes were the same; where it
+                                  left none, as a whole forward may, they are prepared from this call's inputs first */
     int32_t flags;             /* 0 for normal use; FKDA_FLAG_* bits select kernel variants for tests and tuning */
     void* chunk_states;        /* optional bf16 [slots, H, 128 (V), 128 (K)]: the state of every sequence BEFORE each group
                                   of `chunk_states_every` chunks (16 * every tokens), i.e. before tokens 0, 16*every,

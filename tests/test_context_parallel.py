@@ -149,10 +149,10 @@ def test_emulated_shards_match_one_shot_gpu(shards):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("parts", [2, 8])
-def test_sequence_parallel_single_gpu(parts):
+@pytest.mark.parametrize("tokens,parts", [(4096, 2), (4096, 8), (256, 16)])   # the last: pieces of one chunk
+def test_sequence_parallel_single_gpu(tokens, parts):
     import flashkda_b200
-    inp = to_device(_weak_decay_inputs(4096, 4, 23), "cuda")
+    inp = to_device(_weak_decay_inputs(tokens, 4, 23), "cuda")
     one_out, one_hT = torch.zeros_like(inp["out"]), torch.zeros_like(inp["final_state"])
     flashkda_b200.fwd(inp["q"], inp["k"], inp["v"], inp["g"], inp["beta"], inp["scale"], one_out, inp["A_log"],
                       inp["dt_bias"], inp["lower_bound"], inp["initial_state"], one_hT)

@@ -88,3 +88,42 @@ def test_dispatch_line_of_long_ragged_sequences():
     for count, length, expect in ((n, 161, 2), (n, 160, 3), (n - 1, 161, 3)):
         _call(make_inputs(Workload("l", 1, length * count, 1, seq_lens=[length] * count), seed=1))
         assert flashkda_b200.last_launch_count() == expect
+
+
+def _sms():
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.parametrize("kind", ["one_kernel", "one_kernel_ragged", "one_token", "short", "one_chunk", "short_ragged", "two_kernels", "empty"])
+def test_recurrence_alone_behind_any_call(kind):
+    """PHASE_RECURRENCE on a workspace whose last call left no records (a one-kernel form), left records, or left those of other
+    inputs before a call that left none: the result of the whole forward with this call's values, each time."""
+    n = _sms()
+    shape = {"one_kernel": (n, 70, 1, None), "one_kernel_ragged": (1, 70 * 2 * n, 1, [70] * (2 * n)), "one_token": (70, 1, 2, None),
+             "short": (70, 5, 2, None), "one_chunk": (70, 16, 2, None), "short_ragged": (1, 7 * 64, 2, [3, 0, 16, 9] * 16),
+             "two_kernels": (1, 100, 3, None), "empty": (3, 0, 2, None)}[kind]
+    w = Workload("ra", *shape[:3], state_in="fp32", state_out="fp32", lower_bound=-2.0, seq_lens=shape[3])
+    a, b = (to_device(make_inputs(w, seed=s), "cuda") for s in (1, 2))
+    ws = torch.full((flashkda_b200.get_workspace_size(w.tokens, w.H, w.n_seqs),), 0xAB, dtype=torch.uint8, device="cuda")
+
+    def call(d, phase_mask, v=None):
+        flashkda_b200.fwd(d["q"], d["k"], d["v"] if v is None else v, d["g"], d["beta"], d["scale"], d["out"].zero_(), d["A_log"],
+                          d["dt_bias"], d["lower_bound"], d["initial_state"], d["final_state"].zero_(), d["cu_seqlens"],
+                          workspace=ws, phase_mask=phase_mask)
+        assert flashkda_b200.device_status(ws) == 0
+        return d["out"].clone(), d["final_state"].clone()
+
+    v2 = torch.flip(b["v"], [1])
+    general = _lib.FLAG_NO_DECODE | _lib.FLAG_NO_SHORT
+    flashkda_b200.fwd(b["q"], b["k"], v2, b["g"], b["beta"], b["scale"], b["out"].zero_(), b["A_log"], b["dt_bias"], b["lower_bound"],
+                      b["initial_state"], b["final_state"].zero_(), b["cu_seqlens"], flags=general)
+    want = b["out"].clone(), b["final_state"].clone()
+    for before in (0, BOTH, _lib.PHASE_PREPARE, None):   # None: nothing, the records of the call before are still there
+        if before is not None:
+            call(a, _lib.PHASE_PREPARE)
+            call(b, before)
+            if before == 0 and kind in ("one_kernel", "one_kernel_ragged", "one_token", "short", "one_chunk"):
+                assert flashkda_b200.last_launch_count() == (2 if shape[3] else 1)   # no records left
+        for _ in range(2):
+            got = call(b, _lib.PHASE_RECURRENCE, v2)
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), before
