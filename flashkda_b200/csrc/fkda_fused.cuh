@@ -46,6 +46,7 @@ constexpr int kFusedCtrl = kFusedRec + kFusedSlots * kTcRecord;
 // The line of chunks: [lo, hi) is this CTA's range, walked as [b0, hi), [a1, b0), [lo, a1).
 struct FusedRange {
     int64_t lo, hi, a1, b0;
+    int64_t before;       // chunks of the chain at lo that other ranges walk first
     // position of unit u and the end of its run of consecutive positions
     __device__ __forceinline__ int64_t position(int u, int64_t* end) const {
         const int n1 = (int)(hi - b0), n2 = (int)(b0 - a1);
@@ -111,11 +112,13 @@ __device__ __forceinline__ FusedRange fused_range(const TwoPassArgs& a, int rang
     r.lo = fused_bound(a, range);
     r.hi = fused_bound(a, range + 1);
     r.a1 = r.lo;
+    r.before = 0;
     r.b0 = r.hi;
     if (r.lo < r.hi) {
         const FusedSeq f = fused_seq(a, r.lo), l = fused_seq(a, r.hi - 1);
         const int64_t first = r.lo - (r.lo - f.begin) % f.n_chunks;            // starts of the chains that hold the ends
         const int64_t last = r.hi - 1 - (r.hi - 1 - l.begin) % l.n_chunks;
+        r.before = r.lo - first;
         if (first < r.lo) r.a1 = min(r.hi, first + f.n_chunks);
         if (r.hi < last + l.n_chunks) r.b0 = max(r.a1, last);
     }
@@ -182,6 +185,9 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
     const int range = ctl.range;
     const FusedRange r = fused_range(a, range);
     const int n_units = (int)(r.hi - r.lo);
+    // The chain at lo reaches this range when the ranges before have walked its beginning, at a microsecond per chunk: with a
+    // chain much longer than a range that alone may take longer than the limit of a wait, which is for what never comes.
+    const uint64_t wait_ns = a.wait_ns + 8000ull * (uint64_t)r.before;
     bool failed = false;
 
     if (warp >= kFusedWalkers) {
@@ -215,7 +221,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
             const uint32_t phase = 1u ^ ((u / kFusedSlots) & 1);   // of empty[slot]: the first round finds the slots free
             uint8_t* rec = sm + kFusedRec + slot * kTcRecord;
             auto acquire = [&]() {   // the slot is free: leave the note and ask for the value tile
-                if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.empty[slot], phase, abort_flag, a.wait_ns)) == 0) return false;
+                if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.empty[slot], phase, abort_flag, wait_ns)) == 0) return false;
                 if (lane == 0) {
                     FusedInfo& f = ctl.info[slot];
                     f.tok0 = t0;
@@ -265,7 +271,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
         WalkHead<kFusedMt> hd;
         int slot = 0;             // ring slot of the current unit
         uint32_t phase = 0;       // of full[slot]
-        auto wait_full = [&](int sl, uint32_t ph) { return __all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[sl], ph, abort_flag, a.wait_ns)) != 0; };
+        auto wait_full = [&](int sl, uint32_t ph) { return __all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[sl], ph, abort_flag, wait_ns)) != 0; };
         FusedInfo pc;   // of the first chunk of the current piece
         for (int u = 0; u < n_units; u += pc.rest) {
             if (!wait_full(slot, phase)) { failed = true; break; }
@@ -278,7 +284,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
                 const uint64_t begin = global_timer_ns();
                 uint32_t spins = 0;
                 while (load_acquire(a.range_flags + before) < kFusedWalkers) {
-                    if ((++spins & 15u) == 0 && (*abort_flag != 0 || global_timer_ns() - begin > a.wait_ns)) { failed = true; break; }
+                    if ((++spins & 15u) == 0 && (*abort_flag != 0 || global_timer_ns() - begin > wait_ns)) { failed = true; break; }
                     __nanosleep(100);
                 }
                 if (__any_sync(0xffffffffu, failed)) { failed = true; break; }

@@ -18,10 +18,10 @@ from flashkda_b200.synth import Workload, make_inputs, to_device
 pytestmark = pytest.mark.gpu
 
 
-def _call(d, ws, flags=0):
+def _call(d, ws, flags=0, phase_mask=0):
     flashkda_b200.fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], d["scale"], d["out"], A_log=d["A_log"],
                       dt_bias=d["dt_bias"], lower_bound=d["lower_bound"], initial_state=d["initial_state"],
-                      final_state=d["final_state"], cu_seqlens=d["cu_seqlens"], algo="tc", workspace=ws, flags=flags)
+                      final_state=d["final_state"], cu_seqlens=d["cu_seqlens"], algo="tc", workspace=ws, flags=flags, phase_mask=phase_mask)
 
 
 def _many_chains(seed, n_seq=100, H=5):
@@ -81,3 +81,22 @@ def test_two_persistent_launches_on_two_streams():
         for (d, ws), (out, state) in zip(probs, expect):
             assert flashkda_b200.device_status(ws) == 0
             assert torch.equal(d["out"], out) and torch.equal(d["final_state"], state)
+
+
+def test_a_chain_longer_than_the_limit_of_a_wait():
+    """One long sequence among many short ones: its chain is walked range after range, so the last CTA's turn comes when all of it
+    but the end is done (4 ms here, under a limit of 1 ms).  That is no reason to give up."""
+    n = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    lens = [64000 - n] + [1] * (n - 1)
+    w = Workload("lc", 1, sum(lens), 1, state_in="bf16", state_out="bf16", seq_lens=lens, lower_bound=-2.0)
+    d = to_device(make_inputs(w, seed=4), "cuda")
+    ws = torch.empty(flashkda_b200.get_workspace_size(w.tokens, w.H, n), dtype=torch.uint8, device="cuda")
+    _call(d, ws, _lib.flags_wait_ms(1))
+    assert flashkda_b200.last_launch_count() == 2      # the one-kernel form
+    assert flashkda_b200.device_status(ws) == 0
+    out, state = d["out"].clone(), d["final_state"].clone()
+    d["out"].zero_()
+    d["final_state"].zero_()
+    _call(d, ws, phase_mask=_lib.PHASE_PREPARE | _lib.PHASE_RECURRENCE)
+    assert flashkda_b200.device_status(ws) == 0
+    assert torch.equal(d["out"], out) and torch.equal(d["final_state"], state)
