@@ -41,11 +41,16 @@ const at::Tensor& tensor_arg(PyObject* o, const char* name) {
 }
 const at::Tensor* optional_tensor_arg(PyObject* o, const char* name) { return o == Py_None ? nullptr : &tensor_arg(o, name); }
 
+// Whatever float() takes: numpy scalars, one-element tensors, strings.
 double number_arg(PyObject* o) {
-    const double x = PyFloat_AsDouble(o);   // (also what float() accepts: numpy scalars, one-element tensors)
-    if (x == -1.0 && PyErr_Occurred()) throw std::bad_cast();
+    if (PyFloat_Check(o)) return PyFloat_AS_DOUBLE(o);
+    PyObject* f = PyNumber_Float(o);
+    if (f == nullptr) throw std::bad_cast();
+    const double x = PyFloat_AS_DOUBLE(f);
+    Py_DECREF(f);
     return x;
 }
+// Whatever int() takes.
 long integer_arg(PyObject* o) {
     if (PyLong_Check(o)) {
         const long x = PyLong_AsLong(o);
@@ -61,18 +66,15 @@ long integer_arg(PyObject* o) {
 }
 
 int algo_arg(PyObject* o) {
-    const char* s = nullptr;
-    if (o == Py_None) {
-        s = std::getenv("FLASHKDA_B200_ALGO");
-        if (s == nullptr) return FKDA_ALGO_AUTO;
-    } else {
-        s = PyUnicode_AsUTF8(o);
-        if (s == nullptr) throw std::bad_cast();
-        if (s[0] == '\0') {
-            s = std::getenv("FLASHKDA_B200_ALGO");
-            if (s == nullptr) return FKDA_ALGO_AUTO;
-        }
+    const int given = PyObject_IsTrue(o);
+    if (given < 0) throw std::bad_cast();
+    if (given && !PyUnicode_Check(o)) {
+        PyErr_SetObject(PyExc_KeyError, o);
+        throw std::bad_cast();
     }
+    const char* s = given ? PyUnicode_AsUTF8(o) : std::getenv("FLASHKDA_B200_ALGO");
+    if (given && s == nullptr) throw std::bad_cast();
+    if (s == nullptr) return FKDA_ALGO_AUTO;
     if (std::strcmp(s, "auto") == 0) return FKDA_ALGO_AUTO;
     if (std::strcmp(s, "twopass") == 0) return FKDA_ALGO_TWOPASS;
     if (std::strcmp(s, "tc") == 0) return FKDA_ALGO_TC;

@@ -78,3 +78,23 @@ def test_drop_in_module_name():
     params = list(inspect.signature(flash_kda.fwd).parameters)
     assert params[:13] == ["q", "k", "v", "g", "beta", "scale", "out", "A_log", "dt_bias", "lower_bound",
                            "initial_state", "final_state", "cu_seqlens"]
+
+
+@pytest.mark.gpu
+def test_host_side_takes_what_float_and_int_take():
+    import numpy as np
+    d = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in make_inputs(Workload("x", 2, 40, 3), seed=1).items()}
+
+    def call(scale, lower_bound, **kw):
+        d["out"].zero_()
+        flashkda_b200.fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], scale, d["out"], d["A_log"], d["dt_bias"], lower_bound, **kw)
+        return d["out"].clone()
+
+    want = call(0.5, -5.0)
+    for scale, lower_bound in ((np.float32(0.5), -5), ("0.5", "-5"), (torch.tensor(0.5), torch.tensor([-5.0]))):
+        assert torch.equal(call(scale, lower_bound), want)
+    for kw in (dict(algo="", flags=np.int64(0)), dict(algo=0, phase_mask=False), dict(algo=False, flags="0"), dict(phase_mask=0.0)):
+        assert torch.equal(call(0.5, -5.0, **kw), want)
+    for bad, error in ((dict(algo="x"), KeyError), (dict(algo=3), KeyError), (dict(flags="x"), ValueError), (dict(phase_mask=None), TypeError)):
+        with pytest.raises(error):
+            call(0.5, -5.0, **bad)
