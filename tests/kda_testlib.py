@@ -104,8 +104,8 @@ def gate_case_inputs(index, T=8192):
                 final_state=torch.zeros(1, 1, D, D), cu_seqlens=None)
 
 
-# Many-chains case: 8 x 64 = 512 (sequence, head) chains of 64 chunks, more than the 444 chain slots of a B200,
-# so the tensor-core recurrence hands chains from segment to segment through its work queue.
+# Many-chains case: 8 x 64 = 512 (sequence, head) chains of 64 chunks, 3.5 per SM of a B200: the one-kernel forward hands
+# chains from range to range.
 MANY_CHAINS = Workload("many_chains", 8, 1024, 64, lower_bound=-3.0, state_in="fp32", state_out="fp32")
 MANY_CHAINS_OUT_EVERY = 256    # the fixture keeps token rows t % 256 == 255 of every sequence
 MANY_CHAINS_STATE_EVERY = 32   # and the final states of chains (n * H + h) % 32 == 0

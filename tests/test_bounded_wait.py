@@ -1,10 +1,10 @@
 """The give-up path of the device-side waits, and persistent launches that share the GPU.
 
-Every wait inside the kernels (mbarrier, work-queue slot) is bounded: when its limit runs out the kernel
-records FKDA_ERR_DEVICE_STATUS in the workspace header, tells the other warpgroups of its CTA, frees its
-tensor memory and returns, so the context stays usable.  The first test makes that happen without any fault:
-a test-only flag stops finished segments from queueing their follow-ups, so the work queue starves and the
-waiters run out a limit shortened to a few milliseconds.  Nothing here traps, faults or waits without bound.
+Every wait inside the kernels (mbarrier, flag of another range) is bounded: when its limit runs out the kernel
+records FKDA_ERR_DEVICE_STATUS in the workspace header, tells the other warps of its CTA, waits for its own copies in
+flight and returns, so the context stays usable.  The first test makes that happen without any fault: a test-only flag
+stops the one-kernel forward from publishing the states it hands on, so that the ranges behind starve and run out
+a limit shortened to a few milliseconds.  Nothing here traps, faults or waits without bound.
 """
 import time
 
@@ -25,7 +25,7 @@ def _call(d, ws, flags=0, phase_mask=0):
 
 
 def _many_chains(seed, n_seq=100, H=5):
-    # 500 chains (more than the 444 chain slots of a B200: the segment queue is in use), 10 to 40 chunks each
+    # 500 chains of 10 to 40 chunks: the one-kernel forward, with chains cut by the ranges
     gen = torch.Generator().manual_seed(seed)
     lens = torch.randint(160, 640, (n_seq,), generator=gen).tolist()
     w = Workload("bw", 1, sum(lens), H, state_in="fp32", state_out="fp32", seq_lens=lens, lower_bound=-2.0)
@@ -34,32 +34,32 @@ def _many_chains(seed, n_seq=100, H=5):
     return d, ws
 
 
-def test_starved_queue_gives_up_cleanly_and_the_next_call_succeeds():
+def test_starved_ranges_give_up_cleanly_and_the_next_call_succeeds():
     d, ws = _many_chains(1)
     _call(d, ws)                                   # a normal call: the expected result
     assert flashkda_b200.device_status(ws) == 0
     good_out, good_state = d["out"].clone(), d["final_state"].clone()
 
-    flags = _lib.FLAG_TEST_DROP_PUSH | _lib.flags_wait_ms(5) | _lib.flags_seg_chunks(8)
+    flags = _lib.FLAG_TEST_DROP_PUSH | _lib.flags_wait_ms(5)
     t0 = time.perf_counter()
     _call(d, ws, flags)
     status = flashkda_b200.device_status(ws)       # synchronises
     dt = time.perf_counter() - t0
-    assert status == 9, "the starved queue must be reported as FKDA_ERR_DEVICE_STATUS"
+    assert status == 9, "starved ranges must be reported as FKDA_ERR_DEVICE_STATUS"
     assert dt < 2.0, f"the kernel took {dt:.2f} s to give up with a 5 ms limit"
 
-    # the context is intact and the tensor memory was freed: the same call without the hook is correct again
+    # the context is intact: the same call without the hook is correct again
     d["out"].zero_()
     d["final_state"].zero_()
-    _call(d, ws, _lib.flags_seg_chunks(8))
+    _call(d, ws)
     assert flashkda_b200.device_status(ws) == 0
     assert torch.equal(d["out"], good_out) and torch.equal(d["final_state"], good_state)
 
 
 def test_two_persistent_launches_on_two_streams():
-    """Two calls with more chains than chain slots, on two streams at once: the CTAs of the second launch find
-    the SMs taken.  First segments are claimed by whichever CTAs run, so neither launch waits for CTAs that
-    have not started; both must finish with the results of lone calls and a clean status."""
+    """Two calls that each fill the GPU, on two streams at once: the CTAs of the second launch find the SMs taken.  Ranges are
+    numbered by the CTAs as they start, so neither launch waits for CTAs that have not started; both must finish with
+    the results of lone calls and a clean status."""
     probs = [_many_chains(seed) for seed in (2, 3)]
     expect = []
     for d, ws in probs:

@@ -36,7 +36,7 @@ def algo(request):
     return request.param
 
 
-def run_gpu(inp, algo=None, flags=0):
+def run_gpu(inp, algo=None, flags=0, phase_mask=0):
     d = to_device(inp, "cuda")
     w = d["q"]
     n = d["cu_seqlens"].numel() - 1 if d["cu_seqlens"] is not None else w.shape[0]
@@ -44,7 +44,8 @@ def run_gpu(inp, algo=None, flags=0):
                      dtype=torch.uint8, device="cuda")
     flashkda_b200.fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], d["scale"], d["out"], A_log=d["A_log"],
                       dt_bias=d["dt_bias"], lower_bound=d["lower_bound"], initial_state=d["initial_state"],
-                      final_state=d["final_state"], cu_seqlens=d["cu_seqlens"], algo=algo, workspace=ws, flags=flags)
+                      final_state=d["final_state"], cu_seqlens=d["cu_seqlens"], algo=algo, workspace=ws, flags=flags,
+                      phase_mask=phase_mask)
     assert flashkda_b200.device_status(ws) == 0, "a kernel gave up on a bounded wait"
     torch.cuda.synchronize()
     assert flashkda_b200.last_launch_count() > 0
@@ -254,7 +255,7 @@ def test_host_argument_errors_on_gpu():
 
 def test_tensor_core_path_matches_cuda_core_path():
     """Both device implementations share the prepare numerics; the recurrences differ only in the fp32
-    accumulation order inside the contractions (tcgen05.mma vs sequential FMAs), which flips a small
+    accumulation order inside the contractions (mma.sync vs sequential FMAs), which flips a small
     fraction of bf16 roundings."""
     w = Workload("tcv", 2, 2048, 8, state_in="fp32", state_out="fp32")
     inp = make_inputs(w, seed=11)
@@ -268,10 +269,9 @@ def test_tensor_core_path_matches_cuda_core_path():
     assert mism <= 0.05
 
 
-def test_segment_scheduling_many_chains():
-    """More chains than the GPU holds at once (> 444 = 3 per SM): the tensor-core path then schedules
-    segments of chunks and hands the state from one segment to the next through the workspace.  Long and short
-    sequences mixed, so that chains span one to three segments."""
+def test_many_uneven_chains():
+    """500 chains, long and short ones mixed: the one-kernel forward, whose CTAs walk ranges of equal cost that start and end
+    inside chains and hand their states on."""
     gen = torch.Generator().manual_seed(5)
     lens = torch.randint(1, 2500, (100,), generator=gen).tolist()
     lens[7], lens[50], lens[99] = 1, 1024, 3000
@@ -285,7 +285,8 @@ def test_segment_scheduling_many_chains():
     assert oracle.err_ratio(hT2, hT) <= 1e-3
 
 
-def test_segment_scheduling_fixed_batch():
+def test_many_equal_chains():
+    """480 chains of 75 chunks, fp32 states: the one-kernel forward over ranges of a fixed batch."""
     w = Workload("segf", 60, 1200, 8, state_in="fp32", state_out="fp32")
     inp = make_inputs(w, seed=13)
     out, hT = run_gpu(inp, "tc")
@@ -302,26 +303,28 @@ def test_segment_scheduling_fixed_batch():
 
 
 def test_recurrence_kernel_variants_agree():
-    """The tensor-core recurrence has two kernels: three chains per CTA (more chains than SMs) and one chain per
-    CTA with the idle warpgroups sharing the state update (few chains).  Both issue the same tensor-core
-    products in the same order, so their results are identical."""
+    """The tensor-core forward has two forms: one kernel over ranges of chunks (many chains), and a prepare kernel with a
+    recurrence on row slices (few chains).  Both issue the same tensor-core products in the same order, so their results
+    are identical, whichever the dispatch takes."""
     lens = [700, 16, 1, 333, 2048]
     w = Workload("var", 1, sum(lens), 6, state_in="fp32", state_out="fp32", seq_lens=lens)
     inp = make_inputs(w, seed=21)
     ref_out, ref_hT = run_oracle(inp)
-    out_w, hT_w = run_gpu(inp, "tc")                                  # 30 chains: the one-chain-per-CTA kernel
+    out_w, hT_w = run_gpu(inp, "tc")                                  # 30 chains: prefix, prepare, row slices
+    assert flashkda_b200.last_launch_count() == 3
     check_against(out_w, hT_w, ref_out, ref_hT)
-    out_t, hT_t = run_gpu(inp, "tc", flags=_lib.FLAG_NO_WIDE)         # three chains per CTA
+    out_t, hT_t = run_gpu(inp, "tc", flags=_lib.FLAG_NO_WIDE)         # prefix, one kernel
+    assert flashkda_b200.last_launch_count() == 2
     assert torch.equal(out_t, out_w) and torch.equal(hT_t, hT_w)
-    # bf16 states and the segment queue (more than 444 chains), with two forced segment lengths
+    # bf16 states and 480 chains, more row slices than the GPU holds at once
     lens2 = torch.randint(1, 1500, (80,), generator=torch.Generator().manual_seed(3)).tolist()
     w2 = Workload("var2", 1, sum(lens2), 6, state_in="bf16", state_out="bf16", seq_lens=lens2)
     inp2 = make_inputs(w2, seed=22)
     out_a, hT_a = run_gpu(inp2, "tc")
-    out_b, hT_b = run_gpu(inp2, "tc", flags=_lib.flags_seg_chunks(8))
-    out_c, hT_c = run_gpu(inp2, "tc", flags=_lib.flags_seg_chunks(40))
+    assert flashkda_b200.last_launch_count() == 2
+    out_b, hT_b = run_gpu(inp2, "tc", phase_mask=_lib.PHASE_PREPARE | _lib.PHASE_RECURRENCE)
+    assert flashkda_b200.last_launch_count() == 3
     assert torch.equal(out_a, out_b) and torch.equal(hT_a, hT_b)
-    assert torch.equal(out_a, out_c) and torch.equal(hT_a, hT_c)
 
 
 @pytest.mark.parametrize("B,T,H", [(1, 8192, 8), (2, 2100, 4), (1, 1030, 32)])

@@ -1,8 +1,7 @@
 """Seeded random problems (ragged and fixed batches, short and long sequences, all state options): whatever path
-the dispatch picks (decode, fused short-sequence kernel, one-chain-per-CTA kernel with or without the slab pipeline,
-three-chains kernel with or without the segment queue) must give what the plain three-chains kernels give on the
-same inputs, bit for bit (the decode kernel: to its summation-order tolerance), and must agree with the CUDA-core
-implementation within the parity tolerances."""
+the dispatch picks (decode kernel, one-chunk kernel, one-kernel forward, row slices with or without the slab pipeline) must
+give what the plain two-kernel form gives on the same inputs, bit for bit (the decode kernel: to its summation-order
+tolerance), and must agree with the CUDA-core implementation within the parity tolerances."""
 import random
 
 import pytest
@@ -16,7 +15,8 @@ from test_gpu_parity import run_gpu
 
 pytestmark = pytest.mark.gpu
 
-PLAIN = _lib.FLAG_NO_DECODE | _lib.FLAG_NO_SHORT | _lib.FLAG_NO_WIDE | _lib.FLAG_NO_SLABS
+# both stages by name and no one-chunk kernel: prepare and row slices in one launch each
+PLAIN = dict(flags=_lib.FLAG_NO_DECODE | _lib.FLAG_NO_SHORT | _lib.FLAG_NO_SLABS, phase_mask=_lib.PHASE_PREPARE | _lib.PHASE_RECURRENCE)
 
 
 def _random_workload(rng):
@@ -55,7 +55,8 @@ def test_dispatch_paths_agree(seed):
     inp = make_inputs(w, seed=seed)
     out_d, hT_d = run_gpu(inp, "tc")
     launches = flashkda_b200.last_launch_count()
-    out_p, hT_p = run_gpu(inp, "tc", flags=PLAIN)
+    out_p, hT_p = run_gpu(inp, "tc", **PLAIN)
+    assert flashkda_b200.last_launch_count() == (2 if w.seq_lens is None else 3)
     one_token_each = (w.seq_lens is None and w.T == 1) or (w.seq_lens is not None and all(L == 1 for L in w.seq_lens))
     if one_token_each and launches in (1, 5):      # the decode kernel served the call
         assert oracle.err_ratio(out_p, out_d) <= 2e-3

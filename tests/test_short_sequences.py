@@ -81,7 +81,7 @@ def _run_ragged(inp, flags=0):
                       final_state=d["final_state"], cu_seqlens=d["cu_seqlens"], workspace=ws, flags=flags)
     torch.cuda.synchronize()
     assert flashkda_b200.device_status(ws) == 0
-    records_untouched = bool((ws[16384:] == 0xAB).all().item())   # header, prefix tables and queue sit in front
+    records_untouched = bool((ws[16384:] == 0xAB).all().item())   # header and prefix tables sit in front
     return d["out"].cpu(), None if d["final_state"] is None else d["final_state"].cpu(), records_untouched
 
 
@@ -125,12 +125,26 @@ def test_ragged_batch_with_one_longer_sequence_takes_the_general_kernels():
     check_against(out_s, hT_s, ref_out, ref_hT)
 
 
+@pytest.mark.parametrize("state", [None, "bf16", "fp32"])
+def test_longer_sequences_among_many_short_ones(state):
+    """The device decides for the general kernels, in a launch whose CTAs take one row slice after the other (3 200 slices here):
+    sequences of no chunk, one and several in turn, against the two-kernel form with a CTA per slice."""
+    lens = [0, 5, 16, 1, 40, 1, 2, 1] * 25
+    w = Workload("rl", 1, sum(lens), 8, state_in=state, state_out=state, lower_bound=-2.0, seq_lens=lens)
+    inp = make_inputs(w, seed=26)
+    out_s, hT_s, untouched = _run_ragged(inp)
+    assert flashkda_b200.last_launch_count() == 4 and not untouched
+    out_g, hT_g, _ = _run_ragged(inp, flags=_lib.FLAG_NO_SHORT)
+    assert flashkda_b200.last_launch_count() == 3
+    assert torch.equal(out_s, out_g) and (state is None or torch.equal(hT_s, hT_g))
+
+
 def test_ragged_short_batch_without_states_and_many_chains():
     g = torch.Generator().manual_seed(5)
     lens = torch.randint(1, 17, (300,), generator=g).tolist()
-    w = Workload("rm", 1, sum(lens), 8, lower_bound=-1.0, seq_lens=lens)   # 2 400 chains: the segment queue's regime
+    w = Workload("rm", 1, sum(lens), 8, lower_bound=-1.0, seq_lens=lens)   # 2 400 chains: many rounds per CTA
     inp = make_inputs(w, seed=23)
-    out_s, _, _ = _run_ragged(inp)   # (the queue slots of this regime are reset by the host either way)
+    out_s, _, _ = _run_ragged(inp)
     assert flashkda_b200.last_launch_count() == 4
     out_g, _, _ = _run_ragged(inp, flags=_lib.FLAG_NO_SHORT)
     assert torch.equal(out_s, out_g)
