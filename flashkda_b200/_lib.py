@@ -12,10 +12,6 @@ PHASE_PREPARE, PHASE_RECURRENCE = 1, 2
 FLAG_NO_DECODE, FLAG_NO_WIDE, FLAG_NO_SLABS, FLAG_NO_SHORT, FLAG_TEST_DROP_PUSH = 1, 2, 4, 8, 16
 
 
-def flags_seg_chunks(n: int) -> int:
-    return (int(n) & 0xff) << 8
-
-
 def flags_wait_ms(ms: int) -> int:
     return (int(ms) & 0x3fff) << 16
 ALGOS = {"auto": ALGO_AUTO, "twopass": ALGO_TWOPASS, "tc": ALGO_TC}

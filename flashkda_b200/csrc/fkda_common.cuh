@@ -27,8 +27,8 @@ constexpr int kWsMqk = kWsInv + kChunk * kChunk * 2;
 constexpr int kWsRecord = kWsMqk + kChunk * kChunk * 2;  // 13824
 static_assert(kWsRecord == 13824, "workspace record size");
 
-// Record of the tensor-core two-pass workspace: operand tiles in the no-swizzle UMMA canonical
-// layouts (8 x 16-byte "core matrices" of 128 contiguous bytes).  The strides between core matrices are
+// Record of the tensor-core kernels: operand tiles in 8 x 16-byte "core matrices" of 128 contiguous bytes, the matrices
+// that ldmatrix reads.  The strides between core matrices are
 // padded by 16 bytes so that the prepare stage, whose lanes own columns, fills the same tiles in shared
 // memory without bank conflicts and ships them with bulk copies:
 //   B1  [kd; qd] as the K-major B operand [32 rows, K=128]: byte = (k/8)*528 + (r/8)*128 + (r%8)*16 + (k%8)*2
@@ -99,7 +99,6 @@ __device__ __forceinline__ __nv_bfloat16 bfmul(__nv_bfloat16 a, __nv_bfloat16 b)
 __device__ __forceinline__ __nv_bfloat16 bfadd(__nv_bfloat16 a, __nv_bfloat16 b) { return f2bf(bf2f(a) + bf2f(b)); }
 __device__ __forceinline__ __nv_bfloat16 bfsub(__nv_bfloat16 a, __nv_bfloat16 b) { return f2bf(bf2f(a) - bf2f(b)); }
 
-__device__ __forceinline__ float bfbits2f(uint32_t hi16) { return __uint_as_float(hi16 << 16); }
 __device__ __forceinline__ float bf_lo(uint32_t packed) { return __uint_as_float(packed << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t packed) { return __uint_as_float(packed & 0xffff0000u); }
 __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
@@ -179,9 +178,7 @@ __device__ __forceinline__ Frag16 mma16x16_h(const Frag16& a, const Frag16& b) {
 // with fp16 products/accumulators and fp16 additions, result rounded to bf16
 // (csrc/smxx/utils.cuh:262-311; tests/torch_ref.py:221-229).
 // L: the matrix as an mma.sync A / C fragment (what the product that forms it leaves in registers); inv_out:
-// bf16 [16][16], dense row-major (kCanonical = false) or in the UMMA canonical K-major layout (tc_sq_off).
-// All 32 lanes of the warp must call.
-template <bool kCanonical>
+// bf16 [16][16] in core matrices (tc_sq_off).  All 32 lanes of the warp must call.
 __device__ __forceinline__ void neumann_inverse_warp(const Frag16& L, uint8_t* inv_out, int lane) {
     const int g = lane >> 2, t = lane & 3;
     // INV0 = I - L in C-fragment coordinates (register i: row g + 8 (i & 1), columns 2t + 8 (i >> 1), + 1)
@@ -212,8 +209,7 @@ __device__ __forceinline__ void neumann_inverse_warp(const Frag16& L, uint8_t* i
     auto st = [&](int r, int c, uint32_t packed) {
         __half2 h = *reinterpret_cast<__half2*>(&packed);
         float2 f = __half22float2(h);
-        const int off = kCanonical ? tc_sq_off(r, c) : (r * kChunk + c) * 2;
-        *reinterpret_cast<uint32_t*>(inv_out + off) = pack_bf2(f.x, f.y);
+        *reinterpret_cast<uint32_t*>(inv_out + tc_sq_off(r, c)) = pack_bf2(f.x, f.y);
     };
     st(g, 2 * t, inv_c.r[0]);
     st(g + 8, 2 * t, inv_c.r[1]);

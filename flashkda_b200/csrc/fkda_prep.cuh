@@ -301,7 +301,7 @@ __device__ __forceinline__ bool prep_compute(const TwoPassArgs& a, const PrepSrc
             prep_sts(rec + kTcKr + tc_kr_off(8 * hh + i, c), bf2_mul(ki[i].x, etb[0]), bf2_mul(ki[i].y, etb[1]), bf2_mul(ki[i].z, etb[2]),
                      bf2_mul(ki[i].w, etb[3]));
     }
-    neumann_inverse_warp<true>(lfrag, rec_ptr + kTcInv, lane);
+    neumann_inverse_warp(lfrag, rec_ptr + kTcInv, lane);
     __syncwarp();
     return true;
 }

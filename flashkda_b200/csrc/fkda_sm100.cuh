@@ -1,7 +1,5 @@
-// Inline-PTX wrappers for the Blackwell (sm_100a) machinery used by the tensor-core kernels:
-// mbarriers with bounded waits, bulk asynchronous copies (the TMA engine without a tensor map),
-// tensor memory (TMEM) allocation and access, and tcgen05.mma with hand-built shared-memory
-// and instruction descriptors.
+// Inline-PTX wrappers for the sm_100a machinery used by the tensor-core kernels: mbarriers with bounded waits, bulk
+// asynchronous copies (the TMA engine without a tensor map) and tiled copies through a tensor map.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -93,12 +91,9 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ------------------------------------------------------------ proxy fences ----
-// generic-proxy writes to shared memory -> visible to the async proxy (bulk copies, tcgen05.mma)
+// generic-proxy writes to shared memory -> visible to the async proxy (bulk and tiled copies)
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void named_barrier_sync(int id, int n_threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n_threads) : "memory");
 }
 
 // ----------------------------------------------- bulk async copies (1-D TMA) ----
@@ -135,13 +130,6 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, in
         ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
         : "memory");
 }
-// 3-D tile, shared -> global, tracked by the issuing thread's bulk async-group; rows outside the
-// tensor are clipped.
-__device__ __forceinline__ void tma_store_3d(const void* tmap, int c0, int c1, int c2, const void* smem_src) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(tmap),
-                 "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(smem_src))
-                 : "memory");
-}
 // 2-D tiles, as above
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, int c0, int c1, uint64_t* bar) {
     asm volatile(
@@ -152,144 +140,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, in
 __device__ __forceinline__ void tma_store_2d(const void* tmap, int c0, int c1, const void* smem_src) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(tmap), "r"(c0),
                  "r"(c1), "r"(smem_u32(smem_src))
-                 : "memory");
-}
-__device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
-}
-
-// ------------------------------------------------------------------- TMEM ----
-// One full warp allocates `n_cols` (power of two, 32..512) columns; the base address is written to
-// shared memory.  The same warp frees them before the CTA exits.
-__device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t n_cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
-                 "r"(n_cols)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_alloc_permit() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t n_cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(n_cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before_sync() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after_sync() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Each thread of the warp reads its own TMEM lane (lane field of taddr = 32 * (warp % 4)),
-// N consecutive 32-bit columns starting at the column field of taddr.
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-}
-// registers -> 8 consecutive 32-bit columns of the thread's own lane
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3,
-                                         uint32_t r4, uint32_t r5, uint32_t r6, uint32_t r7) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r0),
-                 "r"(r1), "r"(r2), "r"(r3), "r"(r4), "r"(r5), "r"(r6), "r"(r7)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// Fragment-shaped accesses: a warp touches 16 TMEM lanes starting at the lane field of taddr (a multiple of 16
-// inside the warp's own quadrant of 32).  Thread i = 4 g + t of the warp:
-//   16x256b.x2 load:  r0,r1 = (lane g, columns 2t, 2t+1)   r2,r3 = (lane g+8, same columns)
-//                     r4,r5 = (lane g, columns 2t+8, 2t+9) r6,r7 = (lane g+8, same columns)
-//     i.e. 16 fp32 columns arrive as the accumulator fragments of two mma.sync m16n8 tiles;
-//   16x128b.x2 store: r0 -> (lane g, column t), r1 -> (lane g+8, column t), r2 -> (lane g, column t+4),
-//                     r3 -> (lane g+8, column t+4)
-//     i.e. the A fragment {a0,a1,a2,a3} of an mma.sync m16n8k16 (16 rows x 16 bf16 = 8 packed columns) lands as
-//     a K-major tcgen05.mma A operand.
-// (Both mappings were read back on a B200 with a pattern-filling probe.)
-__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_st_16x128b_x2(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-    asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r0), "r"(r1), "r"(r2),
-                 "r"(r3)
-                 : "memory");
-}
-
-// ------------------------------------------------------------ tcgen05.mma ----
-// Shared-memory matrix descriptor, no swizzle ("interleaved" canonical layouts), 16-byte units:
-//   K-major operand  [rows, K]:  byte(r, k) = (r%8)*16 + (r/8)*SBO + (k/8)*LBO + (k%8)*2      (bf16)
-//   MN-major operand [MN, K]:    byte(m, k) = (m%8)*2  + (m/8)*SBO + (k%8)*16 + (k/8)*LBO
-// i.e. "core matrices" of 8 x 16 B = 128 contiguous bytes; one instruction consumes K = 16.
-// Field positions: start address [0,14), LBO [16,30), SBO [32,46) (all >> 4), descriptor version 1 at
-// bit 46, layout type [61,64) = 0 (no swizzle).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr >> 4) & 0x3fffu);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
-// Instruction descriptor for kind::f16 with bf16 A/B and fp32 accumulation:
-// c_format [4,6) = 1 (f32), a_format [7,10) = 1 (bf16), b_format [10,13) = 1 (bf16),
-// a_major bit 15, b_major bit 16 (0 = K-major, 1 = MN-major), N >> 3 at [17,23), M >> 4 at [24,29).
-__host__ __device__ constexpr uint32_t make_idesc_bf16_f32(int M, int N, bool a_mn_major, bool b_mn_major) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) |
-           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.  accumulate = 0 overwrites D.
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand [M = 128 lanes, K = 16] sits in tensor memory, K-major, two
-// 16-bit elements per 32-bit column (8 columns per instruction).  Issued by ONE thread.
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Makes the mbarrier track completion of all tcgen05.mma issued so far by this thread
-// (implies tcgen05.fence::before_thread_sync).
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
 

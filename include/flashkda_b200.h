@@ -109,7 +109,7 @@ enum {
     FKDA_FLAG_TEST_DROP_PUSH = 16  /* TEST ONLY: the one-kernel form does not publish the states it hands over, so that
                                       the waiters starve and their bounded waits give up */
 };
-/* bits 8..15: no effect (once the segment length of a work queue)
+/* bits 8..15: no effect; the macro for them stays for callers that set it
  * bits 16..29: limit of every bounded device-side wait in milliseconds (0 = the default of 2000) */
 #define FKDA_FLAGS_SEG_CHUNKS(x) (((x) & 0xff) << 8)
 #define FKDA_FLAGS_WAIT_MS(x) (((x) & 0x3fff) << 16)
