@@ -57,8 +57,8 @@ def fwd(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state
 
     ``algo`` and ``workspace`` are additions to the reference signature: the implementation
     selector (default from ``$FLASHKDA_B200_ALGO`` or "auto") and an optional caller-owned
-    uint8 scratch tensor of at least ``get_workspace_size(...)`` bytes.  ``phase_mask`` is a
-    measurement aid (see ``fkda_fwd_params.phase_mask``) and ``flags`` selects kernel variants for tests
+    uint8 scratch tensor of at least ``get_workspace_size(...)`` bytes.  ``phase_mask`` runs the
+    two stages of the forward apart (see ``fkda_fwd_params.phase_mask``) and ``flags`` selects kernel variants for tests
     (``fkda_fwd_params.flags``); leave both 0.
 
     ``chunk_states`` (optional, bf16 ``[slots, H, 128, 128]``) receives the state of every sequence before each

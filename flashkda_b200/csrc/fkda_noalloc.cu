@@ -11,8 +11,8 @@
 // loads the library (FKDA_NOALLOC_SCRATCH_BYTES, held until the process exits) and is shared by every
 // call: two calls whose kernels overlap on the GPU (different streams, or different host threads)
 // race on it, so callers must serialise their use of this entry point per device.  The array keeps
-// the previous call's contents; the only part that has to start from zero (the work-queue counter
-// and the device status word in its header) is cleared by every call before the kernels run.
+// the previous call's contents; the only part that has to start from zero (the ticket counter and the
+// device status word in its header) is cleared by every call's first kernel or a memset in front of it.
 #include <atomic>
 
 #include "fkda_internal.h"

@@ -39,8 +39,10 @@ __device__ __forceinline__ bool locate_tile(const TwoPassArgs& a, int64_t tile, 
     return true;
 }
 
-// Warps per CTA: 12 with 168 registers each; 15, as many as have room for a record block, with 128 and spills, 14 % slower
-// per unit, where that makes one round of units out of two (2 176 units: 23 -> 19 us with the prefix kernel).
+// Warps per CTA: 12 with 168 registers each; 15, as many as have room for a record block, with 128 and spills, for 13 to 15 units
+// per SM, where that makes one round of units out of two.  More rounds are not worth it, although there may be one less
+// (us of the stage with 12 and with 15 warps, by units per SM: 12: 14.5 both; 13: 20.6, 16.9; 14: 20.8, 18.4; 15: 21.2, 18.5;
+// 25: 30.0, 31.0; 28: 31.1, 32.6; 30: 32.3, 32.8; 37: 39.9, 43.6; 45: 41.2, 45.1).
 constexpr int kPrepWarps = 12, kPrepWarpsMost = 15;
 
 // The plain record of the CUDA-core recurrence (kWs* layout): kd, qd, kr row-major, INV and Mqk row-major.

@@ -13,9 +13,9 @@
 //   * four preparing warps build the chunk operands of the coming chains in a ring of records (fkda_prep.cuh), the inputs of
 //     their next chain in registers ahead of time.
 // Everything is handed over through mbarriers with bounded waits.
-// Bound by HBM: 32 768 chains of 2 tokens take 344 us with bf16 and 653 us with fp32 states, 0.98 and 1.02 of the copy bandwidth
+// Bound by HBM: 32 768 chains of 2 tokens take 348 us with bf16 and 661 us with fp32 states, 1.01 and 1.05 of the copy bandwidth
 // (554 and 833 us for the predecessor, whose four warps loaded, computed and stored one chain after the other); with 16
-// tokens 472 and 757 us (776, 1 083), where the preparing warps take as long as the states.
+// tokens 476 and 795 us (776, 1 083), where the preparing warps take as long as the states.
 // Numerics and results: those of the chunked kernels on the same inputs (tests/torch_ref.py:153-251 of the reference; the
 // reference itself runs such batches through its two general kernels, csrc/smxx/fwd_kernel1.cuh / fwd_kernel2.cuh).
 #include <cuda.h>

@@ -120,8 +120,7 @@ size_t fkda_workspace_bytes(int64_t T_total, int64_t H, int64_t N, int32_t algo)
 
 /* Scratch bytes THIS call needs (<= fkda_workspace_bytes for the same totals): a fixed batch with at most 16 tokens
  * per sequence (a decode step, T == 1, or a short step, T <= 16) needs nothing (where a workspace is given all the same,
- * its status word is kept), other calls their header,
- * records and queue.  No counterpart in the reference. */
+ * its status word is kept), other calls their header, tables, hand-over states and records.  No counterpart in the reference. */
 size_t fkda_workspace_bytes_for(const fkda_fwd_params* p);
 
 /* Enqueues the forward pass on `stream` (a cudaStream_t passed as void*).
@@ -130,8 +129,10 @@ size_t fkda_workspace_bytes_for(const fkda_fwd_params* p);
  * recurrence on row slices.  For a ragged batch (cu_seqlens) the host knows only the
  * totals: when there are at most 16 tokens per sequence on average (and at least 64 (sequence, head) pairs), a prefix
  * kernel decides on the device whether every sequence has one token, or at most 16, and the kernels of the paths that
- * may apply are all enqueued; those that are not needed return at once.  Results do not depend on the path
- * (the one-token kernel: to the summation order of its dot products). */
+ * may apply are all enqueued; those that are not needed return at once.  Results do not depend on the path, bit for bit,
+ * except for the one-token kernel, which sums its dot products in another order (relative difference below 1e-4).  It
+ * serves decode steps of any size with fp32 states, and of up to 2 048 (sequence, head) pairs with bf16 states: there
+ * the last bits of a sequence's step depend on whether its batch is larger than that. */
 int fkda_fwd(const fkda_fwd_params* p, void* stream);
 
 /* Synchronises `stream`, then reads the device status word that the kernels of the last call
@@ -153,9 +154,9 @@ int fkda_device_status(const void* workspace, void* stream);
  * ignored); the per-chunk scratch comes from a fixed array of FKDA_NOALLOC_SCRATCH_BYTES bytes that
  * every GPU loading this library holds until the process exits.
  *
- * Limit: fkda_workspace_bytes_for(p) must not exceed FKDA_NOALLOC_SCRATCH_BYTES.  With the default
- * algorithm a chunk record takes 14 656 bytes and a (sequence, head) chain 32 KB of hand-over state when
- * the call may be pipelined or queued, so about H * (B*T/16) <= 2 250 chunk records minus 2.2 records per
+ * Limit: fkda_workspace_bytes_for(p) must not exceed FKDA_NOALLOC_SCRATCH_BYTES.  A call that the one-kernel
+ * form serves stays below it whatever its length.  Otherwise, with the default algorithm, a chunk record takes 14 656 bytes and a (sequence, head) chain 32 KB of hand-over state when
+ * the call may be pipelined (fixed batches of up to 58 chains), so about H * (B*T/16) <= 2 250 chunk records minus 2.2 records per
  * chain (algo = twopass: 13 824-byte records, about 2 400); a decode step (T == 1) needs nothing whatever
  * its batch size.  Larger problems return FKDA_ERR_NOALLOC_TOO_LARGE and launch nothing.
  * The call itself performs no cudaMalloc/cudaFree and allocates no device memory through any library.
