@@ -77,7 +77,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches);
 // pause.  The line is where the two cross with bf16 states (2 048 pairs: 30.8 us both, 1 024: 14.4 against 16.8, 32 768: 435
 // against 373); with fp32 states, where the decode kernel's loads are twice as wide, it is the faster one throughout
 // (32 768 pairs: 631 against 671).  The chunk kernel's products are summed in another order: with bf16 states the last bits of a decode
-// step depend on which side of the line the batch is (relative difference 6.5e-5).
+// step depend on which side of the line the batch is (relative difference 6.5e-5), and a state row with an infinity becomes NaN there.
 inline int64_t decode_max_chains(const fkda_fwd_params& p) { return p.state_dtype == FKDA_STATE_FP32 ? 0x7fffffff / 4 : 2048; }
 bool decode_eligible(const fkda_fwd_params& p);
 int launch_decode(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches);
