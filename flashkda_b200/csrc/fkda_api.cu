@@ -89,8 +89,10 @@ int fkda_fwd(const fkda_fwd_params* p, void* stream_v) {
     const int algo = resolve_algo(p->algo);
     if (algo != FKDA_ALGO_TWOPASS && algo != FKDA_ALGO_TC) return FKDA_ERR_BAD_ALGO;
     const size_t need = fkda_workspace_bytes_for(p);
-    if (need > 0 && (p->workspace == nullptr || p->workspace_bytes < need ||
-                     (reinterpret_cast<uintptr_t>(p->workspace) & 255u) != 0))
+    if (need > 0 && p->workspace == nullptr) return FKDA_ERR_WORKSPACE;
+    // (a path that needs none keeps its status word in the header of one that is given)
+    if (p->workspace != nullptr && (p->workspace_bytes < need || p->workspace_bytes < fkda::kWsHeaderBytes ||
+                                    (reinterpret_cast<uintptr_t>(p->workspace) & 255u) != 0))
         return FKDA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
     int launches = 0;

@@ -191,7 +191,8 @@ void fwd_checked(PyObject* const* a) {
     const at::Tensor* ws = optional_tensor_arg(a[14], "workspace");
     c10::DataPtr scratch;   // given back when it goes out of scope; the allocator reuses it in stream order
     if (ws != nullptr) {
-        check(ws->is_cuda() && ws->is_contiguous() && ws->scalar_type() == at::kByte && (size_t)ws->numel() >= need,
+        // (also where none is needed, one that is given has room for the header: the status word goes there)
+        check(ws->is_cuda() && ws->is_contiguous() && ws->scalar_type() == at::kByte && (size_t)ws->numel() >= need && ws->numel() >= 256,
               "workspace must be a contiguous CUDA uint8 tensor of sufficient size");
         p.workspace = ws->data_ptr();
         p.workspace_bytes = (size_t)ws->numel();

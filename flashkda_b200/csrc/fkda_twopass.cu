@@ -296,7 +296,7 @@ void fill_args(const fkda_fwd_params& p, TwoPassArgs* out) {
     uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace);
     a.queue = reinterpret_cast<int32_t*>(base);
     // (a one-kernel path needs no workspace; where the caller gave one, its status word is kept)
-    a.status = base != nullptr && p.workspace_bytes >= kWsHeaderBytes && ((uintptr_t)base & 255u) == 0 ? reinterpret_cast<int32_t*>(base) + 1 : nullptr;
+    a.status = base != nullptr ? reinterpret_cast<int32_t*>(base) + 1 : nullptr;
     a.records = a.status != nullptr ? reinterpret_cast<uint64_t*>(base) + 8 : nullptr;
     a.records_tag = 0;
     a.on_demand = false;

@@ -81,7 +81,8 @@ typedef struct fkda_fwd_params {
     int64_t beta_token_stride; /* elements between consecutive tokens of beta */
     float scale;
     double lower_bound;        /* gate lower bound, -5 <= lower_bound <= 0 */
-    void* workspace;           /* >= fkda_workspace_bytes(B*T, H, N, algo) bytes, 256-byte aligned */
+    void* workspace;           /* >= fkda_workspace_bytes(B*T, H, N, algo) bytes, 256-byte aligned; one that is given holds at
+                                  least the 256-byte header, also where fkda_workspace_bytes_for is 0 */
     size_t workspace_bytes;
     int32_t phase_mask;        /* 0 = whole forward, by whatever kernels serve it best; otherwise a bit set of FKDA_PHASE_*
                                   to run in the two-kernel form (sequences of at most 16 tokens, both bits: as 0).

@@ -62,6 +62,17 @@ def test_null_and_shape_errors_without_gpu():
     assert L.fkda_fwd(p, None) == 1  # A_log / dt_bias missing
 
 
+@pytest.mark.parametrize("T", [1, 16])
+@pytest.mark.parametrize("workspace,workspace_bytes", [(0x10000, 255), (0x10010, 4096)], ids=["small", "misaligned"])
+def test_a_given_workspace_is_checked_also_where_none_is_needed(T, workspace, workspace_bytes):
+    """The status word of a one-chunk call goes into the workspace if there is one; refused before anything is launched."""
+    fake = dict.fromkeys(("q", "k", "v", "g", "beta", "out", "A_log", "dt_bias"), 0x1000)
+    p = _lib.FwdParams(B=1, T=T, H=1, N=1, token_stride=128, beta_token_stride=1, lower_bound=-1.0, workspace=workspace,
+                       workspace_bytes=workspace_bytes, **fake)
+    assert _lib.lib().fkda_workspace_bytes_for(p) == 0
+    assert _lib.lib().fkda_fwd(p, None) == 5
+
+
 def test_host_checks_reject_cpu_tensors():
     inp = make_inputs(Workload("x", 1, 16, 1))
     with pytest.raises(RuntimeError, match="must be on CUDA"):

@@ -52,6 +52,9 @@ def test_short_batch_needs_no_records():
                       final_state=d["final_state"], workspace=ws)
     torch.cuda.synchronize()
     assert flashkda_b200.device_status(ws) == 0 and torch.isfinite(d["out"].float()).all()
+    with pytest.raises(RuntimeError, match="sufficient size"):
+        flashkda_b200.fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], d["scale"], d["out"], A_log=d["A_log"], dt_bias=d["dt_bias"],
+                          lower_bound=d["lower_bound"], workspace=ws[:255])
 
 
 # ---- ragged batches whose sequences all fit one chunk (the device decides: the host sees only the totals) ----
