@@ -338,8 +338,10 @@ def run_ours(a):
     kernel_times = {}
     n_phase = 3
     barrier()
-    decode = w_local.T == 1 and inp.get("cu_seqlens") is None and algo != "twopass" and not (a.flags & 1)
-    short = 2 <= w_local.T <= 16 and inp.get("cu_seqlens") is None and algo != "twopass" and not (a.flags & 8)
+    fixed = inp.get("cu_seqlens") is None and algo != "twopass"
+    # (a decode step with bf16 states and more than 2 048 (sequence, head) pairs: the one-chunk kernel)
+    decode = fixed and w_local.T == 1 and not (a.flags & 1) and ("fp32" in (w.state_in, w.state_out) or w_local.B * w.H <= 2048 or a.flags & 8)
+    short = fixed and 1 <= w_local.T <= 16 and not decode and not (a.flags & 8)
     one_kernel = launches_per_step == (1 if inp.get("cu_seqlens") is None else 2)
     if one_kernel and not cp_mode and a.seq_parts == 1:
         # the library runs ONE kernel (no phases to time apart)
@@ -347,7 +349,7 @@ def run_ours(a):
         kernel_ms = ms_step
         kernel_times[kernel_name] = ms_step
     elif not cp_mode and a.seq_parts == 1:
-        step()
+        step()   # (the recurrence alone also enqueues a prepare launch that returns at once)
         for name, mask in zip(names, (_lib.PHASE_PREPARE, _lib.PHASE_RECURRENCE)):
             p0, p1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             step(mask)
