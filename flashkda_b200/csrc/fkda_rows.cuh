@@ -4,9 +4,16 @@
 // it, and tells the control warp that it is done with the stage.
 //
 // Why this shape: with few chains the forward is a serial walk, (number of chunks) x (latency of a step).  A step is about
-// 115 cycles of dependent latency (u', U, the first update) plus the products of one warp, 52 x 8 cycles of its scheduler's
-// tensor pipe, and four warps put one on each scheduler.  The tcgen05 form of the same step (control warp, accumulators in
-// tensor memory) took 2 100 cycles, of which 1 300 were hand-overs: tensor-memory loads and stores, commits, mbarriers.
+// 115 cycles of dependent latency (u', U, the first update) plus the products of one warp, 52 x 8.5 cycles of its scheduler's
+// tensor pipe, and at most one warp walks on a scheduler.  The tcgen05 form of the same step (control warp, accumulators in
+// tensor memory) took 2 100 cycles, of which 1 300 were hand-overs: tensor-memory loads and stores, commits, mbarriers.  With
+// only the out term's S . qd^T on tcgen05 (the state put into tensor memory block by block, the product started by the control
+// warp, a chunk's out rows stored during the next chunk) a step took 0.46 us against 0.43: eight tcgen05 products and their
+// wait take 300 cycles and slow the mma.sync ones beside them from 8.5 to 10.6 cycles.
+//
+// A stage holds two chunks where shared memory allows it (kPair), which halves the waits, arrivals and branches between chunks
+// (230 of 980 cycles per step were spent there): 131 072 tokens, 32 heads 4.21 -> 3.88 ms together with predicated stores and
+// arrivals and the next chunk's first fragments fetched ahead; 3.75 with products and update strung together (fkda_walk.cuh).
 // Included by fkda_tc.cu.
 #pragma once
 
@@ -14,23 +21,23 @@
 
 namespace fkda {
 
-constexpr int kRowWarps = 4;                      // walking warps per CTA, 16 state rows each
-constexpr int kRowSplit = kD / (16 * kRowWarps);  // CTAs per chain
-constexpr int kRowCols = 16 * kRowWarps;          // value columns (= state rows) of a CTA
-constexpr int kRowThreads = (kRowWarps + 1) * 32;
-constexpr int kRowVBytes = kChunk * kRowCols * 2;              // value tile [16 tokens][64] bf16, 128-byte swizzle
-static_assert(kRowCols == 64 && kRowVBytes % 1024 == 0, "tile alignments");
+// kWarps walking warps per CTA, 16 state rows each: 8 / kWarps CTAs per chain
+__host__ __device__ constexpr int row_split(int warps) { return kD / (16 * warps); }
+__host__ __device__ constexpr int row_threads(int warps) { return (warps + 1) * 32; }
+constexpr int kRowVCols = kD / 2;                               // a CTA of four or fewer warps reads one half of a value row
+constexpr int kRowVBytes = kChunk * kRowVCols * 2;              // value tile [16 tokens][64] bf16, 128-byte swizzle
+static_assert(kRowVBytes % 1024 == 0, "tile alignments");
 
-// Shared memory of a CTA with kStages chunks in flight
-template <int kStages>
+// Shared memory of a CTA with kStages groups of kPair chunks in flight
+template <int kRowWarps, int kStages, int kPair>
 struct RowSmem {
     static constexpr int kV = 0;                                        // value tiles (1024-byte aligned for the swizzle)
-    static constexpr int kOut = kV + kStages * kRowVBytes;              // per warp an out tile [16 tokens][16] bf16
-    static constexpr int kRec = kOut + kRowWarps * 512;                 // chunk records
-    static constexpr int kStaging = kRec + kStages * kTcRecord;         // per warp one staging tile for states
+    static constexpr int kOut = kV + kStages * kPair * kRowVBytes;      // per warp an out tile [16 tokens][16] bf16
+    static constexpr int kRec = kOut + kRowWarps * 512;                    // chunk records
+    static constexpr int kStaging = kRec + kStages * kPair * kTcRecord;   // per warp one staging tile for states
     static constexpr int kCtrl = kStaging + kRowWarps * kWalkStageBytes;
     struct Ctrl {
-        uint64_t full[kStages];    // operands of a chunk have landed (transaction bytes)
+        uint64_t full[kStages];    // operands of a group of chunks have landed (transaction bytes)
         uint64_t empty[kStages];   // a stage has been read by all walking warps
         int32_t abort_flag;
     };
@@ -39,15 +46,18 @@ struct RowSmem {
 };
 
 // kExport: the states before every cs_every-th chunk are written out as well.  kLoop: a CTA takes several slices in turn
-// (for launches that mostly return at once, see launch_tc; the loop alone makes a step 15 % longer).  kRowStages: 8 when every
-// slice has an SM of its own (with the prepare stage of the next slab loading the memory, records arrive up to four steps
-// late: 131 072 tokens, 32 heads: 4.58 -> 4.31 ms against 4 stages), otherwise 4, so that two CTAs fit an SM.
-template <bool kExport, bool kLoop, int kRowStages>
-__global__ void __launch_bounds__(kRowThreads, 2)
+// (for launches that mostly return at once, see launch_tc; the loop alone makes a step 15 % longer).  kRowStages, kPair: 4 stages
+// of two chunks when every slice has an SM of its own (with the prepare stage of the next slab loading the memory, records arrive
+// up to four steps late: 131 072 tokens, 32 heads: 4.58 -> 4.31 ms with 8 chunks in flight against 4), otherwise of one, so that
+// two CTAs fit an SM (with 2 stages of two: 300 + 1 + 211 + 512 tokens of 32 heads 57 us against 51).
+template <bool kExport, bool kLoop, int kRowWarps, int kRowStages, int kPair>
+__global__ void __launch_bounds__(row_threads(kRowWarps), 2)
 recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap map) {
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-    using L = RowSmem<kRowStages>;
+    static_assert(!kLoop || kPair == 1, "slices in turn: a stage of one chunk");
+    constexpr int kRowSplit = row_split(kRowWarps), kRowCols = 16 * kRowWarps;
+    using L = RowSmem<kRowWarps, kRowStages, kPair>;
     typename L::Ctrl& ctl = *reinterpret_cast<typename L::Ctrl*>(sm + L::kCtrl);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
@@ -67,7 +77,7 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
 
     const int64_t n_items = a.N * a.H * kRowSplit;
     bool failed = false;
-    int k0 = 0;   // chunks of the items before: the stages and their phases run on from item to item
+    int k0 = 0;   // groups of the items before: the stages and their phases run on from item to item
     for (int64_t item = blockIdx.x; item < n_items && !failed; item = kLoop ? item + gridDim.x : n_items) {
     // chains come longest first; the second layer of CTAs runs backwards, so that the SMs with the longest chains get the
     // shortest ones beside them (or none)
@@ -82,21 +92,23 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
     if (warp == kRowWarps) {
         // =========================== control warp: keeps the stages filled ===========================
         if (elect_one()) {
-            int t = c0;
-            for (; t < c1; ++t) {
-                const int k = k0 + t - c0, s = k % kRowStages;
+            const int n_groups = (c1 - c0 + kPair - 1) / kPair;
+            int p = 0;
+            for (; p < n_groups; ++p) {
+                const int k = k0 + p, s = k % kRowStages, t = c0 + kPair * p, m = min(kPair, c1 - t);
                 if (k >= kRowStages && !mbar_wait_bounded(&ctl.empty[s], (uint32_t)((k / kRowStages - 1) & 1), abort_flag, a.wait_ns)) {
                     failed = true;
                     break;
                 }
-                mbar_arrive_expect_tx(&ctl.full[s], (uint32_t)(kTcRecord + kRowVBytes));
-                bulk_g2s(sm + L::kRec + s * kTcRecord, ch.rec_base + (int64_t)t * kTcRecord, kTcRecord, &ctl.full[s]);
+                mbar_arrive_expect_tx(&ctl.full[s], (uint32_t)(m * (kTcRecord + kRowVBytes)));
+                bulk_g2s(sm + L::kRec + s * kPair * kTcRecord, ch.rec_base + (int64_t)t * kTcRecord, m * kTcRecord, &ctl.full[s]);
                 // rows past the end of the tensor arrive as zeros; rows of the next sequence are never used
-                tma_load_3d(sm + L::kV + s * kRowVBytes, &map.v, slice * kRowCols, h, (int)(ch.bos + (int64_t)t * kChunk), &ctl.full[s]);
+                for (int e = 0; e < m; ++e)
+                    tma_load_3d(sm + L::kV + (s * kPair + e) * kRowVBytes, &map.v, slice * kRowCols / kRowVCols * kRowVCols, h, (int)(ch.bos + (int64_t)(t + e) * kChunk), &ctl.full[s]);
             }
             if (failed) {   // the copies in flight land before this CTA's shared memory goes
                 *abort_flag = 1;
-                for (int k = max(0, k0 + t - c0 - kRowStages); k < k0 + t - c0; ++k)
+                for (int k = max(0, k0 + p - kRowStages); k < k0 + p; ++k)
                     mbar_wait_bounded(&ctl.full[k % kRowStages], (uint32_t)((k / kRowStages) & 1), nullptr, 100000000ull);
             }
         }
@@ -107,8 +119,8 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         const WalkLane wl = walk_lane(lane);
         uint8_t* stage_tile = sm + L::kStaging + warp * kWalkStageBytes;
         const uint32_t rec0 = smem_u32(sm + L::kRec);
-        // my value columns in the [16 tokens][64] tile: token (lane & 7) + 8 (lane / 16), 16-byte piece 2 warp + (lane / 8) % 2
-        const uint32_t v_off = smem_u32(sm + L::kV) + (uint32_t)(((lane & 7) + 8 * (lane >> 4)) * 128 + (((2 * warp + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+        // my value columns in the [16 tokens][64] tile: token (lane & 7) + 8 (lane / 16), 16-byte piece (my first column) / 8 + (lane / 8) % 2
+        const uint32_t v_off = smem_u32(sm + L::kV) + (uint32_t)(((lane & 7) + 8 * (lane >> 4)) * 128 + (((row0 % kRowVCols / 8 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
         // out tile of my warp, [16 tokens][16] with the two 16-byte pieces of a token swapped in every other group of four:
         // fragments in (token (lane & 7) + 8 (lane / 16), piece (lane / 8) % 2), rows out (token lane / 2, piece lane % 2)
         const int o_tok = (lane & 7) + 8 * (lane >> 4);
@@ -133,55 +145,64 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         } else {
             w.clear();
         }
-        auto full_bar = [&](int i) { return &ctl.full[(k0 + i) % kRowStages]; };
-        auto full_phase = [&](int i) { return (uint32_t)(((k0 + i) / kRowStages) & 1); };
-        auto wait_full = [&](int i) {
-            return __all_sync(0xffffffffu, mbar_wait_bounded(full_bar(i), full_phase(i), abort_flag, a.wait_ns)) != 0;
-        };
+        auto full_phase = [&](int p) { return (uint32_t)(((k0 + p) / kRowStages) & 1); };   // group p of this item
         WalkHead<1> hd;
         int left = (int)min((int64_t)0x7fffffff, ch.seq_len - (int64_t)c0 * kChunk);   // tokens from the current chunk on
-        auto fetch_head = [&](int s, int tokens) {
-            hd.fetch(rec0 + s * kTcRecord, wl);
-            ldmatrix_x4_t(hd.v[0][0], hd.v[0][1], hd.v[0][2], hd.v[0][3], v_off + s * kRowVBytes);
+        auto fetch_head = [&](int slot, int tokens) {   // slot: kPair * stage + chunk of the stage
+            hd.fetch(rec0 + slot * kTcRecord, wl);
+            ldmatrix_x4_t(hd.v[0][0], hd.v[0][1], hd.v[0][2], hd.v[0][3], v_off + slot * kRowVBytes);
             hd.mask(tokens, lane & 3);
         };
         const int n = c1 - c0;
+        int s = k0 % kRowStages;   // stage of the current group
         if (n > 0) {
-            if (!wait_full(0)) failed = true;
+            if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[s], full_phase(0), abort_flag, a.wait_ns)) == 0) failed = true;
             else {
-                w.first(rec0 + k0 % kRowStages * kTcRecord, wl);
-                fetch_head(k0 % kRowStages, left);
+                w.first(rec0 + s * kPair * kTcRecord, wl);
+                fetch_head(s * kPair, left);
             }
         }
-        int s = k0 % kRowStages;   // stage of the current chunk
-        bool ready = false;   // the next chunk's operands have been seen
-        for (int i = 0; i < n && !failed; ++i) {
+        bool ready = false;   // the next group's operands have been seen
+        // Chunk i of the walk, in slot `slot`; `next`: the slot of the chunk after it, or `slot` where there is none.
+        auto step = [&](int i, int slot, int next, auto&& look) {
             if (kExport && (c0 + i) % a.cs_every == 0)   // the state before this group of chunks
                 walk_store_tile(w.s[0], stage_tile, a.chunk_states + ((ch.cs_slot0 + (c0 + i) / a.cs_every) * a.H + h) * (int64_t)(kD * kD) + (int64_t)row0 * kD,
                                 false, lane);
-            const uint32_t rec = rec0 + s * kTcRecord;
-            const int sn = s + 1 == kRowStages ? 0 : s + 1;
-            const bool has_next = i + 1 < n;
-            if (has_next && !ready && !wait_full(i + 1)) { failed = true; break; }
             uint32_t o[1][4];
             uint4 orow;
             const WalkHead<1> cur = hd;
-            w.chunk(rec, has_next ? rec0 + sn * kTcRecord : rec, wl, cur, o, [&](int j) {
-                if (j == 3) fetch_head(has_next ? sn : s, left - kChunk);
-                if (j == 4) ready = __all_sync(0xffffffffu, mbar_test_wait(full_bar(i + 2), full_phase(i + 2))) != 0;
+            w.chunk(rec0 + slot * kTcRecord, rec0 + next * kTcRecord, wl, cur, o, [&](int j) {
+                if (j == 3) fetch_head(next, left - kChunk);
+                if (j == 4) look();
                 // the out rows: fragments through a 512-byte tile, 32 contiguous bytes per token to global memory
                 if (j == 3) {
                     stmatrix_x4_t(o_frag, o[0][0], o[0][1], o[0][2], o[0][3]);
                     __syncwarp();
                 }
                 if (j == 4) orow = lds_u4(o_row);
-                if (j == 6 && (lane >> 1) < left) *reinterpret_cast<uint4*>(og) = orow;
+                if (j == 6) store_if((lane >> 1) < left, og, orow);
             });
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ctl.empty[s]);   // (my warp's last reads of this stage are done)
-            s = sn;
             left -= kChunk;
             og += o_step;
+        };
+#pragma unroll 1
+        for (int i = 0; i < n && !failed; i += kPair) {
+            const int sn = s + 1 == kRowStages ? 0 : s + 1, slot = s * kPair;
+            const int p = i / kPair + 1;   // the next group
+            auto seen = [&](int st, int g) { return __all_sync(0xffffffffu, mbar_test_wait(&ctl.full[st], full_phase(g))) != 0; };
+            const int left_n = n - i;
+            const bool has_next = left_n > kPair;
+            if constexpr (kPair == 2) {
+                step(i, slot, left_n > 1 ? slot + 1 : slot, [&]() { ready = seen(sn, p); });
+                if (left_n == 1) break;
+            }
+            if (has_next && !ready && __all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[sn], full_phase(p), abort_flag, a.wait_ns)) == 0) { failed = true; break; }
+            step(i + kPair - 1, slot + kPair - 1, has_next ? sn * kPair : slot + kPair - 1, [&]() {
+                if (kPair == 1) ready = seen(sn + 1 == kRowStages ? 0 : sn + 1, p + 1);
+            });
+            __syncwarp();
+            mbar_arrive_lane0(&ctl.empty[s], lane);   // (my warp's last reads of this stage are done)
+            s = sn;
         }
         if (!failed) {
             if (c1 < ch.n_chunks) {         // not the last slab
@@ -197,7 +218,7 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
             *abort_flag = 1;   // the other warps leave their waits
         }
     }
-    if constexpr (kLoop) k0 += max(0, c1 - c0);
+    if constexpr (kLoop) k0 += (max(0, c1 - c0) + kPair - 1) / kPair;
     }
     if (failed) atomicExch(a.status, FKDA_ERR_DEVICE_STATUS);
     __syncthreads();   // shared memory stays until every warp, and every copy of the control warp, is done with it

@@ -81,13 +81,14 @@ int device_sm_count() {
     return cache[dev];
 }
 
+constexpr int kRowSplit = row_split(4);   // CTAs per chain of the row-slice kernel, unless there are SMs for more
 constexpr size_t kStateBytes = (size_t)kD * kD * 2;   // a chain's state as bf16 (hand-over buffers)
 
 // Few chains on a fixed batch may run as a slab pipeline (see launch_tc): at least 32 SMs are left beside the row slices.
 static bool slabs_possible(int64_t chains, int sms) { return chains * kRowSplit <= sms - 32; }
 
 // The one-kernel forward serves whole forwards with more than one chunk per chain on average and more row slices than SMs.
-// While every slice has an SM of its own, a step of the row-slice kernel takes 0.52 us against 1.05 us here, which pays for the
+// While every slice has an SM of its own, a step of the row-slice kernel takes 0.45 us against 1.05 us here, which pays for the
 // prepare kernel in front of it (64 chains of 512 chunks: 0.50 ms against 0.57; 96 chains: 0.71 against 0.57).  A ragged batch
 // whose lengths the host does not know may consist of a few long chains, whose walk is then the whole time (128 chains of 1
 // to 32 chunks: 52 us in two kernels against 82): it needs two chains per SM, or 1.6 with more than ten chunks per sequence
@@ -211,7 +212,6 @@ bool encode_state_map(CUtensorMap* m, const void* base, int64_t chains, bool fp3
     const cuuint32_t box[2] = {fp32 ? 32u : 64u, fp32 ? 64u : 128u};
     return encode_map(m, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box);
 }
-static_assert(kRowCols == kD / 2, "a CTA of the row-slice kernel takes one half of a value row");
 
 // What the start and the end of a chain cost a CTA of the one-kernel forward, in chunk steps: the loads and stores of its state,
 // which nothing hides (a chain of c chunks takes 1.2 c + 3.9 us with bf16 states in and out and 1.2 c + 5.7 us with fp32
@@ -246,15 +246,34 @@ static int launch_fused(const fkda_fwd_params& p, TwoPassArgs& a, int sms, cudaS
     if (!(exports ? allow_smem<fused_kernel<true>>(kFusedSmemBytes) : allow_smem<fused_kernel<false>>(kFusedSmemBytes))) return FKDA_ERR_LAUNCH;
     const auto kernel = exports ? fused_kernel<true> : fused_kernel<false>;
     const int64_t ctas = chains < sms ? chains : sms;
-    if (p.cu_seqlens != nullptr) {
-        if (!launch_dependent(kernel, ctas, kFusedThreads, kFusedSmemBytes, stream, a, map)) return FKDA_ERR_LAUNCH;
-    } else {
-        kernel<<<(unsigned)ctas, kFusedThreads, kFusedSmemBytes, stream>>>(a, map);
-    }
-    ++launches;
-    if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
-    *n_launches = launches;
+    if (!launch_dependent(kernel, ctas, kFusedThreads, kFusedSmemBytes, stream, a, map)) return FKDA_ERR_LAUNCH;
+    *n_launches = launches + 1;
     return FKDA_OK;
+}
+
+// The row-slice kernel for a call.
+struct RowsLaunch {
+    void (*kernel)(const TwoPassArgs, const VMap);
+    int smem, threads, split;
+    bool ok;
+};
+template <bool kExport, bool kLoop, int kWarps, int kPair>
+static RowsLaunch rows_launch() {
+    constexpr int kBytes = RowSmem<kWarps, 4, kPair>::kBytes;
+    constexpr auto kKernel = recurrence_rows_kernel<kExport, kLoop, kWarps, 4, kPair>;
+    return RowsLaunch{kKernel, kBytes, row_threads(kWarps), row_split(kWarps), allow_smem<kKernel>(kBytes)};
+}
+// Four CTAs per chain of two warps each instead of two of four, where the SMs last: a step takes 0.43 us against 0.47 (the warps of
+// a CTA share one shared-memory pipe, 8 192 tokens of 8 heads 235 us against 254, 777 tokens of 32 heads 37.6 against 38.9; eight CTAs
+// of one warp: 237 us).  With the prepare stage of the next slab beside it that takes twice as many SMs more as there are chains
+// (8 192 tokens: 16 heads 250 against 257, 32 heads, where the prepare stage comes out of hiding, 380 against 280).
+static RowsLaunch rows_select(const TwoPassArgs& a, int64_t chains, int sms, bool slabs) {
+    if (a.short_flag != nullptr) return rows_launch<false, true, 4, 1>();   // (such a batch exports no states)
+    const bool exports = a.chunk_states != nullptr;
+    if (chains * kRowSplit > sms) return exports ? rows_launch<true, false, 4, 1>() : rows_launch<false, false, 4, 1>();
+    const bool four = slabs ? 4 * chains + 2 * chains <= sms : 4 * chains <= sms;
+    if (four) return exports ? rows_launch<true, false, 2, 2>() : rows_launch<false, false, 2, 2>();
+    return exports ? rows_launch<true, false, 4, 2>() : rows_launch<false, false, 4, 2>();
 }
 
 int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
@@ -286,38 +305,26 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     // A ragged batch whose sequences MAY all fit one chunk (the host sees only the totals): the prefix kernel decides, the
     // one-chunk kernels and the general kernels are all enqueued and all but one return at once.
     if (short_ragged_candidate(p) && !(p.flags & FKDA_FLAG_NO_SHORT)) a.short_flag = a.queue + 8;
-    // every slice has an SM of its own (and the launch is not one that mostly returns at once)
-    const bool roomy = a.short_flag == nullptr && chains * kRowSplit <= sms;
-    const int rows_smem = roomy ? RowSmem<8>::kBytes : RowSmem<4>::kBytes;
-    auto rows_kernel = recurrence_rows_kernel<false, true, 4>;
-    bool smem_ok = true;
-    if (a.short_flag != nullptr) {   // (such a batch exports no states)
-        smem_ok = allow_smem<recurrence_rows_kernel<false, true, 4>>(rows_smem);
-    } else if (a.chunk_states != nullptr) {
-        rows_kernel = roomy ? recurrence_rows_kernel<true, false, 8> : recurrence_rows_kernel<true, false, 4>;
-        smem_ok = roomy ? allow_smem<recurrence_rows_kernel<true, false, 8>>(rows_smem) : allow_smem<recurrence_rows_kernel<true, false, 4>>(rows_smem);
-    } else {
-        rows_kernel = roomy ? recurrence_rows_kernel<false, false, 8> : recurrence_rows_kernel<false, false, 4>;
-        smem_ok = roomy ? allow_smem<recurrence_rows_kernel<false, false, 8>>(rows_smem) : allow_smem<recurrence_rows_kernel<false, false, 4>>(rows_smem);
-    }
-    if (!smem_ok) return FKDA_ERR_LAUNCH;
+    const int64_t tps = (p.T + kChunk - 1) / kChunk;
+    const bool slabs = !varlen && p.phase_mask == 0 && slabs_possible(chains, sms) && tps >= 64 && !(p.flags & FKDA_FLAG_NO_SLABS);
+    const RowsLaunch rows = rows_select(a, chains, sms, slabs);
+    if (!rows.ok) return FKDA_ERR_LAUNCH;
 
     // ---- few chains on a fixed batch: the recurrence is a serial walk on 2 x chains SMs and leaves the others
     //      idle, so the forward is cut into slabs of chunks and the prepare stage of slab i+1 runs on the idle SMs
     //      (side stream) while the recurrence walks slab i; the state of a chain travels through seg_state.
     //      Only stream order and events connect the launches: no kernel waits for another one. ----
-    const int64_t tps = (p.T + kChunk - 1) / kChunk;
-    if (!varlen && p.phase_mask == 0 && slabs_possible(chains, sms) && tps >= 64 && !(p.flags & FKDA_FLAG_NO_SLABS)) {
-        const int idle_sms = sms - (int)chains * kRowSplit;
+    if (slabs) {
+        const int idle_sms = sms - (int)chains * rows.split;
         SlabStreams* ss = slab_streams(dev);
         if (ss == nullptr) return FKDA_ERR_LAUNCH;
         // host threads that call concurrently on one device share the side stream and its events
         std::lock_guard<std::mutex> enqueue_lock(ss->launch_mu);
         // Slab boundaries.  The prepare of slab i+1 (on idle_sms SMs, about 5.8 ns per (chunk, head) on the whole GPU) must
-        // be done when the recurrence (about 0.52 us per chunk) has walked slab i: the slabs grow (or shrink) by the ratio
+        // be done when the recurrence (0.47 us per chunk, 0.43 with four CTAs per chain) has walked slab i: the slabs grow (or shrink) by the ratio
         // of the two speeds (the factor 1.1 measured: 0.9 .. 1.4 tried).  Two or four slabs: more of them leave less of the prepare stage in front of the first one,
         // unhidden, and cost a hand-over of the states and a launch each, about 5 us.
-        const double prep_us = 0.0058 * (double)(chains * tps), walk_us = 0.52 * (double)tps;
+        const double prep_us = 0.0058 * (double)(chains * tps), walk_us = (rows.split == 4 ? 0.43 : 0.47) * (double)tps;
         const double fit = 1.1 * walk_us * (double)idle_sms / (prep_us * (double)sms);
         const double grow = fit < 0.6 ? 0.6 : (fit > 8.0 ? 8.0 : fit);
         int n_slabs = 2;
@@ -354,7 +361,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         for (int i = 0; i < n_slabs; ++i) {
             if (bounds[i + 1] <= bounds[i]) continue;
             if (i > 0 && cudaStreamWaitEvent(stream, ss->done[i], 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
-            rows_kernel<<<(unsigned)(chains * kRowSplit), kRowThreads, rows_smem, stream>>>(slab_args(i), map);
+            rows.kernel<<<(unsigned)(chains * rows.split), rows.threads, rows.smem, stream>>>(slab_args(i), map);
             ++launches;
         }
         if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
@@ -385,13 +392,13 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     }
     if (do_rec) {
         // (behind a device-side decision this launch mostly returns at once: a grid that is resident in one go)
-        int64_t ctas = chains * kRowSplit;
+        int64_t ctas = chains * rows.split;
         if (a.seq_order != nullptr && ctas > sms && ctas <= 2 * sms) a.layer = sms;
         if (a.short_flag != nullptr && ctas > 2 * sms) ctas = 2 * sms;
         if (launches > 0) {
-            if (!launch_dependent(rows_kernel, ctas, kRowThreads, rows_smem, stream, a, map)) return FKDA_ERR_LAUNCH;
+            if (!launch_dependent(rows.kernel, ctas, rows.threads, rows.smem, stream, a, map)) return FKDA_ERR_LAUNCH;
         } else {
-            rows_kernel<<<(unsigned)ctas, kRowThreads, rows_smem, stream>>>(a, map);
+            rows.kernel<<<(unsigned)ctas, rows.threads, rows.smem, stream>>>(a, map);
         }
         ++launches;
     }

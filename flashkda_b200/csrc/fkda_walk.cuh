@@ -56,6 +56,13 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
     return x;
 }
 
+// (predicated: no branch in the middle of a chunk step)
+__device__ __forceinline__ void store_if(bool yes, void* p, const uint4& x) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %0, 0;\n@p st.global.v4.b32 [%1], {%2,%3,%4,%5};\n}\n" ::"r"((int)yes), "l"(p), "r"(x.x),
+                 "r"(x.y), "r"(x.z), "r"(x.w)
+                 : "memory");
+}
+
 // bf(fma(s, e, d)) for a packed pair of state elements
 __device__ __forceinline__ uint32_t update_pair(uint32_t s, const float2& e, float d0, float d1) {
     float y0, y1;
@@ -126,6 +133,7 @@ template <int kMt>
 struct WalkState {
     uint32_t s[kMt][8][4];     // my state rows, A fragments
     float u0[kMt][2][4];       // S . kd^T of the current chunk, token tiles 0 and 1
+    uint32_t qn[2][4];         // qd fragments of the current chunk's first two K steps
 
     __device__ __forceinline__ void clear() {
 #pragma unroll
@@ -162,6 +170,8 @@ struct WalkState {
             fetch_kd(b, rec, wl, j);
             d1_step(u0, b, j);
         }
+        fetch_qd(qn[0], rec, wl, 0);
+        fetch_qd(qn[1], rec, wl, 1);
     }
     // One chunk, record at shared-memory address `rec`, operands of its head in `hd`; S . kd^T of the chunk at `next` is formed
     // on the way (`next` = `rec` when there is none: it is then not used).  `mid(j)` is called after block j of the update:
@@ -173,7 +183,12 @@ struct WalkState {
     // o[mt] = out of tokens 8 (i >> 1) + 2tq, +1 of row g + 8 (i & 1), i = 0 .. 3, complete after block 2.
     template <bool kNext = true, class Mid>
     __device__ __forceinline__ void chunk(uint32_t rec, uint32_t next, const WalkLane& wl, const WalkHead<kMt>& hd, uint32_t (&o)[kMt][4], Mid&& mid) {
-        constexpr int kAhead = 2;   // blocks whose operands (kr, E_tot, kd) are fetched ahead of their products
+        // kStrung: a product takes its pipe for 8.5 cycles and a warp issues in order, so the products of a block are strung together
+        // with the update of the block after it, pair by pair, and neither waits for the other (one row tile per warp, a warp per
+        // scheduler: 131 072 tokens, 32 heads 3.88 -> 3.75 ms).  With two row tiles and the preparing warps beside them (fkda_fused.cuh)
+        // a block's update as one piece is as fast or faster (8 x 32 768 tokens, 64 heads: 8.47 ms against 8.74).
+        constexpr bool kStrung = kMt == 1;
+        constexpr int kAhead = kStrung ? 3 : 2, kAheadB = kStrung ? 2 : 1;   // blocks whose operands (kr and E_tot, kd) are fetched ahead of their products
         uint32_t kr[8][4], b[8][4], q[8][4];
         float2 et[8][2];
         float o0[kMt][2][4];   // S . qd^T
@@ -183,9 +198,16 @@ struct WalkState {
             et[j][1] = lds_f2(rec + wl.et + 64 * j + 32);
         };
 #pragma unroll
-        for (int j = 0; j < 4; ++j) fetch_qd(q[j], rec, wl, j);
+        for (int e = 0; e < 4; ++e) {
+            q[0][e] = qn[0][e];
+            q[1][e] = qn[1][e];
+        }
+        fetch_qd(q[2], rec, wl, 2);
+        fetch_qd(q[3], rec, wl, 3);
         d1_step(o0, q[0], 0);
         d1_step(o0, q[1], 1);
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) fetch_kr(j);
         // ---- u' = (v (-) bf(u0)) (*) bf(beta);  U = bf(u' INV^T) as A fragments (tokens are the K dimension) ----
         uint32_t up[kMt][4], ufr[kMt][4];
 #pragma unroll
@@ -201,9 +223,10 @@ struct WalkState {
             mma_zero(c[mt][0], up[mt], hd.inv[0], hd.inv[1]);
             mma_zero(c[mt][1], up[mt], hd.inv[2], hd.inv[3]);
         }
+        if constexpr (kNext) {
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j) fetch_kr(j);
-        if constexpr (kNext) fetch_kd(b[0], next, wl, 0);
+            for (int j = 0; j < kAheadB; ++j) fetch_kd(b[j], next, wl, j);
+        }
         fetch_qd(q[4], rec, wl, 4);
         fetch_qd(q[5], rec, wl, 5);
         d1_step(o0, q[2], 2);
@@ -223,25 +246,42 @@ struct WalkState {
         };
         dst(0);
         dst(1);
+        fetch_qd(q[6], rec, wl, 6);
+        fetch_qd(q[7], rec, wl, 7);
         d1_step(o0, q[4], 4);
         d1_step(o0, q[5], 5);
+        auto update = [&](int j, int i) {   // pair i of the 4 kMt of block j
+            const int mt = i >> 2, e = i & 3;
+            s[mt][j][e] = update_pair(s[mt][j][e], et[j][e >> 1], d[j][mt][e >> 1][2 * (e & 1)], d[j][mt][e >> 1][2 * (e & 1) + 1]);
+        };
+        if constexpr (kStrung) {
+#pragma unroll
+            for (int i = 0; i < 4 * kMt; ++i) update(0, i);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (j + kAhead < 8) fetch_kr(j + kAhead);
-            if (kNext && j + 1 < 8) fetch_kd(b[j + 1], next, wl, j + 1);
-            if (j == 0) {
-                fetch_qd(q[6], rec, wl, 6);
-                fetch_qd(q[7], rec, wl, 7);
-            }
+            if (kNext && j + kAheadB < 8) fetch_kd(b[j + kAheadB], next, wl, j + kAheadB);
+            if constexpr (kStrung) {
 #pragma unroll
-            for (int mt = 0; mt < kMt; ++mt) {
-                s[mt][j][0] = update_pair(s[mt][j][0], et[j][0], d[j][mt][0][0], d[j][mt][0][1]);
-                s[mt][j][1] = update_pair(s[mt][j][1], et[j][0], d[j][mt][0][2], d[j][mt][0][3]);
-                s[mt][j][2] = update_pair(s[mt][j][2], et[j][1], d[j][mt][1][0], d[j][mt][1][1]);
-                s[mt][j][3] = update_pair(s[mt][j][3], et[j][1], d[j][mt][1][2], d[j][mt][1][3]);
+                for (int i = 0; i < 2 * kMt; ++i) {
+                    if constexpr (kNext) {
+                        if (j == 0) mma_zero(u0[i >> 1][i & 1], s[i >> 1][0], b[0][2 * (i & 1)], b[0][2 * (i & 1) + 1]);
+                        else mma_ord(u0[i >> 1][i & 1], s[i >> 1][j], b[j][2 * (i & 1)], b[j][2 * (i & 1) + 1]);
+                    }
+                    if (j < 7) update(j + 1, i);
+                }
+#pragma unroll
+                for (int i = 0; i < 2 * kMt; ++i) {
+                    if (j + 2 < 8) mma_zero(d[j + 2][i >> 1][i & 1], ufr[i >> 1], kr[j + 2][2 * (i & 1)], kr[j + 2][2 * (i & 1) + 1]);
+                    if (j < 7) update(j + 1, 2 * kMt + i);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4 * kMt; ++i) update(j, i);
+                if constexpr (kNext) d1_step(u0, b[j], j);
+                if (j + 2 < 8) dst(j + 2);
             }
-            if constexpr (kNext) d1_step(u0, b[j], j);
-            if (j + 2 < 8) dst(j + 2);
             if (j == 0) {
                 d1_step(o0, q[6], 6);
                 d1_step(o0, q[7], 7);
@@ -262,6 +302,10 @@ struct WalkState {
                                            pack_bf2(m[mt][i >> 1][2 * (i & 1)], m[mt][i >> 1][2 * (i & 1) + 1]));
             }
             mid(j);
+            if (kNext && j == 5) {   // the next chunk's first products follow this one's last without a wait for their operands
+                fetch_qd(qn[0], next, wl, 0);
+                fetch_qd(qn[1], next, wl, 1);
+            }
         }
     }
 };
