@@ -237,7 +237,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
                 __syncwarp();
                 return true;
             };
-            if (!prep_compute<false>(a, src, len, rec, lane, x, acquire, [] {})) {
+            if (!prep_compute<false, false>(a, src, len, rec, lane, x, acquire, [] {})) {
                 failed = true;
                 *abort_flag = 1;
                 // my value tiles in flight (of my last units, as many as there are slots) land before this CTA's shared memory goes

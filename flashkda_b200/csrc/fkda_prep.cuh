@@ -125,6 +125,26 @@ __device__ __forceinline__ void prep_row_norms(float q, float k, int lane, float
     *ki = up ? v : o;
 }
 
+// 1 / norm of two rows of q and of k from my partial sums of squares, over the 16 lanes of a row.  The first two butterfly steps
+// also split the four sums among the lanes of a row (the sums are those of a plain butterfly: every step adds the same two
+// numbers, whichever lane keeps the result).
+__device__ __forceinline__ void prep_two_norms(const float (&q)[2], const float (&k)[2], int lane, float (&qi)[2], float (&ki)[2]) {
+    const bool up = (lane & 8) != 0, second = (lane & 4) != 0;
+    const float r0 = __shfl_xor_sync(0xffffffffu, up ? q[0] : k[0], 8), r1 = __shfl_xor_sync(0xffffffffu, up ? q[1] : k[1], 8);
+    const float v0 = __fadd_rn(up ? k[0] : q[0], r0), v1 = __fadd_rn(up ? k[1] : q[1], r1);
+    float v = __fadd_rn(second ? v1 : v0, __shfl_xor_sync(0xffffffffu, second ? v0 : v1, 4));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+    v = rsqrt_approx(__fadd_rn(v, 1e-6f));
+    const float w = __shfl_xor_sync(0xffffffffu, v, 4);   // my tensor's other row
+    const float m0 = second ? w : v, m1 = second ? v : w;
+    const float o0 = __shfl_xor_sync(0xffffffffu, m0, 8), o1 = __shfl_xor_sync(0xffffffffu, m1, 8);
+    qi[0] = up ? o0 : m0;
+    qi[1] = up ? o1 : m1;
+    ki[0] = up ? m0 : o0;
+    ki[1] = up ? m1 : o1;
+}
+
 // gate_scale * sigmoid(exp(A_log) * (g + dt_bias)) of two columns, added to their running sum.  sigmoid(x) = tanh(x/2)/2 + 1/2;
 // the halving of x is exact and folded into the factor `ae`.  (The last product is scalar: a packed one followed by the packed
 // sum is contracted into one FMA and loses a rounding.)
@@ -141,7 +161,11 @@ __device__ __forceinline__ f2_t prep_add_gate(f2_t run, uint32_t g, f2_t dt, f2_
 // unit's inputs are used up, before the products: it may load the next unit's head into `x`.
 // kFewRows: units of 8 tokens or fewer are common, their missing rows are skipped (the code for it costs the others 2 %, and
 // the walking warps beside them in fkda_fused.cuh 20 % in registers).
-template <bool kFewRows, class Acquire, class Next>
+// kPaired: the norms of two rows are formed side by side.  A row's norm is a chain of latencies (eight products, five shuffles, the
+// reciprocal root), and the shuffles of a row wait behind the stores of the row before it.  It pays in the kernel that only prepares
+// (8 192 tokens, 32 heads, whole forward 275 -> 266 us; 1 000 tokens 47.3 -> 45.1); beside walking warps its registers cost more
+// (fkda_short.cu: 512 x 16 tokens, 64 heads 489 -> 551 us; fkda_fused.cuh: 3 to 7 % slower).
+template <bool kFewRows, bool kPaired, class Acquire, class Next>
 __device__ __forceinline__ bool prep_compute(const TwoPassArgs& a, const PrepSrc& src, int len, uint8_t* rec_ptr, int lane, PrepHead& x,
                                              Acquire&& acquire, Next&& next) {
     const uint32_t rec = sm100::smem_u32(rec_ptr);
@@ -182,6 +206,21 @@ __device__ __forceinline__ bool prep_compute(const TwoPassArgs& a, const PrepSrc
     const int rows = !kFewRows || len > 8 ? 8 : (len + 1) & ~1;   // rows of each half that are gone through
 #pragma unroll 1
     for (int ib = 0; ib < rows; ib += 2) {
+        float q_norm[2], k_norm[2];
+        if constexpr (kPaired) {
+            float qs[2] = {0.0f, 0.0f}, ks[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t k = (&x.row[u].k.x)[p], q = (&x.row[u].q.x)[p];
+                    qs[u] = __fmaf_rn(bf_lo(q), bf_lo(q), qs[u]);
+                    ks[u] = __fmaf_rn(bf_lo(k), bf_lo(k), ks[u]);
+                    qs[u] = __fmaf_rn(bf_hi(q), bf_hi(q), qs[u]);
+                    ks[u] = __fmaf_rn(bf_hi(k), bf_hi(k), ks[u]);
+                }
+            prep_two_norms(qs, ks, lane, q_norm, k_norm);
+        }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int i = ib + u;
@@ -190,16 +229,21 @@ __device__ __forceinline__ bool prep_compute(const TwoPassArgs& a, const PrepSrc
             const uint32_t qq[4] = {x.row[u].q.x, x.row[u].q.y, x.row[u].q.z, x.row[u].q.w};
             const uint32_t gg[4] = {x.row[u].g.x, x.row[u].g.y, x.row[u].g.z, x.row[u].g.w};
             if (ib < 6) prep_load_row(src, i + 2, x.row[u]);   // two rows ahead of their use
-            float qs = 0.0f, ks = 0.0f;
-#pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                qs = __fmaf_rn(bf_lo(qq[p]), bf_lo(qq[p]), qs);
-                ks = __fmaf_rn(bf_lo(kk[p]), bf_lo(kk[p]), ks);
-                qs = __fmaf_rn(bf_hi(qq[p]), bf_hi(qq[p]), qs);
-                ks = __fmaf_rn(bf_hi(kk[p]), bf_hi(kk[p]), ks);
-            }
             float qi, kj;
-            prep_row_norms(qs, ks, lane, &qi, &kj);
+            if constexpr (kPaired) {
+                qi = q_norm[u];
+                kj = k_norm[u];
+            } else {
+                float qs = 0.0f, ks = 0.0f;
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    qs = __fmaf_rn(bf_lo(qq[p]), bf_lo(qq[p]), qs);
+                    ks = __fmaf_rn(bf_lo(kk[p]), bf_lo(kk[p]), ks);
+                    qs = __fmaf_rn(bf_hi(qq[p]), bf_hi(qq[p]), qs);
+                    ks = __fmaf_rn(bf_hi(kk[p]), bf_hi(kk[p]), ks);
+                }
+                prep_row_norms(qs, ks, lane, &qi, &kj);
+            }
             qi = valid ? qi : 0.0f;
             kj = valid ? kj : 0.0f;
             const float gs = valid ? a.gate_scale : 0.0f;

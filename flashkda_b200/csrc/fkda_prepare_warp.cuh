@@ -39,8 +39,8 @@ __device__ __forceinline__ bool locate_tile(const TwoPassArgs& a, int64_t tile, 
     return true;
 }
 
-// Warps per CTA: 12 with 168 registers each; 15, as many as have room for a record block, with 128 and spills, for 13 to 15 units
-// per SM, where that makes one round of units out of two.  More rounds are not worth it, although there may be one less
+// Warps per CTA: 12 with 168 registers each; 15, as many as have room for a record block, with 128, for 13 to 15 units per SM, where
+// that makes one round of units out of two (so its warps take one unit each, with no next one to ask for and no spills).  More rounds are not worth it, although there may be one less
 // (us of the stage with 12 and with 15 warps, by units per SM: 12: 14.5 both; 13: 20.6, 16.9; 14: 20.8, 18.4; 15: 21.2, 18.5;
 // 25: 30.0, 31.0; 28: 31.1, 32.6; 30: 32.3, 32.8; 37: 39.9, 43.6; 45: 41.2, 45.1).
 constexpr int kPrepWarps = 12, kPrepWarpsMost = 15;
@@ -106,17 +106,18 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) prepare_warp_kernel(const _
         src = prep_src(a, t0, len, h, lane);
         prep_load(a, src, t0, len, h, lane, x);
     }
+    constexpr bool kOneRound = kMaxWarps == kPrepWarpsMost;   // one unit per warp (see launch_prepare_warp)
     while (valid) {
-        const bool next_valid = locate(u + stride, &tile_n, &t0n, &lenn, &hn);
+        const bool next_valid = !kOneRound && locate(u + stride, &tile_n, &t0n, &lenn, &hn);
         uint8_t* ws = a.workspace + ((int64_t)h * a.total_tiles + tile) * (int64_t)(kTc ? kTcRecord : kWsRecord);
-        prep_compute<false>(a, src, len, rec, lane, x,
+        prep_compute<false, true>(a, src, len, rec, lane, x,
                      [&]() {   // the previous record has left the block
                          if (kTc && lane == 0) sm100::bulk_wait_group_read<0>();
                          __syncwarp();
                          return true;
                      },
                      [&]() {   // the head of the next unit travels while the products and the inverse run
-                         if (next_valid) {
+                         if (!kOneRound && next_valid) {
                              src = prep_src(a, t0n, lenn, hn, lane);
                              prep_load(a, src, t0n, lenn, hn, lane, x);
                          }

@@ -187,7 +187,7 @@ short_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ Shor
                     prep_load(a, src, t0n, max(lenn, 1), hn, lane, x);
                 }
             };
-            if (!prep_compute<true>(a, src, len, rec, lane, x, acquire, next)) {
+            if (!prep_compute<true, false>(a, src, len, rec, lane, x, acquire, next)) {
                 failed = true;
                 *abort_flag = 1;
                 // my value tile in flight lands before this CTA's shared memory goes
