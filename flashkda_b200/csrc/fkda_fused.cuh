@@ -8,8 +8,8 @@
 //   * warpgroups 1, 2: eight preparing warps; warp w builds the records of the CTA's chunks w, w + 8, ... in a ring of
 //     kFusedSlots blocks (fkda_prep.cuh), asks for the value tile and leaves a note on where the chunk belongs, so that the
 //     walking warps spend nothing on addresses.  Chunks are handed over through mbarriers, slot by slot.
-// Register shares: the walkers keep 216 registers per thread, the preparing warps 144 (128 x 216 + 256 x 144 = 384 x 168, what
-// the CTA is launched with).
+// Register shares: the walkers keep 232 registers per thread, the preparing warps 136 (128 x 232 + 256 x 136 = 384 x 168, what
+// the CTA is launched with; 216 and 144: 1 % slower, 240 and 128: 2 to 3 %, 200 and 152: 1 to 3 %, 184 and 160: 12 %).
 //
 // Work split: the chunks of all chains form one line, chain after chain, cut into ranges of equal cost, one per CTA.  (Equal
 // numbers of chunks leave the ranges with many short chains far behind: 640 chains of 1 to 16 chunks 110 us against 64, 3 200
@@ -192,7 +192,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
 
     if (warp >= kFusedWalkers) {
         // =========================== preparing warps ===========================
-        reg_dealloc<144>();
+        reg_dealloc<136>();
         FusedSeq sq;          // the sequence of the current unit
         sq.begin = sq.end = sq.n_chunks = -1;
         int h = 0, t = 0;     // its head and chunk
@@ -249,7 +249,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
         }
     } else {
         // =========================== walking warps ===========================
-        reg_alloc<216>();
+        reg_alloc<232>();
         const int row0 = warp * kFusedCols;   // my first state row
         const WalkLane wl = walk_lane(lane);
         uint8_t* stage_tile = sm + kFusedStaging + warp * kWalkStageBytes;
@@ -261,10 +261,15 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
         for (int mt = 0; mt < kFusedMt; ++mt)
             v_off[mt] = smem_u32(sm + kFusedV) + (uint32_t)((warp >> 1) * (kFusedVTile / 2) + v_tok * 128 +
                                                             (((4 * (warp & 1) + 2 * mt + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
-        // out tiles as in recurrence_rows_kernel, one per row tile
+        // out tile of my warp, [16 tokens][32], 64 bytes per token with its 16-byte pieces permuted by the token: fragments of row tile
+        // mt in (token v_tok, piece 2 mt + (lane / 8) % 2), rows out eight tokens at a time (token lane / 4, piece lane % 4), so that a
+        // store touches eight lines, not sixteen (each takes a pass through the L1 of its own)
         const uint32_t o_tile = smem_u32(sm + kFusedOut + warp * kFusedMt * 512);
-        const uint32_t o_frag = o_tile + (uint32_t)(v_tok * 32 + ((((lane >> 3) & 1) ^ ((v_tok >> 2) & 1)) << 4));
-        const uint32_t o_row = o_tile + (uint32_t)((lane >> 1) * 32 + (((lane & 1) ^ ((lane >> 3) & 1)) << 4));
+        auto o_piece = [&](int tok, int piece) { return o_tile + (uint32_t)(tok * 64 + ((piece ^ ((tok >> 1) & 3)) << 4)); };
+        uint32_t o_frag[kFusedMt];
+#pragma unroll
+        for (int mt = 0; mt < kFusedMt; ++mt) o_frag[mt] = o_piece(v_tok, 2 * mt + ((lane >> 3) & 1));
+        const uint32_t o_row = o_piece(lane >> 2, lane & 3);   // tokens 8 .. 15: 512 bytes further (the same permutation)
         const int64_t o_step = kChunk * a.token_stride;
 
         WalkState<kFusedMt> w;
@@ -305,7 +310,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
             // ---- the piece's chunks ----
             const int64_t cs_slot0 = kExport ? cs_first_slot(a, pc.n) : 0;
             int left = pc.left;   // tokens from the current chunk on
-            __nv_bfloat16* og = a.out + (pc.tok0 + (lane >> 1)) * a.token_stride + (int64_t)pc.h * kD + row0 + 8 * (lane & 1);
+            __nv_bfloat16* og = a.out + (pc.tok0 + (lane >> 2)) * a.token_stride + (int64_t)pc.h * kD + row0 + 8 * (lane & 3);
             auto fetch_head = [&](int sl, int tokens) {
                 hd.fetch(rec0 + sl * kTcRecord, wl);
 #pragma unroll
@@ -333,24 +338,24 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
                 uint32_t p2 = pn;
                 if (s2 == kFusedSlots) { s2 = 0; p2 ^= 1u; }
                 uint32_t o[kFusedMt][4];
-                uint4 orow[kFusedMt];
+                uint4 orow[2];
                 const WalkHead<kFusedMt> cur = hd;
                 w.chunk(rec, has_next ? rec0 + sn * kTcRecord : rec, wl, cur, o, [&](int j) {
                     if (j == 3) {
                         fetch_head(has_next ? sn : slot, left - kChunk);
-                        // the out rows: fragments through a 512-byte tile, 32 contiguous bytes per token to global memory
+                        // the out rows: fragments through the tile, 64 contiguous bytes per token to global memory
 #pragma unroll
-                        for (int mt = 0; mt < kFusedMt; ++mt) stmatrix_x4_t(o_frag + mt * 512, o[mt][0], o[mt][1], o[mt][2], o[mt][3]);
+                        for (int mt = 0; mt < kFusedMt; ++mt) stmatrix_x4_t(o_frag[mt], o[mt][0], o[mt][1], o[mt][2], o[mt][3]);
                         __syncwarp();
                     }
                     if (j == 4) {
                         ready = __all_sync(0xffffffffu, mbar_test_wait(&ctl.full[s2], p2)) != 0;
 #pragma unroll
-                        for (int mt = 0; mt < kFusedMt; ++mt) orow[mt] = lds_u4(o_row + mt * 512);
+                        for (int i = 0; i < 2; ++i) orow[i] = lds_u4(o_row + i * 512);
                     }
-                    if (j == 6 && (lane >> 1) < left) {
+                    if (j == 6) {
 #pragma unroll
-                        for (int mt = 0; mt < kFusedMt; ++mt) *reinterpret_cast<uint4*>(og + mt * 16) = orow[mt];
+                        for (int i = 0; i < 2; ++i) store_if((lane >> 2) + 8 * i < left, og + i * 8 * a.token_stride, orow[i]);
                     }
                 });
                 __syncwarp();
