@@ -60,6 +60,7 @@ __device__ __forceinline__ float warp_rows_reduce(float (&x)[kRows], int lane) {
 }
 
 __global__ void __launch_bounds__(128, 4) decode_kernel(const __grid_constant__ TwoPassArgs a) {
+    grid_dep_launch();   // (the next step's launch travels during this one)
     grid_dep_wait();
     // a ragged batch with as many tokens as sequences: mine only if the prefix kernel found one token in each (then
     // sequence n is token n, as in a fixed batch)
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(128, 4) decode_kernel(const __grid_constant__ 
     }
 }
 
-int launch_decode_ragged(const TwoPassArgs& a, cudaStream_t stream) {
+int launch_decode_kernel(const TwoPassArgs& a, cudaStream_t stream) {
     const int64_t chains = a.N * a.H;
     if (chains > 0x7fffffff / kSplit) return FKDA_ERR_BAD_SHAPE;
     return launch_dependent(decode_kernel, chains * kSplit, 128, 0, stream, a) ? FKDA_OK : FKDA_ERR_LAUNCH;
@@ -198,12 +199,9 @@ int launch_decode_ragged(const TwoPassArgs& a, cudaStream_t stream) {
 int launch_decode(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     TwoPassArgs a;
     fill_args(p, &a);
-    const int64_t chains = p.N * p.H;
-    if (chains > 0x7fffffff / kSplit) return FKDA_ERR_BAD_SHAPE;
-    decode_kernel<<<(unsigned)(chains * kSplit), 128, 0, stream>>>(a);
-    if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
-    *n_launches = 1;
-    return FKDA_OK;
+    const int rc = launch_decode_kernel(a, stream);
+    if (rc == FKDA_OK) *n_launches = 1;
+    return rc;
 }
 
 }  // namespace fkda

@@ -91,7 +91,7 @@ int launch_short_ragged(const fkda_fwd_params& p, const TwoPassArgs& a, cudaStre
 // Tensor maps over v and over the states (fkda_tc.cu).
 bool encode_v_map(CUtensorMap* m, const fkda_fwd_params& p);
 bool encode_state_map(CUtensorMap* m, const void* base, int64_t chains, bool fp32);
-int launch_decode_ragged(const TwoPassArgs& a, cudaStream_t stream);   // as many tokens as sequences: maybe one each
+int launch_decode_kernel(const TwoPassArgs& a, cudaStream_t stream);   // (a ragged batch: as many tokens as sequences, maybe one each)
 
 // Allows a kernel its dynamic shared memory on the current device.  The attribute belongs to the function and the device,
 // so it is set once for each and remembered (a driver call on every launch is half a microsecond of host time).
@@ -107,8 +107,10 @@ inline bool allow_smem(int bytes) {
     return true;
 }
 
-// Launches a kernel that begins with grid_dep_wait() (fkda_common.cuh) behind the previous kernel of the same call: its launch
-// and start overlap that kernel's end.
+// Launches a kernel that begins with grid_dep_wait() (fkda_common.cuh) behind whatever kernel is in front of it on the stream,
+// of the same call, the call before or the caller's own: its launch and start overlap that kernel's end, and nothing of it
+// touches memory before that end.  (One token of 32 heads, steps back to back: 4.1 -> 3.1 us; a prompt of 100 tokens, 8 heads:
+// 12.3 -> 11.2; 4 x 1 tokens of 32 heads: 6.2 -> 4.5.)
 template <typename... KernelArgs, typename... Args>
 inline bool launch_dependent(void (*kernel)(KernelArgs...), int64_t ctas, int threads, int smem, cudaStream_t stream, const Args&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -130,7 +132,7 @@ void fill_args(const fkda_fwd_params& p, TwoPassArgs* a);
 // The prefix kernel of a ragged batch: chunk (and state-export) prefix tables, the length order if asked for, and the path
 // decision if a.short_flag is set; clears the header (the note on the records only if the call is going to write new ones
 // or none) and `n_flags` range flags.
-void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags = 0);
+bool launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags = 0);
 // First state-export slot of sequence n.
 __device__ __forceinline__ int64_t cs_first_slot(const TwoPassArgs& a, int64_t n) {
     if (a.cu_seqlens != nullptr) return a.cs_prefix[n];

@@ -374,8 +374,7 @@ static int launch_short_typed(const fkda_fwd_params& p, const TwoPassArgs& a, in
         return launch_dependent(short_kernel<kFp32, true>, ctas, kShortThreads, kShortSmemBytes, stream, a, maps) ? FKDA_OK : FKDA_ERR_LAUNCH;
     }
     if (!allow_smem<short_kernel<kFp32, false>>(kShortSmemBytes)) return FKDA_ERR_LAUNCH;
-    short_kernel<kFp32, false><<<(unsigned)ctas, kShortThreads, kShortSmemBytes, stream>>>(a, maps);
-    return cudaGetLastError() == cudaSuccess ? FKDA_OK : FKDA_ERR_LAUNCH;
+    return launch_dependent(short_kernel<kFp32, false>, ctas, kShortThreads, kShortSmemBytes, stream, a, maps) ? FKDA_OK : FKDA_ERR_LAUNCH;
 }
 
 int launch_short_ragged(const fkda_fwd_params& p, const TwoPassArgs& a, cudaStream_t stream) {

@@ -235,7 +235,7 @@ static int launch_fused(const fkda_fwd_params& p, TwoPassArgs& a, int sms, cudaS
     a.seg_state = reinterpret_cast<uint32_t*>(base + ws_prefix_bytes(p.N) + fused_flag_bytes(sms));
     int launches = 0;
     if (p.cu_seqlens != nullptr) {
-        launch_tile_prefix(a, nullptr, false, stream, sms);
+        if (!launch_tile_prefix(a, nullptr, false, stream, sms)) return FKDA_ERR_LAUNCH;
         ++launches;
     } else if (cudaMemsetAsync(p.workspace, 0, kWsHeaderBytes + (size_t)sms * 4, stream) != cudaSuccess) {
         return FKDA_ERR_LAUNCH;
@@ -348,7 +348,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
             x.slab_chunks = bounds[i + 1] - bounds[i];
             return x;
         };
-        if (launch_prepare_warp<true>(slab_args(0), stream) != FKDA_OK) return FKDA_ERR_LAUNCH;
+        if (launch_prepare_warp<true>(slab_args(0), stream, 0, true) != FKDA_OK) return FKDA_ERR_LAUNCH;
         ++launches;
         if (cudaEventRecord(ss->fork, stream) != cudaSuccess || cudaStreamWaitEvent(ss->side, ss->fork, 0) != cudaSuccess)
             return FKDA_ERR_LAUNCH;
@@ -375,11 +375,11 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     // none (the one-kernel forms), so the tables of a ragged batch are made again and the prepare stage is enqueued in any
     // case: it returns at once where the records are there.
     if (varlen && tables) {
-        launch_tile_prefix(a, const_cast<int32_t*>(a.seq_order), try_decode, stream);
+        if (!launch_tile_prefix(a, const_cast<int32_t*>(a.seq_order), try_decode, stream)) return FKDA_ERR_LAUNCH;
         ++launches;
     }
     if (try_decode) {
-        if (launch_decode_ragged(a, stream) != FKDA_OK) return FKDA_ERR_LAUNCH;
+        if (launch_decode_kernel(a, stream) != FKDA_OK) return FKDA_ERR_LAUNCH;
         ++launches;
     }
     if (a.short_flag != nullptr) {
@@ -387,7 +387,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
         ++launches;
     }
     if (a.total_tiles > 0 && tables) {
-        if (launch_prepare_warp<true>(a, stream, 0, varlen) != FKDA_OK) return FKDA_ERR_LAUNCH;
+        if (launch_prepare_warp<true>(a, stream, 0, true) != FKDA_OK) return FKDA_ERR_LAUNCH;
         ++launches;
     }
     if (do_rec) {

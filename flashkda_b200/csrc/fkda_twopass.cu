@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __rest
                                                            int32_t* __restrict__ header, int keep_records, int32_t* __restrict__ flags,
                                                            int n_flags) {
     grid_dep_launch();
+    grid_dep_wait();   // (the call before may still read its tables)
     __shared__ int64_t part[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < 8) header[tid] = 0;   // ticket counter, device status
@@ -253,10 +254,10 @@ __global__ void __launch_bounds__(128) recurrence_kernel(TwoPassArgs a) {
 // ---------------------------------------------------------------------------------
 // host launcher
 // ---------------------------------------------------------------------------------
-void launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags) {
-    tile_prefix_kernel<<<1, 1024, 0, stream>>>(a.cu_seqlens, a.N, a.tile_prefix, seq_order,
-                                               a.chunk_states != nullptr ? const_cast<int32_t*>(a.cs_prefix) : nullptr, 16 * a.cs_every,
-                                               a.short_flag, decode_enqueued ? 1 : 0, a.queue, a.on_demand ? 1 : 0, a.range_flags, n_flags);
+bool launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags) {
+    return launch_dependent(tile_prefix_kernel, 1, 1024, 0, stream, a.cu_seqlens, a.N, a.tile_prefix, seq_order,
+                            a.chunk_states != nullptr ? const_cast<int32_t*>(a.cs_prefix) : (int32_t*)nullptr, 16 * (int)a.cs_every, a.short_flag,
+                            decode_enqueued ? 1 : 0, a.queue, a.on_demand ? 1 : 0, a.range_flags, n_flags);
 }
 
 size_t twopass_workspace_bytes(int64_t T_total, int64_t H, int64_t N) {
@@ -322,7 +323,7 @@ int launch_twopass(const fkda_fwd_params& p, cudaStream_t stream, int* n_launche
     const bool do_prep = p.phase_mask == 0 || (p.phase_mask & FKDA_PHASE_PREPARE);
     const bool do_rec = p.phase_mask == 0 || (p.phase_mask & FKDA_PHASE_RECURRENCE);
     if (varlen && do_prep) {
-        launch_tile_prefix(a, nullptr, false, stream);
+        if (!launch_tile_prefix(a, nullptr, false, stream)) return FKDA_ERR_LAUNCH;
         ++launches;
     }
     if (a.total_tiles > 0 && do_prep) {
