@@ -178,6 +178,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
         }
         ctl.abort_flag = 0;
         mbar_fence_init();
+        tma_prefetch_map(&map.v);
     }
     grid_dep_wait();
     if (threadIdx.x == 0) ctl.range = atomicAdd(a.queue, 1);

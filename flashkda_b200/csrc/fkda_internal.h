@@ -49,6 +49,7 @@ struct TwoPassArgs {
     int32_t cs_every;
     uint64_t wait_ns;      // limit of every bounded device-side wait (mbarrier, range flag)
     bool state_fp32;
+    bool early_rows;       // the row slices behind the prepare stage take an SM each: their CTAs may come in while it still runs
     bool test_drop_push;   // test hook (FKDA_FLAG_TEST_DROP_PUSH): ranges do not publish the state they hand over
 };
 

@@ -64,7 +64,8 @@ __device__ __forceinline__ void prep_export_plain(uint8_t* ws, const uint8_t* re
 
 template <bool kTc, int kMaxWarps>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1) prepare_warp_kernel(const __grid_constant__ TwoPassArgs a) {
-    // (no early grid_dep_launch(): the recurrence's CTAs would fill the first SMs that fall free two by two)
+    // (otherwise the recurrence's CTAs would fill the first SMs that fall free two by two)
+    if (a.early_rows) grid_dep_launch();
     grid_dep_wait();
     // the first launch of a fixed batch's forward clears the device status (the prefix kernel that of a ragged batch)
     if (a.cu_seqlens == nullptr && a.slab_c0 == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;

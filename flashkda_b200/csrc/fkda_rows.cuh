@@ -69,6 +69,7 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         }
         ctl.abort_flag = 0;
         mbar_fence_init();
+        tma_prefetch_map(&map.v);
     }
     grid_dep_wait();
     // (a ragged batch that a one-kernel path has served: nothing to do)
@@ -148,10 +149,9 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         auto full_phase = [&](int p) { return (uint32_t)(((k0 + p) / kRowStages) & 1); };   // group p of this item
         WalkHead<1> hd;
         int left = (int)min((int64_t)0x7fffffff, ch.seq_len - (int64_t)c0 * kChunk);   // tokens from the current chunk on
-        auto fetch_head = [&](int slot, int tokens) {   // slot: kPair * stage + chunk of the stage
+        auto fetch_head = [&](int slot) {   // slot: kPair * stage + chunk of the stage
             hd.fetch(rec0 + slot * kTcRecord, wl);
             ldmatrix_x4_t(hd.v[0][0], hd.v[0][1], hd.v[0][2], hd.v[0][3], v_off + slot * kRowVBytes);
-            hd.mask(tokens, lane & 3);
         };
         const int n = c1 - c0;
         int s = k0 % kRowStages;   // stage of the current group
@@ -159,7 +159,8 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
             if (__all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[s], full_phase(0), abort_flag, a.wait_ns)) == 0) failed = true;
             else {
                 w.first(rec0 + s * kPair * kTcRecord, wl);
-                fetch_head(s * kPair, left);
+                fetch_head(s * kPair);
+                hd.mask(left, lane & 3);
             }
         }
         bool ready = false;   // the next group's operands have been seen
@@ -172,7 +173,7 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
             uint4 orow;
             const WalkHead<1> cur = hd;
             w.chunk(rec0 + slot * kTcRecord, rec0 + next * kTcRecord, wl, cur, o, [&](int j) {
-                if (j == 3) fetch_head(next, left - kChunk);
+                if (j == 3) fetch_head(next);
                 if (j == 4) look();
                 // the out rows: fragments through a 512-byte tile, 32 contiguous bytes per token to global memory
                 if (j == 3) {
@@ -180,7 +181,10 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
                     __syncwarp();
                 }
                 if (j == 4) orow = lds_u4(o_row);
-                if (j == 6) store_if((lane >> 1) < left, og, orow);
+                if (j == 6) {
+                    hd.mask(left - kChunk, lane & 3);   // (some blocks behind the loads)
+                    store_if((lane >> 1) < left, og, orow);
+                }
             });
             left -= kChunk;
             og += o_step;

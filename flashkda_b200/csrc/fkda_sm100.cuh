@@ -130,6 +130,8 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, in
         ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
         : "memory");
 }
+// Fetches a tensor map (a kernel argument) ahead of its first use.
+__device__ __forceinline__ void tma_prefetch_map(const void* tmap) { asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory"); }
 // 2-D tiles, as above
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, int c0, int c1, uint64_t* bar) {
     asm volatile(

@@ -309,6 +309,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     const bool slabs = !varlen && p.phase_mask == 0 && slabs_possible(chains, sms) && tps >= 64 && !(p.flags & FKDA_FLAG_NO_SLABS);
     const RowsLaunch rows = rows_select(a, chains, sms, slabs);
     if (!rows.ok) return FKDA_ERR_LAUNCH;
+    a.early_rows = a.short_flag == nullptr && chains * rows.split <= sms;
 
     // ---- few chains on a fixed batch: the recurrence is a serial walk on 2 x chains SMs and leaves the others
     //      idle, so the forward is cut into slabs of chunks and the prepare stage of slab i+1 runs on the idle SMs

@@ -19,6 +19,9 @@ namespace fkda {
 // ---------------------------------------------------------------------------------
 // Also ranks the sequences by decreasing length (order[rank] = sequence; ties by index) when the batch is small
 // enough for the quadratic count: the recurrence starts the longest chains first and keeps them apart.
+// One thread per sequence up to 1 024 sequences, in a block no larger than that takes: cu_seqlens is read once and the two tables
+// are summed side by side, so what is left of the kernel is one trip to memory and a few shuffles (1 024 threads whatever the
+// number, a pass for each table: 5.2 us for 4 sequences).
 __global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __restrict__ cu, int64_t N,
                                                            int32_t* __restrict__ prefix, int32_t* __restrict__ order,
                                                            int32_t* __restrict__ cs_prefix, int cs_tokens,
@@ -27,71 +30,78 @@ __global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __rest
                                                            int n_flags) {
     grid_dep_launch();
     grid_dep_wait();   // (the call before may still read its tables)
-    __shared__ int64_t part[32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < 8) header[tid] = 0;   // ticket counter, device status
-    if (!keep_records && (tid == 16 || tid == 17)) header[tid] = 0;
-    for (int i = tid; i < n_flags; i += 1024) flags[i] = 0;
-    const int64_t per = (N + 1023) / 1024;
+    __shared__ int2 part[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = (int)blockDim.x;
+    const int64_t per = (N + threads - 1) / threads;
     const int64_t lo = tid * per, hi = (lo + per < N) ? lo + per : N;
-    // exclusive prefix over the sequences of ceil(len / unit): chunks (unit 16), or state-export groups
-    auto scan = [&](int64_t unit, int32_t* out) {
-        int64_t s = 0;
-        for (int64_t n = lo; n < hi; ++n) {
-            int64_t len = cu[n + 1] - cu[n];
-            if (len < 0) len = 0;
-            s += (len + unit - 1) / unit;
-        }
-        int64_t inc = s;   // inclusive over my warp, then over the warps
+    // of a sequence: chunks (x) and state-export groups (y)
+    auto counts = [&](int64_t len) {
+        if (len < 0) len = 0;
+        int2 c = make_int2((int)((len + kChunk - 1) / kChunk), 0);
+        if (cs_prefix != nullptr)
+            c.y = len <= 0x7fffffff - cs_tokens ? ((int)len + cs_tokens - 1) / cs_tokens : (int)((len + cs_tokens - 1) / cs_tokens);
+        return c;
+    };
+    int64_t raw = 0;   // length of my last sequence (of my only one where per == 1)
+    int2 sum = make_int2(0, 0);
+    int longer = 0, not_one = 0;
+    for (int64_t n = lo; n < hi; ++n) {
+        raw = cu[n + 1] - cu[n];
+        const int2 c = counts(raw);
+        sum.x += c.x;
+        sum.y += c.y;
+        longer |= (raw > kChunk) ? 1 : 0;
+        not_one |= (raw != 1) ? 1 : 0;
+    }
+    for (int i = tid; i < 18; i += threads)   // ticket counter, device status; the note on the records
+        if (i < 8 || (i >= 16 && !keep_records)) header[i] = 0;
+    for (int i = tid; i < n_flags; i += threads) flags[i] = 0;
+    int2 inc = sum;   // inclusive over my warp, then over the warps
+    auto scan_warp = [&](int2& v) {
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            const int64_t x = __shfl_up_sync(0xffffffffu, inc, off);
-            if (lane >= off) inc += x;
+            const int x = __shfl_up_sync(0xffffffffu, v.x, off), y = __shfl_up_sync(0xffffffffu, v.y, off);
+            if (lane >= off) { v.x += x; v.y += y; }
         }
-        __syncthreads();
+    };
+    scan_warp(inc);
+    int2 total = inc, before = make_int2(0, 0);
+    if (threads > 32) {
         if (lane == 31) part[warp] = inc;
         __syncthreads();
-        if (warp == 0) {
-            int64_t w = part[lane];
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int64_t x = __shfl_up_sync(0xffffffffu, w, off);
-                if (lane >= off) w += x;
-            }
-            part[lane] = w;
+        int2 w = lane < (threads >> 5) ? part[lane] : make_int2(0, 0);   // every warp for itself
+        scan_warp(w);
+        total = make_int2(__shfl_sync(0xffffffffu, w.x, 31), __shfl_sync(0xffffffffu, w.y, 31));
+        if (warp > 0) before = make_int2(__shfl_sync(0xffffffffu, w.x, warp - 1), __shfl_sync(0xffffffffu, w.y, warp - 1));
+    }
+    int2 run = make_int2(before.x + inc.x - sum.x, before.y + inc.y - sum.y);
+    for (int64_t n = lo; n < hi; ++n) {
+        prefix[n] = run.x;
+        if (cs_prefix != nullptr) cs_prefix[n] = run.y;
+        if (n + 1 < hi) {
+            const int2 c = counts(cu[n + 1] - cu[n]);
+            run.x += c.x;
+            run.y += c.y;
         }
-        __syncthreads();
-        int64_t run = inc - s + (warp > 0 ? part[warp - 1] : 0);
-        for (int64_t n = lo; n < hi; ++n) {
-            out[n] = (int32_t)run;
-            int64_t len = cu[n + 1] - cu[n];
-            if (len < 0) len = 0;
-            run += (len + unit - 1) / unit;
-        }
-        if (tid == 1023) out[N] = (int32_t)part[31];
-    };
-    scan(kChunk, prefix);
-    if (cs_prefix != nullptr) scan(cs_tokens, cs_prefix);
+    }
+    if (tid == threads - 1) {
+        prefix[N] = total.x;
+        if (cs_prefix != nullptr) cs_prefix[N] = total.y;
+    }
     if (short_flag != nullptr) {   // who serves the call (see TwoPassArgs::short_flag)
-        int longer = 0, not_one = 0;
-        for (int64_t n = lo; n < hi; ++n) {
-            const int64_t len = cu[n + 1] - cu[n];
-            longer |= (len > kChunk) ? 1 : 0;
-            not_one |= (len != 1) ? 1 : 0;
-        }
         longer = __syncthreads_or(longer);
         not_one = __syncthreads_or(not_one);
         if (tid == 0) *short_flag = longer ? 0 : ((decode_enqueued && !not_one) ? 2 : 1);
     }
-    if (order != nullptr) {   // (N <= kSeqOrderMaxN)
+    if (order != nullptr) {   // (N <= kSeqOrderMaxN: a thread per sequence)
         __shared__ int32_t chunks[kSeqOrderMaxN];
-        for (int n = tid; n < (int)N; n += 1024) chunks[n] = (int32_t)((cu[n + 1] - cu[n] + kChunk - 1) / kChunk);
+        const int32_t mine = (int32_t)((raw + kChunk - 1) / kChunk);
+        if (tid < (int)N) chunks[tid] = mine;
         __syncthreads();
-        for (int n = tid; n < (int)N; n += 1024) {
-            const int32_t mine = chunks[n];
+        if (tid < (int)N) {
             int rank = 0;
-            for (int m = 0; m < (int)N; ++m) rank += (chunks[m] > mine || (chunks[m] == mine && m < n)) ? 1 : 0;
-            order[rank] = n;
+            for (int m = 0; m < (int)N; ++m) rank += (chunks[m] > mine || (chunks[m] == mine && m < tid)) ? 1 : 0;
+            order[rank] = tid;
         }
     }
 }
@@ -255,7 +265,8 @@ __global__ void __launch_bounds__(128) recurrence_kernel(TwoPassArgs a) {
 // host launcher
 // ---------------------------------------------------------------------------------
 bool launch_tile_prefix(const TwoPassArgs& a, int32_t* seq_order, bool decode_enqueued, cudaStream_t stream, int n_flags) {
-    return launch_dependent(tile_prefix_kernel, 1, 1024, 0, stream, a.cu_seqlens, a.N, a.tile_prefix, seq_order,
+    const int threads = a.N >= 1024 ? 1024 : ((int)a.N + 31) / 32 * 32;
+    return launch_dependent(tile_prefix_kernel, 1, threads, 0, stream, a.cu_seqlens, a.N, a.tile_prefix, seq_order,
                             a.chunk_states != nullptr ? const_cast<int32_t*>(a.cs_prefix) : (int32_t*)nullptr, 16 * (int)a.cs_every, a.short_flag,
                             decode_enqueued ? 1 : 0, a.queue, a.on_demand ? 1 : 0, a.range_flags, n_flags);
 }
@@ -304,6 +315,7 @@ void fill_args(const fkda_fwd_params& p, TwoPassArgs* out) {
     a.short_flag = nullptr;
     a.range_flags = nullptr;
     a.seg_state = nullptr;
+    a.early_rows = false;
     a.slab_c0 = 0;
     a.slab_chunks = 0;
     a.layer = 0;
