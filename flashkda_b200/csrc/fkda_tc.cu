@@ -342,6 +342,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
             run += part;
         }
         bounds[0] = 0;
+        if (bounds[1] < 2) bounds[1] = 2;
         bounds[n_slabs] = (int)tps;
         auto slab_args = [&](int i) {
             TwoPassArgs x = a;
@@ -349,21 +350,18 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
             x.slab_chunks = bounds[i + 1] - bounds[i];
             return x;
         };
+        // (the side stream forks in front of the first prepare kernel, so that nothing lies between that one and the first walk)
+        if (cudaEventRecord(ss->fork, stream) != cudaSuccess || cudaStreamWaitEvent(ss->side, ss->fork, 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
         if (launch_prepare_warp<true>(slab_args(0), stream, 0, true) != FKDA_OK) return FKDA_ERR_LAUNCH;
-        ++launches;
-        if (cudaEventRecord(ss->fork, stream) != cudaSuccess || cudaStreamWaitEvent(ss->side, ss->fork, 0) != cudaSuccess)
-            return FKDA_ERR_LAUNCH;
+        const int64_t row_ctas = chains * rows.split;
+        if (!launch_dependent(rows.kernel, row_ctas, rows.threads, rows.smem, stream, slab_args(0), map)) return FKDA_ERR_LAUNCH;
+        launches += 2;
         for (int i = 1; i < n_slabs; ++i) {
             if (bounds[i + 1] <= bounds[i]) continue;
             if (launch_prepare_warp<true>(slab_args(i), ss->side, idle_sms) != FKDA_OK) return FKDA_ERR_LAUNCH;
-            ++launches;
-            if (cudaEventRecord(ss->done[i], ss->side) != cudaSuccess) return FKDA_ERR_LAUNCH;
-        }
-        for (int i = 0; i < n_slabs; ++i) {
-            if (bounds[i + 1] <= bounds[i]) continue;
-            if (i > 0 && cudaStreamWaitEvent(stream, ss->done[i], 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
-            rows.kernel<<<(unsigned)(chains * rows.split), rows.threads, rows.smem, stream>>>(slab_args(i), map);
-            ++launches;
+            if (cudaEventRecord(ss->done[i], ss->side) != cudaSuccess || cudaStreamWaitEvent(stream, ss->done[i], 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
+            rows.kernel<<<(unsigned)row_ctas, rows.threads, rows.smem, stream>>>(slab_args(i), map);
+            launches += 2;
         }
         if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
         *n_launches = launches;
