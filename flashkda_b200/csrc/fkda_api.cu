@@ -57,6 +57,12 @@ size_t fkda_workspace_bytes_for(const fkda_fwd_params* p) {
     }
 }
 
+// Scratch bytes this call makes use of: no less than it needs, and more where some more make it faster (same results).
+size_t fkda_workspace_bytes_wanted(const fkda_fwd_params* p) {
+    const size_t need = fkda_workspace_bytes_for(p);
+    return need > 0 && resolve_algo(p->algo) == FKDA_ALGO_TC ? fkda::tc_workspace_bytes_wanted(*p) : need;
+}
+
 int fkda_last_launch_count(void) { return g_last_launches; }
 
 int fkda_device_status(const void* workspace, void* stream_v) {

@@ -57,11 +57,16 @@ struct FusedRange {
     }
 };
 
+// Chunks of each chain of a fixed batch; kSlab: of this launch, which walks only the first a.slab_chunks of them.
+template <bool kSlab>
+__device__ __forceinline__ int64_t fused_chunks(const TwoPassArgs& a) { return kSlab ? a.slab_chunks : (a.T + kChunk - 1) / kChunk; }
+
 // The sequence that holds a position: its chunks of all heads are [begin, end) on the line, head after head.
 struct FusedSeq {
     int64_t begin, end, bos, seq_len;
     int n, n_chunks;      // sequence; chunks of each of its chains
 };
+template <bool kSlab>
 __device__ __forceinline__ FusedSeq fused_seq(const TwoPassArgs& a, int64_t p) {
     FusedSeq s;
     if (a.cu_seqlens != nullptr) {
@@ -78,7 +83,7 @@ __device__ __forceinline__ FusedSeq fused_seq(const TwoPassArgs& a, int64_t p) {
         s.bos = a.cu_seqlens[lo];
         s.seq_len = a.cu_seqlens[lo + 1] - s.bos;
     } else {
-        s.n_chunks = (int)((a.T + kChunk - 1) / kChunk);
+        s.n_chunks = (int)fused_chunks<kSlab>(a);
         const int64_t per = a.H * s.n_chunks;
         s.n = (int)(p / per);
         s.begin = s.n * per;
@@ -90,9 +95,10 @@ __device__ __forceinline__ FusedSeq fused_seq(const TwoPassArgs& a, int64_t p) {
 }
 // Where range `range` starts.  The ranges are equal in cost, not in chunks: a chain counts a.chain_weight chunks more than it
 // has, in front of its first one (a cut that falls there is a cut at the start of the chain).
+template <bool kSlab>
 __device__ __forceinline__ int64_t fused_bound(const TwoPassArgs& a, int range) {
     const int64_t w = a.chain_weight;
-    const int64_t fixed = (a.T + kChunk - 1) / kChunk;
+    const int64_t fixed = fused_chunks<kSlab>(a);
     const int64_t total = a.cu_seqlens != nullptr ? a.H * (a.tile_prefix[a.N] + w * a.N) : a.N * a.H * (fixed + w);
     const int64_t x = total * range / gridDim.x;
     if (a.cu_seqlens == nullptr) return x / (fixed + w) * fixed + max((int64_t)0, x % (fixed + w) - w);
@@ -107,15 +113,16 @@ __device__ __forceinline__ int64_t fused_bound(const TwoPassArgs& a, int range) 
     const int64_t at = x - a.H * (pre[lo] + w * lo);
     return a.H * (int64_t)pre[lo] + min(a.H, at / (n_chunks + w)) * n_chunks + (at < a.H * (n_chunks + w) ? max((int64_t)0, at % (n_chunks + w) - w) : 0);
 }
+template <bool kSlab>
 __device__ __forceinline__ FusedRange fused_range(const TwoPassArgs& a, int range) {
     FusedRange r;
-    r.lo = fused_bound(a, range);
-    r.hi = fused_bound(a, range + 1);
+    r.lo = fused_bound<kSlab>(a, range);
+    r.hi = fused_bound<kSlab>(a, range + 1);
     r.a1 = r.lo;
     r.before = 0;
     r.b0 = r.hi;
     if (r.lo < r.hi) {
-        const FusedSeq f = fused_seq(a, r.lo), l = fused_seq(a, r.hi - 1);
+        const FusedSeq f = fused_seq<kSlab>(a, r.lo), l = fused_seq<kSlab>(a, r.hi - 1);
         const int64_t first = r.lo - (r.lo - f.begin) % f.n_chunks;            // starts of the chains that hold the ends
         const int64_t last = r.hi - 1 - (r.hi - 1 - l.begin) % l.n_chunks;
         r.before = r.lo - first;
@@ -161,8 +168,9 @@ __device__ __forceinline__ int load_acquire(const int32_t* p) {
     return v;
 }
 
-// kExport: the states before every cs_every-th chunk are written out as well
-template <bool kExport>
+// kExport: the states before every cs_every-th chunk are written out as well.  kSlab: only the first a.slab_chunks chunks of every
+// chain are walked, one chain per CTA, and the states handed on to the row-slice kernel (see launch_mid)
+template <bool kExport, bool kSlab>
 __global__ void __launch_bounds__(kFusedThreads, 1)
 fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap map) {
     extern __shared__ uint8_t smem_dyn[];
@@ -184,7 +192,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
     if (threadIdx.x == 0) ctl.range = atomicAdd(a.queue, 1);
     __syncthreads();
     const int range = ctl.range;
-    const FusedRange r = fused_range(a, range);
+    const FusedRange r = fused_range<kSlab>(a, range);
     const int n_units = (int)(r.hi - r.lo);
     // The chain at lo reaches this range when the ranges before have walked its beginning, at a microsecond per chunk: with a
     // chain much longer than a range that alone may take longer than the limit of a wait, which is for what never comes.
@@ -203,7 +211,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
             t += kFusedPrep;
             if (t >= sq.n_chunks || p >= end) {   // another chain, or another run
                 p = r.position(u, &end);
-                if (p < sq.begin || p >= sq.end) sq = fused_seq(a, p);
+                if (p < sq.begin || p >= sq.end) sq = fused_seq<kSlab>(a, p);
                 const int at = (int)(p - sq.begin);
                 h = at / sq.n_chunks;
                 t = at - h * sq.n_chunks;
@@ -286,7 +294,7 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
             // ---- the state this piece starts from ----
             if (pc.chunk > 0) {   // published by the range before this one (the last one that holds any chunks)
                 int before = range - 1;
-                while (before > 0 && fused_bound(a, before) == r.lo) --before;
+                while (before > 0 && fused_bound<kSlab>(a, before) == r.lo) --before;
                 const uint64_t begin = global_timer_ns();
                 uint32_t spins = 0;
                 while (load_acquire(a.range_flags + before) < kFusedWalkers) {
@@ -377,6 +385,12 @@ fused_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap
                 __threadfence();
                 __syncwarp();
                 if (lane == 0 && !a.test_drop_push) atomicAdd(a.range_flags + range, 1);
+            } else if (kSlab) {
+                uint4* dst = reinterpret_cast<uint4*>(a.seg_state) + ((pc.n * a.H + pc.h) * 8 + row0 / 16) * 256 + lane;
+#pragma unroll
+                for (int mt = 0; mt < kFusedMt; ++mt)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) dst[(mt * 8 + j) * 32] = make_uint4(w.s[mt][j][0], w.s[mt][j][1], w.s[mt][j][2], w.s[mt][j][3]);
             } else if (a.final_state != nullptr) {
 #pragma unroll
                 for (int mt = 0; mt < kFusedMt; ++mt)

@@ -197,9 +197,16 @@ void fwd_checked(PyObject* const* a) {
         p.workspace = ws->data_ptr();
         p.workspace_bytes = (size_t)ws->numel();
     } else if (need > 0) {
-        scratch = c10::cuda::CUDACachingAllocator::get()->allocate(need);
+        p.workspace_bytes = fkda_workspace_bytes_wanted(&p);   // more than the path needs only makes it faster
+        if (p.workspace_bytes > need) {
+            try {
+                scratch = c10::cuda::CUDACachingAllocator::get()->allocate(p.workspace_bytes);
+            } catch (const c10::OutOfMemoryError&) {
+                p.workspace_bytes = need;
+            }
+        }
+        if (scratch.get() == nullptr) scratch = c10::cuda::CUDACachingAllocator::get()->allocate(need);
         p.workspace = scratch.get();
-        p.workspace_bytes = need;
     }
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     int rc;

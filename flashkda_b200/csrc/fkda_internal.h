@@ -68,6 +68,7 @@ size_t twopass_workspace_bytes(int64_t T_total, int64_t H, int64_t N);
 int launch_twopass(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches);
 size_t tc_workspace_bytes(int64_t T_total, int64_t H, int64_t N);   // upper bound for these totals
 size_t tc_workspace_bytes_for(const fkda_fwd_params& p);            // what this particular call needs
+size_t tc_workspace_bytes_wanted(const fkda_fwd_params& p);         // what it makes use of
 int device_sm_count();
 // Device address of the built-in scratch of fkda_fwd_noalloc on the current device, or nullptr before that
 // entry point's first call there.

@@ -1,5 +1,5 @@
 // Recurrence over chunk records in HBM / L2, row slices: a (sequence, head) chain is walked by kRowSplit CTAs of
-// kRowWarps warps, each warp with 16 of the 128 state rows in registers (fkda_walk.cuh).  The warps of a chain share nothing
+// kRowWarps warps, each warp with 16 (kMt = 2: 32) of the 128 state rows in registers (fkda_walk.cuh).  The warps of a chain share nothing
 // but the records they read, so a chunk step has no barrier in it: every warp waits for the stage of its next chunk, walks
 // it, and tells the control warp that it is done with the stage.
 //
@@ -21,19 +21,20 @@
 
 namespace fkda {
 
-// kWarps walking warps per CTA, 16 state rows each: 8 / kWarps CTAs per chain
-__host__ __device__ constexpr int row_split(int warps) { return kD / (16 * warps); }
+// kWarps walking warps per CTA, kMt row tiles of 16 state rows each: 8 / (kWarps kMt) CTAs per chain
+__host__ __device__ constexpr int row_split(int warps, int mt) { return kD / (16 * mt * warps); }
 __host__ __device__ constexpr int row_threads(int warps) { return (warps + 1) * 32; }
-constexpr int kRowVCols = kD / 2;                               // a CTA of four or fewer warps reads one half of a value row
-constexpr int kRowVBytes = kChunk * kRowVCols * 2;              // value tile [16 tokens][64] bf16, 128-byte swizzle
-static_assert(kRowVBytes % 1024 == 0, "tile alignments");
+constexpr int kRowVCols = kD / 2;                               // value columns of a tile: a CTA reads one half of a value row, or both
+constexpr int kRowVTile = kChunk * kRowVCols * 2;               // value tile [16 tokens][64] bf16, 128-byte swizzle
+static_assert(kRowVTile % 1024 == 0, "tile alignments");
 
 // Shared memory of a CTA with kStages groups of kPair chunks in flight
-template <int kRowWarps, int kStages, int kPair>
+template <int kMt, int kRowWarps, int kStages, int kPair>
 struct RowSmem {
+    static constexpr int kRowVBytes = (16 * kMt * kRowWarps > kRowVCols ? 2 : 1) * kRowVTile;   // value tiles of a chunk
     static constexpr int kV = 0;                                        // value tiles (1024-byte aligned for the swizzle)
-    static constexpr int kOut = kV + kStages * kPair * kRowVBytes;      // per warp an out tile [16 tokens][16] bf16
-    static constexpr int kRec = kOut + kRowWarps * 512;                    // chunk records
+    static constexpr int kOut = kV + kStages * kPair * kRowVBytes;      // per warp an out tile [16 tokens][16 kMt] bf16
+    static constexpr int kRec = kOut + kRowWarps * kMt * 512;             // chunk records
     static constexpr int kStaging = kRec + kStages * kPair * kTcRecord;   // per warp one staging tile for states
     static constexpr int kCtrl = kStaging + kRowWarps * kWalkStageBytes;
     struct Ctrl {
@@ -50,14 +51,15 @@ struct RowSmem {
 // of two chunks when every slice has an SM of its own (with the prepare stage of the next slab loading the memory, records arrive
 // up to four steps late: 131 072 tokens, 32 heads: 4.58 -> 4.31 ms with 8 chunks in flight against 4), otherwise of one, so that
 // two CTAs fit an SM (with 2 stages of two: 300 + 1 + 211 + 512 tokens of 32 heads 57 us against 51).
-template <bool kExport, bool kLoop, int kRowWarps, int kRowStages, int kPair>
-__global__ void __launch_bounds__(row_threads(kRowWarps), 2)
+template <bool kExport, bool kLoop, int kMt, int kRowWarps, int kRowStages, int kPair>
+__global__ void __launch_bounds__(row_threads(kRowWarps), kMt == 1 ? 2 : 1)
 recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_constant__ VMap map) {
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     static_assert(!kLoop || kPair == 1, "slices in turn: a stage of one chunk");
-    constexpr int kRowSplit = row_split(kRowWarps), kRowCols = 16 * kRowWarps;
-    using L = RowSmem<kRowWarps, kRowStages, kPair>;
+    constexpr int kRowSplit = row_split(kRowWarps, kMt), kRowCols = 16 * kMt * kRowWarps;
+    using L = RowSmem<kMt, kRowWarps, kRowStages, kPair>;
+    constexpr int kRowVBytes = L::kRowVBytes;
     typename L::Ctrl& ctl = *reinterpret_cast<typename L::Ctrl*>(sm + L::kCtrl);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
@@ -105,7 +107,9 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
                 bulk_g2s(sm + L::kRec + s * kPair * kTcRecord, ch.rec_base + (int64_t)t * kTcRecord, m * kTcRecord, &ctl.full[s]);
                 // rows past the end of the tensor arrive as zeros; rows of the next sequence are never used
                 for (int e = 0; e < m; ++e)
-                    tma_load_3d(sm + L::kV + (s * kPair + e) * kRowVBytes, &map.v, slice * kRowCols / kRowVCols * kRowVCols, h, (int)(ch.bos + (int64_t)(t + e) * kChunk), &ctl.full[s]);
+                    for (int half = 0; half < kRowVBytes / kRowVTile; ++half)
+                        tma_load_3d(sm + L::kV + (s * kPair + e) * kRowVBytes + half * kRowVTile, &map.v, slice * kRowCols / kRowVCols * kRowVCols + half * kRowVCols, h,
+                                    (int)(ch.bos + (int64_t)(t + e) * kChunk), &ctl.full[s]);
             }
             if (failed) {   // the copies in flight land before this CTA's shared memory goes
                 *abort_flag = 1;
@@ -116,42 +120,56 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         failed = __any_sync(0xffffffffu, failed) != 0;
     } else {
         // =========================== walking warps ===========================
-        const int row0 = slice * kRowCols + warp * 16;   // my first state row
+        const int row0 = slice * kRowCols + warp * 16 * kMt;   // my first state row
         const WalkLane wl = walk_lane(lane);
         uint8_t* stage_tile = sm + L::kStaging + warp * kWalkStageBytes;
         const uint32_t rec0 = smem_u32(sm + L::kRec);
-        // my value columns in the [16 tokens][64] tile: token (lane & 7) + 8 (lane / 16), 16-byte piece (my first column) / 8 + (lane / 8) % 2
-        const uint32_t v_off = smem_u32(sm + L::kV) + (uint32_t)(((lane & 7) + 8 * (lane >> 4)) * 128 + (((row0 % kRowVCols / 8 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
-        // out tile of my warp, [16 tokens][16] with the two 16-byte pieces of a token swapped in every other group of four:
-        // fragments in (token (lane & 7) + 8 (lane / 16), piece (lane / 8) % 2), rows out (token lane / 2, piece lane % 2)
+        // my value columns in the [16 tokens][64] tiles: token (lane & 7) + 8 (lane / 16), 16-byte piece (my first column) / 8 + (lane / 8) % 2
         const int o_tok = (lane & 7) + 8 * (lane >> 4);
-        const uint32_t o_tile = smem_u32(sm + L::kOut + warp * 512);
-        const uint32_t o_frag = o_tile + (uint32_t)(o_tok * 32 + ((((lane >> 3) & 1) ^ ((o_tok >> 2) & 1)) << 4));
-        const uint32_t o_row = o_tile + (uint32_t)((lane >> 1) * 32 + (((lane & 1) ^ ((lane >> 3) & 1)) << 4));
+        uint32_t v_off[kMt];
+#pragma unroll
+        for (int mt = 0; mt < kMt; ++mt) {
+            const int col = row0 + 16 * mt - slice * kRowCols / kRowVCols * kRowVCols;
+            v_off[mt] = smem_u32(sm + L::kV) + (uint32_t)(col / kRowVCols * kRowVTile + o_tok * 128 + (((col % kRowVCols / 8 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+        }
+        // out tile of my warp, [16 tokens][16 kMt]: 32 bytes per token with the two 16-byte pieces swapped in every other group of four
+        // tokens, or 64 bytes per token as in fused_kernel; rows out 16 / kMt tokens at a time (token lane / (2 kMt), piece lane % (2 kMt))
+        const uint32_t o_tile = smem_u32(sm + L::kOut + warp * kMt * 512);
+        auto o_piece = [&](int tok, int piece) {
+            return o_tile + (uint32_t)(tok * 32 * kMt + ((piece ^ (kMt == 1 ? (tok >> 2) & 1 : (tok >> 1) & 3)) << 4));
+        };
+        uint32_t o_frag[kMt];
+#pragma unroll
+        for (int mt = 0; mt < kMt; ++mt) o_frag[mt] = o_piece(o_tok, 2 * mt + ((lane >> 3) & 1));
+        const int my_tok = lane / (2 * kMt), my_piece = lane % (2 * kMt);
+        const uint32_t o_row = o_piece(my_tok, my_piece);   // (kMt == 2: tokens 8 .. 15 are 512 bytes further, the same permutation)
         const int64_t o_step = kChunk * a.token_stride;
-        __nv_bfloat16* og = a.out + (ch.bos + (int64_t)c0 * kChunk + (lane >> 1)) * a.token_stride + (int64_t)h * kD + row0 + 8 * (lane & 1);
+        __nv_bfloat16* og = a.out + (ch.bos + (int64_t)c0 * kChunk + my_tok) * a.token_stride + (int64_t)h * kD + row0 + 8 * my_piece;
         const int64_t st_base = ((ch.n * a.H + h) * (int64_t)kD + row0) * (int64_t)kD;   // element (row0, 0) of my rows
-        uint4* const handover = reinterpret_cast<uint4*>(a.seg_state) + (chain * 8 + slice * kRowWarps + warp) * 256 + lane;   // + j * 32
+        uint4* const handover = reinterpret_cast<uint4*>(a.seg_state) + (chain * 8 + row0 / 16) * 256 + lane;   // + (8 mt + j) * 32
 
-        WalkState<1> w;
+        WalkState<kMt, true> w;
         if (c0 > 0) {                       // handed over by the previous slab
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint4 x = __ldcg(handover + j * 32);
-                w.s[0][j][0] = x.x; w.s[0][j][1] = x.y; w.s[0][j][2] = x.z; w.s[0][j][3] = x.w;
-            }
+            for (int mt = 0; mt < kMt; ++mt)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint4 x = __ldcg(handover + (8 * mt + j) * 32);
+                    w.s[mt][j][0] = x.x; w.s[mt][j][1] = x.y; w.s[mt][j][2] = x.z; w.s[mt][j][3] = x.w;
+                }
         } else if (a.initial_state != nullptr) {
-            if (a.state_fp32) walk_load_tiles<1, true>(w.s, stage_tile, reinterpret_cast<const float*>(a.initial_state) + st_base, lane);
-            else walk_load_tiles<1, false>(w.s, stage_tile, reinterpret_cast<const unsigned short*>(a.initial_state) + st_base, lane);
+            if (a.state_fp32) walk_load_tiles<kMt, true>(w.s, stage_tile, reinterpret_cast<const float*>(a.initial_state) + st_base, lane);
+            else walk_load_tiles<kMt, false>(w.s, stage_tile, reinterpret_cast<const unsigned short*>(a.initial_state) + st_base, lane);
         } else {
             w.clear();
         }
         auto full_phase = [&](int p) { return (uint32_t)(((k0 + p) / kRowStages) & 1); };   // group p of this item
-        WalkHead<1> hd;
+        WalkHead<kMt> hd;
         int left = (int)min((int64_t)0x7fffffff, ch.seq_len - (int64_t)c0 * kChunk);   // tokens from the current chunk on
         auto fetch_head = [&](int slot) {   // slot: kPair * stage + chunk of the stage
             hd.fetch(rec0 + slot * kTcRecord, wl);
-            ldmatrix_x4_t(hd.v[0][0], hd.v[0][1], hd.v[0][2], hd.v[0][3], v_off + slot * kRowVBytes);
+#pragma unroll
+            for (int mt = 0; mt < kMt; ++mt) ldmatrix_x4_t(hd.v[mt][0], hd.v[mt][1], hd.v[mt][2], hd.v[mt][3], v_off[mt] + slot * kRowVBytes);
         };
         const int n = c1 - c0;
         int s = k0 % kRowStages;   // stage of the current group
@@ -166,24 +184,31 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         bool ready = false;   // the next group's operands have been seen
         // Chunk i of the walk, in slot `slot`; `next`: the slot of the chunk after it, or `slot` where there is none.
         auto step = [&](int i, int slot, int next, auto&& look) {
-            if (kExport && (c0 + i) % a.cs_every == 0)   // the state before this group of chunks
-                walk_store_tile(w.s[0], stage_tile, a.chunk_states + ((ch.cs_slot0 + (c0 + i) / a.cs_every) * a.H + h) * (int64_t)(kD * kD) + (int64_t)row0 * kD,
-                                false, lane);
-            uint32_t o[1][4];
-            uint4 orow;
-            const WalkHead<1> cur = hd;
+            if (kExport && (c0 + i) % a.cs_every == 0) {   // the state before this group of chunks
+                __nv_bfloat16* dst = a.chunk_states + ((ch.cs_slot0 + (c0 + i) / a.cs_every) * a.H + h) * (int64_t)(kD * kD) + (int64_t)row0 * kD;
+#pragma unroll
+                for (int mt = 0; mt < kMt; ++mt) walk_store_tile(w.s[mt], stage_tile, dst + mt * 16 * kD, false, lane);
+            }
+            uint32_t o[kMt][4];
+            uint4 orow[kMt];
+            const WalkHead<kMt> cur = hd;
             w.chunk(rec0 + slot * kTcRecord, rec0 + next * kTcRecord, wl, cur, o, [&](int j) {
                 if (j == 3) fetch_head(next);
                 if (j == 4) look();
-                // the out rows: fragments through a 512-byte tile, 32 contiguous bytes per token to global memory
+                // the out rows: fragments through the warp's tile, 32 kMt contiguous bytes per token to global memory
                 if (j == 3) {
-                    stmatrix_x4_t(o_frag, o[0][0], o[0][1], o[0][2], o[0][3]);
+#pragma unroll
+                    for (int mt = 0; mt < kMt; ++mt) stmatrix_x4_t(o_frag[mt], o[mt][0], o[mt][1], o[mt][2], o[mt][3]);
                     __syncwarp();
                 }
-                if (j == 4) orow = lds_u4(o_row);
+                if (j == 4) {
+#pragma unroll
+                    for (int e = 0; e < kMt; ++e) orow[e] = lds_u4(o_row + e * 512);
+                }
                 if (j == 6) {
                     hd.mask(left - kChunk, lane & 3);   // (some blocks behind the loads)
-                    store_if((lane >> 1) < left, og, orow);
+#pragma unroll
+                    for (int e = 0; e < kMt; ++e) store_if(my_tok + 8 * e < left, og + e * 8 * a.token_stride, orow[e]);
                 }
             });
             left -= kChunk;
@@ -211,12 +236,16 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
         if (!failed) {
             if (c1 < ch.n_chunks) {         // not the last slab
 #pragma unroll
-                for (int j = 0; j < 8; ++j) handover[j * 32] = make_uint4(w.s[0][j][0], w.s[0][j][1], w.s[0][j][2], w.s[0][j][3]);
+                for (int mt = 0; mt < kMt; ++mt)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) handover[(8 * mt + j) * 32] = make_uint4(w.s[mt][j][0], w.s[mt][j][1], w.s[mt][j][2], w.s[mt][j][3]);
             } else if (a.final_state != nullptr) {
-                walk_store_tile(w.s[0], stage_tile,
-                                a.state_fp32 ? (void*)(reinterpret_cast<float*>(a.final_state) + st_base)
-                                             : (void*)(reinterpret_cast<unsigned short*>(a.final_state) + st_base),
-                                a.state_fp32, lane);
+#pragma unroll
+                for (int mt = 0; mt < kMt; ++mt)
+                    walk_store_tile(w.s[mt], stage_tile,
+                                    a.state_fp32 ? (void*)(reinterpret_cast<float*>(a.final_state) + st_base + mt * 16 * kD)
+                                                 : (void*)(reinterpret_cast<unsigned short*>(a.final_state) + st_base + mt * 16 * kD),
+                                    a.state_fp32, lane);
             }
         } else {
             *abort_flag = 1;   // the other warps leave their waits

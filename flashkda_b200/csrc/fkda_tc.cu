@@ -81,7 +81,7 @@ int device_sm_count() {
     return cache[dev];
 }
 
-constexpr int kRowSplit = row_split(4);   // CTAs per chain of the row-slice kernel, unless there are SMs for more
+constexpr int kRowSplit = row_split(4, 1);   // CTAs per chain of the row-slice kernel, unless there are SMs for more
 constexpr size_t kStateBytes = (size_t)kD * kD * 2;   // a chain's state as bf16 (hand-over buffers)
 
 // Few chains on a fixed batch may run as a slab pipeline (see launch_tc): at least 32 SMs are left beside the row slices.
@@ -122,6 +122,21 @@ static TcCarve tc_carve(const fkda_fwd_params& p, int sms) {
     return c;
 }
 
+// Fewer chains than SMs, but too many for two SMs each: launch_mid, while its records take no more than a gigabyte.  The three kernel
+// boundaries cost some 12 us, and what is won grows with the chunks and with the idle SMs: the line lies where the two meet (us, one
+// kernel against this: 128 chunks: 76 chains 154, 134; 112 chains 157, 155; 128 chains 157, 163; 512 chunks: 96 chains 610, 480;
+// 124 chains 634, 572).
+constexpr size_t kMidBytesMost = (size_t)1 << 30;
+static size_t mid_bytes(const fkda_fwd_params& p, int sms) {
+    const int64_t chains = p.N * p.H, tps = (p.T + kChunk - 1) / kChunk;
+    return kWsHeaderBytes + ws_prefix_bytes(p.N) + fused_flag_bytes(sms) + (size_t)chains * kStateBytes + (size_t)(chains * tps) * kTcRecord;
+}
+static bool mid_eligible(const fkda_fwd_params& p, int sms) {
+    const int64_t chains = p.N * p.H;
+    return p.cu_seqlens == nullptr && p.phase_mask == 0 && !(p.flags & (FKDA_FLAG_NO_WIDE | FKDA_FLAG_NO_SLABS)) && chains * kRowSplit > sms &&
+           chains + 24 <= sms && p.T > 63 * kChunk && (p.T + kChunk - 1) / kChunk * (sms - chains) >= 4608 && mid_bytes(p, sms) <= kMidBytesMost;
+}
+
 // Names the records that a call writes or expects: everything that decides where each of them lies.
 static uint64_t records_tag(const fkda_fwd_params& p) {
     uint64_t x = p.cu_seqlens != nullptr ? 2 : 1;
@@ -132,7 +147,7 @@ static uint64_t records_tag(const fkda_fwd_params& p) {
 // Upper bound over every call with these totals (the caller may not know yet whether the batch is ragged).
 size_t tc_workspace_bytes(int64_t T_total, int64_t H, int64_t N) {
     const int sms = device_sm_count();
-    const size_t two_pass = kWsHeaderBytes + ws_prefix_bytes(N) + (slabs_possible(H * N, sms) ? (size_t)(H * N) * kStateBytes : 0) +
+    const size_t two_pass = kWsHeaderBytes + ws_prefix_bytes(N) + (H * N < sms ? fused_flag_bytes(sms) + (size_t)(H * N) * kStateBytes : 0) +
                             (size_t)H * (size_t)ws_tiles_upper_bound(T_total, N) * (size_t)kTcRecord;
     const size_t fused = fused_bytes(N, sms);
     return two_pass > fused ? two_pass : fused;
@@ -145,6 +160,13 @@ size_t tc_workspace_bytes_for(const fkda_fwd_params& p) {
     if (fused_eligible(p, sms)) return fused_bytes(p.N, sms);
     const TcCarve c = tc_carve(p, sms);
     return kWsHeaderBytes + ws_prefix_bytes(p.N) + c.states + c.records;
+}
+
+// What a call makes use of: more than it needs where records of the later chunks make it faster.
+size_t tc_workspace_bytes_wanted(const fkda_fwd_params& p) {
+    const int sms = device_sm_count();
+    const size_t need = tc_workspace_bytes_for(p);
+    return need > 0 && mid_eligible(p, sms) && mid_bytes(p, sms) > need ? mid_bytes(p, sms) : need;
 }
 
 // Side stream and events of the slab pipeline, one set per device, created on first use.
@@ -243,8 +265,8 @@ static int launch_fused(const fkda_fwd_params& p, TwoPassArgs& a, int sms, cudaS
     VMap map;
     if (!encode_v_map(&map.v, p)) return FKDA_ERR_LAUNCH;
     const bool exports = a.chunk_states != nullptr;
-    if (!(exports ? allow_smem<fused_kernel<true>>(kFusedSmemBytes) : allow_smem<fused_kernel<false>>(kFusedSmemBytes))) return FKDA_ERR_LAUNCH;
-    const auto kernel = exports ? fused_kernel<true> : fused_kernel<false>;
+    if (!(exports ? allow_smem<fused_kernel<true, false>>(kFusedSmemBytes) : allow_smem<fused_kernel<false, false>>(kFusedSmemBytes))) return FKDA_ERR_LAUNCH;
+    const auto kernel = exports ? fused_kernel<true, false> : fused_kernel<false, false>;
     const int64_t ctas = chains < sms ? chains : sms;
     if (!launch_dependent(kernel, ctas, kFusedThreads, kFusedSmemBytes, stream, a, map)) return FKDA_ERR_LAUNCH;
     *n_launches = launches + 1;
@@ -257,23 +279,81 @@ struct RowsLaunch {
     int smem, threads, split;
     bool ok;
 };
-template <bool kExport, bool kLoop, int kWarps, int kPair>
+template <bool kExport, bool kLoop, int kMt, int kWarps, int kPair>
 static RowsLaunch rows_launch() {
-    constexpr int kBytes = RowSmem<kWarps, 4, kPair>::kBytes;
-    constexpr auto kKernel = recurrence_rows_kernel<kExport, kLoop, kWarps, 4, kPair>;
-    return RowsLaunch{kKernel, kBytes, row_threads(kWarps), row_split(kWarps), allow_smem<kKernel>(kBytes)};
+    constexpr int kBytes = RowSmem<kMt, kWarps, 4, kPair>::kBytes;
+    static_assert(kBytes <= 232448, "shared memory of an SM");
+    constexpr auto kKernel = recurrence_rows_kernel<kExport, kLoop, kMt, kWarps, 4, kPair>;
+    return RowsLaunch{kKernel, kBytes, row_threads(kWarps), row_split(kWarps, kMt), allow_smem<kKernel>(kBytes)};
 }
 // Four CTAs per chain of two warps each instead of two of four, where the SMs last: a step takes 0.43 us against 0.47 (the warps of
 // a CTA share one shared-memory pipe, 8 192 tokens of 8 heads 235 us against 254, 777 tokens of 32 heads 37.6 against 38.9; eight CTAs
 // of one warp: 237 us).  With the prepare stage of the next slab beside it that takes twice as many SMs more as there are chains
 // (8 192 tokens: 16 heads 250 against 257, 32 heads, where the prepare stage comes out of hiding, 380 against 280).
 static RowsLaunch rows_select(const TwoPassArgs& a, int64_t chains, int sms, bool slabs) {
-    if (a.short_flag != nullptr) return rows_launch<false, true, 4, 1>();   // (such a batch exports no states)
+    if (a.short_flag != nullptr) return rows_launch<false, true, 1, 4, 1>();   // (such a batch exports no states)
     const bool exports = a.chunk_states != nullptr;
-    if (chains * kRowSplit > sms) return exports ? rows_launch<true, false, 4, 1>() : rows_launch<false, false, 4, 1>();
+    if (chains * kRowSplit > sms) return exports ? rows_launch<true, false, 1, 4, 1>() : rows_launch<false, false, 1, 4, 1>();
     const bool four = slabs ? 4 * chains + 2 * chains <= sms : 4 * chains <= sms;
-    if (four) return exports ? rows_launch<true, false, 2, 2>() : rows_launch<false, false, 2, 2>();
-    return exports ? rows_launch<true, false, 4, 2>() : rows_launch<false, false, 4, 2>();
+    if (four) return exports ? rows_launch<true, false, 1, 2, 2>() : rows_launch<false, false, 1, 2, 2>();
+    return exports ? rows_launch<true, false, 1, 4, 2>() : rows_launch<false, false, 1, 4, 2>();
+}
+
+// More chains than half the SMs, but fewer than SMs: in the one-kernel form a chain's SM walks and prepares, and the others idle.  Here
+// they prepare the records of the later chunks meanwhile (side stream), and once the one-kernel form has walked the first chunks a
+// row-slice kernel of one CTA per chain, 32 rows per warp, walks the others without a preparing warp beside it, slab by slab.
+// A step takes about 1.11 us in the one and 0.77 us in the other, a record 0.0050 us of the whole GPU (0.0043, which would hide
+// nothing, to 0.0061 tried): the slabs follow from that.  8 192 tokens of 96 heads: 568 -> 475 us, of 80 heads 579 -> 444.
+static int launch_mid(const fkda_fwd_params& p, TwoPassArgs& a, int sms, int dev, cudaStream_t stream, int* n_launches) {
+    const int chains = (int)(p.N * p.H), idle = sms - chains, tps = (int)((p.T + kChunk - 1) / kChunk);
+    const double records = 0.0050 * sms * chains / idle;   // us for the records of one chunk of every chain
+    const int n_slabs = tps >= 256 ? kMaxSlabs : 3;
+    double size[kMaxSlabs] = {1.0, 1.11 / records, 0.0, 0.0}, total = 0.0, run = 0.0;
+    for (int i = 1; i < n_slabs; ++i) {
+        if (i > 1) size[i] = size[i - 1] * 0.77 / records;
+        if (size[i] > 4.0 * size[i - 1]) size[i] = 4.0 * size[i - 1];
+    }
+    for (int i = 0; i < n_slabs; ++i) total += size[i];
+    int bounds[kMaxSlabs + 1] = {0};
+    for (int i = 0; i < n_slabs; ++i) {
+        run += size[i];
+        bounds[i + 1] = i + 1 == n_slabs ? tps : (int)(run / total * tps + 1.0) / 2 * 2;
+    }
+    a.chain_weight = chain_weight(p);
+    uint8_t* base = reinterpret_cast<uint8_t*>(p.workspace) + kWsHeaderBytes;
+    a.range_flags = reinterpret_cast<int32_t*>(base);
+    uint8_t* states = base + ws_prefix_bytes(p.N) + fused_flag_bytes(sms);
+    a.seg_state = reinterpret_cast<uint32_t*>(states);
+    a.workspace = states + (size_t)chains * kStateBytes;
+    VMap map;
+    if (!encode_v_map(&map.v, p)) return FKDA_ERR_LAUNCH;
+    const bool exports = a.chunk_states != nullptr;
+    if (!(exports ? allow_smem<fused_kernel<true, true>>(kFusedSmemBytes) : allow_smem<fused_kernel<false, true>>(kFusedSmemBytes))) return FKDA_ERR_LAUNCH;
+    const RowsLaunch rows = exports ? rows_launch<true, false, 2, 4, 2>() : rows_launch<false, false, 2, 4, 2>();
+    SlabStreams* ss = slab_streams(dev);
+    if (!rows.ok || ss == nullptr) return FKDA_ERR_LAUNCH;
+    std::lock_guard<std::mutex> enqueue_lock(ss->launch_mu);
+    auto slab_args = [&](int i) {
+        TwoPassArgs x = a;
+        x.slab_c0 = bounds[i];
+        x.slab_chunks = bounds[i + 1] - bounds[i];
+        return x;
+    };
+    if (cudaEventRecord(ss->fork, stream) != cudaSuccess || cudaStreamWaitEvent(ss->side, ss->fork, 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
+    if (cudaMemsetAsync(p.workspace, 0, kWsHeaderBytes + (size_t)sms * 4, stream) != cudaSuccess) return FKDA_ERR_LAUNCH;
+    const auto kernel = exports ? fused_kernel<true, true> : fused_kernel<false, true>;
+    kernel<<<(unsigned)chains, kFusedThreads, kFusedSmemBytes, stream>>>(slab_args(0), map);
+    int launches = 1;
+    for (int i = 1; i < n_slabs; ++i) {
+        if (bounds[i + 1] <= bounds[i]) continue;
+        if (launch_prepare_warp<true>(slab_args(i), ss->side, idle) != FKDA_OK) return FKDA_ERR_LAUNCH;
+        if (cudaEventRecord(ss->done[i], ss->side) != cudaSuccess || cudaStreamWaitEvent(stream, ss->done[i], 0) != cudaSuccess) return FKDA_ERR_LAUNCH;
+        rows.kernel<<<(unsigned)chains, rows.threads, rows.smem, stream>>>(slab_args(i), map);
+        launches += 2;
+    }
+    if (cudaGetLastError() != cudaSuccess) return FKDA_ERR_LAUNCH;
+    *n_launches = launches;
+    return FKDA_OK;
 }
 
 int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
@@ -287,7 +367,10 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     if (cudaGetDevice(&dev) != cudaSuccess) return FKDA_ERR_LAUNCH;
     const int sms = device_sm_count();
     const int64_t T_total = p.B * p.T, chains = p.N * p.H;
-    if (fused_eligible(p, sms)) return launch_fused(p, a, sms, stream, n_launches);
+    if (fused_eligible(p, sms)) {
+        if (mid_eligible(p, sms) && p.workspace_bytes >= mid_bytes(p, sms)) return launch_mid(p, a, sms, dev, stream, n_launches);
+        return launch_fused(p, a, sms, stream, n_launches);
+    }
     if (chains * kRowSplit > 0x7fffffff) return FKDA_ERR_BAD_SHAPE;
     a.records_tag = records_tag(p);
     a.on_demand = do_rec && !do_prep;

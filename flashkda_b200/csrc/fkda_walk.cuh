@@ -129,7 +129,11 @@ struct WalkHead {
     }
 };
 
-template <int kMt>
+// kStrung: a product takes its pipe for 8.5 cycles and a warp issues in order, so the products of a block are strung together with
+// the update of the block after it, pair by pair, and neither waits for the other.  That pays where a walking warp has its scheduler
+// to itself (131 072 tokens, 32 heads 3.88 -> 3.75 ms); with the preparing warps beside it (fkda_fused.cuh) a block's update as one
+// piece is as fast or faster (8 x 32 768 tokens, 64 heads: 8.47 ms against 8.74).
+template <int kMt, bool kStrung = (kMt == 1)>
 struct WalkState {
     uint32_t s[kMt][8][4];     // my state rows, A fragments
     float u0[kMt][2][4];       // S . kd^T of the current chunk, token tiles 0 and 1
@@ -183,11 +187,6 @@ struct WalkState {
     // o[mt] = out of tokens 8 (i >> 1) + 2tq, +1 of row g + 8 (i & 1), i = 0 .. 3, complete after block 2.
     template <bool kNext = true, class Mid>
     __device__ __forceinline__ void chunk(uint32_t rec, uint32_t next, const WalkLane& wl, const WalkHead<kMt>& hd, uint32_t (&o)[kMt][4], Mid&& mid) {
-        // kStrung: a product takes its pipe for 8.5 cycles and a warp issues in order, so the products of a block are strung together
-        // with the update of the block after it, pair by pair, and neither waits for the other (one row tile per warp, a warp per
-        // scheduler: 131 072 tokens, 32 heads 3.88 -> 3.75 ms).  With two row tiles and the preparing warps beside them (fkda_fused.cuh)
-        // a block's update as one piece is as fast or faster (8 x 32 768 tokens, 64 heads: 8.47 ms against 8.74).
-        constexpr bool kStrung = kMt == 1;
         constexpr int kAhead = kStrung ? 3 : 2, kAheadB = kStrung ? 2 : 1;   // blocks whose operands (kr and E_tot, kd) are fetched ahead of their products
         uint32_t kr[8][4], b[8][4], q[8][4];
         float2 et[8][2];

@@ -124,6 +124,11 @@ size_t fkda_workspace_bytes(int64_t T_total, int64_t H, int64_t N, int32_t algo)
  * its status word is kept), other calls their header, tables, hand-over states and records.  No counterpart in the reference. */
 size_t fkda_workspace_bytes_for(const fkda_fwd_params* p);
 
+/* Scratch bytes this call makes use of: what it needs, or more where more makes it faster (a fixed batch of long sequences with fewer
+ * (sequence, head) pairs than SMs but more than half as many: records of the later chunks, up to 1 GiB).  The results are
+ * the same.  No counterpart in the reference. */
+size_t fkda_workspace_bytes_wanted(const fkda_fwd_params* p);
+
 /* Enqueues the forward pass on `stream` (a cudaStream_t passed as void*).
  * Paths: a fixed batch with T == 1 is one state read-modify-write kernel, with 2 <= T <= 16 one fused kernel, a batch
  * with enough (sequence, head) pairs to fill the GPU one persistent kernel, anything else the prepare kernel plus the
