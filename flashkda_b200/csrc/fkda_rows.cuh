@@ -223,9 +223,11 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
             const bool has_next = left_n > kPair;
             if constexpr (kPair == 2) {
                 step(i, slot, left_n > 1 ? slot + 1 : slot, [&]() { ready = seen(sn, p); });
-                if (left_n == 1) break;
             }
-            if (has_next && !ready && __all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[sn], full_phase(p), abort_flag, a.wait_ns)) == 0) { failed = true; break; }
+            if (!(has_next & ready)) {   // (one branch that is rarely taken: a branch costs a lone warp some 25 cycles)
+                if (kPair == 2 && left_n == 1) break;
+                if (has_next && __all_sync(0xffffffffu, mbar_wait_bounded(&ctl.full[sn], full_phase(p), abort_flag, a.wait_ns)) == 0) { failed = true; break; }
+            }
             step(i + kPair - 1, slot + kPair - 1, has_next ? sn * kPair : slot + kPair - 1, [&]() {
                 if (kPair == 1) ready = seen(sn + 1 == kRowStages ? 0 : sn + 1, p + 1);
             });
