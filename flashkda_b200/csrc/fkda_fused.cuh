@@ -21,8 +21,8 @@
 // (or, with a chain longer than a range, for the range before that, and so on): no waiter depends on a CTA that has not
 // started.  A chain longer than a range is walked range after range from time zero, which is its critical path.
 //
-// Bound by issue slots and the shared-memory pipe: 0.56 instructions per cycle and scheduler, 65 % of the shared-memory
-// wavefronts, tensor pipe 44 % (148 chains of 256 chunks, 0.32 ms); a chunk step takes 1.05 us.
+// Bound by the latency of both roles beside each other: 0.57 instructions per cycle and scheduler, 64 % of the L1's wavefronts, tensor
+// pipe 44 % (148 chains of 256 chunks, 0.30 ms); a chunk step takes 1.1 us.  In long runs the power cap takes the clock to 1.8 GHz.
 // Included by fkda_tc.cu.
 #pragma once
 

@@ -2,9 +2,9 @@
 // does the work).  Grid-stride: warp w of the grid takes units w, w + W, ... with the head index fastest, so that
 // neighbouring warps read neighbouring 256-byte rows.  One record block of shared memory per warp; a finished record leaves by
 // a bulk copy (kTc) or, for the CUDA-core recurrence, in that kernel's plain layout.
-// Bound by the latency of a unit (9 us of dependent instructions and loads) at 12 warps per SM: 0.6 of the copy bandwidth on
-// its own 27 KB per unit (16 384 units: 94 us, as with the 16-warp predecessor whose lanes owned 4 columns of all rows; the
-// 1 568 units of a 777-token prompt with 32 heads: 14.7 us against 18.9).
+// Bound by the latency of a unit (7 us of dependent instructions and loads, two thirds of it its rows) at 12 warps per SM: 0.7 of the
+// copy bandwidth on its own 27 KB per unit (16 384 units: 91 us, 96 before two rows shared their norms; on 52 SMs beside a walk
+// 12 ns per unit, 4.3 of the whole GPU's; the 1 568 units of a 777-token prompt with 32 heads: 13.0 us against 14.7).
 #pragma once
 
 #include "fkda_prep.cuh"

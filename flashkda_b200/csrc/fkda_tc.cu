@@ -1,12 +1,13 @@
 // Tensor-core KDA forward for sm_100a: dispatch and launches.
 //
-// Two forms of the forward, both on the same chunk operands (a 14 656-byte record per (chunk, head), fkda_common.cuh), the same
+// The forms of the forward, all on the same chunk operands (a 14 656-byte record per (chunk, head), fkda_common.cuh), the same
 // chunk step on mma.sync with the state in registers (fkda_walk.cuh), and with bit-identical results:
 //   * fkda_fused.cuh: one persistent kernel whose CTAs prepare the records in shared memory and walk them, for batches with
 //     enough chains to fill the GPU: no record ever reaches HBM;
 //   * fkda_prepare_warp.cuh + fkda_rows.cuh: a prepare kernel writes the records to the workspace, a recurrence kernel walks
 //     row slices of the chains; the slices of few chains spread over more SMs than there are chains, and the prepare stage of
-//     later chunks runs on the SMs that are left (the slab pipeline below).
+//     later chunks runs on the SMs that are left (the slab pipeline below);
+//   * both, for chains that leave SMs idle in the first form and have none for slices (launch_mid).
 // An earlier form of both recurrences ran the products on tcgen05 with accumulators in tensor memory: the hand-overs between
 // registers and tensor memory (a store takes 180 cycles, a commit and its wait as long) cost more than products that are 16 to
 // 128 columns wide and 16 deep take on mma.sync (a chunk step of one chain per SM: 1.11 us against 0.52).
