@@ -57,7 +57,9 @@ __host__ __device__ constexpr int tc_sq_off(int i, int j) {
 // ---- programmatic dependent launch: a kernel launched with launch_dependent (fkda_internal.h) may start before the kernel in
 //      front of it has ended; grid_dep_wait() returns when that one is complete and its writes are visible (at once in a
 //      kernel launched otherwise), so every such kernel calls it before anything else.  Each kernel of a call waits for
-//      the one before it, so the one before that is complete as well. ----
+//      the one before it, so the one before that is complete as well.  Behind the wait, everything that an earlier kernel may
+//      have written (inputs, states, tables) is read with ordinary loads: a load that is declared invariant (__ldg, a const
+//      __restrict__ parameter) may be moved in front of the wait, and the wait says nothing of what it finds. ----
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

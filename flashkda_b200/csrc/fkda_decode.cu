@@ -79,9 +79,9 @@ __global__ void __launch_bounds__(128, 4) decode_kernel(const __grid_constant__ 
 
     // ---- the token's q, k, g columns, beta, and my row's v ----
     const int64_t tok = n * a.token_stride + (int64_t)h * kD;
-    const uint2 qraw = __ldg(reinterpret_cast<const uint2*>(a.q + tok + c4));
-    const uint2 kraw = __ldg(reinterpret_cast<const uint2*>(a.k + tok + c4));
-    const uint2 graw = __ldg(reinterpret_cast<const uint2*>(a.g + tok + c4));
+    const uint2 qraw = *reinterpret_cast<const uint2*>(a.q + tok + c4);
+    const uint2 kraw = *reinterpret_cast<const uint2*>(a.k + tok + c4);
+    const uint2 graw = *reinterpret_cast<const uint2*>(a.g + tok + c4);
     const __nv_bfloat16 v_mine = a.v[tok + row0 + my_row];
     const float beta_logit = bf2f(a.beta[n * a.beta_token_stride + h]);
     const float4 dtv = *reinterpret_cast<const float4*>(a.dt_bias + (int64_t)h * kD + c4);

@@ -85,21 +85,21 @@ __device__ __forceinline__ PrepSrc prep_src(const TwoPassArgs& a, int64_t t0, in
 // Row i of my half; a row past the end reads the last valid row (its factors are zero).
 __device__ __forceinline__ void prep_load_row(const PrepSrc& s, int i, PrepRow& x) {
     const uint64_t off = (uint64_t)(uint32_t)min(s.row0 + i, s.last) * s.step;
-    x.k = __ldg(s.k + off);
-    x.q = __ldg(s.q + off);
-    x.g = __ldg(s.g + off);
+    x.k = s.k[off];
+    x.q = s.q[off];
+    x.g = s.g[off];
 }
 __device__ __forceinline__ void prep_load(const TwoPassArgs& a, const PrepSrc& s, int64_t t0, int len, int h, int lane, PrepHead& x) {
     const uint2* g = reinterpret_cast<const uint2*>(a.g + t0 * a.token_stride + (int64_t)h * kD + 4 * lane);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x.g7[i] = __ldg(g + (uint64_t)(uint32_t)min(i, s.last) * (2 * s.step));
+    for (int i = 0; i < 8; ++i) x.g7[i] = g[(uint64_t)(uint32_t)min(i, s.last) * (2 * s.step)];
 #pragma unroll
     for (int i = 0; i < 2; ++i) prep_load_row(s, i, x.row[i]);
     const float4* dt = reinterpret_cast<const float4*>(a.dt_bias + (int64_t)h * kD);
-    x.dt0 = __ldg(dt + 2 * (lane & 15));
-    x.dt1 = __ldg(dt + 2 * (lane & 15) + 1);
-    x.dt7 = __ldg(dt + lane);
-    x.a_log = __ldg(a.A_log + h);
+    x.dt0 = dt[2 * (lane & 15)];
+    x.dt1 = dt[2 * (lane & 15) + 1];
+    x.dt7 = dt[lane];
+    x.a_log = a.A_log[h];
     x.beta = __float2bfloat16_rn(0.0f);
     if (lane < len) x.beta = a.beta[(t0 + lane) * a.beta_token_stride + h];   // len <= 16
 }

@@ -22,12 +22,9 @@ namespace fkda {
 // One thread per sequence up to 1 024 sequences, in a block no larger than that takes: cu_seqlens is read once and the two tables
 // are summed side by side, so what is left of the kernel is one trip to memory and a few shuffles (1 024 threads whatever the
 // number, a pass for each table: 5.2 us for 4 sequences).
-__global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* __restrict__ cu, int64_t N,
-                                                           int32_t* __restrict__ prefix, int32_t* __restrict__ order,
-                                                           int32_t* __restrict__ cs_prefix, int cs_tokens,
-                                                           int32_t* __restrict__ short_flag, int decode_enqueued,
-                                                           int32_t* __restrict__ header, int keep_records, int32_t* __restrict__ flags,
-                                                           int n_flags) {
+__global__ void __launch_bounds__(1024) tile_prefix_kernel(const int64_t* cu, int64_t N, int32_t* prefix, int32_t* order, int32_t* cs_prefix,
+                                                           int cs_tokens, int32_t* short_flag, int decode_enqueued, int32_t* header,
+                                                           int keep_records, int32_t* flags, int n_flags) {
     grid_dep_launch();
     grid_dep_wait();   // (the call before may still read its tables)
     __shared__ int2 part[32];

@@ -328,7 +328,7 @@ __device__ __forceinline__ void walk_load_tiles(uint32_t (&s)[kMt][8][4], uint8_
 #pragma unroll
     for (int mt = 0; mt < kMt; ++mt)
 #pragma unroll
-        for (int i = 0; i < kPer; ++i) x[mt][i] = __ldg(p + 32 * (kPer * mt + i));
+        for (int i = 0; i < kPer; ++i) x[mt][i] = p[32 * (kPer * mt + i)];
 #pragma unroll
     for (int mt = 0; mt < kMt; ++mt) {
 #pragma unroll
