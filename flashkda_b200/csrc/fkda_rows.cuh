@@ -223,6 +223,7 @@ recurrence_rows_kernel(const __grid_constant__ TwoPassArgs a, const __grid_const
             const bool has_next = left_n > kPair;
             if constexpr (kPair == 2) {
                 step(i, slot, left_n > 1 ? slot + 1 : slot, [&]() { ready = seen(sn, p); });
+                __syncwarp();   // (every lane has read its piece of the out tile: the next chunk's rows may go in)
             }
             if (!(has_next & ready)) {   // (one branch that is rarely taken: a branch costs a lone warp some 25 cycles)
                 if (kPair == 2 && left_n == 1) break;

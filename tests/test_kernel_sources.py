@@ -1,4 +1,4 @@
-"""Kernels that start while the kernel in front of them still runs: what their sources may and may not do."""
+"""Orderings that a run cannot be relied on to show: what the kernels' sources have to contain."""
 import glob
 import os
 import re
@@ -27,3 +27,13 @@ def test_no_load_is_declared_invariant():
         for word in ("__ldg(", "__restrict__", "ld.global.nc"):
             assert word not in code, (path, word)
     assert seen >= 6   # decode, short, prefix, prepare, row-slice and one-kernel forms
+
+
+def test_a_warp_barrier_between_the_chunks_of_a_pair():
+    """The out tile of a walking warp is written by all lanes and read by all lanes in every chunk: a barrier lies between one
+    chunk's reads and the next one's writes, also where two chunks share a stage."""
+    code = _code(os.path.join(CSRC, "fkda_rows.cuh"))
+    first, second = (m.start() for m in re.finditer(r"^\s+step\(", code, re.M))
+    assert "__syncwarp();" in code[first:second] and "__syncwarp();" in code[second:]
+    inside = code[code.index("w.chunk("):first]
+    assert inside.index("stmatrix_x4_t(") < inside.index("__syncwarp();") < inside.index("lds_u4(")
