@@ -12,10 +12,13 @@
 
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <optional>
@@ -85,6 +88,39 @@ int algo_arg(PyObject* o) {
 bool shape_is(const at::Tensor& t, std::initializer_list<int64_t> want) {
     const auto s = t.sizes();
     return s.size() == want.size() && std::equal(want.begin(), want.end(), s.begin());
+}
+
+// Whether the allocator can hand out a scratch of `bytes`, up to a gigabyte, that a call can do without, and nobody else pays for it.
+// The device (or what a limit on this process leaves of it) has to have that much unused even if no cached block serves the call:
+// otherwise the allocator would first give every cached block back, synchronising the device, on each such call (2.5 to 3.2 ms of
+// host time).  And twice as much before the first block is cached, so that what made room once makes room again.  The device is
+// asked (68 us) when something has been given back to it since the last time that there was room, or when less is cached than
+// the call takes.  Not under capture: a graph would keep the block for as long as it lives.
+bool spare_memory(c10::DeviceIndex dev, size_t bytes, cudaStream_t stream) {
+    static std::atomic<int64_t> room_since[64];   // per device: blocks given back when there last was room, plus one
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    auto ok = [](cudaError_t e) { return e == cudaSuccess || (cudaGetLastError(), false); };   // (a refusal here is not the call's)
+    if (dev < 0 || dev >= 64 || !ok(cudaStreamIsCapturing(stream, &capture)) || capture != cudaStreamCaptureStatusNone) return false;
+    try {
+        auto* allocator = c10::cuda::CUDACachingAllocator::get();
+        const auto stats = allocator->getDeviceStats(dev);
+        const size_t all = static_cast<size_t>(c10::CachingAllocator::StatType::AGGREGATE);
+        const double reserved = (double)stats.reserved_bytes[all].current;
+        const double cached = std::min(reserved - (double)stats.allocated_bytes[all].current, (double)bytes);
+        const int64_t given_back = stats.num_device_free + 1;
+        if (cached >= (double)bytes && room_since[dev].load(std::memory_order_relaxed) == given_back) return true;
+        size_t unused = 0, total = 0;
+        {
+            c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);   // (another thread may be capturing)
+            if (!ok(cudaMemGetInfo(&unused, &total))) return false;
+        }
+        const double allowed = allocator->getMemoryFraction(dev) * (double)total - reserved;
+        if (std::min((double)unused, allowed) + cached < 2.0 * (double)bytes) return false;
+        room_since[dev].store(given_back, std::memory_order_relaxed);
+        return true;
+    } catch (const c10::Error&) {   // (an allocator that keeps no such figures)
+        return false;
+    }
 }
 
 // fwd(q, k, v, g, beta, scale, out, A_log, dt_bias, lower_bound, initial_state, final_state, cu_seqlens, algo, workspace,
@@ -187,6 +223,7 @@ void fwd_checked(PyObject* const* a) {
     p.chunk_states_every = (int32_t)every;
     c10::cuda::OptionalCUDAGuard guard;
     if (c10::cuda::current_device() != dev.index()) guard.set_index(dev.index());
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     const size_t need = fkda_workspace_bytes_for(&p);   // what this call's path needs (a decode step: nothing)
     const at::Tensor* ws = optional_tensor_arg(a[14], "workspace");
     c10::DataPtr scratch;   // given back when it goes out of scope; the allocator reuses it in stream order
@@ -198,17 +235,17 @@ void fwd_checked(PyObject* const* a) {
         p.workspace_bytes = (size_t)ws->numel();
     } else if (need > 0) {
         p.workspace_bytes = fkda_workspace_bytes_wanted(&p);   // more than the path needs only makes it faster
+        if (p.workspace_bytes > need && !spare_memory(dev.index(), p.workspace_bytes, stream)) p.workspace_bytes = need;
         if (p.workspace_bytes > need) {
             try {
                 scratch = c10::cuda::CUDACachingAllocator::get()->allocate(p.workspace_bytes);
-            } catch (const c10::OutOfMemoryError&) {
+            } catch (const c10::OutOfMemoryError&) {   // (another thread was faster)
                 p.workspace_bytes = need;
             }
         }
         if (scratch.get() == nullptr) scratch = c10::cuda::CUDACachingAllocator::get()->allocate(need);
         p.workspace = scratch.get();
     }
-    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     int rc;
     Py_BEGIN_ALLOW_THREADS   // (a launch may wait for room in the stream's queue; the caller holds the tensors)
     rc = fkda_fwd(&p, stream);
