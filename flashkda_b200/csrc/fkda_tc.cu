@@ -216,8 +216,16 @@ static bool encode_map(CUtensorMap* m, CUtensorMapDataType type, int rank, const
     EncodeTiledFn encode = encode_tiled_fn();
     if (encode == nullptr) return false;
     const cuuint32_t estr[3] = {1u, 1u, 1u};
-    return encode(m, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    auto encoded = [&]() {
+        return encode(m, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult rc = encoded();
+    if (rc == CUDA_ERROR_INVALID_CONTEXT) {   // the first CUDA work of this host thread: nothing has made the device's context its own yet
+        int dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) rc = encoded();
+    }
+    return rc == CUDA_SUCCESS;
 }
 // Map over v viewed as [token][head][128] bf16 with tiles of 16 tokens x 64 columns of one head; the 16-byte pieces of a tile
 // row are permuted by the row (128-byte swizzle), so that transposing reads of the tile (8 rows of one piece) do not collide.
