@@ -170,21 +170,32 @@ size_t tc_workspace_bytes_wanted(const fkda_fwd_params& p) {
     return need > 0 && mid_eligible(p, sms) && mid_bytes(p, sms) > need ? mid_bytes(p, sms) : need;
 }
 
-// Side stream and events of the slab pipeline, one set per device, created on first use.
+// Calls that a host thread makes on the library's own streams concern no stream of the caller: another thread's capture in the
+// strict mode does not forbid them.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Side stream and events, one set per device for the slab pipeline and one for launch_mid, created on first use.
 constexpr int kMaxSlabs = 4;
+enum SideUse { kSideSlabs, kSideMid, kSideUses };
 struct SlabStreams {
-    std::mutex launch_mu;  // one slab pipeline at a time is ENQUEUED per device (event record / wait pairs stay paired)
+    std::mutex launch_mu;  // one call at a time is ENQUEUED per set (event record / wait pairs stay paired)
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, done[kMaxSlabs] = {nullptr, nullptr, nullptr, nullptr};
+    unsigned long long user = 0;   // id of the stream whose call was the last to put work on the side stream (side_free)
     bool ready = false;
 };
-static SlabStreams* slab_streams(int dev) {
+static SlabStreams* slab_streams(int dev, SideUse use) {
     static std::mutex mu;
-    static SlabStreams table[64];
+    static SlabStreams table[64][kSideUses];
     if (dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
-    SlabStreams& t = table[dev];
+    SlabStreams& t = table[dev][use];
     if (!t.ready) {
+        const RelaxedCapture relaxed;
         if (cudaStreamCreateWithFlags(&t.side, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
         if (cudaEventCreateWithFlags(&t.fork, cudaEventDisableTiming) != cudaSuccess) return nullptr;
         for (int i = 0; i < kMaxSlabs; ++i)
@@ -192,6 +203,25 @@ static SlabStreams* slab_streams(int dev) {
         t.ready = true;
     }
     return &t;
+}
+
+// Whether a call on `stream` gets the side stream to itself (launch_mu is held): not while it belongs to another thread's capture,
+// nor while it carries another stream's work, which would put this call behind whatever that stream waits for.
+static bool side_free(SlabStreams& t, cudaStream_t stream) {
+    auto ok = [](cudaError_t e) { return e == cudaSuccess || (cudaGetLastError(), false); };   // (a refusal here is not the call's)
+    cudaStreamCaptureStatus side = cudaStreamCaptureStatusNone, mine = cudaStreamCaptureStatusNone;
+    unsigned long long side_id = 0, my_id = 0;
+    if (!ok(cudaStreamGetCaptureInfo(t.side, &side, &side_id)) || !ok(cudaStreamGetCaptureInfo(stream, &mine, &my_id))) return false;
+    if (side != cudaStreamCaptureStatusNone) return side == cudaStreamCaptureStatusActive && mine == side && my_id == side_id;
+    if (mine != cudaStreamCaptureStatusNone) return true;   // (the graph depends on nothing that was enqueued before it)
+    unsigned long long user = 0;
+    if (!ok(cudaStreamGetId(stream, &user))) return false;
+    if (t.user != user) {
+        const RelaxedCapture relaxed;
+        if (!ok(cudaStreamQuery(t.side))) return false;
+        t.user = user;
+    }
+    return true;
 }
 
 // The driver entry point is looked up through the runtime (no link-time dependency on libcuda, so
@@ -313,6 +343,7 @@ static RowsLaunch rows_select(const TwoPassArgs& a, int64_t chains, int sms, boo
 // row-slice kernel of one CTA per chain, 32 rows per warp, walks the others without a preparing warp beside it, slab by slab.
 // A step takes about 1.11 us in the one and 0.77 us in the other, a record 0.0050 us of the whole GPU (0.0043, which would hide
 // nothing, to 0.0061 tried): the slabs follow from that.  8 192 tokens of 96 heads: 568 -> 475 us, of 80 heads 579 -> 444.
+// The one-kernel form needs the caller's stream alone, so a call that finds the side stream in another's hands takes that form.
 static int launch_mid(const fkda_fwd_params& p, TwoPassArgs& a, int sms, int dev, cudaStream_t stream, int* n_launches) {
     const int chains = (int)(p.N * p.H), idle = sms - chains, tps = (int)((p.T + kChunk - 1) / kChunk);
     const double records = 0.0050 * sms * chains / idle;   // us for the records of one chunk of every chain
@@ -339,9 +370,13 @@ static int launch_mid(const fkda_fwd_params& p, TwoPassArgs& a, int sms, int dev
     const bool exports = a.chunk_states != nullptr;
     if (!(exports ? allow_smem<fused_kernel<true, true>>(kFusedSmemBytes) : allow_smem<fused_kernel<false, true>>(kFusedSmemBytes))) return FKDA_ERR_LAUNCH;
     const RowsLaunch rows = exports ? rows_launch<true, false, 2, 4, 2>() : rows_launch<false, false, 2, 4, 2>();
-    SlabStreams* ss = slab_streams(dev);
+    SlabStreams* ss = slab_streams(dev, kSideMid);
     if (!rows.ok || ss == nullptr) return FKDA_ERR_LAUNCH;
-    std::lock_guard<std::mutex> enqueue_lock(ss->launch_mu);
+    std::unique_lock<std::mutex> enqueue_lock(ss->launch_mu);
+    if (!side_free(*ss, stream)) {   // (same results)
+        enqueue_lock.unlock();
+        return launch_fused(p, a, sms, stream, n_launches);
+    }
     auto slab_args = [&](int i) {
         TwoPassArgs x = a;
         x.slab_c0 = bounds[i];
@@ -409,7 +444,7 @@ int launch_tc(const fkda_fwd_params& p, cudaStream_t stream, int* n_launches) {
     //      Only stream order and events connect the launches: no kernel waits for another one. ----
     if (slabs) {
         const int idle_sms = sms - (int)chains * rows.split;
-        SlabStreams* ss = slab_streams(dev);
+        SlabStreams* ss = slab_streams(dev, kSideSlabs);
         if (ss == nullptr) return FKDA_ERR_LAUNCH;
         // host threads that call concurrently on one device share the side stream and its events
         std::lock_guard<std::mutex> enqueue_lock(ss->launch_mu);
