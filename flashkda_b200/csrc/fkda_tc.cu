@@ -124,9 +124,11 @@ static TcCarve tc_carve(const fkda_fwd_params& p, int sms) {
 }
 
 // Fewer chains than SMs, but too many for two SMs each: launch_mid, while its records take no more than a gigabyte.  The three kernel
-// boundaries cost some 12 us, and what is won grows with the chunks and with the idle SMs: the line lies where the two meet (us, one
-// kernel against this: 128 chunks: 76 chains 154, 134; 112 chains 157, 155; 128 chains 157, 163; 512 chunks: 96 chains 610, 480;
-// 124 chains 634, 572).
+// boundaries cost some 12 us, and what is won grows with the chunks and with the idle SMs: the line lies where the two meet (time of
+// the one kernel over this, 75 to 124 chains by chunks x idle SMs, without exported states: 4 650 .. 4 700: 0.98 to 1.015, 5 200:
+// 1.00 to 1.03, 7 000: 1.01 to 1.08, 8 800: 1.025 to 1.12).  With exported states the line lies higher: the stores of a state hold a walking
+// warp up in both, in the one kernel partly while it would wait for its preparing warps (4 650 .. 4 850: 0.94 to 0.98, 5 800: 0.98 to
+// 0.99, 7 000: 0.99 to 1.03, 9 200: 1.00 to 1.07, from every chunk to every 16th exported).
 constexpr size_t kMidBytesMost = (size_t)1 << 30;
 static size_t mid_bytes(const fkda_fwd_params& p, int sms) {
     const int64_t chains = p.N * p.H, tps = (p.T + kChunk - 1) / kChunk;
@@ -135,7 +137,8 @@ static size_t mid_bytes(const fkda_fwd_params& p, int sms) {
 static bool mid_eligible(const fkda_fwd_params& p, int sms) {
     const int64_t chains = p.N * p.H;
     return p.cu_seqlens == nullptr && p.phase_mask == 0 && !(p.flags & (FKDA_FLAG_NO_WIDE | FKDA_FLAG_NO_SLABS)) && chains * kRowSplit > sms &&
-           chains + 24 <= sms && p.T > 63 * kChunk && (p.T + kChunk - 1) / kChunk * (sms - chains) >= 4608 && mid_bytes(p, sms) <= kMidBytesMost;
+           chains + 24 <= sms && p.T > 63 * kChunk && (p.T + kChunk - 1) / kChunk * (sms - chains) >= (p.chunk_states == nullptr ? 4608 : 6912) &&
+           mid_bytes(p, sms) <= kMidBytesMost;
 }
 
 // Names the records that a call writes or expects: everything that decides where each of them lies.

@@ -132,7 +132,9 @@ size_t fkda_workspace_bytes_wanted(const fkda_fwd_params* p);
 /* Enqueues the forward pass on `stream` (a cudaStream_t passed as void*).
  * Paths: a fixed batch with T == 1 is one state read-modify-write kernel, with 2 <= T <= 16 one fused kernel, a batch
  * with enough (sequence, head) pairs to fill the GPU one persistent kernel, anything else the prepare kernel plus the
- * recurrence on row slices; a fixed batch with 75 to 124 pairs both (with the workspace that fkda_workspace_bytes_wanted asks for).  For a ragged batch (cu_seqlens) the host knows only the
+ * recurrence on row slices; a fixed batch with 75 to 124 pairs (on 148 SMs) both, if it has more than 1 008 tokens per sequence, its chunks
+ * times the SMs that are left come to 4 608 (6 912 with chunk_states), its records fit 1 GiB and the workspace holds what
+ * fkda_workspace_bytes_wanted says, and the library's side stream for such calls is free.  For a ragged batch (cu_seqlens) the host knows only the
  * totals: when there are at most 16 tokens per sequence on average (and at least 64 (sequence, head) pairs), a prefix
  * kernel decides on the device whether every sequence has one token, or at most 16, and the kernels of the paths that
  * may apply are all enqueued; those that are not needed return at once.  Results do not depend on the path, bit for bit,
