@@ -1,5 +1,5 @@
 """The forward pass inside a CUDA graph: with a caller-provided workspace `fwd` allocates nothing and issues
-only stream-ordered work (two memsets, the kernels), so it can be captured once and replayed - the
+only stream-ordered work (the kernels, for some forms a memset), so it can be captured once and replayed - the
 launch-bound regime (short sequences) is where that matters."""
 import pytest
 import torch
@@ -94,3 +94,48 @@ def test_captured_ragged_batch_decides_on_the_device_at_every_replay():
         torch.cuda.synchronize()
         assert flashkda_b200.device_status(ws) == 0
         assert torch.equal(got_out, d["out"][:, :used]) and torch.equal(got_hT, d["final_state"]), name
+
+
+@pytest.mark.parametrize("B,T,H,lens", [(7, 1, 8, None), (9, 5, 8, None), (4, 96, 4, None), (1, 1100, 4, None), (80, 40, 1, None),
+                                        (1, 1100, 80, None), (1, 400, 4, [300, 1, 99])],
+                         ids=["decode", "short", "prompt", "slabs", "one_kernel", "chains_between", "ragged"])
+def test_captured_between_other_work(B, T, H, lens):
+    """A caller's kernel in front, two calls one behind the other (out of the first is v of the second), work of another stream
+    joined, a third call, a caller's kernel behind: programmatic edges where a kernel is in front, full ones elsewhere."""
+    w = Workload("graph", B, T, H, state_in="fp32", state_out="fp32", lower_bound=-0.2, seq_lens=lens)
+    d = to_device(make_inputs(w, seed=3), "cuda")
+    ws = torch.empty(flashkda_b200.get_workspace_size(w.tokens, H, w.n_seqs), dtype=torch.uint8, device="cuda")
+    v0, mid, out, s0, s1, s2, s3 = (torch.zeros_like(d[x]) for x in ("v", "v", "v") + ("initial_state",) * 4)
+    other = torch.cuda.Stream()
+
+    def call(v, o, a, b):
+        flashkda_b200.fwd(d["q"], d["k"], v, d["g"], d["beta"], d["scale"], o, d["A_log"], d["dt_bias"], d["lower_bound"], a, b,
+                          d["cu_seqlens"], workspace=ws)
+
+    def work():
+        torch.mul(d["v"], 0.5, out=v0)
+        s0.copy_(d["initial_state"])
+        call(v0, mid, s0, s1)
+        call(mid, out, s1, s2)
+        other.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(other):
+            v0.mul_(2.0)
+        torch.cuda.current_stream().wait_stream(other)
+        call(v0, mid, s2, s3)
+        out.add_(mid)
+
+    work()
+    torch.cuda.synchronize()
+    want = [t.clone() for t in (out, s3)]
+    assert all(bool(t.isfinite().all()) and bool(t.abs().sum() > 0) for t in want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        work()
+    for _ in range(3):
+        for t in (v0, mid, out, s0, s1, s2, s3):
+            t.fill_(3.0)
+        graph.replay()
+        graph.replay()   # the second follows the first without a wait of the host
+        torch.cuda.synchronize()
+        assert flashkda_b200.device_status(ws) == 0
+        assert all(torch.equal(x, y) for x, y in zip((out, s3), want))
