@@ -32,8 +32,9 @@ __device__ __forceinline__ float row_sumsq(const float (&x)[4], int lane) {
 }
 
 // State rows of a warp; a chain takes 32 / kRows CTAs.  8 rather than 32 rows: a warp has a quarter of the loads, shuffles and
-// stores in its way and 72 registers instead of 168, so the GPU holds seven CTAs per SM (fp32 states, 32 chains 7.2 -> 4.1 us
-// per step, and 2.7 with launches that overlap the step before, 640: 20.7 -> 12.3, 32 768: 679 -> 631, which is 1.06 of the copy bandwidth).  16 rows: 759 us on the last.
+// stores in its way and 72 registers instead of 168, so the GPU holds seven CTAs per SM (fp32 states, each step launched behind
+// the end of the one before: 32 chains 7.2 -> 4.1 us per step, 640: 20.7 -> 12.3, 32 768: 679 -> 631, which is 1.06 of the copy
+// bandwidth).  16 rows: 759 us on the last.
 constexpr int kRows = 8;
 constexpr int kSplit = 32 / kRows;
 

@@ -9,7 +9,8 @@
 //     kFusedSlots blocks (fkda_prep.cuh), asks for the value tile and leaves a note on where the chunk belongs, so that the
 //     walking warps spend nothing on addresses.  Chunks are handed over through mbarriers, slot by slot.
 // Register shares: the walkers keep 232 registers per thread, the preparing warps 136 (128 x 232 + 256 x 136 = 384 x 168, what
-// the CTA is launched with; 216 and 144: 1 % slower, 240 and 128: 2 to 3 %, 200 and 152: 1 to 3 %, 184 and 160: 12 %).
+// the CTA is launched with; 216 and 144: 1 % slower, 240 and 128: 2 to 3 %, 200 and 152: 1 to 3 %, 184 and 160: 12 %).  The build spills
+// 20 bytes (76 of loads).
 //
 // Work split: the chunks of all chains form one line, chain after chain, cut into ranges of equal cost, one per CTA.  (Equal
 // numbers of chunks leave the ranges with many short chains far behind: 640 chains of 1 to 16 chunks 110 us against 64, 3 200

@@ -111,8 +111,8 @@ inline bool allow_smem(int bytes) {
 
 // Launches a kernel that begins with grid_dep_wait() (fkda_common.cuh) behind whatever kernel is in front of it on the stream,
 // of the same call, the call before or the caller's own: its launch and start overlap that kernel's end, and nothing of it
-// touches memory before that end.  (One token of 32 heads, steps back to back: 4.1 -> 3.1 us; a prompt of 100 tokens, 8 heads:
-// 12.3 -> 11.2; 4 x 1 tokens of 32 heads: 6.2 -> 4.5.)
+// touches memory before that end.  (One token of 32 heads, steps back to back through Python: 4.1 -> 2.9 to 3.4 us, by the host; a
+// prompt of 100 tokens, 8 heads: 12.3 -> 11.2; 4 x 1 tokens of 32 heads: 6.2 -> 4.5.  With nothing in front there is nothing to gain.)
 template <typename... KernelArgs, typename... Args>
 inline bool launch_dependent(void (*kernel)(KernelArgs...), int64_t ctas, int threads, int smem, cudaStream_t stream, const Args&... args) {
     cudaLaunchConfig_t cfg = {};

@@ -89,13 +89,15 @@ constexpr size_t kStateBytes = (size_t)kD * kD * 2;   // a chain's state as bf16
 static bool slabs_possible(int64_t chains, int sms) { return chains * kRowSplit <= sms - 32; }
 
 // The one-kernel forward serves whole forwards with more than one chunk per chain on average and more row slices than SMs.
-// While every slice has an SM of its own, a step of the row-slice kernel takes 0.45 us against 1.05 us here, which pays for the
-// prepare kernel in front of it (64 chains of 512 chunks: 0.50 ms against 0.57; 96 chains: 0.71 against 0.57).  A ragged batch
-// whose lengths the host does not know may consist of a few long chains, whose walk is then the whole time (128 chains of 1
-// to 32 chunks: 52 us in two kernels against 82): it needs two chains per SM, or 1.6 with more than ten chunks per sequence
-// on average (256 and 288 chains: 16 chunks 47 to 93 us against 51 to 112, 256 chunks 425 to 568 against 645 to 873, but 4
-// chunks 39 against 34; 192 chains go either way).  With fp32 states to load and to store, which nothing hides here, it needs
-// more than four chunks per sequence on average (3 840 chains of 2 chunks 256 us against 214, of 4 chunks 318 against 289).
+// While every slice has an SM of its own, a step of the row-slice kernel takes 0.45 us against 1.1 us here, which pays for the
+// prepare kernel in front of it (chains of 512 chunks, one prepare and one recurrence kernel against this: 64 chains 395 us, 567;
+// 74 chains 421, 568; 80 chains 627, 568; 96 chains 667, 568).  A ragged batch whose lengths the host does not know may consist of
+// a few long chains, whose walk is then the whole time (128 chains of 1 to 32 chunks: 45.5 us in two kernels against 52.8): it needs
+// two chains per SM, or 1.6 with more than ten chunks per sequence on average (256 and 288 chains of even lengths: 16 chunks 67, 68
+// us in two kernels against 52, 57; 256 chunks 756, 804 against 504, 565; the 4 chunks per sequence that the line keeps out are as fast
+// here by now, 28.4, 29.7 against 25.8, 28.8).  With fp32 states to load and to store, which nothing hides here, it needs more than
+// four chunks per sequence on average (3 840 chains of 2 chunks 199 us in two kernels against 215, of 4 chunks 277 against 268, of 5
+// chunks 319 against 298).
 static bool fused_eligible(const fkda_fwd_params& p, int sms) {
     if (p.phase_mask != 0 || p.B * p.T <= kChunk * p.N) return false;
     if (p.flags & FKDA_FLAG_NO_WIDE) return true;
@@ -345,7 +347,8 @@ static RowsLaunch rows_select(const TwoPassArgs& a, int64_t chains, int sms, boo
 // they prepare the records of the later chunks meanwhile (side stream), and once the one-kernel form has walked the first chunks a
 // row-slice kernel of one CTA per chain, 32 rows per warp, walks the others without a preparing warp beside it, slab by slab.
 // A step takes about 1.11 us in the one and 0.77 us in the other, a record 0.0050 us of the whole GPU (0.0043, which would hide
-// nothing, to 0.0061 tried): the slabs follow from that.  8 192 tokens of 96 heads: 568 -> 475 us, of 80 heads 579 -> 444.
+// nothing, to 0.0061 tried): the slabs follow from that.  8 192 tokens of 96 heads: 568 -> 475 us in runs of some milliseconds, 581 -> 520
+// in long ones, where the power cap takes the clock down; of 80 heads 579 -> 444 in the former.
 // The one-kernel form needs the caller's stream alone, so a call that finds the side stream in another's hands takes that form.
 static int launch_mid(const fkda_fwd_params& p, TwoPassArgs& a, int sms, int dev, cudaStream_t stream, int* n_launches) {
     const int chains = (int)(p.N * p.H), idle = sms - chains, tps = (int)((p.T + kChunk - 1) / kChunk);
